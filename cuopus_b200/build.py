@@ -69,11 +69,7 @@ def build_libcuopus(force=False):
     obj = os.path.join(LIB, "obj")
     os.makedirs(obj, exist_ok=True)
     common = [NVCC, *ARCH, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC,-O2", "-I", CSRC]
-    # The decoder kernel is built at NVVM -O1 and ptxas -O1 (decode_kernel.cu
-    # explains): its machine code is a third smaller than at -O3, and under load
-    # the kernel waits on instruction fetch, so the smaller code decodes faster;
-    # the rest is -O3.
-    _run(common + ["-Xcicc", "-O1", "-Xptxas", "-O1,-v", "-c", os.path.join(CSRC, "decode_kernel.cu"),
+    _run(common + ["-Xptxas", "-v", "-c", os.path.join(CSRC, "decode_kernel.cu"),
                    "-o", os.path.join(obj, "decode_kernel.o")])
     _run(common + ["-Xptxas", "-v", "-c", os.path.join(CSRC, "libcuopus.cu"), "-o", os.path.join(obj, "libcuopus.o")])
     _run(common + ["-Xptxas", "-v", "-c", os.path.join(CSRC, "costmodel.cu"), "-o", os.path.join(obj, "costmodel.o")])
@@ -85,7 +81,7 @@ def build_libcuopus(force=False):
     _run([NVCC, *ARCH, "-shared", "-o", tmp, os.path.join(obj, "decode_kernel.o")] + rest)
     os.replace(tmp, LIBCUOPUS)
     # diagnostic build: the same library with the decoder's stage timers on
-    _run(common + ["-Xcicc", "-O1", "-Xptxas", "-O1", "-DCUO_PHASE_TIMERS", "-c",
+    _run(common + ["-DCUO_PHASE_TIMERS", "-c",
                    os.path.join(CSRC, "decode_kernel.cu"), "-o", os.path.join(obj, "decode_kernel_phases.o")])
     tmp = LIBPHASES + ".tmp"
     _run([NVCC, *ARCH, "-shared", "-o", tmp, os.path.join(obj, "decode_kernel_phases.o")] + rest)

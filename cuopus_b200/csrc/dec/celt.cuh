@@ -101,7 +101,7 @@ DNI void celt_reset(CeltDec *st)
     memset(st->lpc, 0, sizeof(st->lpc));
     memset(st->oldBandE, 0, sizeof(st->oldBandE));
     memset(st->backgroundLogE, 0, sizeof(st->backgroundLogE));
-    for (int i = 0; i < 2 * CELT_NB; i++) st->oldLogE[i] = st->oldLogE2[i] = -28672;   // -QCONST16(28.f, DB_SHIFT)
+    ROLLED for (int i = 0; i < 2 * CELT_NB; i++) st->oldLogE[i] = st->oldLogE2[i] = -28672;   // -QCONST16(28.f, DB_SHIFT)
     st->skip_plc = 1;
 }
 
@@ -250,14 +250,14 @@ DNI void celt_fft(Lanes L, int shift_idx, Cpx *fout)
     int fstride[8];
     fstride[0] = 1;
     int Lf = 0, p, m;
-    do {
+    ROLLED do {
         p = factors[2 * Lf];
         m = factors[2 * Lf + 1];
         fstride[Lf + 1] = fstride[Lf] * p;
         Lf++;
     } while (m != 1);
     m = factors[2 * Lf - 1];
-    for (int i = Lf - 1; i >= 0; i--) {
+    ROLLED for (int i = Lf - 1; i >= 0; i--) {
         int m2 = i != 0 ? factors[2 * i - 1] : 1;
         fft_stage(L, fout, factors[2 * i], fstride[i] << shift, m, fstride[i], m2);
         m = m2;
@@ -274,7 +274,7 @@ DNI void mdct_backward(Lanes L, const int32_t *in, int32_t *out, int shift, int 
 {
     int N = T_CELT_MDCT_N;
     const int16_t *trig = T_celt_mdct_trig;
-    for (int i = 0; i < shift; i++) { N >>= 1; trig += N; }
+    ROLLED for (int i = 0; i < shift; i++) { N >>= 1; trig += N; }
     int N2 = N >> 1, N4 = N >> 2;
     const int16_t *bitrev = fft_bitrev(shift);
     int32_t *yp = out + (CELT_OVERLAP >> 1);
@@ -328,7 +328,7 @@ DNI void denormalise_bands(Lanes L, const int16_t *X, int32_t *freq, const int16
     int bound = M * eB[end];
     if (silence) { bound = 0; start = end = 0; }
     LFOR(L, i, 0, M * eB[start]) freq[i] = 0;
-    for (int b = start; b < end; b++) {
+    ROLLED for (int b = start; b < end; b++) {
         int j0 = M * eB[b], j1 = M * eB[b + 1];
         int16_t lg = c_sat16(wadd(bandLogE[b], shl32((int32_t)T_celt_eMeans[b], 6)));
         int shift = 16 - (lg >> 10);
@@ -356,7 +356,7 @@ DNI void comb_filter(int32_t *y, int32_t *x, int T0, int T1, int N, int16_t g0, 
 {
     const int16_t (*gains)[3] = T_comb_gains;
     if (g0 == 0 && g1 == 0) {
-        if (x != y) for (int i = 0; i < N; i++) y[i] = x[i];
+        if (x != y) ROLLED for (int i = 0; i < N; i++) y[i] = x[i];
         return;
     }
     T0 = imax(T0, 15);
@@ -370,7 +370,7 @@ DNI void comb_filter(int32_t *y, int32_t *x, int T0, int T1, int N, int16_t g0, 
     int32_t x0, x1 = x[-T1 + 1], x2 = x[-T1], x3 = x[-T1 - 1], x4 = x[-T1 - 2];
     if (g0 == g1 && T0 == T1 && tapset0 == tapset1) overlap = 0;
     int i;
-    for (i = 0; i < overlap; i++) {
+    ROLLED for (i = 0; i < overlap; i++) {
         x0 = x[i - T1 + 2];
         int16_t f = (int16_t)c_mul16_q15(window[i], window[i]);
         int32_t v = x[i];
@@ -384,14 +384,14 @@ DNI void comb_filter(int32_t *y, int32_t *x, int T0, int T1, int N, int16_t g0, 
         x4 = x3; x3 = x2; x2 = x1; x1 = x0;
     }
     if (g1 == 0) {
-        if (x != y) for (int k = overlap; k < N; k++) y[k] = x[k];
+        if (x != y) ROLLED for (int k = overlap; k < N; k++) y[k] = x[k];
         return;
     }
     // comb_filter_const_c
     int32_t *yy = y + i, *xx = x + i;
     int Nc = N - i;
     x4 = xx[-T1 - 2]; x3 = xx[-T1 - 1]; x2 = xx[-T1]; x1 = xx[-T1 + 1];
-    for (int k = 0; k < Nc; k++) {
+    ROLLED for (int k = 0; k < Nc; k++) {
         x0 = xx[k - T1 + 2];
         int32_t v = wadd(wadd(wadd(xx[k], c_mul16_32_q15(g10, x2)), c_mul16_32_q15(g11, wadd(x1, x3))),
                          c_mul16_32_q15(g12, wadd(x0, x4)));
@@ -428,7 +428,7 @@ DNI void comb_filter_lanes(Lanes L, int32_t *y, int32_t *x, int T0, int T1, int 
     int16_t g12 = (int16_t)c_mul16_p15(g1, gains[tapset1][2]);
     if (g0 == g1 && T0 == T1 && tapset0 == tapset1) overlap = 0;
     const int B = x == y ? imin(T0, T1) - 2 : imax(N, 1);
-    for (int s = 0; s < overlap; s += B) {
+    ROLLED for (int s = 0; s < overlap; s += B) {
         int e = imin(s + B, overlap);
         LFOR(L, i, s, e) {
             int16_t f = (int16_t)c_mul16_q15(window[i], window[i]);
@@ -450,7 +450,7 @@ DNI void comb_filter_lanes(Lanes L, int32_t *y, int32_t *x, int T0, int T1, int 
         }
         return;
     }
-    for (int s = overlap; s < N; s += B) {
+    ROLLED for (int s = overlap; s < N; s += B) {
         int e = imin(s + B, N);
         LFOR(L, k, s, e) {
             int32_t v = wadd(wadd(wadd(x[k], c_mul16_32_q15(g10, x[k - T1])),
@@ -476,18 +476,18 @@ DNI void deemphasis(Lanes L, int32_t *in0, int32_t *in1, int16_t *pcm, int N, in
         c0 = L.id;
         c1 = L.id < C ? L.id + 1 : L.id;
     }
-    for (int c = c0; c < c1; c++) {
+    ROLLED for (int c = c0; c < c1; c++) {
         const int32_t *x = c == 0 ? in0 : in1;
         int16_t *y = pcm + c;
         int32_t m = mem[c];
         if (accum) {
-            for (int j = 0; j < N; j++) {
+            ROLLED for (int j = 0; j < N; j++) {
                 int32_t tmp = wadd(x[j], m);
                 m = c_mul16_32_q15(coef0, tmp);
                 y[j * C] = c_sat16((int32_t)y[j * C] + c_sig2word16(tmp));
             }
         } else {
-            for (int j = 0; j < N; j++) {
+            ROLLED for (int j = 0; j < N; j++) {
                 int32_t tmp = wadd(x[j], m);
                 m = c_mul16_32_q15(coef0, tmp);
                 y[j * C] = c_sig2word16(tmp);
@@ -514,22 +514,22 @@ DNI void celt_synthesis(Lanes L, CeltScratch *w, const int16_t *X, int32_t **out
         int32_t *freq2 = out_syn[1] + CELT_OVERLAP / 2;
         LFOR(L, i, 0, N) freq2[i] = freq[i];
         lsync(L);
-        for (int b = 0; b < B; b++) mdct_backward(L, &freq2[b], out_syn[0] + NB * b, shift, B);
-        for (int b = 0; b < B; b++) mdct_backward(L, &freq[b], out_syn[1] + NB * b, shift, B);
+        ROLLED for (int b = 0; b < B; b++) mdct_backward(L, &freq2[b], out_syn[0] + NB * b, shift, B);
+        ROLLED for (int b = 0; b < B; b++) mdct_backward(L, &freq[b], out_syn[1] + NB * b, shift, B);
     } else if (CC == 1 && C == 2) {
         int32_t *freq2 = out_syn[0] + CELT_OVERLAP / 2;
         denormalise_bands(L, X, freq, oldBandE, start, effEnd, M, silence);
         denormalise_bands(L, X + N, freq2, oldBandE + CELT_NB, start, effEnd, M, silence);
         LFOR(L, i, 0, N) freq[i] = wadd(freq[i] >> 1, freq2[i] >> 1);
         lsync(L);
-        for (int b = 0; b < B; b++) mdct_backward(L, &freq[b], out_syn[0] + NB * b, shift, B);
+        ROLLED for (int b = 0; b < B; b++) mdct_backward(L, &freq[b], out_syn[0] + NB * b, shift, B);
     } else {
-        for (int c = 0; c < CC; c++) {
+        ROLLED for (int c = 0; c < CC; c++) {
             denormalise_bands(L, X + c * N, freq, oldBandE + c * CELT_NB, start, effEnd, M, silence);
-            for (int b = 0; b < B; b++) mdct_backward(L, &freq[b], out_syn[c] + NB * b, shift, B);
+            ROLLED for (int b = 0; b < B; b++) mdct_backward(L, &freq[b], out_syn[c] + NB * b, shift, B);
         }
     }
-    for (int c = 0; c < CC; c++) {
+    ROLLED for (int c = 0; c < CC; c++) {
         int32_t *o = out_syn[c];
         LFOR(L, i, 0, N) o[i] = c_sat(o[i], CELT_SIG_SAT);
     }
@@ -546,8 +546,8 @@ DNI void unquant_coarse_energy(int start, int end, int16_t *oldEBands, int intra
     if (intra) { coef = 0; beta = T_CELT_BETA_INTRA; }
     else { beta = T_celt_beta_coef[LM]; coef = T_celt_pred_coef[LM]; }
     int32_t budget = dec->storage * 8;
-    for (int i = start; i < end; i++) {
-        for (int c = 0; c < C; c++) {
+    ROLLED for (int i = start; i < end; i++) {
+        ROLLED for (int c = 0; c < C; c++) {
             int qi;
             int32_t tell = rd_tell(dec);
             if (budget - tell >= 15) {
@@ -575,9 +575,9 @@ DNI void unquant_coarse_energy(int start, int end, int16_t *oldEBands, int intra
 DNI void unquant_fine_energy(int start, int end, int16_t *oldEBands, const int32_t *fine_quant, RangeDec *dec,
                              int C)
 {
-    for (int i = start; i < end; i++) {
+    ROLLED for (int i = start; i < end; i++) {
         if (fine_quant[i] <= 0) continue;
-        for (int c = 0; c < C; c++) {
+        ROLLED for (int c = 0; c < C; c++) {
             int q2 = (int)rd_bits(dec, fine_quant[i]);
             int16_t offset = (int16_t)(((shl32(q2, 10) + 512) >> fine_quant[i]) - 512);
             oldEBands[i + c * CELT_NB] = (int16_t)(oldEBands[i + c * CELT_NB] + offset);
@@ -588,10 +588,10 @@ DNI void unquant_fine_energy(int start, int end, int16_t *oldEBands, const int32
 DNI void unquant_energy_finalise(int start, int end, int16_t *oldEBands, const int32_t *fine_quant,
                                  const int32_t *fine_priority, int bits_left, RangeDec *dec, int C)
 {
-    for (int prio = 0; prio < 2; prio++) {
-        for (int i = start; i < end && bits_left >= C; i++) {
+    ROLLED for (int prio = 0; prio < 2; prio++) {
+        ROLLED for (int i = start; i < end && bits_left >= C; i++) {
             if (fine_quant[i] >= 8 || fine_priority[i] != prio) continue;
-            for (int c = 0; c < C; c++) {
+            ROLLED for (int c = 0; c < C; c++) {
                 int q2 = (int)rd_bits(dec, 1);
                 int16_t offset = (int16_t)((int16_t)((uint16_t)q2 << 10) - 512) >> (fine_quant[i] + 1);
                 oldEBands[i + c * CELT_NB] = (int16_t)(oldEBands[i + c * CELT_NB] + offset);
@@ -615,7 +615,7 @@ DFN int bits2pulses(int band, int LM, int bits)
     const uint8_t *cache = pulse_cache(band, LM);
     int lo = 0, hi = cache[0];
     bits--;
-    for (int i = 0; i < 6; i++) {
+    ROLLED for (int i = 0; i < 6; i++) {
         int mid = (lo + hi + 1) >> 1;
         if ((int)cache[mid] >= bits) hi = mid;
         else lo = mid;
@@ -632,7 +632,7 @@ DFN int pulses2bits(int band, int LM, int pulses)
 
 DFN void init_caps(int32_t *cap, int LM, int C)
 {
-    for (int i = 0; i < CELT_NB; i++) {
+    ROLLED for (int i = 0; i < CELT_NB; i++) {
         int N = (T_celt_eBands[i + 1] - T_celt_eBands[i]) << LM;
         cap[i] = (T_celt_cache_caps[CELT_NB * (2 * LM + C - 1) + i] + 64) * C * N >> 2;
     }
@@ -651,11 +651,11 @@ DNI int interp_bits2pulses(int start, int end, int skip_start, const int32_t *bi
     int lo = 0, hi = 1 << 6;
     int32_t psum;
     int done;
-    for (int i = 0; i < 6; i++) {
+    ROLLED for (int i = 0; i < 6; i++) {
         int mid = (lo + hi) >> 1;
         psum = 0;
         done = 0;
-        for (int j = end; j-- > start;) {
+        ROLLED for (int j = end; j-- > start;) {
             int tmp = bits1[j] + (mid * (int32_t)bits2[j] >> 6);
             if (tmp >= thresh[j] || done) {
                 done = 1;
@@ -669,7 +669,7 @@ DNI int interp_bits2pulses(int start, int end, int skip_start, const int32_t *bi
     }
     psum = 0;
     done = 0;
-    for (int j = end; j-- > start;) {
+    ROLLED for (int j = end; j-- > start;) {
         int tmp = bits1[j] + ((int32_t)lo * bits2[j] >> 6);
         if (tmp < thresh[j] && !done) {
             if (tmp >= alloc_floor) tmp = alloc_floor;
@@ -682,7 +682,7 @@ DNI int interp_bits2pulses(int start, int end, int skip_start, const int32_t *bi
         psum += tmp;
     }
     int codedBands;
-    for (codedBands = end;; codedBands--) {
+    ROLLED for (codedBands = end;; codedBands--) {
         int j = codedBands - 1;
         if (j <= skip_start) {
             total += skip_rsv;
@@ -720,15 +720,15 @@ DNI int interp_bits2pulses(int start, int end, int skip_start, const int32_t *bi
     int32_t left = total - psum;
     int32_t percoeff = (int32_t)((uint32_t)left / (uint32_t)(eB[codedBands] - eB[start]));
     left -= (eB[codedBands] - eB[start]) * percoeff;
-    for (int j = start; j < codedBands; j++) bits[j] += (int)percoeff * (eB[j + 1] - eB[j]);
-    for (int j = start; j < codedBands; j++) {
+    ROLLED for (int j = start; j < codedBands; j++) bits[j] += (int)percoeff * (eB[j + 1] - eB[j]);
+    ROLLED for (int j = start; j < codedBands; j++) {
         int tmp = (int)imin(left, eB[j + 1] - eB[j]);
         bits[j] += tmp;
         left -= tmp;
     }
     int32_t balance = 0;
     int j;
-    for (j = start; j < codedBands; j++) {
+    ROLLED for (j = start; j < codedBands; j++) {
         int N0 = eB[j + 1] - eB[j];
         int N = N0 << LM;
         int32_t bit = (int32_t)bits[j] + balance;
@@ -764,7 +764,7 @@ DNI int interp_bits2pulses(int start, int end, int skip_start, const int32_t *bi
         balance = excess;
     }
     *_balance = balance;
-    for (; j < end; j++) {
+    ROLLED for (; j < end; j++) {
         ebits[j] = bits[j] >> stereo >> 3;
         bits[j] = 0;
         fine_priority[j] = ebits[j] < 1;
@@ -793,16 +793,16 @@ DNI int clt_compute_allocation(int start, int end, const int32_t *offsets, const
             total -= dual_stereo_rsv;
         }
     }
-    for (int j = start; j < end; j++) {
+    ROLLED for (int j = start; j < end; j++) {
         thresh[j] = imax(C << 3, (3 * (eB[j + 1] - eB[j]) << LM << 3) >> 4);
         trim_offset[j] = C * (eB[j + 1] - eB[j]) * (alloc_trim - 5 - LM) * (end - j - 1) * (1 << (LM + 3)) >> 6;
         if ((eB[j + 1] - eB[j]) << LM == 1) trim_offset[j] -= C << 3;
     }
     int lo = 1, hi = T_CELT_NBALLOCV - 1;
-    do {
+    ROLLED do {
         int done = 0, psum = 0;
         int mid = (lo + hi) >> 1;
-        for (int j = end; j-- > start;) {
+        ROLLED for (int j = end; j-- > start;) {
             int N = eB[j + 1] - eB[j];
             int bitsj = C * N * T_celt_allocVectors[mid * CELT_NB + j] << LM >> 2;
             if (bitsj > 0) bitsj = imax(0, bitsj + trim_offset[j]);
@@ -818,7 +818,7 @@ DNI int clt_compute_allocation(int start, int end, const int32_t *offsets, const
         else lo = mid + 1;
     } while (lo <= hi);
     hi = lo--;
-    for (int j = start; j < end; j++) {
+    ROLLED for (int j = start; j < end; j++) {
         int N = eB[j + 1] - eB[j];
         int bits1j = C * N * T_celt_allocVectors[lo * CELT_NB + j] << LM >> 2;
         int bits2j = hi >= T_CELT_NBALLOCV ? cap[j] : C * N * T_celt_allocVectors[hi * CELT_NB + j] << LM >> 2;
@@ -853,7 +853,7 @@ DNI int32_t cwrsi(int n, int k, uint32_t idx, int32_t *y)
     int s, k0;
     int16_t val;
     int32_t yy = 0;
-    while (n > 2) {
+    ROLLED while (n > 2) {
         uint32_t q;
         if (k >= n) {
             p = pvq_row(n, k + 1);
@@ -863,10 +863,10 @@ DNI int32_t cwrsi(int n, int k, uint32_t idx, int32_t *y)
             q = pvq_row(n, n);
             if (q > idx) {
                 k = n;
-                do p = pvq_row(--k, n);
+                ROLLED do p = pvq_row(--k, n);
                 while (p > idx);
             } else {
-                for (p = pvq_row(n, k); p > idx; p = pvq_row(n, k)) k--;
+                ROLLED for (p = pvq_row(n, k); p > idx; p = pvq_row(n, k)) k--;
             }
             idx -= p;
             val = (int16_t)((k0 - k + s) ^ s);
@@ -882,7 +882,7 @@ DNI int32_t cwrsi(int n, int k, uint32_t idx, int32_t *y)
                 s = -(idx >= q);
                 idx -= q & s;
                 k0 = k;
-                do p = pvq_row(--k, n);
+                ROLLED do p = pvq_row(--k, n);
                 while (p > idx);
                 idx -= p;
                 val = (int16_t)((k0 - k + s) ^ s);
@@ -919,10 +919,10 @@ DNI void exp_rotation1(int16_t *X, int len, int stride, int16_t c, int16_t s)
 {
     const int16_t ms = (int16_t)-s;
     // forward: i = 0 .. len - stride - 1
-    for (int j = 0; j < stride && j < len - stride; j++) {
+    ROLLED for (int j = 0; j < stride && j < len - stride; j++) {
         int16_t x1 = X[j];
         int i = j;
-        for (; i < len - stride; i += stride) {
+        ROLLED for (; i < len - stride; i += stride) {
             int16_t x2 = X[i + stride];
             X[i] = (int16_t)c_pshr(c_mac16(c_mul16(c, x1), ms, x2), 15);
             x1 = (int16_t)c_pshr(c_mac16(c_mul16(c, x2), s, x1), 15);   // the new X[i + stride]
@@ -932,10 +932,10 @@ DNI void exp_rotation1(int16_t *X, int len, int stride, int16_t c, int16_t s)
     // backward: i = len - 2 stride - 1 .. 0; pair i - stride reads the X[i]
     // pair i has written
     const int top = len - 2 * stride - 1;
-    for (int j = 0; j < stride && top - j >= 0; j++) {
+    ROLLED for (int j = 0; j < stride && top - j >= 0; j++) {
         int i = top - j;
         int16_t x2 = X[i + stride];
-        for (; i >= 0; i -= stride) {
+        ROLLED for (; i >= 0; i -= stride) {
             int16_t x1 = X[i];
             X[i + stride] = (int16_t)c_pshr(c_mac16(c_mul16(c, x2), s, x1), 15);
             x2 = (int16_t)c_pshr(c_mac16(c_mul16(c, x1), ms, x2), 15);   // the new X[i]
@@ -956,10 +956,10 @@ DNI void exp_rotation_dec(int16_t *X, int len, int stride, int K, int spread)
     int stride2 = 0;
     if (len >= 8 * stride) {
         stride2 = 1;
-        while ((stride2 * stride2 + stride2) * stride + (stride >> 2) < len) stride2++;
+        ROLLED while ((stride2 * stride2 + stride2) * stride + (stride >> 2) < len) stride2++;
     }
     len = (int)((unsigned)len / (unsigned)stride);
-    for (int i = 0; i < stride; i++) {
+    ROLLED for (int i = 0; i < stride; i++) {
         if (stride2) exp_rotation1(X + i * len, len, stride2, s, c);
         exp_rotation1(X + i * len, len, 1, c, s);
     }
@@ -1002,9 +1002,9 @@ DNI unsigned alg_unquant(Lanes L, int16_t *X, int N, int K, int spread, int B, R
     if (B <= 1) return 1;
     int N0 = (int)((unsigned)N / (unsigned)B);
     unsigned mask = 0;
-    for (int i = 0; i < B; i++) {
+    ROLLED for (int i = 0; i < B; i++) {
         unsigned tmp = 0;
-        for (int j = 0; j < N0; j++) tmp |= iy[i * N0 + j];
+        ROLLED for (int j = 0; j < N0; j++) tmp |= iy[i * N0 + j];
         mask |= (tmp != 0) << i;
     }
     return mask;
@@ -1032,8 +1032,8 @@ DFN int bitexact_log2tan(int isin, int icos)
 DNI void haar1(int16_t *X, int N0, int stride)
 {
     N0 >>= 1;
-    for (int i = 0; i < stride; i++)
-        for (int j = 0; j < N0; j++) {
+    ROLLED for (int i = 0; i < stride; i++)
+        ROLLED for (int j = 0; j < N0; j++) {
             int32_t t1 = c_mul16(23170, X[stride * 2 * j + i]);
             int32_t t2 = c_mul16(23170, X[stride * (2 * j + 1) + i]);
             X[stride * 2 * j + i] = (int16_t)c_pshr(wadd(t1, t2), 15);
@@ -1046,13 +1046,13 @@ DNI void deinterleave_hadamard(int16_t *X, int N0, int stride, int hadamard, int
     int N = N0 * stride;
     if (hadamard) {
         const int32_t *ordery = T_celt_ordery_table + stride - 2;
-        for (int i = 0; i < stride; i++)
-            for (int j = 0; j < N0; j++) tmp[ordery[i] * N0 + j] = X[j * stride + i];
+        ROLLED for (int i = 0; i < stride; i++)
+            ROLLED for (int j = 0; j < N0; j++) tmp[ordery[i] * N0 + j] = X[j * stride + i];
     } else {
-        for (int i = 0; i < stride; i++)
-            for (int j = 0; j < N0; j++) tmp[i * N0 + j] = X[j * stride + i];
+        ROLLED for (int i = 0; i < stride; i++)
+            ROLLED for (int j = 0; j < N0; j++) tmp[i * N0 + j] = X[j * stride + i];
     }
-    for (int i = 0; i < N; i++) X[i] = tmp[i];
+    ROLLED for (int i = 0; i < N; i++) X[i] = tmp[i];
 }
 
 DNI void interleave_hadamard(int16_t *X, int N0, int stride, int hadamard, int16_t *tmp)
@@ -1060,13 +1060,13 @@ DNI void interleave_hadamard(int16_t *X, int N0, int stride, int hadamard, int16
     int N = N0 * stride;
     if (hadamard) {
         const int32_t *ordery = T_celt_ordery_table + stride - 2;
-        for (int i = 0; i < stride; i++)
-            for (int j = 0; j < N0; j++) tmp[j * stride + i] = X[ordery[i] * N0 + j];
+        ROLLED for (int i = 0; i < stride; i++)
+            ROLLED for (int j = 0; j < N0; j++) tmp[j * stride + i] = X[ordery[i] * N0 + j];
     } else {
-        for (int i = 0; i < stride; i++)
-            for (int j = 0; j < N0; j++) tmp[j * stride + i] = X[i * N0 + j];
+        ROLLED for (int i = 0; i < stride; i++)
+            ROLLED for (int j = 0; j < N0; j++) tmp[j * stride + i] = X[i * N0 + j];
     }
-    for (int i = 0; i < N; i++) X[i] = tmp[i];
+    ROLLED for (int i = 0; i < N; i++) X[i] = tmp[i];
 }
 
 struct BandCtx {
@@ -1174,7 +1174,7 @@ DNI unsigned quant_band_n1(BandCtx *ctx, int16_t *X, int16_t *Y, int16_t *lowban
 {
     int16_t *x = X;
     int stereo = Y != 0;
-    for (int c = 0; c < 1 + stereo; c++) {
+    ROLLED for (int c = 0; c < 1 + stereo; c++) {
         int sign = 0;
         if (ctx->remaining_bits >= 1 << 3) {
             sign = (int)rd_bits(ctx->ec, 1);
@@ -1197,7 +1197,7 @@ DNI unsigned quant_partition_leaf(BandCtx *ctx, int16_t *X, int N, int b, int B,
     int q = bits2pulses(i, LM, b);
     int curr_bits = pulses2bits(i, LM, q);
     ctx->remaining_bits -= curr_bits;
-    while (ctx->remaining_bits < 0 && q > 0) {
+    ROLLED while (ctx->remaining_bits < 0 && q > 0) {
         ctx->remaining_bits += curr_bits;
         q--;
         curr_bits = pulses2bits(i, LM, q);
@@ -1210,16 +1210,16 @@ DNI unsigned quant_partition_leaf(BandCtx *ctx, int16_t *X, int N, int b, int B,
         unsigned cm_mask = (unsigned)(1UL << B) - 1;
         fill &= cm_mask;
         if (!fill) {
-            for (int j = 0; j < N; j++) X[j] = 0;
+            ROLLED for (int j = 0; j < N; j++) X[j] = 0;
         } else {
             if (lowband == 0) {
-                for (int j = 0; j < N; j++) {
+                ROLLED for (int j = 0; j < N; j++) {
                     ctx->seed = c_lcg_rand(ctx->seed);
                     X[j] = (int16_t)((int32_t)ctx->seed >> 20);
                 }
                 cm = cm_mask;
             } else {
-                for (int j = 0; j < N; j++) {
+                ROLLED for (int j = 0; j < N; j++) {
                     ctx->seed = c_lcg_rand(ctx->seed);
                     int16_t tmp = (ctx->seed & 0x8000) ? 4 : -4;   // QCONST16(1.0f/256, 10)
                     X[j] = (int16_t)(lowband[j] + tmp);
@@ -1255,7 +1255,7 @@ DNI unsigned quant_partition(BandCtx *ctx, int16_t *X, int N, int b, int B, int1
     st[0].stage = 0;
     unsigned ret = 0;
     const int i = ctx->i;
-    while (sp >= 0) {
+    ROLLED while (sp >= 0) {
         QPFrame *f = &st[sp];
         QPFrame *c = &st[sp + 1 < 5 ? sp + 1 : 4];
         if (f->stage == 0) {
@@ -1374,16 +1374,16 @@ DNI unsigned quant_band(BandCtx *ctx, int16_t *X, int N, int b, int B, int16_t *
     if (tf_change > 0) recombine = tf_change;
     PHASE_BEGIN(t_tf);
     if (lowband_scratch && lowband && (recombine || ((N_B & 1) == 0 && tf_change < 0) || B0 > 1)) {
-        for (int j = 0; j < N; j++) lowband_scratch[j] = lowband[j];
+        ROLLED for (int j = 0; j < N; j++) lowband_scratch[j] = lowband[j];
         lowband = lowband_scratch;
     }
-    for (int k = 0; k < recombine; k++) {
+    ROLLED for (int k = 0; k < recombine; k++) {
         if (lowband) haar1(lowband, N >> k, 1 << k);
         fill = bit_interleave_table[fill & 0xF] | bit_interleave_table[fill >> 4] << 2;
     }
     B >>= recombine;
     N_B <<= recombine;
-    while ((N_B & 1) == 0 && tf_change < 0) {
+    ROLLED while ((N_B & 1) == 0 && tf_change < 0) {
         if (lowband) haar1(lowband, N_B, B);
         fill |= fill << B;
         B <<= 1;
@@ -1401,13 +1401,13 @@ DNI unsigned quant_band(BandCtx *ctx, int16_t *X, int N, int b, int B, int16_t *
     if (B0 > 1) interleave_hadamard(X, N_B >> recombine, B0 << recombine, longBlocks, ctx->w->tmp);
     N_B = N_B0;
     B = B0;
-    for (int k = 0; k < time_divide; k++) {
+    ROLLED for (int k = 0; k < time_divide; k++) {
         B >>= 1;
         N_B <<= 1;
         cm |= cm >> B;
         haar1(X, N_B, B);
     }
-    for (int k = 0; k < recombine; k++) {
+    ROLLED for (int k = 0; k < recombine; k++) {
         cm = bit_deinterleave_table[cm];
         haar1(X, N0 >> k, 1 << k);
     }
@@ -1415,7 +1415,7 @@ DNI unsigned quant_band(BandCtx *ctx, int16_t *X, int N, int b, int B, int16_t *
     B <<= recombine;
     if (lowband_out) {
         int16_t n = (int16_t)c_sqrt(shl32(N0, 22));
-        for (int j = 0; j < N0; j++) lowband_out[j] = (int16_t)c_mul16_q15(n, X[j]);
+        ROLLED for (int j = 0; j < N0; j++) lowband_out[j] = (int16_t)c_mul16_q15(n, X[j]);
     }
     cm &= (1 << B) - 1;
     return cm;
@@ -1513,7 +1513,7 @@ DNI unsigned quant_band_stereo(BandCtx *ctx, int16_t *X, int16_t *Y, int N, int 
     }
     if (N != 2) stereo_merge(ctx->L, X, Y, mid, N);
     if (inv)
-        for (int j = 0; j < N; j++) Y[j] = (int16_t)-Y[j];
+        ROLLED for (int j = 0; j < N; j++) Y[j] = (int16_t)-Y[j];
     return cm;
 }
 
@@ -1541,7 +1541,7 @@ DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *
     ctx.avoid_split_noise = B > 1;
     ctx.w = w;
     ctx.L = L;
-    for (int i = start; i < end; i++) {
+    ROLLED for (int i = start; i < end; i++) {
         int effective_lowband = -1;
         unsigned x_cm, y_cm;
         ctx.i = i;
@@ -1566,9 +1566,9 @@ DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *
             // special_hybrid_folding
             int n1 = M * (eB[start + 1] - eB[start]);
             int n2 = M * (eB[start + 2] - eB[start + 1]);
-            for (int j = 0; j < n2 - n1; j++) norm[n1 + j] = norm[2 * n1 - n2 + j];
+            ROLLED for (int j = 0; j < n2 - n1; j++) norm[n1 + j] = norm[2 * n1 - n2 + j];
             if (dual_stereo)
-                for (int j = 0; j < n2 - n1; j++) norm2[n1 + j] = norm2[2 * n1 - n2 + j];
+                ROLLED for (int j = 0; j < n2 - n1; j++) norm2[n1 + j] = norm2[2 * n1 - n2 + j];
         }
         int tf_change = tf_res[i];
         ctx.tf_change = tf_change;
@@ -1581,12 +1581,12 @@ DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *
         if (lowband_offset != 0 && (spread != SPREAD_AGGRESSIVE || B > 1 || tf_change < 0)) {
             effective_lowband = imax(0, M * eB[lowband_offset] - norm_offset - N);
             int fold_start = lowband_offset;
-            while (M * eB[--fold_start] > effective_lowband + norm_offset) {}
+            ROLLED while (M * eB[--fold_start] > effective_lowband + norm_offset) {}
             int fold_end = lowband_offset - 1;
-            while (++fold_end < i && M * eB[fold_end] < effective_lowband + norm_offset + N) {}
+            ROLLED while (++fold_end < i && M * eB[fold_end] < effective_lowband + norm_offset + N) {}
             x_cm = y_cm = 0;
             int fold_i = fold_start;
-            do {
+            ROLLED do {
                 x_cm |= collapse_masks[fold_i * C + 0];
                 y_cm |= collapse_masks[fold_i * C + C - 1];
             } while (++fold_i < fold_end);
@@ -1595,7 +1595,7 @@ DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *
         }
         if (dual_stereo && i == intensity) {
             dual_stereo = 0;
-            for (int j = 0; j < M * eB[i] - norm_offset; j++) norm[j] = (int16_t)((norm[j] + norm2[j]) >> 1);
+            ROLLED for (int j = 0; j < M * eB[i] - norm_offset; j++) norm[j] = (int16_t)((norm[j] + norm2[j]) >> 1);
         }
         if (dual_stereo) {
             x_cm = quant_band(&ctx, X, N, b / 2, B, effective_lowband != -1 ? norm + effective_lowband : 0, LM,
@@ -1632,7 +1632,7 @@ DNI void anti_collapse(Lanes L, int16_t *X_, const uint8_t *collapse_masks, int 
                        const int32_t *pulses, uint32_t seed)
 {
     const int16_t *eB = T_celt_eBands;
-    for (int i = start; i < end; i++) {
+    ROLLED for (int i = start; i < end; i++) {
         int N0 = eB[i + 1] - eB[i];
         int depth = (int)((uint32_t)(1 + pulses[i]) / (uint32_t)N0) >> LM;
         int32_t thresh32 = c_exp2((int16_t)-(int16_t)((uint16_t)depth << 7)) >> 1;
@@ -1641,7 +1641,7 @@ DNI void anti_collapse(Lanes L, int16_t *X_, const uint8_t *collapse_masks, int 
         int shift = c_ilog2(t) >> 1;
         t = shl32(t, (7 - shift) << 1);
         int16_t sqrt_1 = c_rsqrt_norm(t);
-        for (int c = 0; c < C; c++) {
+        ROLLED for (int c = 0; c < C; c++) {
             int renormalize = 0;
             int16_t prev1 = prev1logE[c * CELT_NB + i], prev2 = prev2logE[c * CELT_NB + i];
             if (C == 1) {
@@ -1661,9 +1661,9 @@ DNI void anti_collapse(Lanes L, int16_t *X_, const uint8_t *collapse_masks, int 
             r = (int16_t)((thresh < r ? thresh : r) >> 1);
             r = (int16_t)(c_mul16_q15(sqrt_1, r) >> shift);
             int16_t *X = X_ + c * size + (eB[i] << LM);
-            for (int k = 0; k < 1 << LM; k++) {
+            ROLLED for (int k = 0; k < 1 << LM; k++) {
                 if (!(collapse_masks[i * C + c] & 1 << k)) {
-                    for (int j = 0; j < N0; j++) {
+                    ROLLED for (int j = 0; j < N0; j++) {
                         seed = c_lcg_rand(seed);
                         X[(j << LM) + k] = (seed & 0x8000) ? r : (int16_t)-r;
                     }
@@ -1683,7 +1683,7 @@ DNI void tf_decode(int start, int end, int isTransient, int32_t *tf_res, int LM,
     int tf_select_rsv = LM > 0 && tell + logp + 1 <= budget;
     budget -= tf_select_rsv;
     int tf_changed = 0, curr = 0;
-    for (int i = start; i < end; i++) {
+    ROLLED for (int i = start; i < end; i++) {
         if (tell + logp <= budget) {
             curr ^= rd_bit_logp(dec, logp);
             tell = (uint32_t)rd_tell(dec);
@@ -1696,7 +1696,7 @@ DNI void tf_decode(int start, int end, int isTransient, int32_t *tf_res, int LM,
     const int8_t *tt = &T_celt_tf_select_table[LM * 8];
     if (tf_select_rsv && tt[4 * isTransient + 0 + tf_changed] != tt[4 * isTransient + 2 + tf_changed])
         tf_select = rd_bit_logp(dec, 1);
-    for (int i = start; i < end; i++) tf_res[i] = tt[4 * isTransient + 2 * tf_select + tf_res[i]];
+    ROLLED for (int i = start; i < end; i++) tf_res[i] = tt[4 * isTransient + 2 * tf_select + tf_res[i]];
 }
 
 // ------------------------------------------------------------------ PLC (pitch / LPC)
@@ -1709,8 +1709,8 @@ DNI int32_t celt_autocorr(const int16_t *x, int32_t *ac, const int16_t *window, 
     if (overlap == 0) {
         xptr = x;
     } else {
-        for (int i = 0; i < n; i++) xx[i] = x[i];
-        for (int i = 0; i < overlap; i++) {
+        ROLLED for (int i = 0; i < n; i++) xx[i] = x[i];
+        ROLLED for (int i = 0; i < overlap; i++) {
             xx[i] = (int16_t)c_mul16_q15(x[i], window[i]);
             xx[n - i - 1] = (int16_t)c_mul16_q15(x[n - i - 1], window[i]);
         }
@@ -1719,39 +1719,39 @@ DNI int32_t celt_autocorr(const int16_t *x, int32_t *ac, const int16_t *window, 
     {
         int32_t ac0 = 1 + (n << 7);
         if (n & 1) ac0 = wadd(ac0, c_mul16(xptr[0], xptr[0]) >> 9);
-        for (int i = (n & 1); i < n; i += 2) {
+        ROLLED for (int i = (n & 1); i < n; i += 2) {
             ac0 = wadd(ac0, c_mul16(xptr[i], xptr[i]) >> 9);
             ac0 = wadd(ac0, c_mul16(xptr[i + 1], xptr[i + 1]) >> 9);
         }
         shift = c_ilog2(ac0) - 30 + 10;
         shift = shift / 2;
         if (shift > 0) {
-            for (int i = 0; i < n; i++) xx[i] = (int16_t)c_pshr(xptr[i], shift);
+            ROLLED for (int i = 0; i < n; i++) xx[i] = (int16_t)c_pshr(xptr[i], shift);
             xptr = xx;
         } else {
             shift = 0;
         }
     }
-    for (int k = 0; k <= lag; k++) {
+    ROLLED for (int k = 0; k <= lag; k++) {
         int32_t s = 0;
-        for (int j = 0; j < fastN; j++) s = c_mac16(s, xptr[j], xptr[j + k]);
+        ROLLED for (int j = 0; j < fastN; j++) s = c_mac16(s, xptr[j], xptr[j + k]);
         ac[k] = s;
     }
-    for (int k = 0; k <= lag; k++) {
+    ROLLED for (int k = 0; k <= lag; k++) {
         int32_t d = 0;
-        for (int i = k + fastN; i < n; i++) d = c_mac16(d, xptr[i], xptr[i - k]);
+        ROLLED for (int i = k + fastN; i < n; i++) d = c_mac16(d, xptr[i], xptr[i - k]);
         ac[k] = wadd(ac[k], d);
     }
     shift = 2 * shift;
     if (shift <= 0) ac[0] = wadd(ac[0], shl32(1, -shift));
     if (ac[0] < 268435456) {
         int shift2 = 29 - ilog((uint32_t)ac[0]);
-        for (int i = 0; i <= lag; i++) ac[i] = shl32(ac[i], shift2);
+        ROLLED for (int i = 0; i <= lag; i++) ac[i] = shl32(ac[i], shift2);
         shift -= shift2;
     } else if (ac[0] >= 536870912) {
         int shift2 = 1;
         if (ac[0] >= 1073741824) shift2++;
-        for (int i = 0; i <= lag; i++) ac[i] = ac[i] >> shift2;
+        ROLLED for (int i = 0; i <= lag; i++) ac[i] = ac[i] >> shift2;
         shift += shift2;
     }
     return shift;
@@ -1761,15 +1761,15 @@ DNI void celt_lpc(int16_t *_lpc, const int32_t *ac, int p)
 {
     int32_t error = ac[0];
     int32_t lpc[CELT_LPC_ORDER];
-    for (int i = 0; i < p; i++) lpc[i] = 0;
+    ROLLED for (int i = 0; i < p; i++) lpc[i] = 0;
     if (ac[0] != 0) {
-        for (int i = 0; i < p; i++) {
+        ROLLED for (int i = 0; i < p; i++) {
             int32_t rr = 0;
-            for (int j = 0; j < i; j++) rr = wadd(rr, c_mul32_q31(lpc[j], ac[i - j]));
+            ROLLED for (int j = 0; j < i; j++) rr = wadd(rr, c_mul32_q31(lpc[j], ac[i - j]));
             rr = wadd(rr, ac[i + 1] >> 6);
             int32_t r = -c_frac_div32(shl32(rr, 6), error);
             lpc[i] = r >> 6;
-            for (int j = 0; j < (i + 1) >> 1; j++) {
+            ROLLED for (int j = 0; j < (i + 1) >> 1; j++) {
                 int32_t t1 = lpc[j], t2 = lpc[i - 1 - j];
                 lpc[j] = wadd(t1, c_mul32_q31(r, t2));
                 lpc[i - 1 - j] = wadd(t2, c_mul32_q31(r, t1));
@@ -1779,9 +1779,9 @@ DNI void celt_lpc(int16_t *_lpc, const int32_t *ac, int p)
         }
     }
     int iter, idx = 0;
-    for (iter = 0; iter < 10; iter++) {
+    ROLLED for (iter = 0; iter < 10; iter++) {
         int32_t maxabs = 0;
-        for (int i = 0; i < p; i++) {
+        ROLLED for (int i = 0; i < p; i++) {
             int32_t a = lpc[i] < 0 ? -lpc[i] : lpc[i];
             if (a > maxabs) { maxabs = a; idx = i; }
         }
@@ -1790,7 +1790,7 @@ DNI void celt_lpc(int16_t *_lpc, const int32_t *ac, int p)
             maxabs = min32(maxabs, 163838);
             int32_t chirp_Q16 = 65470 - shl32(maxabs - 32767, 14) / (wmul(maxabs, idx + 1) >> 2);
             int32_t cm1 = chirp_Q16 - 65536;
-            for (int i = 0; i < p - 1; i++) {
+            ROLLED for (int i = 0; i < p - 1; i++) {
                 lpc[i] = c_mul32_q16(chirp_Q16, lpc[i]);
                 chirp_Q16 += c_pshr(wmul(chirp_Q16, cm1), 16);
             }
@@ -1802,15 +1802,15 @@ DNI void celt_lpc(int16_t *_lpc, const int32_t *ac, int p)
     if (iter == 10) {
         _lpc[0] = 4096;   // the remaining outputs keep their previous values, as in libopus
     } else {
-        for (int i = 0; i < p; i++) _lpc[i] = (int16_t)c_pshr(lpc[i], 13);
+        ROLLED for (int i = 0; i < p; i++) _lpc[i] = (int16_t)c_pshr(lpc[i], 13);
     }
 }
 
 DNI void celt_fir(const int16_t *x, const int16_t *num, int16_t *y, int N, int ord)
 {
-    for (int i = 0; i < N; i++) {
+    ROLLED for (int i = 0; i < N; i++) {
         int32_t sum = shl32((int32_t)x[i], 12);
-        for (int j = 0; j < ord; j++) sum = c_mac16(sum, num[ord - j - 1], x[i + j - ord]);
+        ROLLED for (int j = 0; j < ord; j++) sum = c_mac16(sum, num[ord - j - 1], x[i + j - ord]);
         y[i] = c_sround16(sum, 12);
     }
 }
@@ -1818,15 +1818,15 @@ DNI void celt_fir(const int16_t *x, const int16_t *num, int16_t *y, int N, int o
 // celt/celt_lpc.c celt_iir (the 4-way unrolled form computes the same values)
 DNI void celt_iir(const int32_t *_x, const int16_t *den, int32_t *_y, int N, int ord, int16_t *mem, int16_t *y)
 {
-    for (int i = 0; i < ord; i++) y[i] = (int16_t)-mem[ord - i - 1];
-    for (int i = ord; i < N + ord; i++) y[i] = 0;
-    for (int i = 0; i < N; i++) {
+    ROLLED for (int i = 0; i < ord; i++) y[i] = (int16_t)-mem[ord - i - 1];
+    ROLLED for (int i = ord; i < N + ord; i++) y[i] = 0;
+    ROLLED for (int i = 0; i < N; i++) {
         int32_t sum = _x[i];
-        for (int j = 0; j < ord; j++) sum = c_mac16(sum, den[ord - j - 1], y[i + j]);
+        ROLLED for (int j = 0; j < ord; j++) sum = c_mac16(sum, den[ord - j - 1], y[i + j]);
         y[i + ord] = (int16_t)-c_sround16(sum, 12);
         _y[i] = sum;
     }
-    for (int i = 0; i < ord; i++) mem[i] = (int16_t)_y[N - i - 1];
+    ROLLED for (int i = 0; i < ord; i++) mem[i] = (int16_t)_y[N - i - 1];
 }
 
 DNI void find_best_pitch(const int32_t *xcorr, const int16_t *y, int len, int max_pitch, int *best_pitch,
@@ -1838,8 +1838,8 @@ DNI void find_best_pitch(const int32_t *xcorr, const int16_t *y, int len, int ma
     int xshift = c_ilog2(maxcorr) - 14;
     best_pitch[0] = 0;
     best_pitch[1] = 1;
-    for (int j = 0; j < len; j++) Syy = wadd(Syy, c_mul16(y[j], y[j]) >> yshift);
-    for (int i = 0; i < max_pitch; i++) {
+    ROLLED for (int j = 0; j < len; j++) Syy = wadd(Syy, c_mul16(y[j], y[j]) >> yshift);
+    ROLLED for (int i = 0; i < max_pitch; i++) {
         if (xcorr[i] > 0) {
             int16_t xcorr16 = (int16_t)c_vshr(xcorr[i], xshift);
             int16_t num = (int16_t)c_mul16_q15(xcorr16, xcorr16);
@@ -1874,20 +1874,20 @@ DNI void pitch_downsample(int32_t *x0, int32_t *x1, int16_t *x_lp, int len, int 
     int shift = c_ilog2(maxabs) - 10;
     if (shift < 0) shift = 0;
     if (C == 2) shift++;
-    for (int i = 1; i < len >> 1; i++)
+    ROLLED for (int i = 1; i < len >> 1; i++)
         x_lp[i] = (int16_t)((x0[2 * i - 1] >> (shift + 2)) + (x0[2 * i + 1] >> (shift + 2)) + (x0[2 * i] >> (shift + 1)));
     x_lp[0] = (int16_t)((x0[1] >> (shift + 2)) + (x0[0] >> (shift + 1)));
     if (C == 2) {
-        for (int i = 1; i < len >> 1; i++)
+        ROLLED for (int i = 1; i < len >> 1; i++)
             x_lp[i] = (int16_t)(x_lp[i] + (x1[2 * i - 1] >> (shift + 2)) + (x1[2 * i + 1] >> (shift + 2)) +
                                 (x1[2 * i] >> (shift + 1)));
         x_lp[0] = (int16_t)(x_lp[0] + (x1[1] >> (shift + 2)) + (x1[0] >> (shift + 1)));
     }
     celt_autocorr(x_lp, ac, 0, 0, 4, len >> 1, xx);
     ac[0] = wadd(ac[0], ac[0] >> 13);
-    for (int i = 1; i <= 4; i++) ac[i] = wsub(ac[i], c_mul16_32_q15(2 * i * i, ac[i]));
+    ROLLED for (int i = 1; i <= 4; i++) ac[i] = wsub(ac[i], c_mul16_32_q15(2 * i * i, ac[i]));
     celt_lpc(lpc, ac, 4);
-    for (int i = 0; i < 4; i++) {
+    ROLLED for (int i = 0; i < 4; i++) {
         tmp = (int16_t)c_mul16_q15(29491, tmp);   // QCONST16(.9f, 15)
         lpc[i] = (int16_t)c_mul16_q15(lpc[i], tmp);
     }
@@ -1898,7 +1898,7 @@ DNI void pitch_downsample(int32_t *x0, int32_t *x1, int16_t *x_lp, int len, int 
     lpc2[4] = (int16_t)c_mul16_q15(c1, lpc[3]);
     // celt_fir5 in place
     int32_t m0 = 0, m1 = 0, m2 = 0, m3 = 0, m4 = 0;
-    for (int i = 0; i < len >> 1; i++) {
+    ROLLED for (int i = 0; i < len >> 1; i++) {
         int32_t sum = shl32((int32_t)x_lp[i], 12);
         sum = c_mac16(sum, lpc2[0], m0);
         sum = c_mac16(sum, lpc2[1], m1);
@@ -1918,13 +1918,13 @@ DNI void pitch_search(Lanes L, const int16_t *x_lp, int16_t *y, int len, int max
     int best_pitch[2] = {0, 0};
     int16_t *x_lp4 = w->x_lp4, *y_lp4 = w->y_lp4;
     int32_t *xcorr = w->xcorr;
-    for (int j = 0; j < len >> 2; j++) x_lp4[j] = x_lp[2 * j];
-    for (int j = 0; j < lag >> 2; j++) y_lp4[j] = y[2 * j];
+    ROLLED for (int j = 0; j < len >> 2; j++) x_lp4[j] = x_lp[2 * j];
+    ROLLED for (int j = 0; j < lag >> 2; j++) y_lp4[j] = y[2 * j];
     int32_t xmax = c_maxabs16(x_lp4, len >> 2), ymax = c_maxabs16(y_lp4, lag >> 2);
     int shift = c_ilog2(max32(1, max32(xmax, ymax))) - 11;
     if (shift > 0) {
-        for (int j = 0; j < len >> 2; j++) x_lp4[j] = (int16_t)(x_lp4[j] >> shift);
-        for (int j = 0; j < lag >> 2; j++) y_lp4[j] = (int16_t)(y_lp4[j] >> shift);
+        ROLLED for (int j = 0; j < len >> 2; j++) x_lp4[j] = (int16_t)(x_lp4[j] >> shift);
+        ROLLED for (int j = 0; j < lag >> 2; j++) y_lp4[j] = (int16_t)(y_lp4[j] >> shift);
         shift *= 2;
     } else {
         shift = 0;
@@ -1933,12 +1933,12 @@ DNI void pitch_search(Lanes L, const int16_t *x_lp, int16_t *y, int len, int max
     // celt_pitch_xcorr: every lag is an independent dot product
     LFOR(L, i, 0, max_pitch >> 2) {
         int32_t s = 0;
-        for (int j = 0; j < len >> 2; j++) s = c_mac16(s, x_lp4[j], y_lp4[i + j]);
+        ROLLED for (int j = 0; j < len >> 2; j++) s = c_mac16(s, x_lp4[j], y_lp4[i + j]);
         xcorr[i] = s;
     }
     lsync(L);
     int32_t maxcorr = 1;
-    for (int i = 0; i < max_pitch >> 2; i++) maxcorr = max32(maxcorr, xcorr[i]);
+    ROLLED for (int i = 0; i < max_pitch >> 2; i++) maxcorr = max32(maxcorr, xcorr[i]);
     find_best_pitch(xcorr, y_lp4, len >> 2, max_pitch >> 2, best_pitch, 0, maxcorr);
     lsync(L);
     LFOR(L, i, 0, max_pitch >> 1) {
@@ -1946,14 +1946,14 @@ DNI void pitch_search(Lanes L, const int16_t *x_lp, int16_t *y, int len, int max
         int d0 = i - 2 * best_pitch[0], d1 = i - 2 * best_pitch[1];
         if (!((d0 < 0 ? -d0 : d0) > 2 && (d1 < 0 ? -d1 : d1) > 2)) {
             int32_t s = 0;
-            for (int j = 0; j < len >> 1; j++) s = wadd(s, c_mul16(x_lp[j], y[i + j]) >> shift);
+            ROLLED for (int j = 0; j < len >> 1; j++) s = wadd(s, c_mul16(x_lp[j], y[i + j]) >> shift);
             xcorr[i] = max32(-1, s);
         }
     }
     lsync(L);
     // libopus tracks max(1, raw sums); the -1 floor and the zeroed lags cannot exceed 1
     maxcorr = 1;
-    for (int i = 0; i < max_pitch >> 1; i++) maxcorr = max32(maxcorr, xcorr[i]);
+    ROLLED for (int i = 0; i < max_pitch >> 1; i++) maxcorr = max32(maxcorr, xcorr[i]);
     find_best_pitch(xcorr, y, len >> 1, max_pitch >> 1, best_pitch, shift + 1, maxcorr);
     int offset;
     if (best_pitch[0] > 0 && best_pitch[0] < (max_pitch >> 1) - 1) {
@@ -1969,12 +1969,12 @@ DNI void pitch_search(Lanes L, const int16_t *x_lp, int16_t *y, int len, int max
 
 DNI void prefilter_and_fold(CeltDec *st, int N, CeltScratch *w)
 {
-    for (int c = 0; c < st->channels; c++) {
+    ROLLED for (int c = 0; c < st->channels; c++) {
         int32_t *dm = st->decode_mem[c];
         comb_filter(w->etmp, dm + CELT_DEC_BUF - N, st->postfilter_period_old, st->postfilter_period, CELT_OVERLAP,
                     (int16_t)-st->postfilter_gain_old, (int16_t)-st->postfilter_gain, st->postfilter_tapset_old,
                     st->postfilter_tapset, 0, 0);
-        for (int i = 0; i < CELT_OVERLAP / 2; i++)
+        ROLLED for (int i = 0; i < CELT_OVERLAP / 2; i++)
             dm[CELT_DEC_BUF - N + i] = wadd(c_mul16_32_q15(T_celt_window[i], w->etmp[CELT_OVERLAP - 1 - i]),
                                             c_mul16_32_q15(T_celt_window[CELT_OVERLAP - i - 1], w->etmp[i]));
     }
@@ -1986,7 +1986,7 @@ DNI void celt_decode_lost(Lanes L, CeltDec *st, int N, int LM, CeltScratch *w)
     const int C = st->channels;
     const int16_t *eB = T_celt_eBands;
     int32_t *out_syn[2];
-    for (int c = 0; c < C; c++) out_syn[c] = st->decode_mem[c] + CELT_DEC_BUF - N;
+    ROLLED for (int c = 0; c < C; c++) out_syn[c] = st->decode_mem[c] + CELT_DEC_BUF - N;
     int loss_duration = st->loss_duration;
     int start = st->start;
     int noise_based = loss_duration >= 40 || start != 0 || st->skip_plc;
@@ -1994,21 +1994,21 @@ DNI void celt_decode_lost(Lanes L, CeltDec *st, int N, int LM, CeltScratch *w)
         int end = st->end;
         int effEnd = imax(start, imin(end, T_CELT_EFFEBANDS));
         int16_t *X = w->X;
-        for (int c = 0; c < C; c++) lshift_copy(L, st->decode_mem[c], CELT_DEC_BUF - N + CELT_OVERLAP, N);
+        ROLLED for (int c = 0; c < C; c++) lshift_copy(L, st->decode_mem[c], CELT_DEC_BUF - N + CELT_OVERLAP, N);
         if (st->prefilter_and_fold) prefilter_and_fold(st, N, w);
         int16_t decay = loss_duration == 0 ? 1536 : 512;   // QCONST16(1.5f / .5f, DB_SHIFT)
-        for (int c = 0; c < C; c++)
-            for (int i = start; i < end; i++) {
+        ROLLED for (int c = 0; c < C; c++)
+            ROLLED for (int i = start; i < end; i++) {
                 int32_t a = st->backgroundLogE[c * CELT_NB + i];
                 int32_t b = st->oldBandE[c * CELT_NB + i] - decay;
                 st->oldBandE[c * CELT_NB + i] = (int16_t)(a > b ? a : b);
             }
         uint32_t seed = st->rng;
-        for (int c = 0; c < C; c++) {
-            for (int i = start; i < effEnd; i++) {
+        ROLLED for (int c = 0; c < C; c++) {
+            ROLLED for (int i = start; i < effEnd; i++) {
                 int boffs = N * c + (eB[i] << LM);
                 int blen = (eB[i + 1] - eB[i]) << LM;
-                for (int j = 0; j < blen; j++) {
+                ROLLED for (int j = 0; j < blen; j++) {
                     seed = c_lcg_rand(seed);
                     X[boffs + j] = (int16_t)((int32_t)seed >> 20);
                 }
@@ -2037,37 +2037,37 @@ DNI void celt_decode_lost(Lanes L, CeltDec *st, int N, int LM, CeltScratch *w)
         int exc_length = imin(2 * pitch_index, CELT_MAX_PERIOD);
         int16_t *exc = w->exc + CELT_LPC_ORDER;
         const int16_t *window = T_celt_window;
-        for (int c = 0; c < C; c++) {
+        ROLLED for (int c = 0; c < C; c++) {
             int32_t *buf = st->decode_mem[c];
             int16_t *lpc = st->lpc[c];
             int32_t S1 = 0;
-            for (int i = 0; i < CELT_MAX_PERIOD + CELT_LPC_ORDER; i++)
+            ROLLED for (int i = 0; i < CELT_MAX_PERIOD + CELT_LPC_ORDER; i++)
                 exc[i - CELT_LPC_ORDER] = c_sround16(buf[CELT_DEC_BUF - CELT_MAX_PERIOD - CELT_LPC_ORDER + i], 12);
             if (loss_duration == 0) {
                 int32_t ac[CELT_LPC_ORDER + 1];
                 celt_autocorr(exc, ac, window, CELT_OVERLAP, CELT_LPC_ORDER, CELT_MAX_PERIOD, w->ac_xx);
                 ac[0] = wadd(ac[0], ac[0] >> 13);
-                for (int i = 1; i <= CELT_LPC_ORDER; i++) ac[i] = wsub(ac[i], c_mul16_32_q15(2 * i * i, ac[i]));
+                ROLLED for (int i = 1; i <= CELT_LPC_ORDER; i++) ac[i] = wsub(ac[i], c_mul16_32_q15(2 * i * i, ac[i]));
                 celt_lpc(lpc, ac, CELT_LPC_ORDER);
-                while (1) {
+                ROLLED while (1) {
                     int16_t tmp = 32767;
                     int32_t sum = 4096;   // QCONST16(1., SIG_SHIFT)
-                    for (int i = 0; i < CELT_LPC_ORDER; i++) sum += lpc[i] < 0 ? -lpc[i] : lpc[i];
+                    ROLLED for (int i = 0; i < CELT_LPC_ORDER; i++) sum += lpc[i] < 0 ? -lpc[i] : lpc[i];
                     if (sum < 65535) break;
-                    for (int i = 0; i < CELT_LPC_ORDER; i++) {
+                    ROLLED for (int i = 0; i < CELT_LPC_ORDER; i++) {
                         tmp = (int16_t)c_mul16_q15(32440, tmp);   // QCONST16(.99f, 15)
                         lpc[i] = (int16_t)c_mul16_q15(lpc[i], tmp);
                     }
                 }
             }
             celt_fir(exc + CELT_MAX_PERIOD - exc_length, lpc, w->fir_tmp, exc_length, CELT_LPC_ORDER);
-            for (int i = 0; i < exc_length; i++) exc[CELT_MAX_PERIOD - exc_length + i] = w->fir_tmp[i];
+            ROLLED for (int i = 0; i < exc_length; i++) exc[CELT_MAX_PERIOD - exc_length + i] = w->fir_tmp[i];
             int16_t decay;
             {
                 int32_t E1 = 1, E2 = 1;
                 int shift = imax(0, 2 * c_zlog2(c_maxabs16(&exc[CELT_MAX_PERIOD - exc_length], exc_length)) - 20);
                 int decay_length = exc_length >> 1;
-                for (int i = 0; i < decay_length; i++) {
+                ROLLED for (int i = 0; i < decay_length; i++) {
                     int16_t e = exc[CELT_MAX_PERIOD - decay_length + i];
                     E1 = wadd(E1, c_mul16(e, e) >> shift);
                     e = exc[CELT_MAX_PERIOD - 2 * decay_length + i];
@@ -2076,11 +2076,11 @@ DNI void celt_decode_lost(Lanes L, CeltDec *st, int N, int LM, CeltScratch *w)
                 E1 = min32(E1, E2);
                 decay = (int16_t)c_sqrt(c_frac_div32(E1 >> 1, E2));
             }
-            for (int i = 0; i < CELT_DEC_BUF - N; i++) buf[i] = buf[i + N];
+            ROLLED for (int i = 0; i < CELT_DEC_BUF - N; i++) buf[i] = buf[i + N];
             int extrapolation_offset = CELT_MAX_PERIOD - pitch_index;
             int extrapolation_len = N + CELT_OVERLAP;
             int16_t attenuation = (int16_t)c_mul16_q15(fade, decay);
-            for (int i = 0, j = 0; i < extrapolation_len; i++, j++) {
+            ROLLED for (int i = 0, j = 0; i < extrapolation_len; i++, j++) {
                 if (j >= pitch_index) {
                     j -= pitch_index;
                     attenuation = (int16_t)c_mul16_q15(attenuation, decay);
@@ -2092,27 +2092,27 @@ DNI void celt_decode_lost(Lanes L, CeltDec *st, int N, int LM, CeltScratch *w)
             }
             {
                 int16_t lpc_mem[CELT_LPC_ORDER];
-                for (int i = 0; i < CELT_LPC_ORDER; i++) lpc_mem[i] = c_sround16(buf[CELT_DEC_BUF - N - 1 - i], 12);
+                ROLLED for (int i = 0; i < CELT_LPC_ORDER; i++) lpc_mem[i] = c_sround16(buf[CELT_DEC_BUF - N - 1 - i], 12);
                 celt_iir(buf + CELT_DEC_BUF - N, lpc, buf + CELT_DEC_BUF - N, extrapolation_len, CELT_LPC_ORDER,
                          lpc_mem, w->iir_y);
-                for (int i = 0; i < extrapolation_len; i++)
+                ROLLED for (int i = 0; i < extrapolation_len; i++)
                     buf[CELT_DEC_BUF - N + i] = c_sat(buf[CELT_DEC_BUF - N + i], CELT_SIG_SAT);
             }
             {
                 int32_t S2 = 0;
-                for (int i = 0; i < extrapolation_len; i++) {
+                ROLLED for (int i = 0; i < extrapolation_len; i++) {
                     int16_t tmp = c_sround16(buf[CELT_DEC_BUF - N + i], 12);
                     S2 = wadd(S2, c_mul16(tmp, tmp) >> 10);
                 }
                 if (!(S1 > (S2 >> 2))) {
-                    for (int i = 0; i < extrapolation_len; i++) buf[CELT_DEC_BUF - N + i] = 0;
+                    ROLLED for (int i = 0; i < extrapolation_len; i++) buf[CELT_DEC_BUF - N + i] = 0;
                 } else if (S1 < S2) {
                     int16_t ratio = (int16_t)c_sqrt(c_frac_div32((S1 >> 1) + 1, S2 + 1));
-                    for (int i = 0; i < CELT_OVERLAP; i++) {
+                    ROLLED for (int i = 0; i < CELT_OVERLAP; i++) {
                         int16_t tmp_g = (int16_t)(32767 - c_mul16_q15(window[i], (int16_t)(32767 - ratio)));
                         buf[CELT_DEC_BUF - N + i] = c_mul16_32_q15(tmp_g, buf[CELT_DEC_BUF - N + i]);
                     }
-                    for (int i = CELT_OVERLAP; i < extrapolation_len; i++)
+                    ROLLED for (int i = CELT_OVERLAP; i < extrapolation_len; i++)
                         buf[CELT_DEC_BUF - N + i] = c_mul16_32_q15(ratio, buf[CELT_DEC_BUF - N + i]);
                 }
             }
@@ -2132,12 +2132,12 @@ DNI void celt_decode_lost(Lanes L, CeltDec *st, int N, int LM, CeltScratch *w)
 DNI void energy_after_loss(CeltDec *st, int start, int end, int LM)
 {
     int16_t *oldBandE = st->oldBandE, *oldLogE = st->oldLogE, *oldLogE2 = st->oldLogE2;
-    for (int c = 0; c < 2; c++) {
+    ROLLED for (int c = 0; c < 2; c++) {
         int16_t safety = 0;
         int missing = imin(10, st->loss_duration >> LM);
         if (LM == 0) safety = 1536;
         else if (LM == 1) safety = 512;
-        for (int i = start; i < end; i++) {
+        ROLLED for (int i = start; i < end; i++) {
             int16_t *e0 = &oldBandE[c * CELT_NB + i];
             int16_t e1 = oldLogE[c * CELT_NB + i], e2 = oldLogE2[c * CELT_NB + i];
             if (*e0 < (e1 > e2 ? e1 : e2)) {
@@ -2164,14 +2164,14 @@ DNI int celt_decode(Lanes L, CeltDec *st, const uint8_t *data, int len, int16_t 
     int C = st->stream_channels;
     int start = st->start, end = st->end;
     int LM;
-    for (LM = 0; LM <= T_CELT_MAXLM; LM++)
+    ROLLED for (LM = 0; LM <= T_CELT_MAXLM; LM++)
         if (T_CELT_SHORTMDCT << LM == frame_size) break;
     if (LM > T_CELT_MAXLM) return -1;   // OPUS_BAD_ARG
     int M = 1 << LM;
     if (len < 0 || len > 1275 || pcm == 0) return -1;
     int N = M * T_CELT_SHORTMDCT;
     int32_t *out_syn[2];
-    for (int c = 0; c < CC; c++) out_syn[c] = st->decode_mem[c] + CELT_DEC_BUF - N;
+    ROLLED for (int c = 0; c < CC; c++) out_syn[c] = st->decode_mem[c] + CELT_DEC_BUF - N;
     if (CC == 1) out_syn[1] = out_syn[0];
     int effEnd = end;
     if (effEnd > T_CELT_EFFEBANDS) effEnd = T_CELT_EFFEBANDS;
@@ -2245,11 +2245,11 @@ DNI int celt_decode(Lanes L, CeltDec *st, const uint8_t *data, int len, int16_t 
         int dynalloc_logp = 6;
         total_bits <<= 3;
         tell = (int32_t)rd_tell_frac(dec);
-        for (int i = start; i < end; i++) {
+        ROLLED for (int i = start; i < end; i++) {
             int width = C * (eB[i + 1] - eB[i]) << LM;
             int quanta = imin(width << 3, imax(6 << 3, width));
             int dll = dynalloc_logp, boost = 0;
-            while (tell + (dll << 3) < total_bits && boost < cap[i]) {
+            ROLLED while (tell + (dll << 3) < total_bits && boost < cap[i]) {
                 int flag = rd_bit_logp(dec, dll);
                 tell = (int32_t)rd_tell_frac(dec);
                 if (!flag) break;
@@ -2283,7 +2283,7 @@ DNI int celt_decode(Lanes L, CeltDec *st, const uint8_t *data, int len, int16_t 
         hv[H_BALANCE] = balance;
         hv[H_CODED] = codedBands;
     });
-    for (int k = 0; k < H_N; k++) hv[k] = lbcast(L, hv[k]);
+    ROLLED for (int k = 0; k < H_N; k++) hv[k] = lbcast(L, hv[k]);
     const int silence = hv[H_SILENCE];
     const int16_t postfilter_gain = (int16_t)hv[H_PF_GAIN];
     const int postfilter_pitch = hv[H_PF_PITCH], postfilter_tapset = hv[H_PF_TAPSET];
@@ -2293,7 +2293,7 @@ DNI int celt_decode(Lanes L, CeltDec *st, const uint8_t *data, int len, int16_t 
     const int32_t balance = hv[H_BALANCE];
     const int codedBands = hv[H_CODED];
     PHASE_BEGIN(t_sh);
-    for (int c = 0; c < CC; c++) lshift_copy(L, st->decode_mem[c], CELT_DEC_BUF - N + CELT_OVERLAP, N);
+    ROLLED for (int c = 0; c < CC; c++) lshift_copy(L, st->decode_mem[c], CELT_DEC_BUF - N + CELT_OVERLAP, N);
     PHASE_END(PH_CELT_SHIFT, t_sh, L.id);
     int16_t *X = w->X;
     // The band shapes: the PVQ split recursion updates its stack, the band
@@ -2317,7 +2317,7 @@ DNI int celt_decode(Lanes L, CeltDec *st, const uint8_t *data, int len, int16_t 
             anti_collapse(lone(L), X, w->collapse_masks, LM, C, N, start, end, oldBandE, oldLogE, oldLogE2, pulses,
                           st->rng);
         if (silence)
-            for (int i = 0; i < C * CELT_NB; i++) oldBandE[i] = -28672;   // -QCONST16(28.f, DB_SHIFT)
+            ROLLED for (int i = 0; i < C * CELT_NB; i++) oldBandE[i] = -28672;   // -QCONST16(28.f, DB_SHIFT)
         if (st->prefilter_and_fold) prefilter_and_fold(st, N, w);
     });
     PHASE_BEGIN(t_sy);
@@ -2329,7 +2329,7 @@ DNI int celt_decode(Lanes L, CeltDec *st, const uint8_t *data, int len, int16_t 
     const int pf_period = imax(st->postfilter_period, 15), pf_period_old = imax(st->postfilter_period_old, 15);
     const int16_t pf_gain = (int16_t)st->postfilter_gain, pf_gain_old = (int16_t)st->postfilter_gain_old;
     const int pf_tapset = st->postfilter_tapset, pf_tapset_old = st->postfilter_tapset_old;
-    for (int c = 0; c < CC; c++) {
+    ROLLED for (int c = 0; c < CC; c++) {
         comb_filter_lanes(L, out_syn[c], out_syn[c], pf_period_old, pf_period, T_CELT_SHORTMDCT, pf_gain_old,
                           pf_gain, pf_tapset_old, pf_tapset, T_celt_window, CELT_OVERLAP);
         if (LM != 0)

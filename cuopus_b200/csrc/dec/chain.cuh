@@ -72,7 +72,7 @@ DFN bool stage_wait(PacketStage &S, int b, int polls = 1 << 20, unsigned long lo
 {
     uint32_t addr = smem_u32(&S.bar[b]), par = (S.parity >> b) & 1u;
     const unsigned long long t0 = limit_ns ? stage_clock_ns() : 0;
-    for (int it = 0;; it++) {
+    ROLLED for (int it = 0;; it++) {
         uint32_t done;
         asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
                      " selp.u32 %0, 1, 0, p;\n}\n"
@@ -142,7 +142,7 @@ DFN bool stage_ready(const Lanes &L, PacketStage &S, int b)
 DFN void stage_drain(const Lanes &L, PacketStage &S)
 {
     bool ok = true;
-    for (int b = 0; b < 2; b++)
+    ROLLED for (int b = 0; b < 2; b++)
         if (S.pending & (1u << b)) ok = stage_wait(S, b, 1 << 20, 1000000000ull) && ok;
     if (!__all_sync(L.mask, ok)) S.ok = 0;
 }
@@ -214,7 +214,7 @@ DNI void decode_chain(Lanes L, ChainSlot *slot, const uint8_t *data, const uint6
 #else
     (void)stage;
 #endif
-    for (uint32_t k = 0; k < npkts; k++) {
+    ROLLED for (uint32_t k = 0; k < npkts; k++) {
         uint64_t p = (uint64_t)first + k;
         const uint8_t *pk = data + off[p];
         int32_t n = (int32_t)len[p];

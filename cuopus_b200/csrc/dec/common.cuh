@@ -22,7 +22,13 @@
 #include <stdint.h>
 #include <string.h>
 
+// ROLLED before a loop keeps it a loop.  The decoder is one large body of code
+// whose warps each run a different part of it, so its size is paid for in
+// instruction fetch: every loop that does not ask for unrolling by name is
+// kept rolled, and the kernel is then compiled at full optimisation (385 KB of
+// kernel code; 764 KB with the compiler's own unrolling).
 #ifdef __CUDACC__
+#define ROLLED _Pragma("unroll 1")
 #define DFN static __device__ __forceinline__
 #define MFN __device__ __forceinline__
 #define DNI static __device__ __noinline__
@@ -30,6 +36,7 @@
 #define TABC(type, decl) static __constant__ type decl
 #define TABG(type, decl) static __device__ const type decl
 #else
+#define ROLLED
 #define DFN static inline
 #define MFN inline
 #define DNI static
@@ -131,7 +138,7 @@ DFN int32_t lbcast(const Lanes &L, int32_t v)
 #ifdef CUO_LFOR_REVERSE
 #define LFOR(L, i, start, end) for (int i = (end) - 1 - (L).id; i >= (start); i -= (L).n)
 #else
-#define LFOR(L, i, start, end) for (int i = (start) + (L).id; i < (end); i += (L).n)
+#define LFOR(L, i, start, end) ROLLED for (int i = (start) + (L).id; i < (end); i += (L).n)
 #endif
 
 // Stage timers of the diagnostic build (CUO_PHASE_TIMERS, libcuopus_phases.so):
@@ -167,7 +174,7 @@ __device__ void cuo_phase_add(int stage, long long cycles);
 DFN int32_t lsum(const Lanes &L, int32_t v)
 {
 #ifdef __CUDA_ARCH__
-    for (int off = L.n >> 1; off > 0; off >>= 1) v = (int32_t)((uint32_t)v + (uint32_t)__shfl_xor_sync(L.mask, v, off));
+    ROLLED for (int off = L.n >> 1; off > 0; off >>= 1) v = (int32_t)((uint32_t)v + (uint32_t)__shfl_xor_sync(L.mask, v, off));
 #elif defined(CUO_LANE_SIM)
     if (L.sim) v = lanesim_sum(L.sim, L.id, v);
 #else
@@ -184,7 +191,7 @@ DFN int32_t lsum(const Lanes &L, int32_t v)
 DFN void lscan_affine(const Lanes &L, uint32_t &a, uint32_t &b)
 {
 #ifdef __CUDA_ARCH__
-    for (int off = 1; off < L.n; off <<= 1) {
+    ROLLED for (int off = 1; off < L.n; off <<= 1) {
         uint32_t pa = __shfl_up_sync(L.mask, a, off, L.n), pb = __shfl_up_sync(L.mask, b, off, L.n);
         if (L.id >= off) {   // this lane's span after the earlier one
             b = a * pb + b;
@@ -221,7 +228,7 @@ DFN void lscan_affine(const Lanes &L, uint32_t &a, uint32_t &b)
 template <class T> DFN void lshift_copy(const Lanes &L, T *buf, int n, int shift)
 {
     lsync(L);
-    for (int b = 0; b < n; b += shift) {
+    ROLLED for (int b = 0; b < n; b += shift) {
         int e = b + shift < n ? b + shift : n;
         LFOR(L, i, b, e) buf[i] = buf[i + shift];
         lsync(L);
@@ -257,6 +264,18 @@ DFN int32_t s_smulwt(int32_t a, int32_t b) { return (int32_t)(((int64_t)a * (b >
 DFN int32_t s_smulbb(int32_t a, int32_t b) { return (int32_t)(int16_t)a * (int32_t)(int16_t)b; }
 DFN int32_t s_smlabb(int32_t a, int32_t b, int32_t c) { return wadd(a, s_smulbb(b, c)); }
 DFN int32_t s_smultt(int32_t a, int32_t b) { return (a >> 16) * (b >> 16); }
+// a + ((b * c) >> 16) wrapping, with the 16-bit factor given as c16 = c << 16:
+// the high word of b * c16 is that product exactly, so a tap is one mad.hi
+DFN int32_t s_smlawh(int32_t a, int32_t b, int32_t c16)
+{
+#ifdef __CUDA_ARCH__
+    int32_t d;
+    asm("mad.hi.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(b), "r"(c16), "r"(a));
+    return d;
+#else
+    return wadd(a, (int32_t)(((int64_t)b * c16) >> 32));
+#endif
+}
 DFN int32_t s_smulww(int32_t a, int32_t b) { return (int32_t)(((int64_t)a * b) >> 16); }
 DFN int32_t s_smlaww(int32_t a, int32_t b, int32_t c) { return wadd(a, s_smulww(b, c)); }
 DFN int32_t s_smmul(int32_t a, int32_t b) { return (int32_t)(((int64_t)a * b) >> 32); }
@@ -408,13 +427,13 @@ DFN int16_t c_sig2word16(int32_t x)
 DFN int32_t c_maxabs16(const int16_t *x, int len)
 {
     int16_t mx = 0, mn = 0;
-    for (int i = 0; i < len; i++) { mx = x[i] > mx ? x[i] : mx; mn = x[i] < mn ? x[i] : mn; }
+    ROLLED for (int i = 0; i < len; i++) { mx = x[i] > mx ? x[i] : mx; mn = x[i] < mn ? x[i] : mn; }
     return max32(mx, -(int32_t)mn);
 }
 DFN int32_t c_maxabs32(const int32_t *x, int len)
 {
     int32_t mx = 0, mn = 0;
-    for (int i = 0; i < len; i++) { mx = max32(mx, x[i]); mn = min32(mn, x[i]); }
+    ROLLED for (int i = 0; i < len; i++) { mx = max32(mx, x[i]); mn = min32(mn, x[i]); }
     return max32(mx, -mn);
 }
 
@@ -424,7 +443,7 @@ DFN unsigned c_isqrt32(uint32_t val)
     unsigned g = 0;
     int bshift = (ilog(val) - 1) >> 1;
     unsigned b = 1u << bshift;
-    do {
+    ROLLED do {
         uint32_t t = (((uint32_t)g << 1) + b) << bshift;
         if (t <= val) { g += b; val -= t; }
         b >>= 1;

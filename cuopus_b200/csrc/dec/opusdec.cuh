@@ -132,7 +132,7 @@ DNI int packet_parse(const uint8_t *data, int32_t len, int16_t *size, int *paylo
         len--;
         if (ch & 0x40) {
             int p;
-            do {
+            ROLLED do {
                 if (len <= 0) return OPUS_INVALID_PACKET;
                 p = *data++;
                 len--;
@@ -144,7 +144,7 @@ DNI int packet_parse(const uint8_t *data, int32_t len, int16_t *size, int *paylo
         int cbr = !(ch & 0x80);
         if (!cbr) {
             last_size = len;
-            for (int i = 0; i < count - 1; i++) {
+            ROLLED for (int i = 0; i < count - 1; i++) {
                 bytes = parse_size(data, len, size + i);
                 len -= bytes;
                 if (size[i] < 0 || size[i] > len) return OPUS_INVALID_PACKET;
@@ -155,7 +155,7 @@ DNI int packet_parse(const uint8_t *data, int32_t len, int16_t *size, int *paylo
         } else {
             last_size = len / count;
             if (last_size * count != len) return OPUS_INVALID_PACKET;
-            for (int i = 0; i < count - 1; i++) size[i] = (int16_t)last_size;
+            ROLLED for (int i = 0; i < count - 1; i++) size[i] = (int16_t)last_size;
         }
         break;
     }
@@ -225,7 +225,7 @@ DNI int opus_frame(Lanes L, OpusDec *st, const uint8_t *data, int32_t len, int16
         }
         if (audiosize > F20) {
             if constexpr (D == 0) {
-                do {
+                ROLLED do {
                     int ret = opus_frame<1>(L, st, 0, 0, pcm, imin(audiosize, F20), w, 0);
                     if (ret < 0) return ret;
                     pcm += ret * C;
@@ -276,7 +276,7 @@ DNI int opus_frame(Lanes L, OpusDec *st, const uint8_t *data, int32_t len, int16
         });
         int lost_flag = data == 0 ? 1 : (fec ? 2 : 0);
         int decoded_samples = 0;
-        do {
+        ROLLED do {
             int first_frame = decoded_samples == 0;
             int32_t silk_frame_size = 0;
             silk_ret = silk_decode(L, &st->silk, &st->DecControl, lost_flag, first_frame, &dec, pcm_ptr,
@@ -423,7 +423,7 @@ template <class Emit>
 DNI int conceal_samples(Lanes L, OpusDec *st, int n, int16_t *frame_buf, OpusScratch *w, Emit &emit)
 {
     int pcm_count = 0;
-    do {
+    ROLLED do {
         int ret = opus_frame<0>(L, st, 0, 0, frame_buf, n - pcm_count, w, 0);
         if (ret < 0) return ret;
         emit(frame_buf, ret);
@@ -508,7 +508,7 @@ DFN int opus_decode_packet(Lanes L, OpusDec *st, const uint8_t *data, int32_t le
         st->stream_channels = packet_stream_channels;
     });
     int nb_samples = 0;
-    for (int i = 0; i < count; i++) {
+    ROLLED for (int i = 0; i < count; i++) {
         int ret = opus_frame<0>(L, st, data, size[i], frame_buf, frame_size - nb_samples, w, 0);
         if (ret < 0) return ret;
         emit(frame_buf, ret);

@@ -70,7 +70,7 @@ DFN int rd_read_byte_end(RangeDec *d)
 
 DFN void rd_normalize(RangeDec *d)
 {
-    while (d->rng <= (1u << 23)) {
+    ROLLED while (d->rng <= (1u << 23)) {
         d->nbits_total += 8;
         d->rng <<= 8;
         int sym = d->rem;
@@ -134,7 +134,7 @@ DNI int rd_icdf(RangeDec *d, const uint8_t *icdf, unsigned ftb)
 {
     uint32_t s = d->rng, v = d->val, r = s >> ftb, t;
     int ret = -1;
-    do {
+    ROLLED do {
         t = s;
         s = r * icdf[++ret];
     } while (v < s);
@@ -149,7 +149,7 @@ DNI uint32_t rd_bits(RangeDec *d, unsigned bits)
     uint32_t window = d->end_window;
     int available = d->nend_bits;
     if ((unsigned)available < bits) {
-        do {
+        ROLLED do {
             window |= (uint32_t)rd_read_byte_end(d) << available;
             available += 8;
         } while (available <= 32 - 8);
@@ -211,7 +211,7 @@ DNI int rd_laplace(RangeDec *d, unsigned fs, int decay)
         val++;
         fl = fs;
         fs = ((32768u - 32u - fs) * (int32_t)(16384 - decay) >> 15) + 1;
-        while (fs > 1 && fm >= fl + 2 * fs) {
+        ROLLED while (fs > 1 && fm >= fl + 2 * fs) {
             fs *= 2;
             fl += fs;
             fs = ((fs - 2) * (int32_t)decay) >> 15;

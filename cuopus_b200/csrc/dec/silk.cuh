@@ -202,7 +202,7 @@ DNI void silk_resampler_init48(SilkResampler *S, int32_t Fs_Hz_in)
     S->batchSize = (int16_t)(S->Fs_in_kHz * 10);
     // IIR_FIR with 2x up-sampling: invRatio = ((Fs_in << 15) / Fs_out) << 2, rounded up
     int32_t inv = shl32((int32_t)(((int64_t)Fs_Hz_in << 15) / 48000), 2);
-    while (s_smulww(inv, 48000) < shl32(Fs_Hz_in, 1)) inv++;
+    ROLLED while (s_smulww(inv, 48000) < shl32(Fs_Hz_in, 1)) inv++;
     S->invRatio_Q16 = inv;
 }
 
@@ -213,10 +213,10 @@ DNI void silk_resampler_init48(SilkResampler *S, int32_t Fs_Hz_in)
 DNI void silk_up2_hq(Lanes L, int32_t *S, int16_t *out, const int16_t *in, int32_t len)
 {
     const int step = L.n > 1 ? 2 : 1;
-    for (int ph = L.n > 1 ? L.id : 0; ph < 2; ph += step) {
+    ROLLED for (int ph = L.n > 1 ? L.id : 0; ph < 2; ph += step) {
         const int16_t *a = ph ? T_silk_resampler_up2_hq_1 : T_silk_resampler_up2_hq_0;
         int32_t s0 = S[3 * ph], s1 = S[3 * ph + 1], s2 = S[3 * ph + 2];
-        for (int32_t k = 0; k < len; k++) {
+        ROLLED for (int32_t k = 0; k < len; k++) {
             int32_t in32 = shl32((int32_t)in[k], 10), Y, X, o1, o2;
             Y = wsub(in32, s0); X = s_smulwb(Y, a[0]); o1 = wadd(s0, X); s0 = wadd(in32, X);
             Y = wsub(o1, s1); X = s_smulwb(Y, a[1]); o2 = wadd(s1, X); s1 = wadd(o1, X);
@@ -236,7 +236,7 @@ DNI int16_t *silk_iir_fir(Lanes L, SilkResampler *S, int16_t *out, const int16_t
     lsync(L);
     const int32_t inc = S->invRatio_Q16;
     int32_t nIn = 0;
-    while (1) {
+    ROLLED while (1) {
         nIn = inLen < S->batchSize ? inLen : S->batchSize;
         silk_up2_hq(L, S->sIIR, &buf[8], in, nIn);
         lsync(L);
@@ -264,7 +264,7 @@ DNI int16_t *silk_iir_fir(Lanes L, SilkResampler *S, int16_t *out, const int16_t
         inLen -= nIn;
         if (inLen > 0) {
             int16_t keep[8];
-            for (int i = 0; i < 8; i++) keep[i] = buf[(nIn << 1) + i];
+            ROLLED for (int i = 0; i < 8; i++) keep[i] = buf[(nIn << 1) + i];
             lsync(L);
             LFOR(L, i, 0, 8) buf[i] = keep[i];
             lsync(L);
@@ -272,7 +272,7 @@ DNI int16_t *silk_iir_fir(Lanes L, SilkResampler *S, int16_t *out, const int16_t
             break;
         }
     }
-    for (int i = 0; i < 8; i++) S->sFIR[i] = buf[(nIn << 1) + i];
+    ROLLED for (int i = 0; i < 8; i++) S->sFIR[i] = buf[(nIn << 1) + i];
     lsync(L);
     return out;
 }
@@ -295,7 +295,7 @@ DNI void silk_resample(Lanes L, SilkResampler *S, int16_t *out, const int16_t *i
 DFN void silk_bwexpander(int16_t *ar, int d, int32_t chirp_Q16)
 {
     int32_t cm1 = chirp_Q16 - 65536;
-    for (int i = 0; i < d - 1; i++) {
+    ROLLED for (int i = 0; i < d - 1; i++) {
         ar[i] = (int16_t)s_rshift_round(wmul(chirp_Q16, ar[i]), 16);
         chirp_Q16 += s_rshift_round(wmul(chirp_Q16, cm1), 16);
     }
@@ -305,7 +305,7 @@ DFN void silk_bwexpander(int16_t *ar, int d, int32_t chirp_Q16)
 DFN void silk_bwexpander_32(int32_t *ar, int d, int32_t chirp_Q16)
 {
     int32_t cm1 = chirp_Q16 - 65536;
-    for (int i = 0; i < d - 1; i++) {
+    ROLLED for (int i = 0; i < d - 1; i++) {
         ar[i] = s_smulww(chirp_Q16, ar[i]);
         chirp_Q16 += s_rshift_round(wmul(chirp_Q16, cm1), 16);
     }
@@ -318,14 +318,14 @@ DNI int32_t silk_lpc_inv_pred_gain(const int16_t *A_Q12, int order, int32_t *A)
     const int32_t A_LIMIT = 16773022;   // SILK_FIX_CONST(0.99975, 24)
     const int32_t MIN_INVG = 107374;    // SILK_FIX_CONST(1 / MAX_PREDICTION_POWER_GAIN, 30)
     int32_t DC = 0;
-    for (int k = 0; k < order; k++) {
+    ROLLED for (int k = 0; k < order; k++) {
         DC += A_Q12[k];
         A[k] = shl32((int32_t)A_Q12[k], 12);
     }
     if (DC >= 4096) return 0;
     int32_t invGain_Q30 = 1 << 30;
     int k;
-    for (k = order - 1; k > 0; k--) {
+    ROLLED for (k = order - 1; k > 0; k--) {
         if (A[k] > A_LIMIT || A[k] < -A_LIMIT) return 0;
         int32_t rc_Q31 = -shl32(A[k], 7);
         int32_t rc_mult1_Q30 = (1 << 30) - s_smmul(rc_Q31, rc_Q31);
@@ -333,7 +333,7 @@ DNI int32_t silk_lpc_inv_pred_gain(const int16_t *A_Q12, int order, int32_t *A)
         if (invGain_Q30 < MIN_INVG) return 0;
         int mult2Q = 32 - s_clz32(s_abs(rc_mult1_Q30));
         int32_t rc_mult2 = s_inverse32_varq(rc_mult1_Q30, mult2Q + 30);
-        for (int n = 0; n < (k + 1) >> 1; n++) {
+        ROLLED for (int n = 0; n < (k + 1) >> 1; n++) {
             int32_t t1 = A[n], t2 = A[k - n - 1];
             int64_t v = s_rshift_round64(s_smull(s_sub_sat32(t1,
                 (int32_t)s_rshift_round64(s_smull(t2, rc_Q31), 31)), rc_mult2), mult2Q);
@@ -357,9 +357,9 @@ DNI int32_t silk_lpc_inv_pred_gain(const int16_t *A_Q12, int order, int32_t *A)
 DNI void silk_lpc_fit(int16_t *a_QOUT, int32_t *a_QIN, int QOUT, int QIN, int d)
 {
     int i, k, idx = 0;
-    for (i = 0; i < 10; i++) {
+    ROLLED for (i = 0; i < 10; i++) {
         int32_t maxabs = 0;
-        for (k = 0; k < d; k++) {
+        ROLLED for (k = 0; k < d; k++) {
             int32_t absval = s_abs(a_QIN[k]);
             if (absval > maxabs) { maxabs = absval; idx = k; }
         }
@@ -373,12 +373,12 @@ DNI void silk_lpc_fit(int16_t *a_QOUT, int32_t *a_QIN, int QOUT, int QIN, int d)
         }
     }
     if (i == 10) {
-        for (k = 0; k < d; k++) {
+        ROLLED for (k = 0; k < d; k++) {
             a_QOUT[k] = (int16_t)s_sat16(s_rshift_round(a_QIN[k], QIN - QOUT));
             a_QIN[k] = shl32((int32_t)a_QOUT[k], QIN - QOUT);
         }
     } else {
-        for (k = 0; k < d; k++) a_QOUT[k] = (int16_t)s_rshift_round(a_QIN[k], QIN - QOUT);
+        ROLLED for (k = 0; k < d; k++) a_QOUT[k] = (int16_t)s_rshift_round(a_QIN[k], QIN - QOUT);
     }
 }
 
@@ -387,10 +387,10 @@ DFN void silk_nlsf2a_poly(int32_t *out, const int32_t *cLSF, int dd)
 {
     out[0] = 1 << 16;
     out[1] = -cLSF[0];
-    for (int k = 1; k < dd; k++) {
+    ROLLED for (int k = 1; k < dd; k++) {
         int32_t ftmp = cLSF[2 * k];
         out[k + 1] = wsub(shl32(out[k - 1], 1), (int32_t)s_rshift_round64(s_smull(ftmp, out[k]), 16));
-        for (int n = k; n > 1; n--)
+        ROLLED for (int n = k; n > 1; n--)
             out[n] = wadd(out[n], wsub(out[n - 2], (int32_t)s_rshift_round64(s_smull(ftmp, out[n - 1]), 16)));
         out[1] = wsub(out[1], ftmp);
     }
@@ -404,7 +404,7 @@ DNI void silk_nlsf2a(int16_t *a_Q12, const int16_t *NLSF, int d, SilkWork *sw)
 {
     const uint8_t *ordering = d == 16 ? T_nlsf2a_ord16 : T_nlsf2a_ord10;
     int32_t *cos_LSF_QA = sw->cos_LSF_QA, *P = sw->P, *Q = sw->Q, *a32_QA1 = sw->a32_QA1;
-    for (int k = 0; k < d; k++) {
+    ROLLED for (int k = 0; k < d; k++) {
         int32_t f_int = NLSF[k] >> 8;
         int32_t f_frac = NLSF[k] - shl32(f_int, 8);
         int32_t cos_val = T_silk_LSFCosTab_FIX_Q12[f_int];
@@ -414,16 +414,16 @@ DNI void silk_nlsf2a(int16_t *a_Q12, const int16_t *NLSF, int d, SilkWork *sw)
     int dd = d >> 1;
     silk_nlsf2a_poly(P, &cos_LSF_QA[0], dd);
     silk_nlsf2a_poly(Q, &cos_LSF_QA[1], dd);
-    for (int k = 0; k < dd; k++) {
+    ROLLED for (int k = 0; k < dd; k++) {
         int32_t Ptmp = wadd(P[k + 1], P[k]);
         int32_t Qtmp = wsub(Q[k + 1], Q[k]);
         a32_QA1[k] = wsub(-Qtmp, Ptmp);
         a32_QA1[d - k - 1] = wsub(Qtmp, Ptmp);
     }
     silk_lpc_fit(a_Q12, a32_QA1, 12, 17, d);
-    for (int i = 0; silk_lpc_inv_pred_gain(a_Q12, d, sw->A) == 0 && i < 16; i++) {
+    ROLLED for (int i = 0; silk_lpc_inv_pred_gain(a_Q12, d, sw->A) == 0 && i < 16; i++) {
         silk_bwexpander_32(a32_QA1, d, 65536 - shl32(2, i));
-        for (int k = 0; k < d; k++) a_Q12[k] = (int16_t)s_rshift_round(a32_QA1[k], 5);
+        ROLLED for (int k = 0; k < d; k++) a_Q12[k] = (int16_t)s_rshift_round(a32_QA1[k], 5);
     }
 }
 
@@ -431,10 +431,10 @@ DNI void silk_nlsf2a(int16_t *a_Q12, const int16_t *NLSF, int d, SilkWork *sw)
 DNI void silk_nlsf_stabilize(int16_t *NLSF_Q15, const int16_t *NDeltaMin_Q15, int L)
 {
     int loops, I = 0;
-    for (loops = 0; loops < 20; loops++) {
+    ROLLED for (loops = 0; loops < 20; loops++) {
         int32_t min_diff = NLSF_Q15[0] - NDeltaMin_Q15[0];
         I = 0;
-        for (int i = 1; i <= L - 1; i++) {
+        ROLLED for (int i = 1; i <= L - 1; i++) {
             int32_t diff = NLSF_Q15[i] - (NLSF_Q15[i - 1] + NDeltaMin_Q15[i]);
             if (diff < min_diff) { min_diff = diff; I = i; }
         }
@@ -447,10 +447,10 @@ DNI void silk_nlsf_stabilize(int16_t *NLSF_Q15, const int16_t *NDeltaMin_Q15, in
             NLSF_Q15[L - 1] = (int16_t)((1 << 15) - NDeltaMin_Q15[L]);
         } else {
             int32_t min_center = 0;
-            for (int k = 0; k < I; k++) min_center += NDeltaMin_Q15[k];
+            ROLLED for (int k = 0; k < I; k++) min_center += NDeltaMin_Q15[k];
             min_center += NDeltaMin_Q15[I] >> 1;
             int32_t max_center = 1 << 15;
-            for (int k = L; k > I; k--) max_center -= NDeltaMin_Q15[k];
+            ROLLED for (int k = L; k > I; k--) max_center -= NDeltaMin_Q15[k];
             max_center -= NDeltaMin_Q15[I] >> 1;
             int16_t center = (int16_t)s_limit(s_rshift_round((int32_t)NLSF_Q15[I - 1] + (int32_t)NLSF_Q15[I], 1),
                                               min_center, max_center);
@@ -459,16 +459,16 @@ DNI void silk_nlsf_stabilize(int16_t *NLSF_Q15, const int16_t *NDeltaMin_Q15, in
         }
     }
     if (loops == 20) {
-        for (int i = 1; i < L; i++) {
+        ROLLED for (int i = 1; i < L; i++) {
             int value = NLSF_Q15[i], j;
-            for (j = i - 1; j >= 0 && value < NLSF_Q15[j]; j--) NLSF_Q15[j + 1] = NLSF_Q15[j];
+            ROLLED for (j = i - 1; j >= 0 && value < NLSF_Q15[j]; j--) NLSF_Q15[j + 1] = NLSF_Q15[j];
             NLSF_Q15[j + 1] = (int16_t)value;
         }
         NLSF_Q15[0] = (int16_t)imax(NLSF_Q15[0], NDeltaMin_Q15[0]);
-        for (int i = 1; i < L; i++)
+        ROLLED for (int i = 1; i < L; i++)
             NLSF_Q15[i] = (int16_t)imax(NLSF_Q15[i], (int16_t)s_sat16(NLSF_Q15[i - 1] + NDeltaMin_Q15[i]));
         NLSF_Q15[L - 1] = (int16_t)imin(NLSF_Q15[L - 1], (1 << 15) - NDeltaMin_Q15[L]);
-        for (int i = L - 2; i >= 0; i--)
+        ROLLED for (int i = L - 2; i >= 0; i--)
             NLSF_Q15[i] = (int16_t)imin(NLSF_Q15[i], NLSF_Q15[i + 1] - NDeltaMin_Q15[i + 1]);
     }
 }
@@ -476,7 +476,7 @@ DNI void silk_nlsf_stabilize(int16_t *NLSF_Q15, const int16_t *NDeltaMin_Q15, in
 DFN void silk_nlsf_unpack(int16_t *ec_ix, uint8_t *pred_Q8, const NlsfCB &cb, int CB1_index)
 {
     const uint8_t *sel = &cb.ec_sel[CB1_index * cb.order / 2];
-    for (int i = 0; i < cb.order; i += 2) {
+    ROLLED for (int i = 0; i < cb.order; i += 2) {
         uint8_t entry = *sel++;
         ec_ix[i] = (int16_t)(((entry >> 1) & 7) * 9);
         pred_Q8[i] = cb.pred_Q8[i + (entry & 1) * (cb.order - 1)];
@@ -492,7 +492,7 @@ DNI void silk_nlsf_decode(int16_t *pNLSF_Q15, const int8_t *NLSFIndices, const N
     int16_t *ec_ix = sw->ec_ix, *res_Q10 = sw->res_Q10;
     silk_nlsf_unpack(ec_ix, pred_Q8, cb, NLSFIndices[0]);
     int32_t out_Q10 = 0;
-    for (int i = cb.order - 1; i >= 0; i--) {
+    ROLLED for (int i = cb.order - 1; i >= 0; i--) {
         int32_t pred_Q10 = s_smulbb(out_Q10, (int16_t)pred_Q8[i]) >> 8;
         out_Q10 = shl32(NLSFIndices[i + 1], 10);
         if (out_Q10 > 0) out_Q10 -= 102;            // SILK_FIX_CONST(NLSF_QUANT_LEVEL_ADJ, 10)
@@ -502,7 +502,7 @@ DNI void silk_nlsf_decode(int16_t *pNLSF_Q15, const int8_t *NLSFIndices, const N
     }
     const uint8_t *el = &cb.CB1_NLSF_Q8[NLSFIndices[0] * cb.order];
     const int16_t *w = &cb.CB1_Wght_Q9[NLSFIndices[0] * cb.order];
-    for (int i = 0; i < cb.order; i++) {
+    ROLLED for (int i = 0; i < cb.order; i++) {
         int32_t t = wadd(shl32((int32_t)res_Q10[i], 14) / w[i], shl32((int16_t)el[i], 7));
         pNLSF_Q15[i] = (int16_t)s_limit(t, 0, 32767);
     }
@@ -516,7 +516,7 @@ DNI void silk_lpc_analysis_filter(Lanes L, int16_t *out, const int16_t *in,
     LFOR(L, ix, d, len) {
         const int16_t *ip = &in[ix - 1];
         int32_t acc = s_smulbb(ip[0], B[0]);
-        for (int j = 1; j < d; j++) acc = s_smlabb(acc, ip[-j], B[j]);
+        ROLLED for (int j = 1; j < d; j++) acc = s_smlabb(acc, ip[-j], B[j]);
         acc = wsub(shl32((int32_t)ip[1], 12), acc);
         out[ix] = (int16_t)s_sat16(s_rshift_round(acc, 12));
     }
@@ -529,7 +529,7 @@ DNI void silk_sum_sqr_shift(int32_t *energy, int *shift, const int16_t *x, int l
 {
     int i, shft = 31 - s_clz32(len);
     int32_t nrg = len;
-    for (i = 0; i < len - 1; i += 2) {
+    ROLLED for (i = 0; i < len - 1; i += 2) {
         uint32_t t = (uint32_t)s_smulbb(x[i], x[i]);
         t = (uint32_t)s_smlabb((int32_t)t, x[i + 1], x[i + 1]);
         nrg = (int32_t)((uint32_t)nrg + (t >> shft));
@@ -537,7 +537,7 @@ DNI void silk_sum_sqr_shift(int32_t *energy, int *shift, const int16_t *x, int l
     if (i < len) nrg = (int32_t)((uint32_t)nrg + ((uint32_t)s_smulbb(x[i], x[i]) >> shft));
     shft = imax(0, shft + 3 - s_clz32(nrg));
     nrg = 0;
-    for (i = 0; i < len - 1; i += 2) {
+    ROLLED for (i = 0; i < len - 1; i += 2) {
         uint32_t t = (uint32_t)s_smulbb(x[i], x[i]);
         t = (uint32_t)s_smlabb((int32_t)t, x[i + 1], x[i + 1]);
         nrg = (int32_t)((uint32_t)nrg + (t >> shft));
@@ -552,7 +552,7 @@ DNI void silk_sum_sqr_shift(int32_t *energy, int *shift, const int16_t *x, int l
 DFN void silk_cng_reset(SilkChan *c)
 {
     int32_t step = 32767 / (c->LPC_order + 1), acc = 0;
-    for (int i = 0; i < c->LPC_order; i++) {
+    ROLLED for (int i = 0; i < c->LPC_order; i++) {
         acc += step;
         c->sCNG.CNG_smth_NLSF_Q15[i] = (int16_t)acc;
     }
@@ -642,13 +642,13 @@ DNI void silk_decode_indices(SilkChan *c, RangeDec *rd, int FrameIndex, int deco
         ix->GainsIndices[0] = (int8_t)shl32(rd_icdf(rd, &T_silk_gain_iCDF[ix->signalType * 8], 8), 3);
         ix->GainsIndices[0] = (int8_t)(ix->GainsIndices[0] + rd_icdf(rd, T_silk_uniform8_iCDF, 8));
     }
-    for (int i = 1; i < c->nb_subfr; i++) ix->GainsIndices[i] = (int8_t)rd_icdf(rd, T_silk_delta_gain_iCDF, 8);
+    ROLLED for (int i = 1; i < c->nb_subfr; i++) ix->GainsIndices[i] = (int8_t)rd_icdf(rd, T_silk_delta_gain_iCDF, 8);
 
     NlsfCB cb = silk_nlsf_cb(c->LPC_order);
     ix->NLSFIndices[0] = (int8_t)rd_icdf(rd, &cb.CB1_iCDF[(ix->signalType >> 1) * cb.nVectors], 8);
     int16_t *ec_ix = sw->ec_ix;
     silk_nlsf_unpack(ec_ix, sw->pred_Q8, cb, ix->NLSFIndices[0]);
-    for (int i = 0; i < cb.order; i++) {
+    ROLLED for (int i = 0; i < cb.order; i++) {
         Ix = rd_icdf(rd, &cb.ec_iCDF[ec_ix[i]], 8);
         if (Ix == 0) Ix -= rd_icdf(rd, T_silk_NLSF_EXT_iCDF, 8);
         else if (Ix == 8) Ix += rd_icdf(rd, T_silk_NLSF_EXT_iCDF, 8);
@@ -676,7 +676,7 @@ DNI void silk_decode_indices(SilkChan *c, RangeDec *rd, int FrameIndex, int deco
         ix->PERIndex = (int8_t)rd_icdf(rd, T_silk_LTP_per_index_iCDF, 8);
         const uint8_t *gt = ix->PERIndex == 0 ? T_silk_LTP_gain_iCDF_0
                           : (ix->PERIndex == 1 ? T_silk_LTP_gain_iCDF_1 : T_silk_LTP_gain_iCDF_2);
-        for (int k = 0; k < c->nb_subfr; k++) ix->LTPIndex[k] = (int8_t)rd_icdf(rd, gt, 8);
+        ROLLED for (int k = 0; k < c->nb_subfr; k++) ix->LTPIndex[k] = (int8_t)rd_icdf(rd, gt, 8);
         if (condCoding == CODE_INDEP) ix->LTP_scaleIndex = (int8_t)rd_icdf(rd, T_silk_LTPscale_iCDF, 8);
         else ix->LTP_scaleIndex = 0;
     }
@@ -694,7 +694,7 @@ DNI void silk_shell_decoder(int16_t *p0, RangeDec *rd, int pulses4, int16_t *tre
 {
     int sp = 0;
     tree[sp++] = (int16_t)(pulses4 | 3 << 5);                 // count | level << 5 | first position << 8
-    while (sp > 0) {
+    ROLLED while (sp > 0) {
         int node = tree[--sp];
         int p = node & 31, lvl = (node >> 5) & 3, pos = node >> 8;
         int left = 0;
@@ -725,29 +725,29 @@ DNI void silk_decode_pulses(RangeDec *rd, int16_t *pulses, int signalType, int q
     int iter = frame_length >> 4;
     if (iter * 16 < frame_length) iter++;
     const uint8_t *cdf = &T_silk_pulses_per_block_iCDF[RateLevelIndex * 18];
-    for (int i = 0; i < iter; i++) {
+    ROLLED for (int i = 0; i < iter; i++) {
         nLshifts[i] = 0;
         sum_pulses[i] = rd_icdf(rd, cdf, 8);
-        while (sum_pulses[i] == 17) {
+        ROLLED while (sum_pulses[i] == 17) {
             nLshifts[i]++;
             sum_pulses[i] = rd_icdf(rd, &T_silk_pulses_per_block_iCDF[9 * 18] + (nLshifts[i] == 10), 8);
         }
     }
-    for (int i = 0; i < iter; i++) {
+    ROLLED for (int i = 0; i < iter; i++) {
         if (sum_pulses[i] > 0) {
             PHASE_BEGIN(t_sh);
             silk_shell_decoder(&pulses[i * 16], rd, sum_pulses[i], sw->shell);
             PHASE_END(PH_SILK_SHELL, t_sh, 0);
         }
-        else for (int k = 0; k < 16; k++) pulses[i * 16 + k] = 0;
+        else ROLLED for (int k = 0; k < 16; k++) pulses[i * 16 + k] = 0;
     }
-    for (int i = 0; i < iter; i++) {
+    ROLLED for (int i = 0; i < iter; i++) {
         if (nLshifts[i] > 0) {
             int nLS = nLshifts[i];
             int16_t *pp = &pulses[i * 16];
-            for (int k = 0; k < 16; k++) {
+            ROLLED for (int k = 0; k < 16; k++) {
                 int abs_q = pp[k];
-                for (int j = 0; j < nLS; j++) {
+                ROLLED for (int j = 0; j < nLS; j++) {
                     abs_q = shl32(abs_q, 1);
                     abs_q += rd_icdf(rd, T_silk_lsb_iCDF, 8);
                 }
@@ -762,11 +762,11 @@ DNI void silk_decode_pulses(RangeDec *rd, int16_t *pulses, int signalType, int q
     const uint8_t *icdf_ptr = &T_silk_sign_iCDF[7 * (quantOffsetType + (signalType << 1))];
     int len = (frame_length + 8) >> 4;
     int16_t *q = pulses;
-    for (int i = 0; i < len; i++) {
+    ROLLED for (int i = 0; i < len; i++) {
         int p = sum_pulses[i];
         if (p > 0) {
             icdf[0] = icdf_ptr[imin(p & 0x1F, 6)];
-            for (int j = 0; j < 16; j++)
+            ROLLED for (int j = 0; j < 16; j++)
                 if (q[j] > 0) q[j] = (int16_t)(q[j] * (shl32(rd_icdf(rd, icdf, 8), 1) - 1));
         }
         q += 16;
@@ -780,11 +780,11 @@ DNI void silk_stereo_decode_pred(RangeDec *rd, int32_t *pred_Q13)
     int n = rd_icdf(rd, T_silk_stereo_pred_joint_iCDF, 8);
     ix[0][2] = n / 5;
     ix[1][2] = n - 5 * ix[0][2];
-    for (n = 0; n < 2; n++) {
+    ROLLED for (n = 0; n < 2; n++) {
         ix[n][0] = rd_icdf(rd, T_silk_uniform3_iCDF, 8);
         ix[n][1] = rd_icdf(rd, T_silk_uniform5_iCDF, 8);
     }
-    for (n = 0; n < 2; n++) {
+    ROLLED for (n = 0; n < 2; n++) {
         ix[n][0] += 3 * ix[n][2];
         int32_t low = T_silk_stereo_pred_quant_Q13[ix[n][0]];
         int32_t step = s_smulwb(T_silk_stereo_pred_quant_Q13[ix[n][0] + 1] - low, 6554);
@@ -808,7 +808,7 @@ DNI void silk_decode_pitch(int lagIndex, int contourIndex, int32_t *pitch_lags, 
     }
     int min_lag = 2 * Fs_kHz, max_lag = 18 * Fs_kHz;
     int lag = min_lag + lagIndex;
-    for (int k = 0; k < nb_subfr; k++) {
+    ROLLED for (int k = 0; k < nb_subfr; k++) {
         pitch_lags[k] = lag + cb[k * cbk_size + contourIndex];
         pitch_lags[k] = s_limit(pitch_lags[k], min_lag, max_lag);
     }
@@ -817,7 +817,7 @@ DNI void silk_decode_pitch(int lagIndex, int contourIndex, int32_t *pitch_lags, 
 DNI void silk_gains_dequant(int32_t *gain_Q16, const int8_t *ind, int32_t *prev_ind, int conditional,
                             int nb_subfr)
 {
-    for (int k = 0; k < nb_subfr; k++) {
+    ROLLED for (int k = 0; k < nb_subfr; k++) {
         if (k == 0 && conditional == 0) {
             *prev_ind = imax(ind[k], *prev_ind - 16);
         } else {
@@ -843,14 +843,14 @@ DNI void silk_decode_parameters(SilkChan *c, SilkCtrl *ctrl, int condCoding, Sil
     silk_nlsf2a(ctrl->PredCoef_Q12[1], pNLSF_Q15, c->LPC_order, sw);
     if (c->first_frame_after_reset == 1) ix->NLSFInterpCoef_Q2 = 4;
     if (ix->NLSFInterpCoef_Q2 < 4) {
-        for (int i = 0; i < c->LPC_order; i++)
+        ROLLED for (int i = 0; i < c->LPC_order; i++)
             pNLSF0_Q15[i] = (int16_t)(c->prevNLSF_Q15[i] +
                 ((ix->NLSFInterpCoef_Q2 * (pNLSF_Q15[i] - c->prevNLSF_Q15[i])) >> 2));
         silk_nlsf2a(ctrl->PredCoef_Q12[0], pNLSF0_Q15, c->LPC_order, sw);
     } else {
-        for (int i = 0; i < c->LPC_order; i++) ctrl->PredCoef_Q12[0][i] = ctrl->PredCoef_Q12[1][i];
+        ROLLED for (int i = 0; i < c->LPC_order; i++) ctrl->PredCoef_Q12[0][i] = ctrl->PredCoef_Q12[1][i];
     }
-    for (int i = 0; i < c->LPC_order; i++) c->prevNLSF_Q15[i] = pNLSF_Q15[i];
+    ROLLED for (int i = 0; i < c->LPC_order; i++) c->prevNLSF_Q15[i] = pNLSF_Q15[i];
     if (c->lossCnt) {
         silk_bwexpander(ctrl->PredCoef_Q12[0], c->LPC_order, 63570);
         silk_bwexpander(ctrl->PredCoef_Q12[1], c->LPC_order, 63570);
@@ -859,20 +859,93 @@ DNI void silk_decode_parameters(SilkChan *c, SilkCtrl *ctrl, int condCoding, Sil
         silk_decode_pitch(ix->lagIndex, ix->contourIndex, ctrl->pitchL, c->fs_kHz, c->nb_subfr);
         const int8_t *cbk = ix->PERIndex == 0 ? T_silk_LTP_gain_vq_0
                           : (ix->PERIndex == 1 ? T_silk_LTP_gain_vq_1 : T_silk_LTP_gain_vq_2);
-        for (int k = 0; k < c->nb_subfr; k++) {
+        ROLLED for (int k = 0; k < c->nb_subfr; k++) {
             int I = ix->LTPIndex[k];
-            for (int i = 0; i < 5; i++) ctrl->LTPCoef_Q14[k * 5 + i] = (int16_t)shl32(cbk[I * 5 + i], 7);
+            ROLLED for (int i = 0; i < 5; i++) ctrl->LTPCoef_Q14[k * 5 + i] = (int16_t)shl32(cbk[I * 5 + i], 7);
         }
         ctrl->LTP_scale_Q14 = T_silk_LTPScales_table_Q14[ix->LTP_scaleIndex];
     } else {
-        for (int k = 0; k < c->nb_subfr; k++) ctrl->pitchL[k] = 0;
-        for (int k = 0; k < 5 * c->nb_subfr; k++) ctrl->LTPCoef_Q14[k] = 0;
+        ROLLED for (int k = 0; k < c->nb_subfr; k++) ctrl->pitchL[k] = 0;
+        ROLLED for (int k = 0; k < 5 * c->nb_subfr; k++) ctrl->LTPCoef_Q14[k] = 0;
         ix->PERIndex = 0;
         ctrl->LTP_scale_Q14 = 0;
     }
 }
 
 // ------------------------------------------------------------------ synthesis
+
+// LPC synthesis of one subframe (silk/decode_core.c): v[i] = sat(e[i] +
+// lshift_sat(p, 4)), p = order/2 + sum of the order's truncated tap products
+// on the previous outputs.  win holds the last 16 outputs (win[15] newest).
+//
+// The recursion is the longest serial chain of a SILK frame, so it is laid out
+// for dependency latency: four samples at a time, the taps on outputs older
+// than the four summed first in four independent accumulators (wrap-around
+// sums may be taken in any order), then the few taps inside the four; the
+// order is a compile-time constant and the window stays in registers.  A
+// sample's own path is one mad.hi and one add-shift.  That leaves saturation
+// out; it is checked per four samples (|p| < 2^26 and |e| < 2^30 cannot
+// saturate) and, when that does not hold, the four are redone with the
+// saturating operators.  The int16 outputs are scaled from v afterwards, lanes
+// splitting them.
+template <int ORD>
+DNI void silk_lpc_synth(Lanes L, int32_t *hist, const int16_t *A_Q12, const int32_t *exc, int32_t *v, int n)
+{
+    int32_t a[ORD], win[16];
+#pragma unroll
+    for (int j = 0; j < ORD; j++) a[j] = shl32((int32_t)A_Q12[j], 16);
+#pragma unroll
+    for (int t = 0; t < 16; t++) win[t] = hist[t];
+    lsync(L);   // every lane has read the window before it is written back
+    ROLLED for (int i = 0; i < n; i += 4) {
+        int32_t e[4], p[4], o[4];
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+            e[s] = exc[i + s];
+            p[s] = ORD >> 1;
+        }
+        // taps on the window: sample s's tap j reads win[15 + s - j], j >= s
+#pragma unroll
+        for (int j = ORD - 1; j >= 0; j--) {
+#pragma unroll
+            for (int s = 0; s < 4; s++)
+                if (j >= s) p[s] = s_smlawh(p[s], win[15 + s - j], a[j]);
+        }
+        const int32_t h1 = p[1], h2 = p[2], h3 = p[3];
+        o[0] = wadd(e[0], shl32(p[0], 4));
+        p[1] = s_smlawh(h1, o[0], a[0]);
+        o[1] = wadd(e[1], shl32(p[1], 4));
+        p[2] = s_smlawh(s_smlawh(h2, o[0], a[1]), o[1], a[0]);
+        o[2] = wadd(e[2], shl32(p[2], 4));
+        p[3] = s_smlawh(s_smlawh(s_smlawh(h3, o[0], a[2]), o[1], a[1]), o[2], a[0]);
+        o[3] = wadd(e[3], shl32(p[3], 4));
+        uint32_t far_p = 0, far_e = 0;
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+            far_p |= (uint32_t)p[s] + (1u << 26);
+            far_e |= (uint32_t)e[s] + (1u << 30);
+        }
+        if ((far_p >> 27) | (far_e >> 31)) {
+            o[0] = s_add_sat32(e[0], s_lshift_sat32(p[0], 4));
+            p[1] = s_smlawh(h1, o[0], a[0]);
+            o[1] = s_add_sat32(e[1], s_lshift_sat32(p[1], 4));
+            p[2] = s_smlawh(s_smlawh(h2, o[0], a[1]), o[1], a[0]);
+            o[2] = s_add_sat32(e[2], s_lshift_sat32(p[2], 4));
+            p[3] = s_smlawh(s_smlawh(s_smlawh(h3, o[0], a[2]), o[1], a[1]), o[2], a[0]);
+            o[3] = s_add_sat32(e[3], s_lshift_sat32(p[3], 4));
+        }
+#pragma unroll
+        for (int t = 0; t < 12; t++) win[t] = win[t + 4];
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+            win[12 + s] = o[s];
+            v[i + s] = o[s];
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < 16; t++) hist[t] = win[t];
+    lsync(L);
+}
 
 // silk/decode_core.c: excitation, LTP and LPC synthesis for one frame
 DNI void silk_decode_core(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *xq, const int16_t *pulses,
@@ -895,13 +968,13 @@ DNI void silk_decode_core(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *xq, con
         const int run = (n + L.n - 1) / L.n;
         const int i0 = imin(n, L.id * run), i1 = imin(n, i0 + run);
         uint32_t ma = 1, mb = 0;
-        for (int i = i0; i < i1; i++) {
+        ROLLED for (int i = i0; i < i1; i++) {
             mb = A * (mb + (uint32_t)(int32_t)pulses[i]) + B;
             ma = A * ma;
         }
         lscan_affine(L, ma, mb);
         uint32_t t = ma * (uint32_t)s_rand(ix->Seed) + mb;
-        for (int i = i0; i < i1; i++) {
+        ROLLED for (int i = i0; i < i1; i++) {
             int32_t e = shl32((int32_t)pulses[i], 14);
             if (e > 0) e -= 80 << 4;
             else if (e < 0) e += 80 << 4;
@@ -912,22 +985,15 @@ DNI void silk_decode_core(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *xq, con
         }
         lsync(L);
     }
-    // LPC synthesis history: the last 16 outputs, in registers (win[15] newest);
-    // the previous subframe's gain, also in a register: both are written back
-    // after the frame's last barrier
+    // the previous subframe's gain, in a register until the frame's last barrier
     int32_t prev_gain_Q16 = c->prev_gain_Q16;
-    int32_t win[16];
-#pragma unroll
-    for (int t = 0; t < 16; t++) win[t] = c->sLPC_Q14_buf[t];
     const int32_t *pexc = c->exc_Q14;
     int16_t *pxq = xq;
     int sLTP_buf_idx = c->ltp_mem_length;
     int lag = 0;
-    for (int k = 0; k < c->nb_subfr; k++) {
+    ROLLED for (int k = 0; k < c->nb_subfr; k++) {
         const int32_t *pres;
-        int16_t A_Q12[16];
-        const int16_t *Acoef = ctrl->PredCoef_Q12[k >> 1];
-        for (int i = 0; i < c->LPC_order; i++) A_Q12[i] = Acoef[i];
+        const int16_t *A_Q12 = ctrl->PredCoef_Q12[k >> 1];
         int16_t *B_Q14 = &ctrl->LTPCoef_Q14[k * 5];
         int signalType = ix->signalType;
         int32_t Gain_Q10 = ctrl->Gains_Q16[k] >> 6;
@@ -935,14 +1001,14 @@ DNI void silk_decode_core(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *xq, con
         int32_t gain_adj_Q16;
         if (ctrl->Gains_Q16[k] != prev_gain_Q16) {
             gain_adj_Q16 = s_div32_varq(prev_gain_Q16, ctrl->Gains_Q16[k], 16);
-#pragma unroll
-            for (int t = 0; t < 16; t++) win[t] = s_smulww(gain_adj_Q16, win[t]);
+            LFOR(L, t, 0, 16) c->sLPC_Q14_buf[t] = s_smulww(gain_adj_Q16, c->sLPC_Q14_buf[t]);
+            lsync(L);
         } else {
             gain_adj_Q16 = 1 << 16;
         }
         prev_gain_Q16 = ctrl->Gains_Q16[k];
         if (c->lossCnt && c->prevSignalType == SIG_VOICED && ix->signalType != SIG_VOICED && k < 2) {
-            for (int i = 0; i < 5; i++) B_Q14[i] = 0;
+            ROLLED for (int i = 0; i < 5; i++) B_Q14[i] = 0;
             B_Q14[2] = 4096;   // SILK_FIX_CONST(0.25, 14)
             signalType = SIG_VOICED;
             ctrl->pitchL[k] = c->lagPrev;
@@ -975,7 +1041,7 @@ DNI void silk_decode_core(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *xq, con
             // block, blocks run in order
             const int32_t *pl = &sLTP_Q15[sLTP_buf_idx - lag + 2];
             const int blk = imax(lag - 2, 1);   // lag >= 16 in a valid stream
-            for (int s0 = 0; s0 < c->subfr_length; s0 += blk) {
+            ROLLED for (int s0 = 0; s0 < c->subfr_length; s0 += blk) {
                 int e0 = imin(s0 + blk, c->subfr_length);
                 LFOR(L, i, s0, e0) {
                     int32_t p = 2;
@@ -997,40 +1063,16 @@ DNI void silk_decode_core(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *xq, con
         }
         PHASE_END(PH_SILK_LTP, t_ltp, L.id);
         PHASE_BEGIN(t_lpc);
-        // LPC synthesis: order-10/16 recursion per sample.  The prediction is
-        // order/2 plus one truncated product per tap, summed with wrap-around
-        // adds, so the sum may be taken in any order: the taps on samples
-        // older than the newest one are summed while the newest sample is
-        // still being computed, and only tap 0 stays on the recursion's path.
-        const int order = c->LPC_order;
-        int32_t pold = order >> 1;     // order/2 + taps 1.. on the current window
-#pragma unroll
-        for (int j = 1; j < 16; j++)
-            if (j < order) pold = wadd(pold, s_smulwb(win[15 - j], A_Q12[j]));
-        for (int i = 0; i < c->subfr_length; i++) {
-            int32_t p = wadd(pold, s_smulwb(win[15], A_Q12[0]));
-            // taps 1.. of the next sample read win[16 - j]: known already
-            int32_t pa = order >> 1, pb = 0;
-#pragma unroll
-            for (int j = 1; j < 16; j += 2) {
-                if (j < order) pa = wadd(pa, s_smulwb(win[16 - j], A_Q12[j]));
-                if (j + 1 < order) pb = wadd(pb, s_smulwb(win[15 - j], A_Q12[j + 1]));
-            }
-            pold = wadd(pa, pb);
-            int32_t v = s_add_sat32(pres[i], s_lshift_sat32(p, 4));
-#pragma unroll
-            for (int t = 0; t < 15; t++) win[t] = win[t + 1];
-            win[15] = v;
-            pxq[i] = (int16_t)s_sat16(s_rshift_round(s_smulww(v, Gain_Q10), 8));
-        }
+        int32_t *v = w->sLPC_Q14;
+        if (c->LPC_order == 16) silk_lpc_synth<16>(L, c->sLPC_Q14_buf, A_Q12, pres, v, c->subfr_length);
+        else silk_lpc_synth<10>(L, c->sLPC_Q14_buf, A_Q12, pres, v, c->subfr_length);
+        LFOR(L, i, 0, c->subfr_length) pxq[i] = (int16_t)s_sat16(s_rshift_round(s_smulww(v[i], Gain_Q10), 8));
         pexc += c->subfr_length;
         pxq += c->subfr_length;
         PHASE_END(PH_SILK_LPC, t_lpc, L.id);
         lsync(L);   // the next subframe's LTP rewrites res_Q14, which this one's synthesis reads
     }
     lsync(L);
-#pragma unroll
-    for (int t = 0; t < 16; t++) c->sLPC_Q14_buf[t] = win[t];
     c->prev_gain_Q16 = prev_gain_Q16;
     lsync(L);
 }
@@ -1043,30 +1085,30 @@ DNI void silk_plc_update(SilkChan *c, const SilkCtrl *ctrl)
     c->prevSignalType = c->indices.signalType;
     int32_t LTP_Gain_Q14 = 0;
     if (c->indices.signalType == SIG_VOICED) {
-        for (int j = 0; j * c->subfr_length < ctrl->pitchL[c->nb_subfr - 1]; j++) {
+        ROLLED for (int j = 0; j * c->subfr_length < ctrl->pitchL[c->nb_subfr - 1]; j++) {
             if (j == c->nb_subfr) break;
             int32_t t = 0;
-            for (int i = 0; i < 5; i++) t += ctrl->LTPCoef_Q14[(c->nb_subfr - 1 - j) * 5 + i];
+            ROLLED for (int i = 0; i < 5; i++) t += ctrl->LTPCoef_Q14[(c->nb_subfr - 1 - j) * 5 + i];
             if (t > LTP_Gain_Q14) {
                 LTP_Gain_Q14 = t;
-                for (int i = 0; i < 5; i++) p->LTPCoef_Q14[i] = ctrl->LTPCoef_Q14[(c->nb_subfr - 1 - j) * 5 + i];
+                ROLLED for (int i = 0; i < 5; i++) p->LTPCoef_Q14[i] = ctrl->LTPCoef_Q14[(c->nb_subfr - 1 - j) * 5 + i];
                 p->pitchL_Q8 = shl32(ctrl->pitchL[c->nb_subfr - 1 - j], 8);
             }
         }
-        for (int i = 0; i < 5; i++) p->LTPCoef_Q14[i] = 0;
+        ROLLED for (int i = 0; i < 5; i++) p->LTPCoef_Q14[i] = 0;
         p->LTPCoef_Q14[2] = (int16_t)LTP_Gain_Q14;
         if (LTP_Gain_Q14 < 11469) {
             int32_t scale_Q10 = shl32(11469, 10) / imax(LTP_Gain_Q14, 1);
-            for (int i = 0; i < 5; i++) p->LTPCoef_Q14[i] = (int16_t)(s_smulbb(p->LTPCoef_Q14[i], scale_Q10) >> 10);
+            ROLLED for (int i = 0; i < 5; i++) p->LTPCoef_Q14[i] = (int16_t)(s_smulbb(p->LTPCoef_Q14[i], scale_Q10) >> 10);
         } else if (LTP_Gain_Q14 > 15565) {
             int32_t scale_Q14 = shl32(15565, 14) / imax(LTP_Gain_Q14, 1);
-            for (int i = 0; i < 5; i++) p->LTPCoef_Q14[i] = (int16_t)(s_smulbb(p->LTPCoef_Q14[i], scale_Q14) >> 14);
+            ROLLED for (int i = 0; i < 5; i++) p->LTPCoef_Q14[i] = (int16_t)(s_smulbb(p->LTPCoef_Q14[i], scale_Q14) >> 14);
         }
     } else {
         p->pitchL_Q8 = shl32(s_smulbb(c->fs_kHz, 18), 8);
-        for (int i = 0; i < 5; i++) p->LTPCoef_Q14[i] = 0;
+        ROLLED for (int i = 0; i < 5; i++) p->LTPCoef_Q14[i] = 0;
     }
-    for (int i = 0; i < c->LPC_order; i++) p->prevLPC_Q12[i] = ctrl->PredCoef_Q12[1][i];
+    ROLLED for (int i = 0; i < c->LPC_order; i++) p->prevLPC_Q12[i] = ctrl->PredCoef_Q12[1][i];
     p->prevLTP_scale_Q14 = (int16_t)ctrl->LTP_scale_Q14;
     p->prevGain_Q16[0] = ctrl->Gains_Q16[c->nb_subfr - 2];
     p->prevGain_Q16[1] = ctrl->Gains_Q16[c->nb_subfr - 1];
@@ -1093,15 +1135,15 @@ DNI void silk_plc_conceal(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *frame, 
     lead(L, [&]() CUO_INLINE {
         prevGain_Q10[0] = p->prevGain_Q16[0] >> 6;
         prevGain_Q10[1] = p->prevGain_Q16[1] >> 6;
-        if (c->first_frame_after_reset) for (int i = 0; i < 16; i++) p->prevLPC_Q12[i] = 0;
+        if (c->first_frame_after_reset) ROLLED for (int i = 0; i < 16; i++) p->prevLPC_Q12[i] = 0;
 
         // silk_PLC_energy
         int32_t energy1, energy2;
         int shift1, shift2;
         {
             int16_t *eb = w->plc_exc;
-            for (int k = 0; k < 2; k++)
-                for (int i = 0; i < c->subfr_length; i++)
+            ROLLED for (int k = 0; k < 2; k++)
+                ROLLED for (int i = 0; i < c->subfr_length; i++)
                     eb[k * c->subfr_length + i] = (int16_t)s_sat16(s_smulww(
                         c->exc_Q14[i + (k + c->nb_subfr - 2) * c->subfr_length], prevGain_Q10[k]) >> 8);
             silk_sum_sqr_shift(&energy1, &shift1, eb, c->subfr_length);
@@ -1120,7 +1162,7 @@ DNI void silk_plc_conceal(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *frame, 
         if (c->lossCnt == 0) {
             rand_scale_Q14 = 1 << 14;
             if (c->prevSignalType == SIG_VOICED) {
-                for (int i = 0; i < 5; i++) rand_scale_Q14 = (int16_t)(rand_scale_Q14 - B_Q14[i]);
+                ROLLED for (int i = 0; i < 5; i++) rand_scale_Q14 = (int16_t)(rand_scale_Q14 - B_Q14[i]);
                 rand_scale_Q14 = rand_scale_Q14 > 3277 ? rand_scale_Q14 : 3277;
                 rand_scale_Q14 = (int16_t)(s_smulbb(rand_scale_Q14, p->prevLTP_scale_Q14) >> 14);
             } else {
@@ -1133,7 +1175,7 @@ DNI void silk_plc_conceal(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *frame, 
         }
     });
     int16_t A_Q12[16];
-    for (int i = 0; i < c->LPC_order; i++) A_Q12[i] = p->prevLPC_Q12[i];
+    ROLLED for (int i = 0; i < c->LPC_order; i++) A_Q12[i] = p->prevLPC_Q12[i];
     int lag = s_rshift_round(p->pitchL_Q8, 8);
     int idx = c->ltp_mem_length - lag - c->LPC_order - 2;
     silk_lpc_analysis_filter(L, &sLTP[idx], &c->outBuf[idx], A_Q12, c->ltp_mem_length - idx, c->LPC_order);
@@ -1143,9 +1185,9 @@ DNI void silk_plc_conceal(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *frame, 
     lead(L, [&]() CUO_INLINE {
         int32_t rand_seed = p->rand_seed;
         int sLTP_buf_idx = c->ltp_mem_length;
-        for (int k = 0; k < c->nb_subfr; k++) {
+        ROLLED for (int k = 0; k < c->nb_subfr; k++) {
             const int32_t *pl = &sLTP_Q14[sLTP_buf_idx - lag + 2];
-            for (int i = 0; i < c->subfr_length; i++) {
+            ROLLED for (int i = 0; i < c->subfr_length; i++) {
                 int32_t pr = 2;
                 pr = s_smlawb(pr, pl[i], B_Q14[0]);
                 pr = s_smlawb(pr, pl[i - 1], B_Q14[1]);
@@ -1157,24 +1199,24 @@ DNI void silk_plc_conceal(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *frame, 
                 sLTP_Q14[sLTP_buf_idx] = shl32(s_smlawb(pr, rand_ptr[ri], rand_scale_Q14), 2);
                 sLTP_buf_idx++;
             }
-            for (int j = 0; j < 5; j++) B_Q14[j] = (int16_t)(s_smulbb(harm_Gain_Q15, B_Q14[j]) >> 15);
+            ROLLED for (int j = 0; j < 5; j++) B_Q14[j] = (int16_t)(s_smulbb(harm_Gain_Q15, B_Q14[j]) >> 15);
             rand_scale_Q14 = (int16_t)(s_smulbb(rand_scale_Q14, rand_Gain_Q15) >> 15);
             p->pitchL_Q8 = s_smlawb(p->pitchL_Q8, p->pitchL_Q8, 655);
             p->pitchL_Q8 = min32(p->pitchL_Q8, shl32(s_smulbb(18, c->fs_kHz), 8));
             lag = s_rshift_round(p->pitchL_Q8, 8);
         }
         int32_t *sl = &sLTP_Q14[c->ltp_mem_length - 16];
-        for (int i = 0; i < 16; i++) sl[i] = c->sLPC_Q14_buf[i];
-        for (int i = 0; i < c->frame_length; i++) {
+        ROLLED for (int i = 0; i < 16; i++) sl[i] = c->sLPC_Q14_buf[i];
+        ROLLED for (int i = 0; i < c->frame_length; i++) {
             int32_t pr = c->LPC_order >> 1;
-            for (int j = 0; j < c->LPC_order; j++) pr = s_smlawb(pr, sl[16 + i - j - 1], A_Q12[j]);
+            ROLLED for (int j = 0; j < c->LPC_order; j++) pr = s_smlawb(pr, sl[16 + i - j - 1], A_Q12[j]);
             sl[16 + i] = s_add_sat32(sl[16 + i], s_lshift_sat32(pr, 4));
             frame[i] = (int16_t)s_sat16(s_sat16(s_rshift_round(s_smulww(sl[16 + i], prevGain_Q10[1]), 8)));
         }
-        for (int i = 0; i < 16; i++) c->sLPC_Q14_buf[i] = sl[c->frame_length + i];
+        ROLLED for (int i = 0; i < 16; i++) c->sLPC_Q14_buf[i] = sl[c->frame_length + i];
         p->rand_seed = rand_seed;
         p->randScale_Q14 = rand_scale_Q14;
-        for (int i = 0; i < 4; i++) ctrl->pitchL[i] = lag;
+        ROLLED for (int i = 0; i < 4; i++) ctrl->pitchL[i] = lag;
     });
 }
 
@@ -1216,7 +1258,7 @@ DNI void silk_plc_glue_frames(SilkChan *c, int16_t *frame, int length)
                 int32_t gain_Q16 = shl32(s_sqrt_approx(frac_Q24), 4);
                 int32_t slope_Q16 = ((1 << 16) - gain_Q16) / length;
                 slope_Q16 = shl32(slope_Q16, 2);
-                for (int i = 0; i < length; i++) {
+                ROLLED for (int i = 0; i < length; i++) {
                     frame[i] = (int16_t)s_smulwb(gain_Q16, frame[i]);
                     gain_Q16 += slope_Q16;
                     if (gain_Q16 > (1 << 16)) break;
@@ -1247,24 +1289,24 @@ DNI void silk_cng_generate(SilkChan *c, int16_t *frame, int length, SilkScratch 
     int32_t gain_Q10 = gain_Q16 >> 6;
     // silk_CNG_exc
     int exc_mask = 255;
-    while (exc_mask > length) exc_mask >>= 1;
+    ROLLED while (exc_mask > length) exc_mask >>= 1;
     int32_t seed = g->rand_seed;
-    for (int i = 0; i < length; i++) {
+    ROLLED for (int i = 0; i < length; i++) {
         seed = s_rand(seed);
         sig[16 + i] = g->CNG_exc_buf_Q14[(seed >> 24) & exc_mask];
     }
     g->rand_seed = seed;
     int16_t A_Q12[16];
     silk_nlsf2a(A_Q12, g->CNG_smth_NLSF_Q15, c->LPC_order, &w->sw);
-    for (int i = 0; i < 16; i++) sig[i] = g->CNG_synth_state[i];
-    for (int i = 0; i < length; i++) {
+    ROLLED for (int i = 0; i < 16; i++) sig[i] = g->CNG_synth_state[i];
+    ROLLED for (int i = 0; i < length; i++) {
         int32_t pr = c->LPC_order >> 1;
-        for (int j = 0; j < c->LPC_order; j++) pr = s_smlawb(pr, sig[16 + i - j - 1], A_Q12[j]);
+        ROLLED for (int j = 0; j < c->LPC_order; j++) pr = s_smlawb(pr, sig[16 + i - j - 1], A_Q12[j]);
         sig[16 + i] = s_add_sat32(sig[16 + i], s_lshift_sat32(pr, 4));
         frame[i] = (int16_t)s_sat16((int32_t)frame[i] +
             s_sat16(s_rshift_round(s_smulww(sig[16 + i], gain_Q10), 8)));
     }
-    for (int i = 0; i < 16; i++) g->CNG_synth_state[i] = sig[length + i];
+    ROLLED for (int i = 0; i < 16; i++) g->CNG_synth_state[i] = sig[length + i];
 }
 
 DNI void silk_cng(Lanes L, SilkChan *c, const SilkCtrl *ctrl, int16_t *frame, int length, SilkScratch *w)
@@ -1278,26 +1320,26 @@ DNI void silk_cng(Lanes L, SilkChan *c, const SilkCtrl *ctrl, int16_t *frame, in
             g->fs_kHz = c->fs_kHz;
         }
         if (c->lossCnt == 0 && c->prevSignalType == SIG_NO_VOICE)
-            for (int i = 0; i < c->LPC_order; i++)
+            ROLLED for (int i = 0; i < c->LPC_order; i++)
                 g->CNG_smth_NLSF_Q15[i] = (int16_t)(g->CNG_smth_NLSF_Q15[i] +
                     s_smulwb((int32_t)c->prevNLSF_Q15[i] - (int32_t)g->CNG_smth_NLSF_Q15[i], 16348));
     });
     if (c->lossCnt == 0 && c->prevSignalType == SIG_NO_VOICE) {
         int32_t max_Gain_Q16 = 0;
         int subfr = 0;
-        for (int i = 0; i < c->nb_subfr; i++)
+        ROLLED for (int i = 0; i < c->nb_subfr; i++)
             if (ctrl->Gains_Q16[i] > max_Gain_Q16) { max_Gain_Q16 = ctrl->Gains_Q16[i]; subfr = i; }
         // the excitation history moves up by one subframe: blocks of one
         // subframe from the top, each reading only what the block before it
         // has already moved; lanes split a block
         const int S = c->subfr_length;
-        for (int hi = (c->nb_subfr - 1) * S; hi > 0; hi -= S) {
+        ROLLED for (int hi = (c->nb_subfr - 1) * S; hi > 0; hi -= S) {
             LFOR(L, i, hi - S, hi) g->CNG_exc_buf_Q14[S + i] = g->CNG_exc_buf_Q14[i];
             lsync(L);
         }
         LFOR(L, i, 0, S) g->CNG_exc_buf_Q14[i] = c->exc_Q14[subfr * S + i];
         lead(L, [&]() CUO_INLINE {
-            for (int i = 0; i < c->nb_subfr; i++) {
+            ROLLED for (int i = 0; i < c->nb_subfr; i++) {
                 g->CNG_smth_Gain_Q16 += s_smulwb(ctrl->Gains_Q16[i] - g->CNG_smth_Gain_Q16, 4634);
                 if (s_smulww(g->CNG_smth_Gain_Q16, 46396) > ctrl->Gains_Q16[i])
                     g->CNG_smth_Gain_Q16 = ctrl->Gains_Q16[i];
@@ -1307,7 +1349,7 @@ DNI void silk_cng(Lanes L, SilkChan *c, const SilkCtrl *ctrl, int16_t *frame, in
     lead(L, [&]() CUO_INLINE {
         if (c->lossCnt) silk_cng_generate(c, frame, length, w);
         else
-            for (int i = 0; i < c->LPC_order; i++) g->CNG_synth_state[i] = 0;
+            ROLLED for (int i = 0; i < c->LPC_order; i++) g->CNG_synth_state[i] = 0;
     });
 }
 
@@ -1414,8 +1456,8 @@ DNI void silk_stereo_ms_to_lr(Lanes L, SilkStereo *st, int16_t *x1, int16_t *x2,
 DNI int silk_skip_lbrr(SilkChan *cs, int nChannelsInternal, RangeDec *rd, int32_t *MS_pred_Q13,
                        int decode_only_middle, SilkScratch *w)
 {
-    for (int i = 0; i < cs[0].nFramesPerPacket; i++) {
-        for (int n = 0; n < nChannelsInternal; n++) {
+    ROLLED for (int i = 0; i < cs[0].nFramesPerPacket; i++) {
+        ROLLED for (int n = 0; n < nChannelsInternal; n++) {
             if (cs[n].LBRR_flags[i]) {
                 if (nChannelsInternal == 2 && n == 0) {
                     silk_stereo_decode_pred(rd, MS_pred_Q13);
@@ -1448,14 +1490,14 @@ DNI int silk_decode(Lanes L, SilkDec *dec, SilkDecControl *ctl, int lostFlag, in
     int32_t ms_pred[2] = {0, 0};
         int decode_only_middle = 0;
         if (newPacketFlag)
-            for (int n = 0; n < ctl->nChannelsInternal; n++) cs[n].nFramesDecoded = 0;
+            ROLLED for (int n = 0; n < ctl->nChannelsInternal; n++) cs[n].nFramesDecoded = 0;
         if (ctl->nChannelsInternal > dec->nChannelsInternal) {
             silk_reset_chan(&cs[1]);   // silk_init_decoder
         }
         hdr[2] = ctl->nChannelsInternal == 1 && dec->nChannelsInternal == 2 &&
                              ctl->internalSampleRate == 1000 * cs[0].fs_kHz;
         if (cs[0].nFramesDecoded == 0) {
-            for (int n = 0; n < ctl->nChannelsInternal; n++) {
+            ROLLED for (int n = 0; n < ctl->nChannelsInternal; n++) {
                 int ms = ctl->payloadSize_ms;
                 if (ms == 0 || ms == 10) { cs[n].nFramesPerPacket = 1; cs[n].nb_subfr = 2; }
                 else if (ms == 20) { cs[n].nFramesPerPacket = 1; cs[n].nb_subfr = 4; }
@@ -1477,11 +1519,11 @@ DNI int silk_decode(Lanes L, SilkDec *dec, SilkDecControl *ctl, int lostFlag, in
         dec->nChannelsInternal = ctl->nChannelsInternal;
 
         if (lostFlag != LOSS_LOST && cs[0].nFramesDecoded == 0) {
-            for (int n = 0; n < ctl->nChannelsInternal; n++) {
-                for (int i = 0; i < cs[n].nFramesPerPacket; i++) cs[n].VAD_flags[i] = rd_bit_logp(rd, 1);
+            ROLLED for (int n = 0; n < ctl->nChannelsInternal; n++) {
+                ROLLED for (int i = 0; i < cs[n].nFramesPerPacket; i++) cs[n].VAD_flags[i] = rd_bit_logp(rd, 1);
                 cs[n].LBRR_flag = rd_bit_logp(rd, 1);
             }
-            for (int n = 0; n < ctl->nChannelsInternal; n++) {
+            ROLLED for (int n = 0; n < ctl->nChannelsInternal; n++) {
                 cs[n].LBRR_flags[0] = cs[n].LBRR_flags[1] = cs[n].LBRR_flags[2] = 0;
                 if (cs[n].LBRR_flag) {
                     if (cs[n].nFramesPerPacket == 1) {
@@ -1490,7 +1532,7 @@ DNI int silk_decode(Lanes L, SilkDec *dec, SilkDecControl *ctl, int lostFlag, in
                         const uint8_t *t = cs[n].nFramesPerPacket == 2 ? T_silk_LBRR_flags_2_iCDF
                                                                        : T_silk_LBRR_flags_3_iCDF;
                         int sym = rd_icdf(rd, t, 8) + 1;
-                        for (int i = 0; i < cs[n].nFramesPerPacket; i++) cs[n].LBRR_flags[i] = (sym >> i) & 1;
+                        ROLLED for (int i = 0; i < cs[n].nFramesPerPacket; i++) cs[n].LBRR_flags[i] = (sym >> i) & 1;
                     }
                 }
             }
@@ -1527,13 +1569,13 @@ DNI int silk_decode(Lanes L, SilkDec *dec, SilkDecControl *ctl, int lostFlag, in
         hdr[3] = ms_pred[0];
         hdr[4] = ms_pred[1];
     });
-    for (int k = 0; k < 6; k++) hdr[k] = lbcast(L, hdr[k]);
+    ROLLED for (int k = 0; k < 6; k++) hdr[k] = lbcast(L, hdr[k]);
     if (hdr[0]) return hdr[0];
     const int decode_only_middle = hdr[1], stereo_to_mono = hdr[2], has_side = hdr[5];
     MS_pred_Q13[0] = hdr[3];
     MS_pred_Q13[1] = hdr[4];
     int16_t *tmp[2] = {w->tmp[0], w->tmp[1]};
-    for (int n = 0; n < ctl->nChannelsInternal; n++) {
+    ROLLED for (int n = 0; n < ctl->nChannelsInternal; n++) {
         if (n == 0 || has_side) {
             int FrameIndex = cs[0].nFramesDecoded - n;
             int cond;
@@ -1565,7 +1607,7 @@ DNI int silk_decode(Lanes L, SilkDec *dec, SilkDecControl *ctl, int lostFlag, in
     *nSamplesOut = nSamplesOutDec * ctl->API_sampleRate / s_smulbb(cs[0].fs_kHz, 1000);
     int16_t *rs_out = ctl->nChannelsAPI == 2 ? w->rs_out : samplesOut;
     int nres = imin(ctl->nChannelsAPI, ctl->nChannelsInternal);
-    for (int n = 0; n < nres; n++) {
+    ROLLED for (int n = 0; n < nres; n++) {
         PHASE_BEGIN(t_rs);
         silk_resample(L, &cs[n].resampler_state, rs_out, &tmp[n][1], nSamplesOutDec, w->rs_buf);
         PHASE_END(PH_SILK_RESAMPLE, t_rs, L.id);
@@ -1585,7 +1627,7 @@ DNI int silk_decode(Lanes L, SilkDec *dec, SilkDecControl *ctl, int lostFlag, in
     }
     lead(L, [&]() CUO_INLINE {
         if (lostFlag == LOSS_LOST) {
-            for (int i = 0; i < dec->nChannelsInternal; i++) cs[i].LastGainIndex = 10;
+            ROLLED for (int i = 0; i < dec->nChannelsInternal; i++) cs[i].LastGainIndex = 10;
         } else {
             dec->prev_decode_only_middle = decode_only_middle;
         }

@@ -1,18 +1,14 @@
 // Translation unit of the chain decoder kernel (k_decode_chains).
 //
-// It is compiled apart from the rest of libcuopus, at NVVM -O1 and ptxas -O1:
-//   * code size: the kernel is one large body of codec paths (SILK, CELT,
-//     hybrid, PLC), and with every decoder slot busy its warps stall mostly on
-//     instruction fetch (ncu: 6.1 cycles per issued instruction).  NVVM -O1
-//     unrolls and duplicates less; the machine code shrinks from 1.17 MB to
-//     0.79 MB and a loaded GPU decodes about 20 % more audio per second, with
-//     identical output;
-//   * with NVVM -O3, ptxas -O2 and -O3 decoded stereo SILK and hybrid frames
-//     with wrong samples (the mid/side to left/right stage diverged from
-//     libopus on the first stereo frame), while ptxas -O0 / -O1, nvcc -G and
-//     the same sources built for the host with g++ (also under ASan / UBSan,
-//     and with every local variable pattern-initialised) were bit-exact.
-// The GPU parity tests hold the shipped build to libopus on stereo streams.
+// The kernel is one large body of codec paths (SILK, CELT, hybrid, PLC), each
+// warp at a different place in it, so instruction fetch is paid for by size.
+// It is compiled at full optimisation with its loops rolled (ROLLED in
+// dec/common.cuh): 385 KB of kernel code.  Built at NVVM -O1 and ptxas -O1 to
+// keep it small (342 KB) the arrays that the unrolled loops index stayed in
+// local memory: the LPC recursion took 2,300 cycles a sample (160 now) and
+// 64 one-second voice clips took 29.0 ms (14.8 now); at -O3 with the
+// compiler's own unrolling (764 KB) a loaded GPU was slower than either (30
+// files, 1,085 s: 172 ms against 122 and 117 ms).
 #define CUO_DECODE_KERNEL_TU 1
 #include <cuda_runtime.h>
 #include <stdio.h>

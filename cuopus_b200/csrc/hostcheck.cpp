@@ -179,6 +179,15 @@ int hc_silk_resample(int fs_in, const int16_t *in, int n_in, int frame, int16_t 
     return o;
 }
 
+// LPC synthesis of n samples (order 10 or 16): hist is the 16-sample window in
+// and out, v receives the outputs.
+void hc_silk_lpc_synth(int order, int32_t *hist, const int16_t *A_Q12, const int32_t *exc, int32_t *v, int n)
+{
+    cuo::Lanes L{0, 1, 1u};
+    if (order == 16) cuo::silk_lpc_synth<16>(L, hist, A_Q12, exc, v, n);
+    else cuo::silk_lpc_synth<10>(L, hist, A_Q12, exc, v, n);
+}
+
 // The decoder's comb (post-)filter in place on buf + off: the serial form
 // (lanes = 0) or the block-parallel form the decoder runs (lanes = 1, here
 // with a single lane walking the same blocks).
