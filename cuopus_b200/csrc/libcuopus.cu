@@ -212,9 +212,10 @@ int ensure_taps(cudaStream_t st, Err &err)
     CK(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lk(g_taps_mu);
     if (G.taps_dev == dev) return RC_OK;
-    float taps[cuo::RS_TAPS];
+    float taps[cuo::RS_TAPS], pairs[2 * cuo::RS_TAPS];
     make_taps(taps);
-    CK(cudaMemcpyToSymbolAsync(cuo::c_rs_taps, taps, sizeof taps, 0, cudaMemcpyHostToDevice, st));
+    for (int t = 0; t < cuo::RS_TAPS; t++) pairs[2 * t] = pairs[2 * t + 1] = taps[t];
+    CK(cudaMemcpyToSymbolAsync(cuo::c_rs_taps, pairs, sizeof pairs, 0, cudaMemcpyHostToDevice, st));
     CK(cudaStreamSynchronize(st));
     G.taps_dev = dev;
     return RC_OK;
@@ -732,9 +733,15 @@ int resample(const int16_t *in, int64_t avail, int64_t n_out, float *out, cudaSt
     if (n_out <= 0) return RC_OK;
     int rc = ensure_taps(st, err);
     if (rc) return rc;
-    long long blocks = (n_out + cuo::RS_TILE_OUT - 1) / cuo::RS_TILE_OUT;
-    if (blocks > 0x7fffffffLL) return err.set(RC_ARG, "resample length too large");
-    cuo::k_resample48to16<<<(unsigned)blocks, cuo::RS_THREADS, 0, st>>>(in, avail, n_out, out, chans);
+    if ((rc = ensure_occupancy(err))) return rc;
+    const int run = cuo::rs_run(n_out, G.sm_count);
+    long long tiles = (n_out + cuo::rs_tile(run) - 1) / cuo::rs_tile(run);
+    if (tiles > 0x7fffffffLL) return err.set(RC_ARG, "resample length too large");
+    const long long blocks = std::min<long long>(tiles, (long long)G.sm_count * cuo::RS_BLOCKS);
+    if (run == 9)
+        cuo::k_resample48to16<9><<<(unsigned)blocks, cuo::RS_THREADS, 0, st>>>(in, avail, n_out, out, chans);
+    else
+        cuo::k_resample48to16<3><<<(unsigned)blocks, cuo::RS_THREADS, 0, st>>>(in, avail, n_out, out, chans);
     CK(cudaGetLastError());
     return RC_OK;
 }
