@@ -309,7 +309,7 @@ DNI int opus_frame(Lanes L, OpusDec *st, const uint8_t *data, int32_t len, int16
                 redundancy_bytes = 0;
                 redundancy = 0;
             }
-            dec.storage -= redundancy_bytes;
+            rd_shrink(&dec, redundancy_bytes);
         }
     }
     if (mode != MODE_CELT_ONLY) start_band = 17;

@@ -9,7 +9,7 @@
 // (all lanes decode the same symbols).  `buf` points at the frame bytes; the
 // chain kernel stages those into shared memory when it can.
 #pragma once
-#include "common.cuh"
+#include "hottabs.cuh"
 
 namespace cuo {
 
@@ -25,6 +25,7 @@ struct RangeDec {
     uint32_t val;
     uint32_t ext;
     int rem;
+    int next;        // the byte at offs (0 past the end), read ahead of its use
     int error;
 };
 
@@ -45,6 +46,7 @@ DFN void rd_bcast(const Lanes &L, RangeDec *d)
     d->val = __shfl_sync(L.mask, d->val, src);
     d->ext = __shfl_sync(L.mask, d->ext, src);
     d->rem = __shfl_sync(L.mask, d->rem, src);
+    d->next = __shfl_sync(L.mask, d->next, src);
     d->error = __shfl_sync(L.mask, d->error, src);
 #elif defined(CUO_LANE_SIM)
     if (L.sim) lanesim_bcast(L.sim, L.id, d, (int)sizeof *d);
@@ -62,7 +64,22 @@ template <class F> DFN void lead_rd(const Lanes &L, RangeDec *rd, F &&body)
     rd_bcast(L, rd);
 }
 
-DFN int rd_read_byte(RangeDec *d) { return d->offs < d->storage ? d->buf[d->offs++] : 0; }
+DFN int rd_peek(const RangeDec *d) { return d->offs < d->storage ? d->buf[d->offs] : 0; }
+// The frame's next byte.  The one after it is loaded here, so that its latency
+// is over by the time a symbol needs it.
+DFN int rd_read_byte(RangeDec *d)
+{
+    int b = d->next;
+    d->offs += d->offs < d->storage;
+    d->next = rd_peek(d);
+    return b;
+}
+// The frame lost its last bytes (redundancy): what is read ahead may be one of them.
+DFN void rd_shrink(RangeDec *d, uint32_t bytes)
+{
+    d->storage -= bytes;
+    d->next = rd_peek(d);
+}
 DFN int rd_read_byte_end(RangeDec *d)
 {
     return d->end_offs < d->storage ? d->buf[d->storage - ++(d->end_offs)] : 0;
@@ -89,6 +106,7 @@ DNI void rd_init(RangeDec *d, const uint8_t *buf, uint32_t storage)
     d->nend_bits = 0;
     d->nbits_total = 33 - 24;   // EC_CODE_BITS+1 - ((EC_CODE_BITS-EC_CODE_EXTRA)/8)*8
     d->offs = 0;
+    d->next = rd_peek(d);
     d->rng = 1u << 7;
     d->rem = rd_read_byte(d);
     d->val = d->rng - 1 - (d->rem >> 1);
@@ -119,7 +137,12 @@ DNI void rd_update(RangeDec *d, unsigned fl, unsigned fh, unsigned ft)
     rd_normalize(d);
 }
 
-DNI int rd_bit_logp(RangeDec *d, unsigned logp)
+// The symbol functions come twice: inlined (rdi_), for the loops that decode
+// many symbols and keep a copy of the decoder state in registers while they
+// do (a copy whose address goes to no call), and as calls (rd_) that update
+// the state in memory, for everything else.  A symbol took 500-1,000 cycles as
+// a call in a SILK frame's pulses, mostly the state's round trips.
+DFN int rdi_bit_logp(RangeDec *d, unsigned logp)
 {
     uint32_t r = d->rng, v = d->val;
     uint32_t s = r >> logp;
@@ -129,8 +152,9 @@ DNI int rd_bit_logp(RangeDec *d, unsigned logp)
     rd_normalize(d);
     return ret;
 }
+DNI int rd_bit_logp(RangeDec *d, unsigned logp) { return rdi_bit_logp(d, logp); }
 
-DNI int rd_icdf(RangeDec *d, const uint8_t *icdf, unsigned ftb)
+DFN int rdi_icdf(RangeDec *d, const uint8_t *icdf, unsigned ftb)
 {
     uint32_t s = d->rng, v = d->val, r = s >> ftb, t;
     int ret = -1;
@@ -140,6 +164,45 @@ DNI int rd_icdf(RangeDec *d, const uint8_t *icdf, unsigned ftb)
     } while (v < s);
     d->val = v - s;
     d->rng = t - s;
+    rd_normalize(d);
+    return ret;
+}
+DNI int rd_icdf(RangeDec *d, const uint8_t *icdf, unsigned ftb) { return rdi_icdf(d, icdf, ftb); }
+
+// rdi_icdf (8-bit probabilities) over a row of HotTabs: four entries a step,
+// their products side by side, where the plain search waits for one entry
+// after the other.
+DFN int rdi_icdf_row(RangeDec *d, const uint32_t *row)
+{
+    const uint32_t v = d->val, r = d->rng >> 8;
+    uint32_t t = d->rng, s0, s1, s2, s3;
+    int at = 0;
+    ROLLED while (1) {
+        const uint32_t w = row[at >> 2];
+        s0 = r * (w & 0xff);
+        s1 = r * ((w >> 8) & 0xff);
+        s2 = r * ((w >> 16) & 0xff);
+        s3 = r * (w >> 24);
+        if (v >= s3) break;
+        t = s3;
+        at += 4;
+    }
+    const int a0 = v < s0, a1 = v < s1, a2 = v < s2;   // entries above v: a prefix
+    const uint32_t s = a2 ? s3 : a1 ? s2 : a0 ? s1 : s0;
+    t = a2 ? s2 : a1 ? s1 : a0 ? s0 : t;
+    d->val = v - s;
+    d->rng = t - s;
+    rd_normalize(d);
+    return at + a0 + a1 + a2;
+}
+
+// rdi_icdf over the two-entry table {p, 0}
+DFN int rdi_icdf_bit(RangeDec *d, unsigned p)
+{
+    const uint32_t s = (d->rng >> 8) * p;
+    const int ret = d->val < s;
+    d->rng = ret ? s : d->rng - s;
+    if (!ret) d->val -= s;
     rd_normalize(d);
     return ret;
 }

@@ -128,18 +128,17 @@ struct SilkDecControl {   // silk_DecControlStruct (decoder fields)
 struct SilkWork {
     int32_t A[16];                                        // silk_lpc_inv_pred_gain
     int32_t cos_LSF_QA[16], P[9], Q[9], a32_QA1[16];      // silk_nlsf2a
-    int16_t ec_ix[16], res_Q10[16];                       // NLSF unpack / residuals
+    int16_t ec_ix[16], res_Q10[16];                       // NLSF unpack (codebook selectors) / residuals
     uint8_t pred_Q8[16];
     int16_t pNLSF_Q15[16], pNLSF0_Q15[16];                // silk_decode_parameters
     int32_t sum_pulses[20], nLshifts[20];                 // silk_decode_pulses
-    int16_t shell[14];                                    // shell split tree walk: stack
-    uint8_t sign_icdf[2];
+    uint16_t nonzero[20];                                 // per block of 16: which have pulses
 };
 
 struct SilkScratch {
     SilkWork sw;
-    int16_t pulses[SILK_MAX_FRAME + 16];
-    int16_t lbrr_pulses[SILK_MAX_FRAME + 16];
+    alignas(16) int16_t pulses[SILK_MAX_FRAME + 16];
+    alignas(16) int16_t lbrr_pulses[SILK_MAX_FRAME + 16];
     int16_t sLTP[SILK_MAX_FRAME];
     int32_t sLTP_Q15[2 * SILK_MAX_FRAME];
     int32_t res_Q14[SILK_MAX_SUBFR_LEN];
@@ -478,9 +477,9 @@ DFN void silk_nlsf_unpack(int16_t *ec_ix, uint8_t *pred_Q8, const NlsfCB &cb, in
     const uint8_t *sel = &cb.ec_sel[CB1_index * cb.order / 2];
     ROLLED for (int i = 0; i < cb.order; i += 2) {
         uint8_t entry = *sel++;
-        ec_ix[i] = (int16_t)(((entry >> 1) & 7) * 9);
+        ec_ix[i] = (int16_t)((entry >> 1) & 7);
         pred_Q8[i] = cb.pred_Q8[i + (entry & 1) * (cb.order - 1)];
-        ec_ix[i + 1] = (int16_t)(((entry >> 5) & 7) * 9);
+        ec_ix[i + 1] = (int16_t)((entry >> 5) & 7);
         pred_Q8[i + 1] = cb.pred_Q8[i + ((entry >> 4) & 1) * (cb.order - 1) + 1];
     }
 }
@@ -648,11 +647,17 @@ DNI void silk_decode_indices(SilkChan *c, RangeDec *rd, int FrameIndex, int deco
     ix->NLSFIndices[0] = (int8_t)rd_icdf(rd, &cb.CB1_iCDF[(ix->signalType >> 1) * cb.nVectors], 8);
     int16_t *ec_ix = sw->ec_ix;
     silk_nlsf_unpack(ec_ix, sw->pred_Q8, cb, ix->NLSFIndices[0]);
-    ROLLED for (int i = 0; i < cb.order; i++) {
-        Ix = rd_icdf(rd, &cb.ec_iCDF[ec_ix[i]], 8);
-        if (Ix == 0) Ix -= rd_icdf(rd, T_silk_NLSF_EXT_iCDF, 8);
-        else if (Ix == 8) Ix += rd_icdf(rd, T_silk_NLSF_EXT_iCDF, 8);
-        ix->NLSFIndices[i + 1] = (int8_t)(Ix - 4);
+    {
+        RangeDec d = *rd;
+        ROLLED for (int i = 0; i < cb.order; i++) {
+            Ix = rdi_icdf_row(&d, hot_tabs().nlsf[cb.order == 16][ec_ix[i]]);
+            if (Ix == 0 || Ix == 8) {
+                int e = rdi_icdf(&d, T_silk_NLSF_EXT_iCDF, 8);
+                Ix += Ix == 0 ? -e : e;
+            }
+            ix->NLSFIndices[i + 1] = (int8_t)(Ix - 4);
+        }
+        *rd = d;
     }
     if (c->nb_subfr == 4) ix->NLSFInterpCoef_Q2 = (int8_t)rd_icdf(rd, T_silk_NLSF_interpolation_factor_iCDF, 8);
     else ix->NLSFInterpCoef_Q2 = 4;
@@ -689,31 +694,35 @@ DNI void silk_decode_indices(SilkChan *c, RangeDec *rd, int FrameIndex, int deco
 // before right half, which reads the splits in the same order.  A node at
 // level L (3 = the root) holds the pulse count of 2^(L+1) positions; its split
 // gives the left child's count from the level-L table, the right child gets
-// the rest.  `tree` is scratch for the walk's stack (8 entries).
-DNI void silk_shell_decoder(int16_t *p0, RangeDec *rd, int pulses4, int16_t *tree)
+// the rest.
+// Nodes without pulses are never visited: the 16 positions start as zeros.
+// The nodes yet to be visited (at most one per level) are the 16-bit fields of
+// one register: count | level << 5 | first position << 7.  Returns the mask of
+// the positions that got pulses.  Every node takes the same path: with several
+// chains in a warp their nodes are decoded side by side, and a shorter path for
+// nodes of one pulse, no faster on one chain (a voice second 9.7 ms either
+// way), took that away (the 2 h file at 8 lanes a chain 143 ms against 113).
+DFN unsigned silk_shell_decoder(int16_t *p0, RangeDec *rd, int pulses)
 {
-    int sp = 0;
-    tree[sp++] = (int16_t)(pulses4 | 3 << 5);                 // count | level << 5 | first position << 8
-    ROLLED while (sp > 0) {
-        int node = tree[--sp];
-        int p = node & 31, lvl = (node >> 5) & 3, pos = node >> 8;
-        int left = 0;
-        if (p > 0) {
-            const uint8_t *t = lvl == 3 ? T_silk_shell_code_table3
-                             : lvl == 2 ? T_silk_shell_code_table2
-                             : lvl == 1 ? T_silk_shell_code_table1 : T_silk_shell_code_table0;
-            left = rd_icdf(rd, &t[T_silk_shell_code_table_offsets[p]], 8);
-        }
-        int right = p - left;
+    memset(__builtin_assume_aligned(p0, 16), 0, 16 * sizeof(int16_t));
+    unsigned nonzero = 0;
+    uint64_t todo = (uint64_t)(pulses | 3 << 5);
+    ROLLED while (todo) {
+        const unsigned node = (unsigned)todo & 0xffff, p = node & 31;
+        const unsigned lvl = (node >> 5) & 3, pos = node >> 7;
+        todo >>= 16;
+        const unsigned left = (unsigned)rdi_icdf_row(rd, hot_tabs().shell[lvl][p]), right = p - left;
         if (lvl == 0) {
             p0[pos] = (int16_t)left;
             p0[pos + 1] = (int16_t)right;
+            nonzero |= (left ? 1u << pos : 0u) | (right ? 2u << pos : 0u);
         } else {
-            int half = 1 << lvl;                                  // positions under each child
-            tree[sp++] = (int16_t)(right | (lvl - 1) << 5 | (pos + half) << 8);
-            tree[sp++] = (int16_t)(left | (lvl - 1) << 5 | pos << 8);
+            const unsigned child = node - p - 32, half = 1u << lvl;   // level - 1; positions under each child
+            if (right) todo = todo << 16 | (child + right + (half << 7));
+            if (left) todo = todo << 16 | (child + left);
         }
     }
+    return nonzero;
 }
 
 // silk/decode_pulses.c + code_signs.c silk_decode_signs
@@ -721,56 +730,59 @@ DNI void silk_decode_pulses(RangeDec *rd, int16_t *pulses, int signalType, int q
                             int frame_length, SilkWork *sw)
 {
     int32_t *sum_pulses = sw->sum_pulses, *nLshifts = sw->nLshifts;
-    int RateLevelIndex = rd_icdf(rd, &T_silk_rate_levels_iCDF[(signalType >> 1) * 9], 8);
+    RangeDec d = *rd;   // in registers for the whole frame (rangedec.cuh)
+    int RateLevelIndex = rdi_icdf_row(&d, hot_tabs().rate[signalType >> 1]);
     int iter = frame_length >> 4;
     if (iter * 16 < frame_length) iter++;
-    const uint8_t *cdf = &T_silk_pulses_per_block_iCDF[RateLevelIndex * 18];
+    const uint32_t *cdf = hot_tabs().pulses[RateLevelIndex];
     ROLLED for (int i = 0; i < iter; i++) {
-        nLshifts[i] = 0;
-        sum_pulses[i] = rd_icdf(rd, cdf, 8);
-        ROLLED while (sum_pulses[i] == 17) {
-            nLshifts[i]++;
-            sum_pulses[i] = rd_icdf(rd, &T_silk_pulses_per_block_iCDF[9 * 18] + (nLshifts[i] == 10), 8);
+        int shifts = 0, sum = rdi_icdf_row(&d, cdf);
+        ROLLED while (sum == 17) {
+            shifts++;
+            sum = rdi_icdf_row(&d, hot_tabs().pulses[shifts == 10 ? 10 : 9]);
+        }
+        nLshifts[i] = shifts;
+        sum_pulses[i] = sum;
+    }
+    PHASE_BEGIN(t_sh);
+    ROLLED for (int i = 0; i < iter; i++) {
+        if (sum_pulses[i] > 0) sw->nonzero[i] = (uint16_t)silk_shell_decoder(&pulses[i * 16], &d, sum_pulses[i]);
+        else {
+            memset(__builtin_assume_aligned(&pulses[i * 16], 16), 0, 16 * sizeof(int16_t));
+            sw->nonzero[i] = 0;
         }
     }
-    ROLLED for (int i = 0; i < iter; i++) {
-        if (sum_pulses[i] > 0) {
-            PHASE_BEGIN(t_sh);
-            silk_shell_decoder(&pulses[i * 16], rd, sum_pulses[i], sw->shell);
-            PHASE_END(PH_SILK_SHELL, t_sh, 0);
-        }
-        else ROLLED for (int k = 0; k < 16; k++) pulses[i * 16 + k] = 0;
-    }
+    PHASE_END(PH_SILK_SHELL, t_sh, 0);
     ROLLED for (int i = 0; i < iter; i++) {
         if (nLshifts[i] > 0) {
             int nLS = nLshifts[i];
             int16_t *pp = &pulses[i * 16];
+            unsigned nonzero = 0;
             ROLLED for (int k = 0; k < 16; k++) {
                 int abs_q = pp[k];
-                ROLLED for (int j = 0; j < nLS; j++) {
-                    abs_q = shl32(abs_q, 1);
-                    abs_q += rd_icdf(rd, T_silk_lsb_iCDF, 8);
-                }
+                ROLLED for (int j = 0; j < nLS; j++) abs_q = shl32(abs_q, 1) + rdi_icdf_bit(&d, T_silk_lsb_iCDF[0]);
                 pp[k] = (int16_t)abs_q;
+                nonzero |= (unsigned)(pp[k] > 0) << k;
             }
             sum_pulses[i] |= nLS << 5;
+            sw->nonzero[i] = (uint16_t)nonzero;
         }
     }
-    // signs
-    uint8_t *icdf = sw->sign_icdf;
-    icdf[1] = 0;
+    // signs, of the positions that have pulses
     const uint8_t *icdf_ptr = &T_silk_sign_iCDF[7 * (quantOffsetType + (signalType << 1))];
     int len = (frame_length + 8) >> 4;
-    int16_t *q = pulses;
     ROLLED for (int i = 0; i < len; i++) {
-        int p = sum_pulses[i];
+        const int p = sum_pulses[i];
         if (p > 0) {
-            icdf[0] = icdf_ptr[imin(p & 0x1F, 6)];
-            ROLLED for (int j = 0; j < 16; j++)
-                if (q[j] > 0) q[j] = (int16_t)(q[j] * (shl32(rd_icdf(rd, icdf, 8), 1) - 1));
+            const unsigned icdf0 = icdf_ptr[imin(p & 0x1F, 6)];
+            int16_t *q = &pulses[i * 16];
+            ROLLED for (unsigned left = sw->nonzero[i]; left; left &= left - 1) {
+                const int j = ilog(left & (0u - left)) - 1;
+                if (!rdi_icdf_bit(&d, icdf0)) q[j] = (int16_t)-q[j];
+            }
         }
-        q += 16;
     }
+    *rd = d;
 }
 
 // silk/stereo_decode_pred.c

@@ -111,6 +111,8 @@ __device__ __forceinline__ unsigned queue_next(const DecodeArgs &a, int light)
 template <int MIN_BLOCKS>
 __global__ void __launch_bounds__(128, MIN_BLOCKS) k_decode_chains(DecodeArgs a)
 {
+    hot_fill(&s_hot_tabs, threadIdx.x, blockDim.x);
+    __syncthreads();
     const int W = a.width;
     const int lane = threadIdx.x & 31;
     const int sub = lane / W;
