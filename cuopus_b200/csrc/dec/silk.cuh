@@ -208,20 +208,60 @@ DNI void silk_resampler_init48(SilkResampler *S, int32_t Fs_Hz_in)
 // silk/resampler_private_up2_HQ.c: 2x up-sampling by two 3-stage all-pass chains
 // The even and the odd outputs come from two all-pass cascades that share
 // only the input (states S[0..2] and S[3..5]), so two lanes run one cascade
-// each; a group of one lane runs them one after the other.
+// each; a group of one lane runs them one after the other.  The cascade's
+// three sections are skewed: step k runs section 1 on input k, section 2 on
+// section 1's output of k - 1 and section 3 on section 2's of k - 2, so a step
+// waits for one section and not for three.  Inputs come eight ahead.
 DNI void silk_up2_hq(Lanes L, int32_t *S, int16_t *out, const int16_t *in, int32_t len)
 {
     const int step = L.n > 1 ? 2 : 1;
     ROLLED for (int ph = L.n > 1 ? L.id : 0; ph < 2; ph += step) {
         const int16_t *a = ph ? T_silk_resampler_up2_hq_1 : T_silk_resampler_up2_hq_0;
+        const int32_t a0 = shl32(a[0], 16), a1 = shl32(a[1], 16), a2 = shl32(a[2], 16);
         int32_t s0 = S[3 * ph], s1 = S[3 * ph + 1], s2 = S[3 * ph + 2];
-        ROLLED for (int32_t k = 0; k < len; k++) {
-            int32_t in32 = shl32((int32_t)in[k], 10), Y, X, o1, o2;
-            Y = wsub(in32, s0); X = s_smulwb(Y, a[0]); o1 = wadd(s0, X); s0 = wadd(in32, X);
-            Y = wsub(o1, s1); X = s_smulwb(Y, a[1]); o2 = wadd(s1, X); s1 = wadd(o1, X);
-            Y = wsub(o2, s2); X = s_smlawb(Y, Y, a[2]); o1 = wadd(s2, X); s2 = wadd(o2, X);
-            out[2 * k + ph] = (int16_t)s_sat16(s_rshift_round(o1, 10));
+        int32_t i1 = 0, i2 = 0;   // the inputs of sections 2 and 3
+        int16_t *o = out + ph;
+        // section 1 of `x`; section 2 and 3 of what came before when on
+        auto step3 = [&](int32_t x, int on2, int on3, int16_t *dst) CUO_INLINE {
+            int32_t Y2 = wsub(i2, s2), X2 = s_smlawh(Y2, Y2, a2), o2 = wadd(s2, X2);
+            int32_t Y1 = wsub(i1, s1), X1 = s_smlawh(0, Y1, a1), o1 = wadd(s1, X1);
+            int32_t in32 = shl32(x, 10);
+            int32_t Y0 = wsub(in32, s0), X0 = s_smlawh(0, Y0, a0), o0 = wadd(s0, X0);
+            if (on3) {
+                s2 = wadd(i2, X2);
+                *dst = (int16_t)s_sat16(s_rshift_round(o2, 10));
+            }
+            if (on2) s1 = wadd(i1, X1);
+            s0 = wadd(in32, X0);
+            i2 = o1;
+            i1 = o0;
+        };
+        // the first two steps fill the cascade, the last two drain it
+        int32_t k = 0;
+        if (len > 0) step3(in[0], 0, 0, o);
+        if (len > 1) step3(in[1], 1, 0, o);
+        k = 2;
+        ROLLED for (; k + 8 <= len; k += 8) {
+            int32_t x[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) x[j] = in[k + j];
+#pragma unroll
+            for (int j = 0; j < 8; j++) step3(x[j], 1, 1, o + 2 * (k + j - 2));
         }
+        ROLLED for (; k < len; k++) step3(in[k], 1, 1, o + 2 * (k - 2));
+        const int32_t keep0 = s0;
+        if (len > 1) {
+            step3(0, 1, 1, o + 2 * (len - 2));
+            const int32_t keep1 = s1;
+            step3(0, 0, 1, o + 2 * (len - 1));
+            s1 = keep1;
+        } else if (len == 1) {
+            step3(0, 1, 0, o);
+            const int32_t keep1 = s1;
+            step3(0, 0, 1, o);
+            s1 = keep1;
+        }
+        s0 = keep0;
         S[3 * ph] = s0; S[3 * ph + 1] = s1; S[3 * ph + 2] = s2;
     }
     lsync(L);
@@ -908,12 +948,17 @@ DNI void silk_lpc_synth(Lanes L, int32_t *hist, const int16_t *A_Q12, const int3
     for (int j = 0; j < ORD; j++) a[j] = shl32((int32_t)A_Q12[j], 16);
 #pragma unroll
     for (int t = 0; t < 16; t++) win[t] = hist[t];
+    int32_t ahead[4];   // the next four inputs, loaded while these four are computed
+#pragma unroll
+    for (int s = 0; s < 4; s++) ahead[s] = exc[s];
     lsync(L);   // every lane has read the window before it is written back
     ROLLED for (int i = 0; i < n; i += 4) {
         int32_t e[4], p[4], o[4];
+        const int nx = i + 4 < n ? i + 4 : i;
 #pragma unroll
         for (int s = 0; s < 4; s++) {
-            e[s] = exc[i + s];
+            e[s] = ahead[s];
+            ahead[s] = exc[nx + s];
             p[s] = ORD >> 1;
         }
         // taps on the window: sample s's tap j reads win[15 + s - j], j >= s
