@@ -46,13 +46,11 @@ struct CeltDec {
     int16_t oldBandE[2 * CELT_NB], oldLogE[2 * CELT_NB], oldLogE2[2 * CELT_NB], backgroundLogE[2 * CELT_NB];
 };
 
-// One frame of quant_partition's explicit stack (the state of one split level).
-struct QPFrame {
-    int16_t *X, *Y, *lowband, *next_lowband2;
-    int N, b, B, B0, LM, fill, mbits, sbits, itheta, stage;
-    int32_t rebalance;
-    int16_t gain, mid, side;
-    unsigned cm;
+// A split of quant_partition: what its second half needs.
+struct QPSplit {
+    int16_t *X, *lowband;
+    int32_t bits, first_bits, rebalance, N, B, B0, LM, fill, mid_first, fixed;
+    int16_t gain;
 };
 
 // Per lane group, in the decoder slot.  Besides the frame buffers it holds
@@ -61,7 +59,7 @@ struct QPFrame {
 // of them (a per-lane stack copy would multiply the memory these stages touch
 // by the group width).
 struct CeltScratch {
-    QPFrame qp[5];                    // quant_partition's split stack
+    QPSplit qp[4];                    // quant_partition's splits, outermost first
     int32_t bits1[CELT_NB], bits2[CELT_NB], thresh[CELT_NB], trim_offset[CELT_NB];   // allocation
     int16_t X[2 * 960];
     int32_t freq[960];
@@ -846,35 +844,52 @@ DFN uint32_t pvq_u(int n, int k)
 DFN uint32_t pvq_v(int n, int k) { return pvq_u(n, k) + pvq_u(n, k + 1); }
 DFN uint32_t pvq_row(int r, int c) { return T_celt_pvq_u_data[T_celt_pvq_u_row[r] + c]; }
 
-// celt/cwrs.c cwrsi: combinatorial index -> pulse vector; returns sum of squares
+// celt/cwrs.c cwrsi: combinatorial index -> pulse vector; returns sum of squares.
+// With fewer pulses than positions most positions stay empty, so the two counts
+// that decide the next position are loaded while this one is decided, for the
+// case that it stays empty; with no pulse left (idx is 0 then) zeros follow.
 DNI int32_t cwrsi(int n, int k, uint32_t idx, int32_t *y)
 {
-    uint32_t p;
-    int s, k0;
+    uint32_t p, q;
+    int s, k0, rows = -1;   // rows: the k that row and row1 are for
     int16_t val;
     int32_t yy = 0;
+    const uint32_t *row = T_celt_pvq_u_data, *row1 = row;
+    uint32_t pn = 0, qn = 0;
     ROLLED while (n > 2) {
-        uint32_t q;
         if (k >= n) {
-            p = pvq_row(n, k + 1);
+            const uint32_t *rn = T_celt_pvq_u_data + T_celt_pvq_u_row[n];
+            p = rn[k + 1];
             s = -(idx >= p);
             idx -= p & s;
             k0 = k;
-            q = pvq_row(n, n);
-            if (q > idx) {
+            if (rn[n] > idx) {
                 k = n;
                 ROLLED do p = pvq_row(--k, n);
                 while (p > idx);
             } else {
-                ROLLED for (p = pvq_row(n, k); p > idx; p = pvq_row(n, k)) k--;
+                ROLLED for (p = rn[k]; p > idx; p = rn[k]) k--;
             }
             idx -= p;
             val = (int16_t)((k0 - k + s) ^ s);
             *y++ = val;
             yy = c_mac16(yy, val, val);
         } else {
-            p = pvq_row(k, n);
-            q = pvq_row(k + 1, n);
+            if (k == 0) {
+                ROLLED for (; n > 0; n--) *y++ = 0;
+                return yy;
+            }
+            if (rows != k) {
+                rows = k;
+                row = T_celt_pvq_u_data + T_celt_pvq_u_row[k];
+                row1 = T_celt_pvq_u_data + T_celt_pvq_u_row[k + 1];
+                pn = row[n];
+                qn = row1[n];
+            }
+            p = pn;
+            q = qn;
+            pn = row[n - 1];
+            qn = row1[n - 1];   // not a count when n - 1 == k, and not used then
             if (p <= idx && idx < q) {
                 idx -= p;
                 *y++ = 0;
@@ -908,44 +923,57 @@ DNI int32_t cwrsi(int n, int k, uint32_t idx, int32_t *y)
     return yy;
 }
 
-// celt/vq.c exp_rotation1.  Each pass rotates the pairs (X[i], X[i + stride])
-// in order, and pair i + stride reads the element pair i has just written:
-// the pass is `stride` independent recurrences, one per residue class of i
-// mod stride.  Here each class runs on its own with the element it carries
-// into the next pair kept in a register rather than stored and loaded back
-// (a store-then-load round trip per step); every element gets the same
-// arithmetic as in the serial pass.
-DNI void exp_rotation1(int16_t *X, int len, int stride, int16_t c, int16_t s)
+// celt/vq.c exp_rotation1 on one residue class.  Each pass rotates the pairs
+// (X[i], X[i + stride]) in order, and pair i + stride reads the element pair i
+// has just written: the pass is `stride` independent recurrences, one per
+// residue class r of i mod stride, which the lanes share out.  A class's
+// carried element stays in a register; its other inputs are loaded four
+// ahead.  The coefficients come doubled: the rounded product sums are then the
+// high halves of wrap-around 32-bit sums ((v << 1) >> 16 is (int16_t)(v >> 15)),
+// so a step waits for one multiply-add and one shift.
+DFN void exp_rotation_class(int16_t *X, int len, int stride, int32_t c, int32_t s, int r)
 {
-    const int16_t ms = (int16_t)-s;
-    // forward: i = 0 .. len - stride - 1
-    ROLLED for (int j = 0; j < stride && j < len - stride; j++) {
-        int16_t x1 = X[j];
-        int i = j;
-        ROLLED for (; i < len - stride; i += stride) {
-            int16_t x2 = X[i + stride];
-            X[i] = (int16_t)c_pshr(c_mac16(c_mul16(c, x1), ms, x2), 15);
-            x1 = (int16_t)c_pshr(c_mac16(c_mul16(c, x2), s, x1), 15);   // the new X[i + stride]
+    const int32_t c2 = 2 * c, s2 = 2 * s, rnd = 32768;
+    const int n = (len - r + stride - 1) / stride - 1;   // pairs of the class
+    if (n <= 0) return;
+    int16_t *x = X + r;
+    // forward: pairs 0 .. n - 1
+    int32_t x1 = x[0];
+    ROLLED for (int i = 0; i < n; i += 4) {
+        int32_t v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = x[imin(i + j + 1, n) * stride];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if (i + j < n) {
+                const int32_t x2 = v[j];
+                x[(i + j) * stride] = (int16_t)(wadd(wadd(wmul(c2, x1), rnd), -wmul(s2, x2)) >> 16);
+                x1 = wadd(wadd(wmul(c2, x2), rnd), wmul(s2, x1)) >> 16;
+            }
         }
-        X[i] = x1;
     }
-    // backward: i = len - 2 stride - 1 .. 0; pair i - stride reads the X[i]
-    // pair i has written
-    const int top = len - 2 * stride - 1;
-    ROLLED for (int j = 0; j < stride && top - j >= 0; j++) {
-        int i = top - j;
-        int16_t x2 = X[i + stride];
-        ROLLED for (; i >= 0; i -= stride) {
-            int16_t x1 = X[i];
-            X[i + stride] = (int16_t)c_pshr(c_mac16(c_mul16(c, x2), s, x1), 15);
-            x2 = (int16_t)c_pshr(c_mac16(c_mul16(c, x1), ms, x2), 15);   // the new X[i]
+    x[n * stride] = (int16_t)x1;
+    // backward: pairs n - 2 .. 0 (libopus's second pass starts at len - 2 stride - 1)
+    if (n < 2) return;
+    int32_t x2 = x[(n - 1) * stride];
+    ROLLED for (int i = n - 2; i >= 0; i -= 4) {
+        int32_t v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = x[imax(i - j, 0) * stride];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if (i - j >= 0) {
+                const int32_t w = v[j];
+                x[(i - j + 1) * stride] = (int16_t)(wadd(wadd(wmul(c2, x2), rnd), wmul(s2, w)) >> 16);
+                x2 = wadd(wadd(wmul(c2, w), rnd), -wmul(s2, x2)) >> 16;
+            }
         }
-        X[i + stride] = x2;
     }
+    x[0] = (int16_t)x2;
 }
 
 // celt/vq.c exp_rotation, dir = -1 (decoder)
-DNI void exp_rotation_dec(int16_t *X, int len, int stride, int K, int spread)
+DNI void exp_rotation_dec(Lanes L, int16_t *X, int len, int stride, int K, int spread)
 {
     if (2 * K >= len || spread == SPREAD_NONE) return;
     int factor = spread == 1 ? 15 : spread == 2 ? 10 : 5;   // SPREAD_FACTOR[spread - 1] = {15, 10, 5}
@@ -959,10 +987,15 @@ DNI void exp_rotation_dec(int16_t *X, int len, int stride, int K, int spread)
         ROLLED while ((stride2 * stride2 + stride2) * stride + (stride >> 2) < len) stride2++;
     }
     len = (int)((unsigned)len / (unsigned)stride);
-    ROLLED for (int i = 0; i < stride; i++) {
-        if (stride2) exp_rotation1(X + i * len, len, stride2, s, c);
-        exp_rotation1(X + i * len, len, 1, c, s);
+    if (stride2) {
+        LFOR(L, q, 0, stride * stride2) {
+            const int i = q / stride2;
+            exp_rotation_class(X + i * len, len, stride2, s, c, q - i * stride2);
+        }
+        lsync(L);
     }
+    LFOR(L, i, 0, stride) exp_rotation_class(X + i * len, len, 1, c, s, 0);
+    lsync(L);
 }
 
 // celt/vq.c renormalise_vector
@@ -982,32 +1015,32 @@ DNI void renormalise_vector(Lanes L, int16_t *X, int N, int16_t gain)
     PHASE_END(PH_PVQ_RENORM, t_rn, L.id);
 }
 
-// celt/vq.c alg_unquant
-DNI unsigned alg_unquant(Lanes L, int16_t *X, int N, int K, int spread, int B, RangeDec *dec, int16_t gain,
+// celt/vq.c alg_unquant.  Every lane decodes the codeword (same index, same
+// pulses) and the lanes share out the vector work.
+DFN unsigned alg_unquant(const Lanes &L, int16_t *X, int N, int K, int spread, int B, RangeDec *dec, int16_t gain,
                          int32_t *iy)
 {
     PHASE_BEGIN(t_cw);
-    int32_t Ryy = cwrsi(N, K, rd_uint(dec, pvq_v(N, K)), iy);
+    const uint32_t idx = rdi_uint(dec, pvq_v(N, K));
+    lsync(L);   // every lane is done with the last partition's pulses
+    int32_t Ryy = cwrsi(N, K, idx, iy);
     PHASE_END(PH_PVQ_CWRSI, t_cw, L.id);
     // normalise_residual (every element on its own)
     int k = c_ilog2(Ryy) >> 1;
     int32_t t = c_vshr(Ryy, 2 * (k - 7));
     int16_t g = (int16_t)c_mul16_p15(c_rsqrt_norm(t), gain);
+    lsync(L);
     LFOR(L, i, 0, N) X[i] = (int16_t)c_pshr(c_mul16(g, iy[i]), k + 1);
     lsync(L);
     PHASE_BEGIN(t_rt);
-    exp_rotation_dec(X, N, B, K, spread);
+    exp_rotation_dec(L, X, N, B, K, spread);
     PHASE_END(PH_PVQ_ROT, t_rt, L.id);
     // extract_collapse_mask
     if (B <= 1) return 1;
-    int N0 = (int)((unsigned)N / (unsigned)B);
+    const int N0 = (int)((unsigned)N / (unsigned)B);
     unsigned mask = 0;
-    ROLLED for (int i = 0; i < B; i++) {
-        unsigned tmp = 0;
-        ROLLED for (int j = 0; j < N0; j++) tmp |= iy[i * N0 + j];
-        mask |= (tmp != 0) << i;
-    }
-    return mask;
+    LFOR(L, i, 0, N) if (iy[i]) mask |= 1u << (i / N0);
+    return lor(L, mask);
 }
 
 // ------------------------------------------------------------------ bands
@@ -1029,57 +1062,50 @@ DFN int bitexact_log2tan(int isin, int icos)
            c_frac_mul16(icos, c_frac_mul16(icos, -2597) + 7932);
 }
 
-DNI void haar1(int16_t *X, int N0, int stride)
+// In place over independent pairs: the lanes split them.
+DFN void haar1(const Lanes &L, int16_t *X, int N0, int stride)
 {
-    N0 >>= 1;
-    ROLLED for (int i = 0; i < stride; i++)
-        ROLLED for (int j = 0; j < N0; j++) {
-            int32_t t1 = c_mul16(23170, X[stride * 2 * j + i]);
-            int32_t t2 = c_mul16(23170, X[stride * (2 * j + 1) + i]);
-            X[stride * 2 * j + i] = (int16_t)c_pshr(wadd(t1, t2), 15);
-            X[stride * (2 * j + 1) + i] = (int16_t)c_pshr(wsub(t1, t2), 15);
-        }
-}
-
-DNI void deinterleave_hadamard(int16_t *X, int N0, int stride, int hadamard, int16_t *tmp)
-{
-    int N = N0 * stride;
-    if (hadamard) {
-        const int32_t *ordery = T_celt_ordery_table + stride - 2;
-        ROLLED for (int i = 0; i < stride; i++)
-            ROLLED for (int j = 0; j < N0; j++) tmp[ordery[i] * N0 + j] = X[j * stride + i];
-    } else {
-        ROLLED for (int i = 0; i < stride; i++)
-            ROLLED for (int j = 0; j < N0; j++) tmp[i * N0 + j] = X[j * stride + i];
+    LFOR(L, q, 0, (N0 >> 1) * stride) {
+        const int j = q / stride, i = q - j * stride;
+        int16_t *x = X + stride * 2 * j + i;
+        int32_t t1 = c_mul16(23170, x[0]);
+        int32_t t2 = c_mul16(23170, x[stride]);
+        x[0] = (int16_t)c_pshr(wadd(t1, t2), 15);
+        x[stride] = (int16_t)c_pshr(wsub(t1, t2), 15);
     }
-    ROLLED for (int i = 0; i < N; i++) X[i] = tmp[i];
+    lsync(L);
 }
 
-DNI void interleave_hadamard(int16_t *X, int N0, int stride, int hadamard, int16_t *tmp)
+// celt/bands.c deinterleave_hadamard (to = 1) and interleave_hadamard (to = 0)
+DNI void hadamard_order(Lanes L, int16_t *X, int N0, int stride, int hadamard, int to, int16_t *tmp)
 {
-    int N = N0 * stride;
-    if (hadamard) {
-        const int32_t *ordery = T_celt_ordery_table + stride - 2;
-        ROLLED for (int i = 0; i < stride; i++)
-            ROLLED for (int j = 0; j < N0; j++) tmp[j * stride + i] = X[ordery[i] * N0 + j];
-    } else {
-        ROLLED for (int i = 0; i < stride; i++)
-            ROLLED for (int j = 0; j < N0; j++) tmp[j * stride + i] = X[i * N0 + j];
+    const int32_t *ordery = T_celt_ordery_table + stride - 2;
+    const int N = N0 * stride;
+    LFOR(L, q, 0, N) {
+        const int j = q / stride, i = q - j * stride;       // element i of group j, interleaved at q
+        const int at = (hadamard ? ordery[i] : i) * N0 + j;   // its place with the blocks apart
+        tmp[to ? at : q] = X[to ? q : at];
     }
-    ROLLED for (int i = 0; i < N; i++) X[i] = tmp[i];
+    lsync(L);
+    LFOR(L, i, 0, N) X[i] = tmp[i];
+    lsync(L);
 }
 
+// Band decoding runs on every lane of the group: each lane holds the range
+// decoder and the bit budget in its registers and decodes the same symbols,
+// and the lanes share out the work on the band vectors.  (On the first lane
+// alone, with the decoder's state in memory, a full-band mono 20 ms frame of
+// 250 bytes took 530 k cycles, BANDS_MEASURED.)
 struct BandCtx {
     Lanes L;
+    RangeDec d;
     int i;
     int intensity;
     int spread;
     int tf_change;
-    RangeDec *ec;
     int32_t remaining_bits;
     uint32_t seed;
     int disable_inv;
-    int avoid_split_noise;
     CeltScratch *w;
 };
 
@@ -1109,249 +1135,253 @@ DFN int compute_qn(int N, int b, int offset, int pulse_cap, int stereo)
 }
 
 // celt/bands.c compute_theta (decoder side)
-DNI void compute_theta(BandCtx *ctx, SplitCtx *sctx, int N, int *b, int B, int B0, int LM, int stereo, int *fill)
+DFN void compute_theta(BandCtx &ctx, SplitCtx &sctx, int N, int &b, int B, int B0, int LM, int stereo, int &fill)
 {
     int itheta = 0, delta, imid, iside, inv = 0;
-    RangeDec *ec = ctx->ec;
-    int i = ctx->i;
+    RangeDec *ec = &ctx.d;
+    int i = ctx.i;
     int pulse_cap = T_celt_logN[i] + LM * (1 << 3);
     int offset = (pulse_cap >> 1) - (stereo && N == 2 ? 16 : 4);
-    int qn = compute_qn(N, *b, offset, pulse_cap, stereo);
-    if (stereo && i >= ctx->intensity) qn = 1;
+    int qn = compute_qn(N, b, offset, pulse_cap, stereo);
+    if (stereo && i >= ctx.intensity) qn = 1;
     int32_t tell = (int32_t)rd_tell_frac(ec);
     if (qn != 1) {
-        if (stereo && N > 2) {
-            int p0 = 3, x0 = qn / 2, ft = p0 * (x0 + 1) + x0, x;
-            int fs = (int)rd_decode(ec, ft);
-            if (fs < (x0 + 1) * p0) x = fs / p0;
-            else x = x0 + 1 + (fs - (x0 + 1) * p0);
-            rd_update(ec, x <= x0 ? p0 * x : (x - 1 - x0) + (x0 + 1) * p0,
-                      x <= x0 ? p0 * (x + 1) : (x - x0) + (x0 + 1) * p0, ft);
-            itheta = x;
-        } else if (B0 > 1 || stereo) {
-            itheta = (int)rd_uint(ec, qn + 1);
+        // the three models of the angle: a step, uniform, a triangle; each is
+        // one decode of a total and one update with the range it falls in
+        const int step = stereo && N > 2, uniform = !step && (B0 > 1 || stereo);
+        const int x0 = qn / 2, half = qn >> 1;
+        if (uniform && qn + 1 > 256) {   // more than eight bits: part of them raw
+            itheta = (int)rdi_uint(ec, qn + 1);
         } else {
-            int fs = 1, fl = 0, ft = ((qn >> 1) + 1) * ((qn >> 1) + 1);
-            int fm = (int)rd_decode(ec, ft);
-            if (fm < ((qn >> 1) * ((qn >> 1) + 1) >> 1)) {
-                itheta = (int)(c_isqrt32(8 * (uint32_t)fm + 1) - 1) >> 1;
-                fs = itheta + 1;
-                fl = itheta * (itheta + 1) >> 1;
+            const unsigned ft = step ? (unsigned)(3 * (x0 + 1) + x0) : uniform ? (unsigned)(qn + 1)
+                                                                               : (unsigned)((half + 1) * (half + 1));
+            const int fm = (int)rdi_decode(ec, ft);
+            unsigned fl, fh;
+            if (step) {
+                const int p0 = 3;
+                itheta = fm < (x0 + 1) * p0 ? fm / p0 : x0 + 1 + (fm - (x0 + 1) * p0);
+                fl = itheta <= x0 ? p0 * itheta : (itheta - 1 - x0) + (x0 + 1) * p0;
+                fh = itheta <= x0 ? p0 * (itheta + 1) : (itheta - x0) + (x0 + 1) * p0;
+            } else if (uniform) {
+                itheta = fm;
+                fl = fm;
+                fh = fm + 1;
             } else {
-                itheta = (2 * (qn + 1) - (int)c_isqrt32(8 * (uint32_t)(ft - fm - 1) + 1)) >> 1;
-                fs = qn + 1 - itheta;
-                fl = ft - ((qn + 1 - itheta) * (qn + 2 - itheta) >> 1);
+                const int low = fm < (half * (half + 1) >> 1);
+                const int root = (int)c_isqrt32(8 * (uint32_t)(low ? fm : (int)ft - fm - 1) + 1);
+                int fs;
+                if (low) {
+                    itheta = (root - 1) >> 1;
+                    fs = itheta + 1;
+                    fl = itheta * (itheta + 1) >> 1;
+                } else {
+                    itheta = (2 * (qn + 1) - root) >> 1;
+                    fs = qn + 1 - itheta;
+                    fl = ft - ((qn + 1 - itheta) * (qn + 2 - itheta) >> 1);
+                }
+                fh = fl + fs;
             }
-            rd_update(ec, fl, fl + fs, ft);
+            rdi_update(ec, fl, fh, ft);
         }
         itheta = (int)((uint32_t)((int32_t)itheta * 16384) / (uint32_t)qn);
     } else if (stereo) {
-        if (*b > 2 << 3 && ctx->remaining_bits > 2 << 3) inv = rd_bit_logp(ec, 2);
+        if (b > 2 << 3 && ctx.remaining_bits > 2 << 3) inv = rdi_bit_logp(ec, 2);
         else inv = 0;
-        if (ctx->disable_inv) inv = 0;
+        if (ctx.disable_inv) inv = 0;
         itheta = 0;
     }
     int qalloc = (int)rd_tell_frac(ec) - tell;
-    *b -= qalloc;
+    b -= qalloc;
     if (itheta == 0) {
         imid = 32767; iside = 0;
-        *fill &= (1 << B) - 1;
+        fill &= (1 << B) - 1;
         delta = -16384;
     } else if (itheta == 16384) {
         imid = 0; iside = 32767;
-        *fill &= ((1 << B) - 1) << B;
+        fill &= ((1 << B) - 1) << B;
         delta = 16384;
     } else {
         imid = bitexact_cos((int16_t)itheta);
         iside = bitexact_cos((int16_t)(16384 - itheta));
         delta = c_frac_mul16((N - 1) << 7, bitexact_log2tan(iside, imid));
     }
-    sctx->inv = inv; sctx->imid = imid; sctx->iside = iside;
-    sctx->delta = delta; sctx->itheta = itheta; sctx->qalloc = qalloc;
+    sctx.inv = inv; sctx.imid = imid; sctx.iside = iside;
+    sctx.delta = delta; sctx.itheta = itheta; sctx.qalloc = qalloc;
 }
 
-DNI unsigned quant_band_n1(BandCtx *ctx, int16_t *X, int16_t *Y, int16_t *lowband_out)
+// Ends with a barrier: the group's lanes may read X, Y and lowband_out.
+DFN unsigned quant_band_n1(BandCtx &ctx, int16_t *X, int16_t *Y, int16_t *lowband_out)
 {
-    int16_t *x = X;
-    int stereo = Y != 0;
-    ROLLED for (int c = 0; c < 1 + stereo; c++) {
-        int sign = 0;
-        if (ctx->remaining_bits >= 1 << 3) {
-            sign = (int)rd_bits(ctx->ec, 1);
-            ctx->remaining_bits -= 1 << 3;
+    int sign[2] = {0, 0};
+    ROLLED for (int c = 0; c < 1 + (Y != 0); c++) {
+        if (ctx.remaining_bits >= 1 << 3) {
+            const int v = (int)rdi_bits(&ctx.d, 1);
+            if (c) sign[1] = v;
+            else sign[0] = v;
+            ctx.remaining_bits -= 1 << 3;
         }
-        x[0] = sign ? -16384 : 16384;
-        x = Y;
     }
-    if (lowband_out) lowband_out[0] = (int16_t)(X[0] >> 4);
+    lead(ctx.L, [&]() CUO_INLINE {
+        X[0] = sign[0] ? -16384 : 16384;
+        if (Y) Y[0] = sign[1] ? -16384 : 16384;
+        if (lowband_out) lowband_out[0] = (int16_t)(X[0] >> 4);
+    });
     return 1;
+}
+
+// celt/bands.c celt_lcg_rand k steps on: the seed as an affine map of the seed
+// now (x -> A^k x + B_k mod 2^32), by binary powers.
+DFN uint32_t lcg_jump(uint32_t seed, unsigned k)
+{
+    uint32_t a = 1664525u, c = 1013904223u;
+    ROLLED for (; k; k >>= 1) {
+        if (k & 1) seed = a * seed + c;
+        c = a * c + c;
+        a = a * a;
+    }
+    return seed;
 }
 
 // celt/bands.c quant_partition, leaf: pulses for the band piece (PVQ) or,
 // with none, folding / noise fill.
-DNI unsigned quant_partition_leaf(BandCtx *ctx, int16_t *X, int N, int b, int B, int16_t *lowband, int LM,
+DFN unsigned quant_partition_leaf(BandCtx &ctx, int16_t *X, int N, int b, int B, int16_t *lowband, int LM,
                                   int16_t gain, int fill)
 {
-    const int i = ctx->i;
+    const int i = ctx.i;
     unsigned cm = 0;
     int q = bits2pulses(i, LM, b);
     int curr_bits = pulses2bits(i, LM, q);
-    ctx->remaining_bits -= curr_bits;
-    ROLLED while (ctx->remaining_bits < 0 && q > 0) {
-        ctx->remaining_bits += curr_bits;
+    ctx.remaining_bits -= curr_bits;
+    ROLLED while (ctx.remaining_bits < 0 && q > 0) {
+        ctx.remaining_bits += curr_bits;
         q--;
         curr_bits = pulses2bits(i, LM, q);
-        ctx->remaining_bits -= curr_bits;
+        ctx.remaining_bits -= curr_bits;
     }
     if (q != 0) {
         int K = get_pulses(q);
-        cm = alg_unquant(ctx->L, X, N, K, ctx->spread, B, ctx->ec, gain, ctx->w->iy);
+        cm = alg_unquant(ctx.L, X, N, K, ctx.spread, B, &ctx.d, gain, ctx.w->iy);
     } else {
         unsigned cm_mask = (unsigned)(1UL << B) - 1;
         fill &= cm_mask;
         if (!fill) {
-            ROLLED for (int j = 0; j < N; j++) X[j] = 0;
+            LFOR(ctx.L, j, 0, N) X[j] = 0;
+            lsync(ctx.L);
         } else {
-            if (lowband == 0) {
-                ROLLED for (int j = 0; j < N; j++) {
-                    ctx->seed = c_lcg_rand(ctx->seed);
-                    X[j] = (int16_t)((int32_t)ctx->seed >> 20);
-                }
-                cm = cm_mask;
-            } else {
-                ROLLED for (int j = 0; j < N; j++) {
-                    ctx->seed = c_lcg_rand(ctx->seed);
-                    int16_t tmp = (ctx->seed & 0x8000) ? 4 : -4;   // QCONST16(1.0f/256, 10)
+            // sample j takes the seed j + 1 steps on: a lane jumps to its first
+            // sample's seed and from one of its samples to the next
+            uint32_t seed = lcg_jump(ctx.seed, ctx.L.id + 1);
+            const uint32_t c = lcg_jump(0, ctx.L.n), a = lcg_jump(1, ctx.L.n) - c;
+            ROLLED for (int j = ctx.L.id; j < N; j += ctx.L.n) {
+                if (lowband == 0) {
+                    X[j] = (int16_t)((int32_t)seed >> 20);
+                } else {
+                    int16_t tmp = (seed & 0x8000) ? 4 : -4;   // QCONST16(1.0f/256, 10)
                     X[j] = (int16_t)(lowband[j] + tmp);
                 }
-                cm = fill;
+                seed = a * seed + c;
             }
-            renormalise_vector(ctx->L, X, N, gain);
+            ctx.seed = lcg_jump(ctx.seed, N);
+            cm = lowband == 0 ? cm_mask : fill;
+            lsync(ctx.L);
+            renormalise_vector(ctx.L, X, N, gain);
         }
     }
     return cm;
 }
 
 // celt/bands.c quant_partition.  libopus recurses into the two halves of a
-// split band; here one loop walks an explicit stack of frames instead, so a
-// single copy of the code serves every depth (the split depth is bounded by
-// LM + 1 <= 4, five frames).  A frame resumes after each half: stage 1 / 2
-// when the mid half went first, 3 / 4 when the side half did; the bit
-// rebalancing between the halves and the collapse-mask combination happen at
-// those points, in libopus's order.
-DNI unsigned quant_partition(BandCtx *ctx, int16_t *X, int N, int b, int B, int16_t *lowband, int LM,
+// split band; here one loop walks down to a leaf and back up, so a single copy
+// of the code serves every depth (the split depth is bounded by LM + 1 <= 4).
+// What the second half of a split needs is kept in the group's memory, written
+// once when the band splits; the collapse mask of the first half (8 bits per
+// depth) and which halves are done are registers.  The bit rebalancing between
+// the halves and the collapse-mask combination happen in libopus's order.
+DFN unsigned quant_partition(BandCtx &ctx, int16_t *X, int N, int b, int B, int16_t *lowband, int LM,
                              int16_t gain, int fill)
 {
-    QPFrame *st = ctx->w->qp;
-    int sp = 0;
-    st[0].X = X;
-    st[0].N = N;
-    st[0].b = b;
-    st[0].B = B;
-    st[0].lowband = lowband;
-    st[0].LM = LM;
-    st[0].gain = gain;
-    st[0].fill = fill;
-    st[0].stage = 0;
-    unsigned ret = 0;
-    const int i = ctx->i;
-    ROLLED while (sp >= 0) {
-        QPFrame *f = &st[sp];
-        QPFrame *c = &st[sp + 1 < 5 ? sp + 1 : 4];
-        if (f->stage == 0) {
-            const uint8_t *cache = T_celt_cache_bits + T_celt_cache_index[(f->LM + 1) * CELT_NB + i];
-            if (f->LM != -1 && f->b > cache[cache[0]] + 12 && f->N > 2 && sp < 4) {
-                SplitCtx sctx;
-                int B0 = f->B;
-                int N2 = f->N >> 1;
-                int fill2 = f->fill;
-                if (f->B == 1) fill2 = (fill2 & 1) | (fill2 << 1);
-                int B2 = (f->B + 1) >> 1;
-                int LM2 = f->LM - 1;
-                int b2 = f->b;
-                PHASE_BEGIN(t_th);
-                compute_theta(ctx, &sctx, N2, &b2, B2, B0, LM2, 0, &fill2);
-                PHASE_END(PH_PVQ_THETA, t_th, ctx->L.id);
-                int delta = sctx.delta, itheta = sctx.itheta;
-                if (B0 > 1 && (itheta & 0x3fff)) {
-                    if (itheta > 8192) delta -= delta >> (4 - LM2);
-                    else delta = imin(0, delta + (N2 << 3 >> (5 - LM2)));
-                }
-                int mbits = imax(0, imin(b2, (b2 - delta) / 2));
-                int sbits = b2 - mbits;
-                ctx->remaining_bits -= sctx.qalloc;
-                f->Y = f->X + N2;
-                f->N = N2;
-                f->B = B2;
-                f->B0 = B0;
-                f->LM = LM2;
-                f->fill = fill2;
-                f->mid = (int16_t)sctx.imid;
-                f->side = (int16_t)sctx.iside;
-                f->itheta = itheta;
-                f->mbits = mbits;
-                f->sbits = sbits;
-                f->next_lowband2 = f->lowband ? f->lowband + N2 : 0;
-                f->rebalance = ctx->remaining_bits;
-                c->stage = 0;
-                c->N = N2;
-                c->B = B2;
-                c->LM = LM2;
-                if (mbits >= sbits) {
-                    f->stage = 1;
-                    c->X = f->X;
-                    c->b = mbits;
-                    c->lowband = f->lowband;
-                    c->gain = (int16_t)c_mul16_p15(f->gain, f->mid);
-                    c->fill = fill2;
-                } else {
-                    f->stage = 3;
-                    c->X = f->Y;
-                    c->b = sbits;
-                    c->lowband = f->next_lowband2;
-                    c->gain = (int16_t)c_mul16_p15(f->gain, f->side);
-                    c->fill = fill2 >> B2;
-                }
-                sp++;
-                continue;
+    QPSplit *st = ctx.w->qp;
+    const Lanes &L = ctx.L;
+    const int i = ctx.i;
+    int sp = 0;                          // splits above the current piece
+    unsigned second = 0, cms = 0;        // bit d: split d is in its second half; byte d: first half's mask
+    ROLLED while (1) {
+        // down: split while the piece has more bits than one codeword takes
+        const uint8_t *cache = pulse_cache(i, LM);
+        if (LM != -1 && b > cache[cache[0]] + 12 && N > 2 && sp < 4) {
+            SplitCtx sctx;
+            const int B0 = B, n2 = N >> 1, parent_gain = gain;
+            N = n2;
+            if (B == 1) fill = (fill & 1) | (fill << 1);
+            B = (B + 1) >> 1;
+            LM--;
+            PHASE_BEGIN(t_th);
+            compute_theta(ctx, sctx, N, b, B, B0, LM, 0, fill);
+            PHASE_END(PH_PVQ_THETA, t_th, L.id);
+            int delta = sctx.delta;
+            const int itheta = sctx.itheta;
+            if (B0 > 1 && (itheta & 0x3fff)) {
+                if (itheta > 8192) delta -= delta >> (4 - LM);
+                else delta = imin(0, delta + (N << 3 >> (5 - LM)));
             }
-            ret = quant_partition_leaf(ctx, f->X, f->N, f->b, f->B, f->lowband, f->LM, f->gain, f->fill);
-            sp--;
-            continue;
-        }
-        if (f->stage == 1 || f->stage == 3) {
-            c->stage = 0;
-            c->N = f->N;
-            c->B = f->B;
-            c->LM = f->LM;
-            if (f->stage == 1) {            // mid half done: rebalance, then the side half
-                f->cm = ret;
-                int32_t rebalance = f->mbits - (f->rebalance - ctx->remaining_bits);
-                if (rebalance > 3 << 3 && f->itheta != 0) f->sbits += rebalance - (3 << 3);
-                c->X = f->Y;
-                c->b = f->sbits;
-                c->lowband = f->next_lowband2;
-                c->gain = (int16_t)c_mul16_p15(f->gain, f->side);
-                c->fill = f->fill >> f->B;
-                f->stage = 2;
-            } else {                        // side half done: rebalance, then the mid half
-                f->cm = ret << (f->B0 >> 1);
-                int32_t rebalance = f->sbits - (f->rebalance - ctx->remaining_bits);
-                if (rebalance > 3 << 3 && f->itheta != 16384) f->mbits += rebalance - (3 << 3);
-                c->X = f->X;
-                c->b = f->mbits;
-                c->lowband = f->lowband;
-                c->gain = (int16_t)c_mul16_p15(f->gain, f->mid);
-                c->fill = f->fill;
-                f->stage = 4;
+            const int mbits = imax(0, imin(b, (b - delta) / 2));
+            const int sbits = b - mbits;
+            ctx.remaining_bits -= sctx.qalloc;
+            const int mid_first = mbits >= sbits;
+            const int16_t gmid = (int16_t)c_mul16_p15(parent_gain, (int16_t)sctx.imid);
+            const int16_t gside = (int16_t)c_mul16_p15(parent_gain, (int16_t)sctx.iside);
+            int16_t *const Y = X + N, *const lowband2 = lowband ? lowband + N : 0;
+            QPSplit *f = &st[sp];
+            lsync(L);   // every lane has read what an earlier split left here
+            f->X = mid_first ? Y : X;
+            f->lowband = mid_first ? lowband2 : lowband;
+            f->bits = mid_first ? sbits : mbits;
+            f->first_bits = mid_first ? mbits : sbits;
+            f->rebalance = ctx.remaining_bits;
+            f->N = N;
+            f->B = B;
+            f->B0 = B0;
+            f->LM = LM;
+            f->fill = mid_first ? fill >> B : fill;
+            f->gain = mid_first ? gside : gmid;
+            f->mid_first = mid_first;
+            // no rebalancing towards a half that gets no energy
+            f->fixed = mid_first ? itheta == 0 : itheta == 16384;
+            lsync(L);
+            if (!mid_first) {
+                X = Y;
+                lowband = lowband2;
+                fill >>= B;
             }
+            b = mid_first ? mbits : sbits;
+            gain = mid_first ? gmid : gside;
+            second &= ~(1u << sp);
             sp++;
             continue;
         }
-        ret = f->stage == 2 ? f->cm | (ret << (f->B0 >> 1)) : f->cm | ret;
-        sp--;
+        unsigned cm = quant_partition_leaf(ctx, X, N, b, B, lowband, LM, gain, fill);
+        // up: to the nearest split whose second half is still to come
+        ROLLED while (sp > 0 && (second >> (sp - 1) & 1)) {
+            sp--;
+            const unsigned first = cms >> (8 * sp) & 0xff;
+            const int shift = st[sp].B0 >> 1;
+            cm = st[sp].mid_first ? first | cm << shift : first << shift | cm;
+        }
+        if (sp == 0) return cm;
+        const QPSplit *f = &st[sp - 1];
+        X = f->X;
+        lowband = f->lowband;
+        N = f->N;
+        B = f->B;
+        LM = f->LM;
+        fill = f->fill;
+        gain = f->gain;
+        b = f->bits;
+        const int32_t rebalance = f->first_bits - (f->rebalance - ctx.remaining_bits);
+        if (rebalance > 3 << 3 && !f->fixed) b += rebalance - (3 << 3);
+        cms = (cms & ~(0xffu << (8 * (sp - 1)))) | (cm & 0xff) << (8 * (sp - 1));
+        second |= 1u << (sp - 1);
     }
-    return ret;
 }
 
 // bit_interleave_table / bit_deinterleave_table of celt/bands.c quant_band
@@ -1359,32 +1389,34 @@ TABC(uint8_t, T_bit_interleave[16]) = {0, 1, 1, 1, 2, 3, 3, 3, 2, 3, 3, 3, 2, 3,
 TABC(uint8_t, T_bit_deinterleave[16]) = {0x00, 0x03, 0x0C, 0x0F, 0x30, 0x33, 0x3C, 0x3F,
                                          0xC0, 0xC3, 0xCC, 0xCF, 0xF0, 0xF3, 0xFC, 0xFF};
 
-// celt/bands.c quant_band (decoder, resynth always on)
-DNI unsigned quant_band(BandCtx *ctx, int16_t *X, int N, int b, int B, int16_t *lowband, int LM,
+// celt/bands.c quant_band (decoder, resynth always on).  Ends with a barrier.
+DFN unsigned quant_band(BandCtx &ctx, int16_t *X, int N, int b, int B, int16_t *lowband, int LM,
                         int16_t *lowband_out, int16_t gain, int16_t *lowband_scratch, int fill)
 {
+    const Lanes &L = ctx.L;
     const uint8_t *bit_interleave_table = T_bit_interleave;
     const uint8_t *bit_deinterleave_table = T_bit_deinterleave;
     int N0 = N, N_B = N, N_B0, B0 = B, time_divide = 0, recombine = 0;
     int longBlocks = B0 == 1;
     unsigned cm = 0;
-    int tf_change = ctx->tf_change;
+    int tf_change = ctx.tf_change;
     N_B = (int)((unsigned)N_B / (unsigned)B);
     if (N == 1) return quant_band_n1(ctx, X, 0, lowband_out);
     if (tf_change > 0) recombine = tf_change;
     PHASE_BEGIN(t_tf);
     if (lowband_scratch && lowband && (recombine || ((N_B & 1) == 0 && tf_change < 0) || B0 > 1)) {
-        ROLLED for (int j = 0; j < N; j++) lowband_scratch[j] = lowband[j];
+        LFOR(L, j, 0, N) lowband_scratch[j] = lowband[j];
+        lsync(L);
         lowband = lowband_scratch;
     }
     ROLLED for (int k = 0; k < recombine; k++) {
-        if (lowband) haar1(lowband, N >> k, 1 << k);
+        if (lowband) haar1(L, lowband, N >> k, 1 << k);
         fill = bit_interleave_table[fill & 0xF] | bit_interleave_table[fill >> 4] << 2;
     }
     B >>= recombine;
     N_B <<= recombine;
     ROLLED while ((N_B & 1) == 0 && tf_change < 0) {
-        if (lowband) haar1(lowband, N_B, B);
+        if (lowband) haar1(L, lowband, N_B, B);
         fill |= fill << B;
         B <<= 1;
         N_B >>= 1;
@@ -1394,28 +1426,29 @@ DNI unsigned quant_band(BandCtx *ctx, int16_t *X, int N, int b, int B, int16_t *
     B0 = B;
     N_B0 = N_B;
     if (B0 > 1 && lowband)
-        deinterleave_hadamard(lowband, N_B >> recombine, B0 << recombine, longBlocks, ctx->w->tmp);
-    PHASE_END(PH_PVQ_TF, t_tf, ctx->L.id);
+        hadamard_order(L, lowband, N_B >> recombine, B0 << recombine, longBlocks, 1, ctx.w->tmp);
+    PHASE_END(PH_PVQ_TF, t_tf, L.id);
     cm = quant_partition(ctx, X, N, b, B, lowband, LM, gain, fill);
     PHASE_BEGIN(t_tf2);
-    if (B0 > 1) interleave_hadamard(X, N_B >> recombine, B0 << recombine, longBlocks, ctx->w->tmp);
+    if (B0 > 1) hadamard_order(L, X, N_B >> recombine, B0 << recombine, longBlocks, 0, ctx.w->tmp);
     N_B = N_B0;
     B = B0;
     ROLLED for (int k = 0; k < time_divide; k++) {
         B >>= 1;
         N_B <<= 1;
         cm |= cm >> B;
-        haar1(X, N_B, B);
+        haar1(L, X, N_B, B);
     }
     ROLLED for (int k = 0; k < recombine; k++) {
         cm = bit_deinterleave_table[cm];
-        haar1(X, N0 >> k, 1 << k);
+        haar1(L, X, N0 >> k, 1 << k);
     }
-    PHASE_END(PH_PVQ_TF, t_tf2, ctx->L.id);
+    PHASE_END(PH_PVQ_TF, t_tf2, L.id);
     B <<= recombine;
     if (lowband_out) {
         int16_t n = (int16_t)c_sqrt(shl32(N0, 22));
-        ROLLED for (int j = 0; j < N0; j++) lowband_out[j] = (int16_t)c_mul16_q15(n, X[j]);
+        LFOR(L, j, 0, N0) lowband_out[j] = (int16_t)c_mul16_q15(n, X[j]);
+        lsync(L);
     }
     cm &= (1 << B) - 1;
     return cm;
@@ -1457,67 +1490,11 @@ DNI void stereo_merge(Lanes L, int16_t *X, int16_t *Y, int16_t mid, int N)
     lsync(L);
 }
 
-DNI unsigned quant_band_stereo(BandCtx *ctx, int16_t *X, int16_t *Y, int N, int b, int B, int16_t *lowband,
-                               int LM, int16_t *lowband_out, int16_t *lowband_scratch, int fill)
-{
-    unsigned cm = 0;
-    SplitCtx sctx;
-    if (N == 1) return quant_band_n1(ctx, X, Y, lowband_out);
-    int orig_fill = fill;
-    PHASE_BEGIN(t_th);
-    compute_theta(ctx, &sctx, N, &b, B, B, LM, 1, &fill);
-    PHASE_END(PH_PVQ_THETA, t_th, ctx->L.id);
-    int inv = sctx.inv, delta = sctx.delta, itheta = sctx.itheta, qalloc = sctx.qalloc;
-    int16_t mid = (int16_t)sctx.imid, side = (int16_t)sctx.iside;
-    int mbits, sbits;
-    if (N == 2) {
-        int sign = 0;
-        mbits = b;
-        sbits = 0;
-        if (itheta != 0 && itheta != 16384) sbits = 1 << 3;
-        mbits -= sbits;
-        int c = itheta > 8192;
-        ctx->remaining_bits -= qalloc + sbits;
-        int16_t *x2 = c ? Y : X, *y2 = c ? X : Y;
-        if (sbits) sign = (int)rd_bits(ctx->ec, 1);
-        sign = 1 - 2 * sign;
-        cm = quant_band(ctx, x2, N, mbits, B, lowband, LM, lowband_out, 32767, lowband_scratch, orig_fill);
-        y2[0] = (int16_t)(-sign * x2[1]);
-        y2[1] = (int16_t)(sign * x2[0]);
-        X[0] = (int16_t)c_mul16_q15(mid, X[0]);
-        X[1] = (int16_t)c_mul16_q15(mid, X[1]);
-        Y[0] = (int16_t)c_mul16_q15(side, Y[0]);
-        Y[1] = (int16_t)c_mul16_q15(side, Y[1]);
-        int16_t tmp = X[0];
-        X[0] = (int16_t)(tmp - Y[0]);
-        Y[0] = (int16_t)(tmp + Y[0]);
-        tmp = X[1];
-        X[1] = (int16_t)(tmp - Y[1]);
-        Y[1] = (int16_t)(tmp + Y[1]);
-    } else {
-        mbits = imax(0, imin(b, (b - delta) / 2));
-        sbits = b - mbits;
-        ctx->remaining_bits -= qalloc;
-        int32_t rebalance = ctx->remaining_bits;
-        if (mbits >= sbits) {
-            cm = quant_band(ctx, X, N, mbits, B, lowband, LM, lowband_out, 32767, lowband_scratch, fill);
-            rebalance = mbits - (rebalance - ctx->remaining_bits);
-            if (rebalance > 3 << 3 && itheta != 0) sbits += rebalance - (3 << 3);
-            cm |= quant_band(ctx, Y, N, sbits, B, 0, LM, 0, side, 0, fill >> B);
-        } else {
-            cm = quant_band(ctx, Y, N, sbits, B, 0, LM, 0, side, 0, fill >> B);
-            rebalance = sbits - (rebalance - ctx->remaining_bits);
-            if (rebalance > 3 << 3 && itheta != 16384) mbits += rebalance - (3 << 3);
-            cm |= quant_band(ctx, X, N, mbits, B, lowband, LM, lowband_out, 32767, lowband_scratch, fill);
-        }
-    }
-    if (N != 2) stereo_merge(ctx->L, X, Y, mid, N);
-    if (inv)
-        ROLLED for (int j = 0; j < N; j++) Y[j] = (int16_t)-Y[j];
-    return cm;
-}
-
-// celt/bands.c quant_all_bands, decoder path (encode = 0, resynth = 1, no theta RDO)
+// celt/bands.c quant_all_bands, decoder path (encode = 0, resynth = 1, no theta
+// RDO), with quant_band_stereo.  A band takes one pass through quant_band or
+// two: mono, stereo of two samples and a band coded mid only: X; dual stereo: X
+// then Y; mid / side stereo: whichever half has more bits, then the other.
+// One call site serves them all.
 DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *Y_, uint8_t *collapse_masks,
                              const int32_t *pulses, int shortBlocks, int spread, int dual_stereo, int intensity,
                              const int32_t *tf_res, int32_t total_bits, int32_t balance, RangeDec *ec, int LM,
@@ -1533,14 +1510,13 @@ DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *
     int16_t *lowband_scratch = X_ + M * eB[T_CELT_EFFEBANDS - 1];
     int lowband_offset = 0, update_lowband = 1;
     BandCtx ctx;
-    ctx.ec = ec;
+    ctx.L = L;
+    ctx.d = *ec;
     ctx.intensity = intensity;
     ctx.seed = *seed;
     ctx.spread = spread;
     ctx.disable_inv = disable_inv;
-    ctx.avoid_split_noise = B > 1;
     ctx.w = w;
-    ctx.L = L;
     ROLLED for (int i = start; i < end; i++) {
         int effective_lowband = -1;
         unsigned x_cm, y_cm;
@@ -1549,7 +1525,7 @@ DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *
         int16_t *X = X_ + M * eB[i];
         int16_t *Y = Y_ != 0 ? Y_ + M * eB[i] : 0;
         int N = M * eB[i + 1] - M * eB[i];
-        int32_t tell = (int32_t)rd_tell_frac(ec);
+        int32_t tell = (int32_t)rd_tell_frac(&ctx.d);
         if (i != start) balance -= tell;
         int32_t remaining_bits = total_bits - tell - 1;
         ctx.remaining_bits = remaining_bits;
@@ -1566,9 +1542,12 @@ DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *
             // special_hybrid_folding
             int n1 = M * (eB[start + 1] - eB[start]);
             int n2 = M * (eB[start + 2] - eB[start + 1]);
-            ROLLED for (int j = 0; j < n2 - n1; j++) norm[n1 + j] = norm[2 * n1 - n2 + j];
-            if (dual_stereo)
-                ROLLED for (int j = 0; j < n2 - n1; j++) norm2[n1 + j] = norm2[2 * n1 - n2 + j];
+            // the copied range starts where the copy's source ends or later
+            LFOR(L, j, 0, n2 - n1) {
+                norm[n1 + j] = norm[2 * n1 - n2 + j];
+                if (dual_stereo) norm2[n1 + j] = norm2[2 * n1 - n2 + j];
+            }
+            lsync(L);
         }
         int tf_change = tf_res[i];
         ctx.tf_change = tf_change;
@@ -1595,32 +1574,119 @@ DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *
         }
         if (dual_stereo && i == intensity) {
             dual_stereo = 0;
-            ROLLED for (int j = 0; j < M * eB[i] - norm_offset; j++) norm[j] = (int16_t)((norm[j] + norm2[j]) >> 1);
+            lsync(L);
+            LFOR(L, j, 0, M * eB[i] - norm_offset) norm[j] = (int16_t)((norm[j] + norm2[j]) >> 1);
+            lsync(L);
         }
-        if (dual_stereo) {
-            x_cm = quant_band(&ctx, X, N, b / 2, B, effective_lowband != -1 ? norm + effective_lowband : 0, LM,
-                              last ? 0 : norm + M * eB[i] - norm_offset, 32767, lowband_scratch, (int)x_cm);
-            y_cm = quant_band(&ctx, Y, N, b / 2, B, effective_lowband != -1 ? norm2 + effective_lowband : 0, LM,
-                              last ? 0 : norm2 + M * eB[i] - norm_offset, 32767, lowband_scratch, (int)y_cm);
+        int16_t *const lowband = effective_lowband != -1 ? norm + effective_lowband : 0;
+        int16_t *const lowband_out = last ? 0 : norm + M * eB[i] - norm_offset;
+        const int orig_fill = (int)(x_cm | y_cm);
+        if (Y != 0 && !dual_stereo && N == 1) {
+            x_cm = y_cm = quant_band_n1(ctx, X, Y, lowband_out);
         } else {
-            if (Y != 0) {
-                x_cm = quant_band_stereo(&ctx, X, Y, N, b, B,
-                                         effective_lowband != -1 ? norm + effective_lowband : 0, LM,
-                                         last ? 0 : norm + M * eB[i] - norm_offset, lowband_scratch,
-                                         (int)(x_cm | y_cm));
-            } else {
-                x_cm = quant_band(&ctx, X, N, b, B, effective_lowband != -1 ? norm + effective_lowband : 0, LM,
-                                  last ? 0 : norm + M * eB[i] - norm_offset, 32767, lowband_scratch,
-                                  (int)(x_cm | y_cm));
+            // the passes: vector, bits, folding source and target, gain, fill
+            int16_t *px = X, *plow = lowband, *pout = lowband_out, *pscratch = lowband_scratch;
+            int pb = b, pfill = orig_fill, passes = 1, mid_first = 1, second_bits = 0;
+            int16_t pgain = 32767;
+            SplitCtx sctx = {0, 0, 0, 0, 0, 0};
+            int sign = 0, fill = orig_fill;
+            int32_t rebalance = 0;
+            if (dual_stereo) {
+                pb = b / 2;
+                pfill = (int)x_cm;
+                passes = 2;
+            } else if (Y != 0) {
+                int left = b;   // without the angle's bits
+                PHASE_BEGIN(t_th);
+                compute_theta(ctx, sctx, N, left, B, B, LM, 1, fill);
+                PHASE_END(PH_PVQ_THETA, t_th, L.id);
+                if (N == 2) {
+                    int sbits = 0;
+                    if (sctx.itheta != 0 && sctx.itheta != 16384) sbits = 1 << 3;
+                    pb = left - sbits;
+                    ctx.remaining_bits -= sctx.qalloc + sbits;
+                    px = sctx.itheta > 8192 ? Y : X;
+                    if (sbits) sign = (int)rdi_bits(&ctx.d, 1);
+                    sign = 1 - 2 * sign;
+                } else {
+                    const int mbits = imax(0, imin(left, (left - sctx.delta) / 2)), sbits = left - mbits;
+                    ctx.remaining_bits -= sctx.qalloc;
+                    rebalance = ctx.remaining_bits;
+                    passes = 2;
+                    mid_first = mbits >= sbits;
+                    pb = mid_first ? mbits : sbits;
+                    second_bits = mid_first ? sbits : mbits;
+                    pfill = fill;
+                    if (!mid_first) {
+                        px = Y;
+                        plow = pout = pscratch = 0;
+                        pgain = (int16_t)sctx.iside;
+                        pfill = fill >> B;
+                    }
+                }
             }
-            y_cm = x_cm;
+            unsigned cm[2] = {0, 0};
+            ROLLED for (int pass = 0; pass < passes; pass++) {
+                const unsigned m = quant_band(ctx, px, N, pb, B, plow, LM, pout, pgain, pscratch, pfill);
+                if (pass) cm[1] = m;
+                else cm[0] = m;
+                // the second pass
+                const int first_bits = pb;
+                px = dual_stereo || mid_first ? Y : X;
+                if (dual_stereo) {
+                    plow = effective_lowband != -1 ? norm2 + effective_lowband : 0;
+                    pout = last ? 0 : norm2 + M * eB[i] - norm_offset;
+                    pfill = (int)y_cm;
+                } else {
+                    const int32_t gained = first_bits - (rebalance - ctx.remaining_bits);
+                    pb = second_bits;
+                    if (gained > 3 << 3 && sctx.itheta != (mid_first ? 0 : 16384)) pb += gained - (3 << 3);
+                    plow = mid_first ? 0 : lowband;
+                    pout = mid_first ? 0 : lowband_out;
+                    pscratch = mid_first ? 0 : lowband_scratch;
+                    pgain = mid_first ? (int16_t)sctx.iside : (int16_t)32767;
+                    pfill = mid_first ? fill >> B : fill;
+                }
+            }
+            x_cm = cm[0];
+            y_cm = cm[1];
+            if (!dual_stereo) {
+                x_cm = y_cm = cm[0] | cm[1];
+                if (Y != 0) {
+                    const int16_t mid = (int16_t)sctx.imid, side = (int16_t)sctx.iside;
+                    if (N == 2) {
+                        lead(L, [&]() CUO_INLINE {
+                            int16_t *x2 = sctx.itheta > 8192 ? Y : X, *y2 = sctx.itheta > 8192 ? X : Y;
+                            y2[0] = (int16_t)(-sign * x2[1]);
+                            y2[1] = (int16_t)(sign * x2[0]);
+                            X[0] = (int16_t)c_mul16_q15(mid, X[0]);
+                            X[1] = (int16_t)c_mul16_q15(mid, X[1]);
+                            Y[0] = (int16_t)c_mul16_q15(side, Y[0]);
+                            Y[1] = (int16_t)c_mul16_q15(side, Y[1]);
+                            int16_t tmp = X[0];
+                            X[0] = (int16_t)(tmp - Y[0]);
+                            Y[0] = (int16_t)(tmp + Y[0]);
+                            tmp = X[1];
+                            X[1] = (int16_t)(tmp - Y[1]);
+                            Y[1] = (int16_t)(tmp + Y[1]);
+                        });
+                    } else {
+                        stereo_merge(L, X, Y, mid, N);
+                    }
+                    if (sctx.inv) {
+                        LFOR(L, j, 0, N) Y[j] = (int16_t)-Y[j];
+                        lsync(L);
+                    }
+                }
+            }
         }
         collapse_masks[i * C + 0] = (uint8_t)x_cm;
         collapse_masks[i * C + C - 1] = (uint8_t)y_cm;
         balance += pulses[i] + tell;
         update_lowband = b > (N << 3);
-        ctx.avoid_split_noise = 0;
     }
+    lsync(L);
+    *ec = ctx.d;
     *seed = ctx.seed;
     lsync(L);
 }
@@ -2296,15 +2362,13 @@ DNI int celt_decode(Lanes L, CeltDec *st, const uint8_t *data, int len, int16_t 
     ROLLED for (int c = 0; c < CC; c++) lshift_copy(L, st->decode_mem[c], CELT_DEC_BUF - N + CELT_OVERLAP, N);
     PHASE_END(PH_CELT_SHIFT, t_sh, L.id);
     int16_t *X = w->X;
-    // The band shapes: the PVQ split recursion updates its stack, the band
-    // vectors and the folding buffer in place from entropy-decoded values,
-    // so it runs on the first lane as a group of one.
+    // the band shapes
     PHASE_BEGIN(t_qb);
-    lead_rd(L, dec, [&]() CUO_INLINE {
-        quant_all_bands_dec(lone(L), start, end, X, C == 2 ? X + N : 0, w->collapse_masks, pulses, shortBlocks,
+    {
+        quant_all_bands_dec(L, start, end, X, C == 2 ? X + N : 0, w->collapse_masks, pulses, shortBlocks,
                             spread_decision, dual_stereo, intensity, tf_res, len * (8 << 3) - anti_collapse_rsv,
                             balance, dec, LM, codedBands, &st->rng, st->disable_inv, w);
-    });
+    }
     PHASE_END(PH_CELT_BANDS, t_qb, L.id);
     int anti_collapse_on = 0;
     lead_rd(L, dec, [&]() CUO_INLINE {

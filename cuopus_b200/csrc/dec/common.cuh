@@ -60,6 +60,7 @@ namespace cuo {
 struct LaneSim;
 void lanesim_sync(LaneSim *s, int id);
 int32_t lanesim_sum(LaneSim *s, int id, int32_t v);
+uint32_t lanesim_or(LaneSim *s, int id, uint32_t v);
 void lanesim_scan_affine(LaneSim *s, int id, uint32_t *a, uint32_t *b);
 void lanesim_bcast(LaneSim *s, int id, void *p, int bytes);
 #endif
@@ -174,9 +175,24 @@ __device__ void cuo_phase_add(int stage, long long cycles);
 DFN int32_t lsum(const Lanes &L, int32_t v)
 {
 #ifdef __CUDA_ARCH__
+    if (L.n == 32) return __reduce_add_sync(0xffffffffu, v);
     ROLLED for (int off = L.n >> 1; off > 0; off >>= 1) v = (int32_t)((uint32_t)v + (uint32_t)__shfl_xor_sync(L.mask, v, off));
 #elif defined(CUO_LANE_SIM)
     if (L.sim) v = lanesim_sum(L.sim, L.id, v);
+#else
+    (void)L;
+#endif
+    return v;
+}
+
+// Bitwise or of v over the lanes of the group; every lane gets it.
+DFN uint32_t lor(const Lanes &L, uint32_t v)
+{
+#ifdef __CUDA_ARCH__
+    if (L.n == 32) return __reduce_or_sync(0xffffffffu, v);
+    ROLLED for (int off = L.n >> 1; off > 0; off >>= 1) v |= __shfl_xor_sync(L.mask, v, off);
+#elif defined(CUO_LANE_SIM)
+    if (L.sim) v = lanesim_or(L.sim, L.id, v);
 #else
     (void)L;
 #endif

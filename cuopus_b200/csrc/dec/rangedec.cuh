@@ -114,34 +114,37 @@ DNI void rd_init(RangeDec *d, const uint8_t *buf, uint32_t storage)
     rd_normalize(d);
 }
 
-DNI unsigned rd_decode(RangeDec *d, unsigned ft)
+// The symbol functions come twice: inlined (rdi_), for the loops that decode
+// many symbols and keep a copy of the decoder state in registers while they
+// do (a copy whose address goes to no call), and as calls (rd_) that update
+// the state in memory, for everything else.  A symbol took 500-1,000 cycles as
+// a call in a SILK frame's pulses, mostly the state's round trips.
+DFN unsigned rdi_decode(RangeDec *d, unsigned ft)
 {
     d->ext = d->rng / ft;
     unsigned s = d->val / d->ext;
     return ft - (s + 1 < ft ? s + 1 : ft);
 }
+DNI unsigned rd_decode(RangeDec *d, unsigned ft) { return rdi_decode(d, ft); }
 
-DNI unsigned rd_decode_bin(RangeDec *d, unsigned bits)
+DFN unsigned rdi_decode_bin(RangeDec *d, unsigned bits)
 {
     d->ext = d->rng >> bits;
     unsigned s = d->val / d->ext;
     unsigned t = 1u << bits;
     return t - (s + 1u < t ? s + 1u : t);
 }
+DNI unsigned rd_decode_bin(RangeDec *d, unsigned bits) { return rdi_decode_bin(d, bits); }
 
-DNI void rd_update(RangeDec *d, unsigned fl, unsigned fh, unsigned ft)
+DFN void rdi_update(RangeDec *d, unsigned fl, unsigned fh, unsigned ft)
 {
     uint32_t s = d->ext * (ft - fh);
     d->val -= s;
     d->rng = fl > 0 ? d->ext * (fh - fl) : d->rng - s;
     rd_normalize(d);
 }
+DNI void rd_update(RangeDec *d, unsigned fl, unsigned fh, unsigned ft) { rdi_update(d, fl, fh, ft); }
 
-// The symbol functions come twice: inlined (rdi_), for the loops that decode
-// many symbols and keep a copy of the decoder state in registers while they
-// do (a copy whose address goes to no call), and as calls (rd_) that update
-// the state in memory, for everything else.  A symbol took 500-1,000 cycles as
-// a call in a SILK frame's pulses, mostly the state's round trips.
 DFN int rdi_bit_logp(RangeDec *d, unsigned logp)
 {
     uint32_t r = d->rng, v = d->val;
@@ -207,7 +210,7 @@ DFN int rdi_icdf_bit(RangeDec *d, unsigned p)
     return ret;
 }
 
-DNI uint32_t rd_bits(RangeDec *d, unsigned bits)
+DFN uint32_t rdi_bits(RangeDec *d, unsigned bits)
 {
     uint32_t window = d->end_window;
     int available = d->nend_bits;
@@ -225,26 +228,28 @@ DNI uint32_t rd_bits(RangeDec *d, unsigned bits)
     d->nbits_total += bits;
     return ret;
 }
+DNI uint32_t rd_bits(RangeDec *d, unsigned bits) { return rdi_bits(d, bits); }
 
-DNI uint32_t rd_uint(RangeDec *d, uint32_t ft)
+DFN uint32_t rdi_uint(RangeDec *d, uint32_t ft)
 {
     ft--;
     int ftb = ilog(ft);
     if (ftb > 8) {
         ftb -= 8;
         unsigned f = (unsigned)(ft >> ftb) + 1;
-        unsigned s = rd_decode(d, f);
-        rd_update(d, s, s + 1, f);
-        uint32_t t = (uint32_t)s << ftb | rd_bits(d, ftb);
+        unsigned s = rdi_decode(d, f);
+        rdi_update(d, s, s + 1, f);
+        uint32_t t = (uint32_t)s << ftb | rdi_bits(d, ftb);
         if (t <= ft) return t;
         d->error = 1;
         return ft;
     }
     ft++;
-    unsigned s = rd_decode(d, (unsigned)ft);
-    rd_update(d, s, s + 1, (unsigned)ft);
+    unsigned s = rdi_decode(d, (unsigned)ft);
+    rdi_update(d, s, s + 1, (unsigned)ft);
     return s;
 }
+DNI uint32_t rd_uint(RangeDec *d, uint32_t ft) { return rdi_uint(d, ft); }
 
 DFN int rd_tell(const RangeDec *d) { return d->nbits_total - ilog(d->rng); }
 
@@ -265,11 +270,11 @@ DFN uint32_t rd_tell_frac(const RangeDec *d)
 }
 
 // celt/laplace.c ec_laplace_decode (LAPLACE_MINP 1, LAPLACE_NMIN 16)
-DNI int rd_laplace(RangeDec *d, unsigned fs, int decay)
+DFN int rdi_laplace(RangeDec *d, unsigned fs, int decay)
 {
     int val = 0;
     unsigned fl = 0;
-    unsigned fm = rd_decode_bin(d, 15);
+    unsigned fm = rdi_decode_bin(d, 15);
     if (fm >= fs) {
         val++;
         fl = fs;
@@ -289,8 +294,9 @@ DNI int rd_laplace(RangeDec *d, unsigned fs, int decay)
         if (fm < fl + fs) val = -val;
         else fl += fs;
     }
-    rd_update(d, fl, (fl + fs) < 32768u ? fl + fs : 32768u, 32768);
+    rdi_update(d, fl, (fl + fs) < 32768u ? fl + fs : 32768u, 32768);
     return val;
 }
+DNI int rd_laplace(RangeDec *d, unsigned fs, int decay) { return rdi_laplace(d, fs, decay); }
 
 } // namespace cuo

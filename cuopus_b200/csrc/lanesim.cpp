@@ -212,6 +212,17 @@ int32_t lanesim_sum(LaneSim *s, int id, int32_t v)
     return (int32_t)t;
 }
 
+uint32_t lanesim_or(LaneSim *s, int id, uint32_t v) NOINSTR;
+uint32_t lanesim_or(LaneSim *s, int id, uint32_t v)
+{
+    s->xv[id] = (int32_t)v;
+    lanesim_sync(s, id);
+    uint32_t t = 0;
+    for (int i = 0; i < s->n; i++) t |= (uint32_t)s->xv[i];
+    lanesim_sync(s, id);
+    return t;
+}
+
 void lanesim_scan_affine(LaneSim *s, int id, uint32_t *a, uint32_t *b) NOINSTR;
 void lanesim_scan_affine(LaneSim *s, int id, uint32_t *a, uint32_t *b)
 {
