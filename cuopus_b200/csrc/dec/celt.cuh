@@ -129,6 +129,7 @@ DFN Cpx cmul(Cpx a, int16_t br, int16_t bi)
 // Every butterfly touches its own p outputs, so the N*m of them are spread over lanes.
 DNI void fft_stage(Lanes L, Cpx *F, int p, int fstride, int m, int N, int mm)
 {
+    const int inv = (int)((65536u + m - 1) / (unsigned)m);   // q / m == q * inv >> 16 for q < 480, m <= 120
     const int16_t *tw = T_fft_twiddles;
     if (p == 2) {
         // kf_bfly2 (m == 4 in the static mode)
@@ -165,7 +166,7 @@ DNI void fft_stage(Lanes L, Cpx *F, int p, int fstride, int m, int N, int mm)
             }
         } else {
             LFOR(L, q, 0, N * m) {
-                int i = q / m, j = q - i * m;
+                int i = q * inv >> 16, j = q - i * m;
                 Cpx *Fo = F + i * mm + j, s[6];
                 s[0] = cmul(Fo[m], tw[2 * (j * fstride)], tw[2 * (j * fstride) + 1]);
                 s[1] = cmul(Fo[2 * m], tw[2 * (2 * j * fstride)], tw[2 * (2 * j * fstride) + 1]);
@@ -183,7 +184,7 @@ DNI void fft_stage(Lanes L, Cpx *F, int p, int fstride, int m, int N, int mm)
     } else if (p == 3) {
         const int16_t epi3i = -28378;
         LFOR(L, q, 0, N * m) {
-            int i = q / m, j = q - i * m;
+            int i = q * inv >> 16, j = q - i * m;
             Cpx *Fo = F + i * mm + j, s[4];
             s[1] = cmul(Fo[m], tw[2 * (j * fstride)], tw[2 * (j * fstride) + 1]);
             s[2] = cmul(Fo[2 * m], tw[2 * (2 * j * fstride)], tw[2 * (2 * j * fstride) + 1]);
@@ -203,7 +204,7 @@ DNI void fft_stage(Lanes L, Cpx *F, int p, int fstride, int m, int N, int mm)
         // kf_bfly5
         const int16_t yar = 10126, yai = -31164, ybr = -26510, ybi = -19261;
         LFOR(L, q, 0, N * m) {
-            int i = q / m, u = q - i * m;
+            int i = q * inv >> 16, u = q - i * m;
             Cpx *F0 = F + i * mm + u, *F1 = F0 + m, *F2 = F0 + 2 * m, *F3 = F0 + 3 * m, *F4 = F0 + 4 * m;
             Cpx s[13];
             s[0] = *F0;
@@ -464,7 +465,11 @@ DNI void comb_filter_lanes(Lanes L, int32_t *y, int32_t *x, int T0, int T1, int 
 DNI void deemphasis(Lanes L, int32_t *in0, int32_t *in1, int16_t *pcm, int N, int C, int32_t *mem,
                     int accum)
 {
-    const int16_t coef0 = T_CELT_PREEMPH0;
+    // One step is m = (coef0 (x + m)) >> 15: with c the 32-bit value of coef0 * 2^17
+    // less 2^32, tmp + (tmp c >> 32) is that product exactly, so a step waits for
+    // one add and one mad.hi.  Inputs (and the samples added to) are loaded four
+    // ahead.  960 samples: 81 k cycles one at a time with a 64-bit product, 38 k now.
+    const int32_t cm = (int32_t)(((uint32_t)T_CELT_PREEMPH0 << 17));
     // The channels are independent recursions: with two or more lanes, lane c
     // runs channel c, so a stereo frame's two recursions execute side by side
     // in the same instructions; a single lane runs them one after the other.
@@ -478,17 +483,28 @@ DNI void deemphasis(Lanes L, int32_t *in0, int32_t *in1, int16_t *pcm, int N, in
         const int32_t *x = c == 0 ? in0 : in1;
         int16_t *y = pcm + c;
         int32_t m = mem[c];
-        if (accum) {
-            ROLLED for (int j = 0; j < N; j++) {
-                int32_t tmp = wadd(x[j], m);
-                m = c_mul16_32_q15(coef0, tmp);
-                y[j * C] = c_sat16((int32_t)y[j * C] + c_sig2word16(tmp));
+        int32_t xa[4], ya[4] = {0, 0, 0, 0};   // N is a multiple of 4
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            xa[k] = x[k];
+            if (accum) ya[k] = y[k * C];
+        }
+        ROLLED for (int j = 0; j < N; j += 4) {
+            int32_t xb[4], yb[4];
+            const int nx = j + 4 < N ? j + 4 : j;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                xb[k] = xa[k];
+                yb[k] = ya[k];
+                xa[k] = x[nx + k];
+                if (accum) ya[k] = y[(nx + k) * C];
             }
-        } else {
-            ROLLED for (int j = 0; j < N; j++) {
-                int32_t tmp = wadd(x[j], m);
-                m = c_mul16_32_q15(coef0, tmp);
-                y[j * C] = c_sig2word16(tmp);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int32_t tmp = wadd(xb[k], m);
+                m = s_smlawh(tmp, tmp, cm);
+                const int16_t v = c_sig2word16(tmp);
+                y[(j + k) * C] = accum ? c_sat16(yb[k] + v) : v;
             }
         }
         mem[c] = m;
@@ -536,8 +552,9 @@ DNI void celt_synthesis(Lanes L, CeltScratch *w, const int16_t *X, int32_t **out
 
 // ------------------------------------------------------------------ energy
 
-DNI void unquant_coarse_energy(int start, int end, int16_t *oldEBands, int intra, RangeDec *dec, int C, int LM)
+DNI void unquant_coarse_energy(int start, int end, int16_t *oldEBands, int intra, RangeDec *rd, int C, int LM)
 {
+    RangeDec dd = *rd, *dec = &dd;   // in registers
     const uint8_t *prob = &T_celt_e_prob_model[(LM * 2 + intra) * 42];
     int32_t prev[2] = {0, 0};
     int16_t coef, beta;
@@ -550,12 +567,12 @@ DNI void unquant_coarse_energy(int start, int end, int16_t *oldEBands, int intra
             int32_t tell = rd_tell(dec);
             if (budget - tell >= 15) {
                 int pi = 2 * imin(i, 20);
-                qi = rd_laplace(dec, prob[pi] << 7, prob[pi + 1] << 6);
+                qi = rdi_laplace(dec, prob[pi] << 7, prob[pi + 1] << 6);
             } else if (budget - tell >= 2) {
-                qi = rd_icdf(dec, T_celt_small_energy_icdf, 2);
+                qi = rdi_icdf(dec, T_celt_small_energy_icdf, 2);
                 qi = (qi >> 1) ^ -(qi & 1);
             } else if (budget - tell >= 1) {
-                qi = -rd_bit_logp(dec, 1);
+                qi = -rdi_bit_logp(dec, 1);
             } else {
                 qi = -1;
             }
@@ -568,35 +585,40 @@ DNI void unquant_coarse_energy(int start, int end, int16_t *oldEBands, int intra
             prev[c] = wsub(wadd(prev[c], shl32(q, 7)), c_mul16(beta, c_pshr(q, 8)));
         }
     }
+    *rd = dd;
 }
 
-DNI void unquant_fine_energy(int start, int end, int16_t *oldEBands, const int32_t *fine_quant, RangeDec *dec,
+DNI void unquant_fine_energy(int start, int end, int16_t *oldEBands, const int32_t *fine_quant, RangeDec *rd,
                              int C)
 {
+    RangeDec dd = *rd, *dec = &dd;   // in registers
     ROLLED for (int i = start; i < end; i++) {
         if (fine_quant[i] <= 0) continue;
         ROLLED for (int c = 0; c < C; c++) {
-            int q2 = (int)rd_bits(dec, fine_quant[i]);
+            int q2 = (int)rdi_bits(dec, fine_quant[i]);
             int16_t offset = (int16_t)(((shl32(q2, 10) + 512) >> fine_quant[i]) - 512);
             oldEBands[i + c * CELT_NB] = (int16_t)(oldEBands[i + c * CELT_NB] + offset);
         }
     }
+    *rd = dd;
 }
 
 DNI void unquant_energy_finalise(int start, int end, int16_t *oldEBands, const int32_t *fine_quant,
-                                 const int32_t *fine_priority, int bits_left, RangeDec *dec, int C)
+                                 const int32_t *fine_priority, int bits_left, RangeDec *rd, int C)
 {
+    RangeDec dd = *rd, *dec = &dd;   // in registers
     ROLLED for (int prio = 0; prio < 2; prio++) {
         ROLLED for (int i = start; i < end && bits_left >= C; i++) {
             if (fine_quant[i] >= 8 || fine_priority[i] != prio) continue;
             ROLLED for (int c = 0; c < C; c++) {
-                int q2 = (int)rd_bits(dec, 1);
+                int q2 = (int)rdi_bits(dec, 1);
                 int16_t offset = (int16_t)((int16_t)((uint16_t)q2 << 10) - 512) >> (fine_quant[i] + 1);
                 oldEBands[i + c * CELT_NB] = (int16_t)(oldEBands[i + c * CELT_NB] + offset);
                 bits_left--;
             }
         }
     }
+    *rd = dd;
 }
 
 // ------------------------------------------------------------------ allocation
@@ -636,9 +658,33 @@ DFN void init_caps(int32_t *cap, int LM, int C)
     }
 }
 
-DNI int interp_bits2pulses(int start, int end, int skip_start, const int32_t *bits1, const int32_t *bits2,
-                           const int32_t *thresh, const int32_t *cap, int32_t total, int32_t *_balance,
-                           int skip_rsv, int *intensity, int intensity_rsv, int *dual_stereo,
+// Bit allocation.  It runs on every lane of the group: the lanes split the
+// bands (band j of a search step adds its own share to the total, up to the
+// highest band that reaches its threshold), and the symbols between the
+// searches are decoded by all of them from a range decoder in registers.  One
+// lane walking the bands took 52 k cycles a full-band frame, this 16 k.
+
+// Sum over the bands of what each takes when it asks for want(j) bits: bands up
+// to the highest that reaches its threshold take what they ask for, at most
+// their cap; the ones above take the floor when they reach that.
+template <class F>
+DFN int32_t alloc_sum(const Lanes &L, int start, int end, const int32_t *thresh, const int32_t *cap, int alloc_floor,
+                      F want)
+{
+    int top = -1;
+    LFOR(L, j, start, end) if (want(j) >= thresh[j]) top = imax(top, j);
+    top = lmax(L, top);
+    int32_t sum = 0;
+    LFOR(L, j, start, end) {
+        const int bits = want(j);
+        sum += j <= top ? imin(bits, cap[j]) : bits >= alloc_floor ? alloc_floor : 0;
+    }
+    return lsum(L, sum);
+}
+
+DFN int interp_bits2pulses(const Lanes &L, int start, int end, int skip_start, const int32_t *bits1,
+                           const int32_t *bits2, const int32_t *thresh, const int32_t *cap, int32_t total,
+                           int32_t *_balance, int skip_rsv, int *intensity, int intensity_rsv, int *dual_stereo,
                            int dual_stereo_rsv, int32_t *bits, int32_t *ebits, int32_t *fine_priority, int C,
                            int LM, RangeDec *ec)
 {
@@ -647,38 +693,29 @@ DNI int interp_bits2pulses(int start, int end, int skip_start, const int32_t *bi
     int stereo = C > 1;
     int logM = LM << 3;
     int lo = 0, hi = 1 << 6;
-    int32_t psum;
-    int done;
     ROLLED for (int i = 0; i < 6; i++) {
         int mid = (lo + hi) >> 1;
-        psum = 0;
-        done = 0;
-        ROLLED for (int j = end; j-- > start;) {
-            int tmp = bits1[j] + (mid * (int32_t)bits2[j] >> 6);
-            if (tmp >= thresh[j] || done) {
-                done = 1;
-                psum += imin(tmp, cap[j]);
-            } else if (tmp >= alloc_floor) {
-                psum += alloc_floor;
-            }
-        }
+        const int32_t psum = alloc_sum(L, start, end, thresh, cap, alloc_floor,
+                                       [&](int j) CUO_INLINE { return bits1[j] + (mid * bits2[j] >> 6); });
         if (psum > total) hi = mid;
         else lo = mid;
     }
-    psum = 0;
-    done = 0;
-    ROLLED for (int j = end; j-- > start;) {
-        int tmp = bits1[j] + ((int32_t)lo * bits2[j] >> 6);
-        if (tmp < thresh[j] && !done) {
-            if (tmp >= alloc_floor) tmp = alloc_floor;
-            else tmp = 0;
-        } else {
-            done = 1;
-        }
+    int top = -1;
+    LFOR(L, j, start, end) if (bits1[j] + (lo * bits2[j] >> 6) >= thresh[j]) top = imax(top, j);
+    top = lmax(L, top);
+    int32_t psum = 0;
+    LFOR(L, j, start, end) {
+        int tmp = bits1[j] + (lo * bits2[j] >> 6);
+        if (j > top) tmp = tmp >= alloc_floor ? alloc_floor : 0;
         tmp = imin(tmp, cap[j]);
         bits[j] = tmp;
         psum += tmp;
     }
+    psum = lsum(L, psum);
+    lsync(L);
+    // which of the highest bands are skipped: every lane reads the bands' bits
+    // as they are; the skipped bands' new ones are written after the loop
+    unsigned floored = 0;
     int codedBands;
     ROLLED for (codedBands = end;; codedBands--) {
         int j = codedBands - 1;
@@ -693,7 +730,7 @@ DNI int interp_bits2pulses(int start, int end, int skip_start, const int32_t *bi
         int band_width = eB[codedBands] - eB[j];
         int band_bits = (int)(bits[j] + percoeff * band_width + rem);
         if (band_bits >= imax(thresh[j], alloc_floor + (1 << 3))) {
-            if (rd_bit_logp(ec, 1)) break;
+            if (rdi_bit_logp(ec, 1)) break;
             psum += 1 << 3;
             band_bits -= 1 << 3;
         }
@@ -702,82 +739,92 @@ DNI int interp_bits2pulses(int start, int end, int skip_start, const int32_t *bi
         psum += intensity_rsv;
         if (band_bits >= alloc_floor) {
             psum += alloc_floor;
-            bits[j] = alloc_floor;
-        } else {
-            bits[j] = 0;
+            floored |= 1u << j;
         }
     }
-    if (intensity_rsv > 0) *intensity = start + (int)rd_uint(ec, codedBands + 1 - start);
+    if (intensity_rsv > 0) *intensity = start + (int)rdi_uint(ec, codedBands + 1 - start);
     else *intensity = 0;
     if (*intensity <= start) {
         total += dual_stereo_rsv;
         dual_stereo_rsv = 0;
     }
-    if (dual_stereo_rsv > 0) *dual_stereo = rd_bit_logp(ec, 1);
+    if (dual_stereo_rsv > 0) *dual_stereo = rdi_bit_logp(ec, 1);
     else *dual_stereo = 0;
     int32_t left = total - psum;
     int32_t percoeff = (int32_t)((uint32_t)left / (uint32_t)(eB[codedBands] - eB[start]));
     left -= (eB[codedBands] - eB[start]) * percoeff;
-    ROLLED for (int j = start; j < codedBands; j++) bits[j] += (int)percoeff * (eB[j + 1] - eB[j]);
-    ROLLED for (int j = start; j < codedBands; j++) {
-        int tmp = (int)imin(left, eB[j + 1] - eB[j]);
-        bits[j] += tmp;
-        left -= tmp;
-    }
-    int32_t balance = 0;
-    int j;
-    ROLLED for (j = start; j < codedBands; j++) {
-        int N0 = eB[j + 1] - eB[j];
-        int N = N0 << LM;
-        int32_t bit = (int32_t)bits[j] + balance;
-        int32_t excess;
-        if (N > 1) {
-            excess = max32(bit - cap[j], 0);
-            bits[j] = bit - excess;
-            int den = C * N + ((C == 2 && N > 2 && !*dual_stereo && j < *intensity) ? 1 : 0);
-            int NClogN = den * (T_celt_logN[j] + logM);
-            int offset = (NClogN >> 1) - den * 21;   // FINE_OFFSET
-            if (N == 2) offset += den << 3 >> 2;
-            if (bits[j] + offset < den * 2 << 3) offset += NClogN >> 2;
-            else if (bits[j] + offset < den * 3 << 3) offset += NClogN >> 3;
-            ebits[j] = imax(0, bits[j] + offset + (den << 2));
-            ebits[j] = (int32_t)((uint32_t)ebits[j] / (uint32_t)den) >> 3;
-            if (C * ebits[j] > (bits[j] >> 3)) ebits[j] = bits[j] >> stereo >> 3;
-            ebits[j] = imin(ebits[j], 8);
-            fine_priority[j] = ebits[j] * (den << 3) >= bits[j] + offset;
-            bits[j] -= C * ebits[j] << 3;
+    lsync(L);
+    LFOR(L, j, start, end) {
+        if (j >= codedBands) {
+            bits[j] = floored >> j & 1 ? alloc_floor : 0;
         } else {
-            excess = max32(0, bit - (C << 3));
-            bits[j] = bit - excess;
-            ebits[j] = 0;
-            fine_priority[j] = 1;
+            const int width = eB[j + 1] - eB[j];
+            bits[j] += percoeff * width + imax(0, imin(left - (eB[j] - eB[start]), width));
         }
-        if (excess > 0) {
-            int extra_fine = imin(excess >> (stereo + 3), 8 - ebits[j]);
-            ebits[j] += extra_fine;
-            int extra_bits = extra_fine * C << 3;
-            fine_priority[j] = extra_bits >= excess - balance;
-            excess -= extra_bits;
+    }
+    // fine energy against shapes, band after band: what a band cannot use goes
+    // to the next
+    int32_t balance = 0;
+    lead(L, [&]() CUO_INLINE {
+        int j;
+        ROLLED for (j = start; j < codedBands; j++) {
+            int N0 = eB[j + 1] - eB[j];
+            int N = N0 << LM;
+            int32_t bit = (int32_t)bits[j] + balance;
+            int32_t excess;
+            int32_t bj, ej, fp;
+            if (N > 1) {
+                excess = max32(bit - cap[j], 0);
+                bj = bit - excess;
+                int den = C * N + ((C == 2 && N > 2 && !*dual_stereo && j < *intensity) ? 1 : 0);
+                int NClogN = den * (T_celt_logN[j] + logM);
+                int offset = (NClogN >> 1) - den * 21;   // FINE_OFFSET
+                if (N == 2) offset += den << 3 >> 2;
+                if (bj + offset < den * 2 << 3) offset += NClogN >> 2;
+                else if (bj + offset < den * 3 << 3) offset += NClogN >> 3;
+                ej = imax(0, bj + offset + (den << 2));
+                ej = (int32_t)((uint32_t)ej / (uint32_t)den) >> 3;
+                if (C * ej > (bj >> 3)) ej = bj >> stereo >> 3;
+                ej = imin(ej, 8);
+                fp = ej * (den << 3) >= bj + offset;
+                bj -= C * ej << 3;
+            } else {
+                excess = max32(0, bit - (C << 3));
+                bj = bit - excess;
+                ej = 0;
+                fp = 1;
+            }
+            if (excess > 0) {
+                int extra_fine = imin(excess >> (stereo + 3), 8 - ej);
+                ej += extra_fine;
+                int extra_bits = extra_fine * C << 3;
+                fp = extra_bits >= excess - balance;
+                excess -= extra_bits;
+            }
+            bits[j] = bj;
+            ebits[j] = ej;
+            fine_priority[j] = fp;
+            balance = excess;
         }
-        balance = excess;
-    }
-    *_balance = balance;
-    ROLLED for (; j < end; j++) {
-        ebits[j] = bits[j] >> stereo >> 3;
-        bits[j] = 0;
-        fine_priority[j] = ebits[j] < 1;
-    }
+        ROLLED for (; j < end; j++) {
+            ebits[j] = bits[j] >> stereo >> 3;
+            bits[j] = 0;
+            fine_priority[j] = ebits[j] < 1;
+        }
+    });
+    *_balance = lbcast(L, balance);
     return codedBands;
 }
 
-DNI int clt_compute_allocation(int start, int end, const int32_t *offsets, const int32_t *cap, int alloc_trim,
-                               int *intensity, int *dual_stereo, int32_t total, int32_t *balance, int32_t *pulses,
-                               int32_t *ebits, int32_t *fine_priority, int C, int LM, RangeDec *ec, CeltScratch *w)
+DNI int clt_compute_allocation(Lanes L, int start, int end, const int32_t *offsets, const int32_t *cap,
+                               int alloc_trim, int *intensity, int *dual_stereo, int32_t total, int32_t *balance,
+                               int32_t *pulses, int32_t *ebits, int32_t *fine_priority, int C, int LM,
+                               RangeDec *rd, CeltScratch *w)
 {
     const int16_t *eB = T_celt_eBands;
     int32_t *bits1 = w->bits1, *bits2 = w->bits2, *thresh = w->thresh, *trim_offset = w->trim_offset;
+    RangeDec d = *rd;
     total = max32(total, 0);
-    int skip_start = start;
     int skip_rsv = total >= 1 << 3 ? 1 << 3 : 0;
     total -= skip_rsv;
     int intensity_rsv = 0, dual_stereo_rsv = 0;
@@ -791,32 +838,26 @@ DNI int clt_compute_allocation(int start, int end, const int32_t *offsets, const
             total -= dual_stereo_rsv;
         }
     }
-    ROLLED for (int j = start; j < end; j++) {
+    LFOR(L, j, start, end) {
         thresh[j] = imax(C << 3, (3 * (eB[j + 1] - eB[j]) << LM << 3) >> 4);
         trim_offset[j] = C * (eB[j + 1] - eB[j]) * (alloc_trim - 5 - LM) * (end - j - 1) * (1 << (LM + 3)) >> 6;
         if ((eB[j + 1] - eB[j]) << LM == 1) trim_offset[j] -= C << 3;
     }
+    lsync(L);
     int lo = 1, hi = T_CELT_NBALLOCV - 1;
     ROLLED do {
-        int done = 0, psum = 0;
         int mid = (lo + hi) >> 1;
-        ROLLED for (int j = end; j-- > start;) {
-            int N = eB[j + 1] - eB[j];
-            int bitsj = C * N * T_celt_allocVectors[mid * CELT_NB + j] << LM >> 2;
+        const int32_t psum = alloc_sum(L, start, end, thresh, cap, C << 3, [&](int j) CUO_INLINE {
+            int bitsj = C * (eB[j + 1] - eB[j]) * T_celt_allocVectors[mid * CELT_NB + j] << LM >> 2;
             if (bitsj > 0) bitsj = imax(0, bitsj + trim_offset[j]);
-            bitsj += offsets[j];
-            if (bitsj >= thresh[j] || done) {
-                done = 1;
-                psum += imin(bitsj, cap[j]);
-            } else if (bitsj >= C << 3) {
-                psum += C << 3;
-            }
-        }
+            return bitsj + offsets[j];
+        });
         if (psum > total) hi = mid - 1;
         else lo = mid + 1;
     } while (lo <= hi);
     hi = lo--;
-    ROLLED for (int j = start; j < end; j++) {
+    int boosted = -1;
+    LFOR(L, j, start, end) {
         int N = eB[j + 1] - eB[j];
         int bits1j = C * N * T_celt_allocVectors[lo * CELT_NB + j] << LM >> 2;
         int bits2j = hi >= T_CELT_NBALLOCV ? cap[j] : C * N * T_celt_allocVectors[hi * CELT_NB + j] << LM >> 2;
@@ -824,14 +865,18 @@ DNI int clt_compute_allocation(int start, int end, const int32_t *offsets, const
         if (bits2j > 0) bits2j = imax(0, bits2j + trim_offset[j]);
         if (lo > 0) bits1j += offsets[j];
         bits2j += offsets[j];
-        if (offsets[j] > 0) skip_start = j;
+        if (offsets[j] > 0) boosted = imax(boosted, j);
         bits2j = imax(0, bits2j - bits1j);
         bits1[j] = bits1j;
         bits2[j] = bits2j;
     }
-    return interp_bits2pulses(start, end, skip_start, bits1, bits2, thresh, cap, total, balance, skip_rsv,
-                              intensity, intensity_rsv, dual_stereo, dual_stereo_rsv, pulses, ebits,
-                              fine_priority, C, LM, ec);
+    const int skip_start = imax(start, lmax(L, boosted));
+    lsync(L);
+    const int coded = interp_bits2pulses(L, start, end, skip_start, bits1, bits2, thresh, cap, total, balance,
+                                         skip_rsv, intensity, intensity_rsv, dual_stereo, dual_stereo_rsv, pulses,
+                                         ebits, fine_priority, C, LM, &d);
+    *rd = d;
+    return coded;
 }
 
 // ------------------------------------------------------------------ PVQ
@@ -938,37 +983,51 @@ DFN void exp_rotation_class(int16_t *X, int len, int stride, int32_t c, int32_t 
     if (n <= 0) return;
     int16_t *x = X + r;
     // forward: pairs 0 .. n - 1
-    int32_t x1 = x[0];
-    ROLLED for (int i = 0; i < n; i += 4) {
-        int32_t v[4];
+    auto fwd = [&](int i, int32_t x2, int32_t &x1) CUO_INLINE {
+        x[i * stride] = (int16_t)(wadd(wadd(wmul(c2, x1), rnd), -wmul(s2, x2)) >> 16);
+        x1 = wadd(wadd(wmul(c2, x2), rnd), wmul(s2, x1)) >> 16;
+    };
+    int32_t x1 = x[0], v[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) v[j] = x[imin(i + j + 1, n) * stride];
+    for (int j = 0; j < 4; j++) v[j] = x[imin(j + 1, n) * stride];
+    int i = 0;
+    ROLLED for (; i + 4 <= n; i += 4) {
+        int32_t u[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            if (i + j < n) {
-                const int32_t x2 = v[j];
-                x[(i + j) * stride] = (int16_t)(wadd(wadd(wmul(c2, x1), rnd), -wmul(s2, x2)) >> 16);
-                x1 = wadd(wadd(wmul(c2, x2), rnd), wmul(s2, x1)) >> 16;
-            }
+            u[j] = v[j];
+            v[j] = x[imin(i + j + 5, n) * stride];
         }
+#pragma unroll
+        for (int j = 0; j < 4; j++) fwd(i + j, u[j], x1);
     }
+    if (i < n) fwd(i, v[0], x1);
+    if (i + 1 < n) fwd(i + 1, v[1], x1);
+    if (i + 2 < n) fwd(i + 2, v[2], x1);
     x[n * stride] = (int16_t)x1;
     // backward: pairs n - 2 .. 0 (libopus's second pass starts at len - 2 stride - 1)
     if (n < 2) return;
+    auto bwd = [&](int i, int32_t w, int32_t &x2) CUO_INLINE {
+        x[(i + 1) * stride] = (int16_t)(wadd(wadd(wmul(c2, x2), rnd), wmul(s2, w)) >> 16);
+        x2 = wadd(wadd(wmul(c2, w), rnd), -wmul(s2, x2)) >> 16;
+    };
     int32_t x2 = x[(n - 1) * stride];
-    ROLLED for (int i = n - 2; i >= 0; i -= 4) {
-        int32_t v[4];
+    i = n - 2;
 #pragma unroll
-        for (int j = 0; j < 4; j++) v[j] = x[imax(i - j, 0) * stride];
+    for (int j = 0; j < 4; j++) v[j] = x[imax(i - j, 0) * stride];
+    ROLLED for (; i >= 3; i -= 4) {
+        int32_t u[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            if (i - j >= 0) {
-                const int32_t w = v[j];
-                x[(i - j + 1) * stride] = (int16_t)(wadd(wadd(wmul(c2, x2), rnd), wmul(s2, w)) >> 16);
-                x2 = wadd(wadd(wmul(c2, w), rnd), -wmul(s2, x2)) >> 16;
-            }
+            u[j] = v[j];
+            v[j] = x[imax(i - j - 4, 0) * stride];
         }
+#pragma unroll
+        for (int j = 0; j < 4; j++) bwd(i - j, u[j], x2);
     }
+    if (i >= 0) bwd(i, v[0], x2);
+    if (i >= 1) bwd(i - 1, v[1], x2);
+    if (i >= 2) bwd(i - 2, v[2], x2);
     x[0] = (int16_t)x2;
 }
 
@@ -987,15 +1046,16 @@ DNI void exp_rotation_dec(Lanes L, int16_t *X, int len, int stride, int K, int s
         ROLLED while ((stride2 * stride2 + stride2) * stride + (stride >> 2) < len) stride2++;
     }
     len = (int)((unsigned)len / (unsigned)stride);
-    if (stride2) {
-        LFOR(L, q, 0, stride * stride2) {
-            const int i = q / stride2;
-            exp_rotation_class(X + i * len, len, stride2, s, c, q - i * stride2);
+    // first the residue classes of stride2 with the coefficients swapped, then
+    // the whole blocks
+    ROLLED for (int pass = stride2 ? 0 : 1; pass < 2; pass++) {
+        const int st = pass ? 1 : stride2;
+        ROLLED for (int q = L.id; q < stride * st; q += L.n) {
+            const int i = pass ? q : (int)((unsigned)q / (unsigned)st);
+            exp_rotation_class(X + i * len, len, st, pass ? c : s, pass ? s : c, q - i * st);
         }
         lsync(L);
     }
-    LFOR(L, i, 0, stride) exp_rotation_class(X + i * len, len, 1, c, s, 0);
-    lsync(L);
 }
 
 // celt/vq.c renormalise_vector
@@ -1021,7 +1081,7 @@ DFN unsigned alg_unquant(const Lanes &L, int16_t *X, int N, int K, int spread, i
                          int32_t *iy)
 {
     PHASE_BEGIN(t_cw);
-    const uint32_t idx = rdi_uint(dec, pvq_v(N, K));
+    const uint32_t idx = rd_uint(dec, pvq_v(N, K));
     lsync(L);   // every lane is done with the last partition's pulses
     int32_t Ryy = cwrsi(N, K, idx, iy);
     PHASE_END(PH_PVQ_CWRSI, t_cw, L.id);
@@ -1063,7 +1123,7 @@ DFN int bitexact_log2tan(int isin, int icos)
 }
 
 // In place over independent pairs: the lanes split them.
-DFN void haar1(const Lanes &L, int16_t *X, int N0, int stride)
+DNI void haar1(Lanes L, int16_t *X, int N0, int stride)
 {
     LFOR(L, q, 0, (N0 >> 1) * stride) {
         const int j = q / stride, i = q - j * stride;
@@ -1091,14 +1151,17 @@ DNI void hadamard_order(Lanes L, int16_t *X, int N0, int stride, int hadamard, i
     lsync(L);
 }
 
-// Band decoding runs on every lane of the group: each lane holds the range
-// decoder and the bit budget in its registers and decodes the same symbols,
-// and the lanes share out the work on the band vectors.  (On the first lane
-// alone, with the decoder's state in memory, a full-band mono 20 ms frame of
-// 250 bytes took 530 k cycles, BANDS_MEASURED.)
+// Band decoding runs on every lane of the group: each lane decodes the same
+// symbols from its own copy of the range decoder and the lanes share out the
+// work on the band vectors.  The loop over the bands is the kernel's largest
+// and what it costs above all is instruction fetch (an SM's first instruction
+// cache holds a part of it), so everything a band does once or twice is a call
+// and every inlined piece has one call site: 29 KB of code, where everything
+// inlined came to 53 KB and decoded no faster (12 stereo files 60.3 ms against
+// 58.5 now, 30 files to int16 115 against 108).
 struct BandCtx {
     Lanes L;
-    RangeDec d;
+    RangeDec *d;
     int i;
     int intensity;
     int spread;
@@ -1134,16 +1197,16 @@ DFN int compute_qn(int N, int b, int offset, int pulse_cap, int stereo)
     return qn;
 }
 
-// celt/bands.c compute_theta (decoder side)
-DFN void compute_theta(BandCtx &ctx, SplitCtx &sctx, int N, int &b, int B, int B0, int LM, int stereo, int &fill)
+// celt/bands.c compute_theta (decoder side).  may_invert: bit 0, there are bits
+// left for the inversion flag; bit 1, the flag counts.
+DNI void compute_theta(RangeDec *ec, SplitCtx *sctx, int i, int intensity, int may_invert, int N, int *b, int B,
+                       int B0, int LM, int stereo, int *fill)
 {
     int itheta = 0, delta, imid, iside, inv = 0;
-    RangeDec *ec = &ctx.d;
-    int i = ctx.i;
     int pulse_cap = T_celt_logN[i] + LM * (1 << 3);
     int offset = (pulse_cap >> 1) - (stereo && N == 2 ? 16 : 4);
-    int qn = compute_qn(N, b, offset, pulse_cap, stereo);
-    if (stereo && i >= ctx.intensity) qn = 1;
+    int qn = compute_qn(N, *b, offset, pulse_cap, stereo);
+    if (stereo && i >= intensity) qn = 1;
     int32_t tell = (int32_t)rd_tell_frac(ec);
     if (qn != 1) {
         // the three models of the angle: a step, uniform, a triangle; each is
@@ -1151,11 +1214,11 @@ DFN void compute_theta(BandCtx &ctx, SplitCtx &sctx, int N, int &b, int B, int B
         const int step = stereo && N > 2, uniform = !step && (B0 > 1 || stereo);
         const int x0 = qn / 2, half = qn >> 1;
         if (uniform && qn + 1 > 256) {   // more than eight bits: part of them raw
-            itheta = (int)rdi_uint(ec, qn + 1);
+            itheta = (int)rd_uint(ec, qn + 1);
         } else {
             const unsigned ft = step ? (unsigned)(3 * (x0 + 1) + x0) : uniform ? (unsigned)(qn + 1)
                                                                                : (unsigned)((half + 1) * (half + 1));
-            const int fm = (int)rdi_decode(ec, ft);
+            const int fm = (int)rd_decode(ec, ft);
             unsigned fl, fh;
             if (step) {
                 const int p0 = 3;
@@ -1181,66 +1244,69 @@ DFN void compute_theta(BandCtx &ctx, SplitCtx &sctx, int N, int &b, int B, int B
                 }
                 fh = fl + fs;
             }
-            rdi_update(ec, fl, fh, ft);
+            rd_update(ec, fl, fh, ft);
         }
         itheta = (int)((uint32_t)((int32_t)itheta * 16384) / (uint32_t)qn);
     } else if (stereo) {
-        if (b > 2 << 3 && ctx.remaining_bits > 2 << 3) inv = rdi_bit_logp(ec, 2);
-        else inv = 0;
-        if (ctx.disable_inv) inv = 0;
+        if (*b > 2 << 3 && (may_invert & 1)) inv = rd_bit_logp(ec, 2);
+        if (!(may_invert & 2)) inv = 0;
         itheta = 0;
     }
     int qalloc = (int)rd_tell_frac(ec) - tell;
-    b -= qalloc;
+    *b -= qalloc;
     if (itheta == 0) {
         imid = 32767; iside = 0;
-        fill &= (1 << B) - 1;
+        *fill &= (1 << B) - 1;
         delta = -16384;
     } else if (itheta == 16384) {
         imid = 0; iside = 32767;
-        fill &= ((1 << B) - 1) << B;
+        *fill &= ((1 << B) - 1) << B;
         delta = 16384;
     } else {
         imid = bitexact_cos((int16_t)itheta);
         iside = bitexact_cos((int16_t)(16384 - itheta));
         delta = c_frac_mul16((N - 1) << 7, bitexact_log2tan(iside, imid));
     }
-    sctx.inv = inv; sctx.imid = imid; sctx.iside = iside;
-    sctx.delta = delta; sctx.itheta = itheta; sctx.qalloc = qalloc;
+    sctx->inv = inv; sctx->imid = imid; sctx->iside = iside;
+    sctx->delta = delta; sctx->itheta = itheta; sctx->qalloc = qalloc;
 }
 
-// Ends with a barrier: the group's lanes may read X, Y and lowband_out.
-DFN unsigned quant_band_n1(BandCtx &ctx, int16_t *X, int16_t *Y, int16_t *lowband_out)
+// celt/bands.c quant_band_n1; returns the bits left.  Ends with a barrier: the
+// group's lanes may read X, Y and lowband_out.
+DNI int quant_band_n1(Lanes L, RangeDec *d, int remaining_bits, int16_t *X, int16_t *Y, int16_t *lowband_out)
 {
     int sign[2] = {0, 0};
     ROLLED for (int c = 0; c < 1 + (Y != 0); c++) {
-        if (ctx.remaining_bits >= 1 << 3) {
-            const int v = (int)rdi_bits(&ctx.d, 1);
+        if (remaining_bits >= 1 << 3) {
+            const int v = (int)rd_bits(d, 1);
             if (c) sign[1] = v;
             else sign[0] = v;
-            ctx.remaining_bits -= 1 << 3;
+            remaining_bits -= 1 << 3;
         }
     }
-    lead(ctx.L, [&]() CUO_INLINE {
+    lead(L, [&]() CUO_INLINE {
         X[0] = sign[0] ? -16384 : 16384;
         if (Y) Y[0] = sign[1] ? -16384 : 16384;
         if (lowband_out) lowband_out[0] = (int16_t)(X[0] >> 4);
     });
-    return 1;
+    return remaining_bits;
 }
 
-// celt/bands.c celt_lcg_rand k steps on: the seed as an affine map of the seed
-// now (x -> A^k x + B_k mod 2^32), by binary powers.
-DFN uint32_t lcg_jump(uint32_t seed, unsigned k)
-{
-    uint32_t a = 1664525u, c = 1013904223u;
-    ROLLED for (; k; k >>= 1) {
-        if (k & 1) seed = a * seed + c;
-        c = a * c + c;
-        a = a * a;
+// celt/bands.c celt_lcg_rand k steps on is the affine map seed -> a[k] seed +
+// c[k] mod 2^32; k up to the longest band.
+struct LcgPowers {
+    uint32_t a[177], c[177];
+    constexpr LcgPowers() : a(), c()
+    {
+        a[0] = 1;
+        c[0] = 0;
+        for (int k = 1; k < 177; k++) {
+            a[k] = 1664525u * a[k - 1];
+            c[k] = 1664525u * c[k - 1] + 1013904223u;
+        }
     }
-    return seed;
-}
+};
+TABG(LcgPowers, T_lcg) = LcgPowers();
 
 // celt/bands.c quant_partition, leaf: pulses for the band piece (PVQ) or,
 // with none, folding / noise fill.
@@ -1260,7 +1326,7 @@ DFN unsigned quant_partition_leaf(BandCtx &ctx, int16_t *X, int N, int b, int B,
     }
     if (q != 0) {
         int K = get_pulses(q);
-        cm = alg_unquant(ctx.L, X, N, K, ctx.spread, B, &ctx.d, gain, ctx.w->iy);
+        cm = alg_unquant(ctx.L, X, N, K, ctx.spread, B, ctx.d, gain, ctx.w->iy);
     } else {
         unsigned cm_mask = (unsigned)(1UL << B) - 1;
         fill &= cm_mask;
@@ -1268,20 +1334,17 @@ DFN unsigned quant_partition_leaf(BandCtx &ctx, int16_t *X, int N, int b, int B,
             LFOR(ctx.L, j, 0, N) X[j] = 0;
             lsync(ctx.L);
         } else {
-            // sample j takes the seed j + 1 steps on: a lane jumps to its first
-            // sample's seed and from one of its samples to the next
-            uint32_t seed = lcg_jump(ctx.seed, ctx.L.id + 1);
-            const uint32_t c = lcg_jump(0, ctx.L.n), a = lcg_jump(1, ctx.L.n) - c;
-            ROLLED for (int j = ctx.L.id; j < N; j += ctx.L.n) {
+            // sample j takes the seed j + 1 steps on
+            LFOR(ctx.L, j, 0, N) {
+                const uint32_t seed = T_lcg.a[j + 1] * ctx.seed + T_lcg.c[j + 1];
                 if (lowband == 0) {
                     X[j] = (int16_t)((int32_t)seed >> 20);
                 } else {
                     int16_t tmp = (seed & 0x8000) ? 4 : -4;   // QCONST16(1.0f/256, 10)
                     X[j] = (int16_t)(lowband[j] + tmp);
                 }
-                seed = a * seed + c;
             }
-            ctx.seed = lcg_jump(ctx.seed, N);
+            ctx.seed = T_lcg.a[N] * ctx.seed + T_lcg.c[N];
             cm = lowband == 0 ? cm_mask : fill;
             lsync(ctx.L);
             renormalise_vector(ctx.L, X, N, gain);
@@ -1316,7 +1379,7 @@ DFN unsigned quant_partition(BandCtx &ctx, int16_t *X, int N, int b, int B, int1
             B = (B + 1) >> 1;
             LM--;
             PHASE_BEGIN(t_th);
-            compute_theta(ctx, sctx, N, b, B, B0, LM, 0, fill);
+            compute_theta(ctx.d, &sctx, i, ctx.intensity, 0, N, &b, B, B0, LM, 0, &fill);
             PHASE_END(PH_PVQ_THETA, t_th, L.id);
             int delta = sctx.delta;
             const int itheta = sctx.itheta;
@@ -1401,7 +1464,10 @@ DFN unsigned quant_band(BandCtx &ctx, int16_t *X, int N, int b, int B, int16_t *
     unsigned cm = 0;
     int tf_change = ctx.tf_change;
     N_B = (int)((unsigned)N_B / (unsigned)B);
-    if (N == 1) return quant_band_n1(ctx, X, 0, lowband_out);
+    if (N == 1) {
+        ctx.remaining_bits = quant_band_n1(L, ctx.d, ctx.remaining_bits, X, 0, lowband_out);
+        return 1;
+    }
     if (tf_change > 0) recombine = tf_change;
     PHASE_BEGIN(t_tf);
     if (lowband_scratch && lowband && (recombine || ((N_B & 1) == 0 && tf_change < 0) || B0 > 1)) {
@@ -1490,6 +1556,19 @@ DNI void stereo_merge(Lanes L, int16_t *X, int16_t *Y, int16_t mid, int N)
     lsync(L);
 }
 
+// Band of a bin of the shortest frame (eBands inverted).
+struct BandOf {
+    uint8_t b[101];
+    constexpr BandOf() : b()
+    {
+        const int e[22] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16, 20, 24, 28, 34, 40, 48, 60, 78, 100};
+        for (int k = 0; k < 21; k++)
+            for (int u = e[k]; u < e[k + 1]; u++) b[u] = (uint8_t)k;
+        b[100] = 21;
+    }
+};
+TABC(BandOf, T_band_of) = BandOf();
+
 // celt/bands.c quant_all_bands, decoder path (encode = 0, resynth = 1, no theta
 // RDO), with quant_band_stereo.  A band takes one pass through quant_band or
 // two: mono, stereo of two samples and a band coded mid only: X; dual stereo: X
@@ -1511,7 +1590,7 @@ DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *
     int lowband_offset = 0, update_lowband = 1;
     BandCtx ctx;
     ctx.L = L;
-    ctx.d = *ec;
+    ctx.d = ec;
     ctx.intensity = intensity;
     ctx.seed = *seed;
     ctx.spread = spread;
@@ -1525,13 +1604,14 @@ DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *
         int16_t *X = X_ + M * eB[i];
         int16_t *Y = Y_ != 0 ? Y_ + M * eB[i] : 0;
         int N = M * eB[i + 1] - M * eB[i];
-        int32_t tell = (int32_t)rd_tell_frac(&ctx.d);
+        int32_t tell = (int32_t)rd_tell_frac(ec);
         if (i != start) balance -= tell;
         int32_t remaining_bits = total_bits - tell - 1;
         ctx.remaining_bits = remaining_bits;
         int b;
         if (i <= codedBands - 1) {
-            int32_t curr_balance = balance / imin(3, codedBands - i);
+            const int share = codedBands - i;
+            int32_t curr_balance = share >= 3 ? balance / 3 : share == 2 ? balance / 2 : balance;
             b = imax(0, imin(16383, imin(remaining_bits + 1, pulses[i] + curr_balance)));
         } else {
             b = 0;
@@ -1559,10 +1639,11 @@ DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *
         if (last) lowband_scratch = 0;
         if (lowband_offset != 0 && (spread != SPREAD_AGGRESSIVE || B > 1 || tf_change < 0)) {
             effective_lowband = imax(0, M * eB[lowband_offset] - norm_offset - N);
-            int fold_start = lowband_offset;
-            ROLLED while (M * eB[--fold_start] > effective_lowband + norm_offset) {}
-            int fold_end = lowband_offset - 1;
-            ROLLED while (++fold_end < i && M * eB[fold_end] < effective_lowband + norm_offset + N) {}
+            // the bands the folding source covers, from the lowest at or below its
+            // first bin to the one its last bin is in (of the bands decoded)
+            const int first = effective_lowband + norm_offset;
+            const int fold_start = imin(lowband_offset - 1, T_band_of.b[first >> LM]);
+            const int fold_end = imin(i, imax(lowband_offset, T_band_of.b[(first + N - 1) >> LM] + 1));
             x_cm = y_cm = 0;
             int fold_i = fold_start;
             ROLLED do {
@@ -1582,7 +1663,8 @@ DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *
         int16_t *const lowband_out = last ? 0 : norm + M * eB[i] - norm_offset;
         const int orig_fill = (int)(x_cm | y_cm);
         if (Y != 0 && !dual_stereo && N == 1) {
-            x_cm = y_cm = quant_band_n1(ctx, X, Y, lowband_out);
+            ctx.remaining_bits = quant_band_n1(L, ctx.d, ctx.remaining_bits, X, Y, lowband_out);
+            x_cm = y_cm = 1;
         } else {
             // the passes: vector, bits, folding source and target, gain, fill
             int16_t *px = X, *plow = lowband, *pout = lowband_out, *pscratch = lowband_scratch;
@@ -1598,7 +1680,8 @@ DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *
             } else if (Y != 0) {
                 int left = b;   // without the angle's bits
                 PHASE_BEGIN(t_th);
-                compute_theta(ctx, sctx, N, left, B, B, LM, 1, fill);
+                compute_theta(ctx.d, &sctx, i, ctx.intensity, (ctx.remaining_bits > 2 << 3) | (ctx.disable_inv ? 0 : 2), N,
+                              &left, B, B, LM, 1, &fill);
                 PHASE_END(PH_PVQ_THETA, t_th, L.id);
                 if (N == 2) {
                     int sbits = 0;
@@ -1606,7 +1689,7 @@ DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *
                     pb = left - sbits;
                     ctx.remaining_bits -= sctx.qalloc + sbits;
                     px = sctx.itheta > 8192 ? Y : X;
-                    if (sbits) sign = (int)rdi_bits(&ctx.d, 1);
+                    if (sbits) sign = (int)rd_bits(ctx.d, 1);
                     sign = 1 - 2 * sign;
                 } else {
                     const int mbits = imax(0, imin(left, (left - sctx.delta) / 2)), sbits = left - mbits;
@@ -1686,7 +1769,6 @@ DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *
         update_lowband = b > (N << 3);
     }
     lsync(L);
-    *ec = ctx.d;
     *seed = ctx.seed;
     lsync(L);
 }
@@ -1741,8 +1823,9 @@ DNI void anti_collapse(Lanes L, int16_t *X_, const uint8_t *collapse_masks, int 
     }
 }
 
-DNI void tf_decode(int start, int end, int isTransient, int32_t *tf_res, int LM, RangeDec *dec)
+DNI void tf_decode(int start, int end, int isTransient, int32_t *tf_res, int LM, RangeDec *rd)
 {
+    RangeDec dd = *rd, *dec = &dd;   // in registers
     uint32_t budget = dec->storage * 8;
     uint32_t tell = (uint32_t)rd_tell(dec);
     int logp = isTransient ? 2 : 4;
@@ -1751,7 +1834,7 @@ DNI void tf_decode(int start, int end, int isTransient, int32_t *tf_res, int LM,
     int tf_changed = 0, curr = 0;
     ROLLED for (int i = start; i < end; i++) {
         if (tell + logp <= budget) {
-            curr ^= rd_bit_logp(dec, logp);
+            curr ^= rdi_bit_logp(dec, logp);
             tell = (uint32_t)rd_tell(dec);
             tf_changed |= curr;
         }
@@ -1761,8 +1844,9 @@ DNI void tf_decode(int start, int end, int isTransient, int32_t *tf_res, int LM,
     int tf_select = 0;
     const int8_t *tt = &T_celt_tf_select_table[LM * 8];
     if (tf_select_rsv && tt[4 * isTransient + 0 + tf_changed] != tt[4 * isTransient + 2 + tf_changed])
-        tf_select = rd_bit_logp(dec, 1);
+        tf_select = rdi_bit_logp(dec, 1);
     ROLLED for (int i = start; i < end; i++) tf_res[i] = tt[4 * isTransient + 2 * tf_select + tf_res[i]];
+    *rd = dd;
 }
 
 // ------------------------------------------------------------------ PLC (pitch / LPC)
@@ -2260,11 +2344,10 @@ DNI int celt_decode(Lanes L, CeltDec *st, const uint8_t *data, int len, int16_t 
     }
     int32_t *tf_res = w->tf_res;
     int32_t *pulses = w->pulses, *fine_quant = w->fine_quant, *fine_priority = w->fine_priority;
-    // The frame header, the energies and the bit allocation: entropy decoding
-    // and state updates in place, on the first lane; every lane gets the
-    // outcome (the per-band tables stay in the scratch).
-    enum { H_SILENCE, H_PF_GAIN, H_PF_PITCH, H_PF_TAPSET, H_TRANSIENT, H_SPREAD, H_AC_RSV, H_INTENSITY, H_DUAL,
-           H_BALANCE, H_CODED, H_N };
+    // The frame header and the energies: entropy decoding and state updates in
+    // place, on the first lane; every lane gets the outcome (the per-band tables
+    // stay in the scratch).
+    enum { H_SILENCE, H_PF_GAIN, H_PF_PITCH, H_PF_TAPSET, H_TRANSIENT, H_SPREAD, H_AC_RSV, H_TRIM, H_BITS, H_N };
     int32_t hv[H_N] = {0};
     lead_rd(L, dec, [&]() CUO_INLINE {
         if (st->loss_duration == 0) st->skip_plc = 0;
@@ -2310,14 +2393,15 @@ DNI int celt_decode(Lanes L, CeltDec *st, const uint8_t *data, int len, int16_t 
         init_caps(cap, LM, C);
         int dynalloc_logp = 6;
         total_bits <<= 3;
-        tell = (int32_t)rd_tell_frac(dec);
+        RangeDec d = *dec;   // in registers for the boosts
+        tell = (int32_t)rd_tell_frac(&d);
         ROLLED for (int i = start; i < end; i++) {
             int width = C * (eB[i + 1] - eB[i]) << LM;
             int quanta = imin(width << 3, imax(6 << 3, width));
             int dll = dynalloc_logp, boost = 0;
             ROLLED while (tell + (dll << 3) < total_bits && boost < cap[i]) {
-                int flag = rd_bit_logp(dec, dll);
-                tell = (int32_t)rd_tell_frac(dec);
+                int flag = rdi_bit_logp(&d, dll);
+                tell = (int32_t)rd_tell_frac(&d);
                 if (!flag) break;
                 boost += quanta;
                 total_bits -= quanta;
@@ -2326,17 +2410,11 @@ DNI int celt_decode(Lanes L, CeltDec *st, const uint8_t *data, int len, int16_t 
             offsets[i] = boost;
             if (boost > 0) dynalloc_logp = imax(2, dynalloc_logp - 1);
         }
+        *dec = d;
         int alloc_trim = tell + (6 << 3) <= total_bits ? rd_icdf(dec, T_celt_trim_icdf, 7) : 5;
         int32_t bits = (((int32_t)len * 8) << 3) - (int32_t)rd_tell_frac(dec) - 1;
         int anti_collapse_rsv = isTransient && LM >= 2 && bits >= ((LM + 2) << 3) ? (1 << 3) : 0;
         bits -= anti_collapse_rsv;
-        int intensity = 0, dual_stereo = 0;
-        int32_t balance;
-        PHASE_BEGIN(t_al);
-        int codedBands = clt_compute_allocation(start, end, offsets, cap, alloc_trim, &intensity, &dual_stereo,
-                                                bits, &balance, pulses, fine_quant, fine_priority, C, LM, dec, w);
-        PHASE_END(PH_CELT_ALLOC, t_al, L.id);
-        unquant_fine_energy(start, end, oldBandE, fine_quant, dec, C);
         hv[H_SILENCE] = silence;
         hv[H_PF_GAIN] = postfilter_gain;
         hv[H_PF_PITCH] = postfilter_pitch;
@@ -2344,20 +2422,23 @@ DNI int celt_decode(Lanes L, CeltDec *st, const uint8_t *data, int len, int16_t 
         hv[H_TRANSIENT] = isTransient;
         hv[H_SPREAD] = spread_decision;
         hv[H_AC_RSV] = anti_collapse_rsv;
-        hv[H_INTENSITY] = intensity;
-        hv[H_DUAL] = dual_stereo;
-        hv[H_BALANCE] = balance;
-        hv[H_CODED] = codedBands;
+        hv[H_TRIM] = alloc_trim;
+        hv[H_BITS] = bits;
     });
-    ROLLED for (int k = 0; k < H_N; k++) hv[k] = lbcast(L, hv[k]);
+    for (int k = 0; k < H_N; k++) hv[k] = lbcast(L, hv[k]);
+    int intensity = 0, dual_stereo = 0;
+    int32_t balance;
+    PHASE_BEGIN(t_al);
+    const int codedBands = clt_compute_allocation(L, start, end, w->offsets, w->cap, hv[H_TRIM], &intensity,
+                                                  &dual_stereo, hv[H_BITS], &balance, pulses, fine_quant,
+                                                  fine_priority, C, LM, dec, w);
+    PHASE_END(PH_CELT_ALLOC, t_al, L.id);
+    lead_rd(L, dec, [&]() CUO_INLINE { unquant_fine_energy(start, end, oldBandE, fine_quant, dec, C); });
     const int silence = hv[H_SILENCE];
     const int16_t postfilter_gain = (int16_t)hv[H_PF_GAIN];
     const int postfilter_pitch = hv[H_PF_PITCH], postfilter_tapset = hv[H_PF_TAPSET];
     const int isTransient = hv[H_TRANSIENT], shortBlocks = isTransient ? M : 0;
     const int spread_decision = hv[H_SPREAD], anti_collapse_rsv = hv[H_AC_RSV];
-    const int intensity = hv[H_INTENSITY], dual_stereo = hv[H_DUAL];
-    const int32_t balance = hv[H_BALANCE];
-    const int codedBands = hv[H_CODED];
     PHASE_BEGIN(t_sh);
     ROLLED for (int c = 0; c < CC; c++) lshift_copy(L, st->decode_mem[c], CELT_DEC_BUF - N + CELT_OVERLAP, N);
     PHASE_END(PH_CELT_SHIFT, t_sh, L.id);

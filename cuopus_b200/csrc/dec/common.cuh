@@ -61,6 +61,7 @@ struct LaneSim;
 void lanesim_sync(LaneSim *s, int id);
 int32_t lanesim_sum(LaneSim *s, int id, int32_t v);
 uint32_t lanesim_or(LaneSim *s, int id, uint32_t v);
+int32_t lanesim_max(LaneSim *s, int id, int32_t v);
 void lanesim_scan_affine(LaneSim *s, int id, uint32_t *a, uint32_t *b);
 void lanesim_bcast(LaneSim *s, int id, void *p, int bytes);
 #endif
@@ -193,6 +194,23 @@ DFN uint32_t lor(const Lanes &L, uint32_t v)
     ROLLED for (int off = L.n >> 1; off > 0; off >>= 1) v |= __shfl_xor_sync(L.mask, v, off);
 #elif defined(CUO_LANE_SIM)
     if (L.sim) v = lanesim_or(L.sim, L.id, v);
+#else
+    (void)L;
+#endif
+    return v;
+}
+
+// Maximum of v over the lanes of the group; every lane gets it.
+DFN int32_t lmax(const Lanes &L, int32_t v)
+{
+#ifdef __CUDA_ARCH__
+    if (L.n == 32) return __reduce_max_sync(0xffffffffu, v);
+    ROLLED for (int off = L.n >> 1; off > 0; off >>= 1) {
+        const int32_t o = __shfl_xor_sync(L.mask, v, off);
+        v = v > o ? v : o;
+    }
+#elif defined(CUO_LANE_SIM)
+    if (L.sim) v = lanesim_max(L.sim, L.id, v);
 #else
     (void)L;
 #endif

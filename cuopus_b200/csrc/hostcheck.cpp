@@ -215,7 +215,7 @@ int hc_alloc(const uint8_t *buf, uint32_t len, int start, int end, const int32_t
     cuo::RangeDec d;
     cuo::init_caps(cap, LM, C);
     cuo::rd_init(&d, buf, len);
-    int coded = cuo::clt_compute_allocation(start, end, offsets, cap, alloc_trim, &intensity, &dual_stereo, total,
+    int coded = cuo::clt_compute_allocation(cuo::Lanes{0, 1, 1u}, start, end, offsets, cap, alloc_trim, &intensity, &dual_stereo, total,
                                             &balance, pulses, ebits, fine_priority, C, LM, &d, &w);
     int k = 0;
     out[k++] = coded;
@@ -247,7 +247,7 @@ int hc_bands(const uint8_t *buf, uint32_t len, int start, int end, const int32_t
     cuo::init_caps(cap, LM, C);
     cuo::rd_init(&d, buf, len);
     int32_t bits = (int32_t)(len * 8 << 3) - (int32_t)cuo::rd_tell_frac(&d) - 1;
-    int coded = cuo::clt_compute_allocation(start, end, offsets, cap, alloc_trim, &intensity, &dual_stereo, bits,
+    int coded = cuo::clt_compute_allocation(cuo::Lanes{0, 1, 1u}, start, end, offsets, cap, alloc_trim, &intensity, &dual_stereo, bits,
                                             &balance, pulses, ebits, fine_priority, C, LM, &d, &w);
     uint32_t s = seed;
     cuo::quant_all_bands_dec(L, start, end, w.X, C == 2 ? w.X + N : nullptr, w.collapse_masks, pulses, shortBlocks,
@@ -274,7 +274,7 @@ int hc_energy(const uint8_t *buf, uint32_t len, int start, int end, int intra, c
     cuo::unquant_coarse_energy(start, end, oldE, intra, &d, C, LM);
     cuo::init_caps(cap, LM, C);
     int32_t bits = (int32_t)(len * 8 << 3) - (int32_t)cuo::rd_tell_frac(&d) - 1;
-    cuo::clt_compute_allocation(start, end, offsets, cap, alloc_trim, &intensity, &dual_stereo, bits, &balance,
+    cuo::clt_compute_allocation(cuo::Lanes{0, 1, 1u}, start, end, offsets, cap, alloc_trim, &intensity, &dual_stereo, bits, &balance,
                                 pulses, ebits, fine_priority, C, LM, &d, &w);
     cuo::unquant_fine_energy(start, end, oldE, ebits, &d, C);
     cuo::unquant_energy_finalise(start, end, oldE, ebits, fine_priority, (int)len * 8 - cuo::rd_tell(&d), &d, C);

@@ -212,6 +212,17 @@ int32_t lanesim_sum(LaneSim *s, int id, int32_t v)
     return (int32_t)t;
 }
 
+int32_t lanesim_max(LaneSim *s, int id, int32_t v) NOINSTR;
+int32_t lanesim_max(LaneSim *s, int id, int32_t v)
+{
+    s->xv[id] = v;
+    lanesim_sync(s, id);
+    int32_t t = v;
+    for (int i = 0; i < s->n; i++) t = s->xv[i] > t ? s->xv[i] : t;
+    lanesim_sync(s, id);
+    return t;
+}
+
 uint32_t lanesim_or(LaneSim *s, int id, uint32_t v) NOINSTR;
 uint32_t lanesim_or(LaneSim *s, int id, uint32_t v)
 {
