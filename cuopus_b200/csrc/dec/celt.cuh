@@ -77,7 +77,6 @@ struct CeltScratch {
     int16_t y_lp4[(CELT_DEC_BUF - 720 + 620) >> 2];    // (len + max_pitch) >> 2
     int32_t xcorr[CELT_MAX_PERIOD >> 1];
     int16_t ac_xx[CELT_MAX_PERIOD];
-    int16_t iir_y[CELT_MAX_PERIOD + CELT_OVERLAP + CELT_LPC_ORDER];
     int32_t etmp[CELT_OVERLAP];
 };
 
@@ -1850,61 +1849,85 @@ DNI void tf_decode(int start, int end, int isTransient, int32_t *tf_res, int LM,
 }
 
 // ------------------------------------------------------------------ PLC (pitch / LPC)
+//
+// Concealment runs on every lane: sums that wrap are split over the lanes, and
+// so are the sample loops; recursions keep their window in registers.  (On the
+// first lane alone a lost 20 ms CELT frame took several million cycles: the
+// correlations, the FIR and the IIR are 25 k multiply-adds each, one load pair
+// at a time.)
 
-DNI int32_t celt_autocorr(const int16_t *x, int32_t *ac, const int16_t *window, int overlap, int lag, int n,
-                          int16_t *xx)
+// celt/mathops.h celt_maxabs16 / celt_maxabs32 over the lanes
+template <class T> DFN int32_t c_maxabs_lanes(const Lanes &L, const T *x, int len)
 {
-    int fastN = n - lag, shift;
-    const int16_t *xptr;
-    if (overlap == 0) {
-        xptr = x;
-    } else {
-        ROLLED for (int i = 0; i < n; i++) xx[i] = x[i];
-        ROLLED for (int i = 0; i < overlap; i++) {
-            xx[i] = (int16_t)c_mul16_q15(x[i], window[i]);
-            xx[n - i - 1] = (int16_t)c_mul16_q15(x[n - i - 1], window[i]);
+    int32_t mx = 0, mn = 0;
+    LFOR(L, i, 0, len) {
+        const int32_t v = x[i];
+        mx = max32(mx, v);
+        mn = min32(mn, v);
+    }
+    return lmax(L, max32(mx, -mn));
+}
+
+// sum of x[i] y[i], n a multiple of 4, this lane alone
+DFN int32_t c_dot4(const int16_t *x, const int16_t *y, int n)
+{
+    int32_t s0 = 0, s1 = 0, s2 = 0, s3 = 0;
+    ROLLED for (int j = 0; j < n; j += 4) {
+        s0 = c_mac16(s0, x[j], y[j]);
+        s1 = c_mac16(s1, x[j + 1], y[j + 1]);
+        s2 = c_mac16(s2, x[j + 2], y[j + 2]);
+        s3 = c_mac16(s3, x[j + 3], y[j + 3]);
+    }
+    return wadd(wadd(s0, s1), wadd(s2, s3));
+}
+
+// Writes ac[0 .. lag] (the group's memory) and ends with a barrier.
+DNI void celt_autocorr(Lanes L, const int16_t *x, int32_t *ac, const int16_t *window, int overlap, int lag, int n,
+                       int16_t *xx)
+{
+    const int16_t *xptr = x;
+    int shift;
+    if (overlap) {
+        LFOR(L, i, 0, n) {
+            int16_t v = x[i];
+            if (i < overlap) v = (int16_t)c_mul16_q15(v, window[i]);
+            if (n - 1 - i < overlap) v = (int16_t)c_mul16_q15(x[i], window[n - 1 - i]);
+            xx[i] = v;
         }
+        lsync(L);
         xptr = xx;
     }
-    {
-        int32_t ac0 = 1 + (n << 7);
-        if (n & 1) ac0 = wadd(ac0, c_mul16(xptr[0], xptr[0]) >> 9);
-        ROLLED for (int i = (n & 1); i < n; i += 2) {
-            ac0 = wadd(ac0, c_mul16(xptr[i], xptr[i]) >> 9);
-            ac0 = wadd(ac0, c_mul16(xptr[i + 1], xptr[i + 1]) >> 9);
-        }
-        shift = c_ilog2(ac0) - 30 + 10;
-        shift = shift / 2;
-        if (shift > 0) {
-            ROLLED for (int i = 0; i < n; i++) xx[i] = (int16_t)c_pshr(xptr[i], shift);
-            xptr = xx;
-        } else {
-            shift = 0;
-        }
+    int32_t ac0 = 0;
+    LFOR(L, i, 0, n) ac0 = wadd(ac0, c_mul16(xptr[i], xptr[i]) >> 9);
+    ac0 = wadd(lsum(L, ac0), 1 + (n << 7));
+    shift = c_ilog2(ac0) - 30 + 10;
+    shift = shift / 2;
+    if (shift > 0) {
+        lsync(L);
+        LFOR(L, i, 0, n) xx[i] = (int16_t)c_pshr(xptr[i], shift);
+        lsync(L);
+        xptr = xx;
+    } else {
+        shift = 0;
     }
-    ROLLED for (int k = 0; k <= lag; k++) {
-        int32_t s = 0;
-        ROLLED for (int j = 0; j < fastN; j++) s = c_mac16(s, xptr[j], xptr[j + k]);
+    LFOR(L, k, 0, lag + 1) {
+        const int len = n - k, main = len & ~3;
+        int32_t s = c_dot4(xptr, xptr + k, main);
+        ROLLED for (int j = main; j < len; j++) s = c_mac16(s, xptr[j], xptr[j + k]);
         ac[k] = s;
     }
-    ROLLED for (int k = 0; k <= lag; k++) {
-        int32_t d = 0;
-        ROLLED for (int i = k + fastN; i < n; i++) d = c_mac16(d, xptr[i], xptr[i - k]);
-        ac[k] = wadd(ac[k], d);
-    }
-    shift = 2 * shift;
-    if (shift <= 0) ac[0] = wadd(ac[0], shl32(1, -shift));
-    if (ac[0] < 268435456) {
-        int shift2 = 29 - ilog((uint32_t)ac[0]);
-        ROLLED for (int i = 0; i <= lag; i++) ac[i] = shl32(ac[i], shift2);
-        shift -= shift2;
-    } else if (ac[0] >= 536870912) {
-        int shift2 = 1;
-        if (ac[0] >= 1073741824) shift2++;
-        ROLLED for (int i = 0; i <= lag; i++) ac[i] = ac[i] >> shift2;
-        shift += shift2;
-    }
-    return shift;
+    lead(L, [&]() CUO_INLINE {
+        shift = 2 * shift;
+        if (shift <= 0) ac[0] = wadd(ac[0], shl32(1, -shift));
+        if (ac[0] < 268435456) {
+            int shift2 = 29 - ilog((uint32_t)ac[0]);
+            ROLLED for (int i = 0; i <= lag; i++) ac[i] = shl32(ac[i], shift2);
+        } else if (ac[0] >= 536870912) {
+            int shift2 = 1;
+            if (ac[0] >= 1073741824) shift2++;
+            ROLLED for (int i = 0; i <= lag; i++) ac[i] = ac[i] >> shift2;
+        }
+    });
 }
 
 DNI void celt_lpc(int16_t *_lpc, const int32_t *ac, int p)
@@ -1956,39 +1979,80 @@ DNI void celt_lpc(int16_t *_lpc, const int32_t *ac, int p)
     }
 }
 
-DNI void celt_fir(const int16_t *x, const int16_t *num, int16_t *y, int N, int ord)
+// every output on its own: the lanes split them
+DNI void celt_fir(Lanes L, const int16_t *x, const int16_t *num, int16_t *y, int N)
 {
-    ROLLED for (int i = 0; i < N; i++) {
-        int32_t sum = shl32((int32_t)x[i], 12);
-        ROLLED for (int j = 0; j < ord; j++) sum = c_mac16(sum, num[ord - j - 1], x[i + j - ord]);
-        y[i] = c_sround16(sum, 12);
+    int32_t a[CELT_LPC_ORDER];
+#pragma unroll
+    for (int j = 0; j < CELT_LPC_ORDER; j++) a[j] = num[j];
+    LFOR(L, i, 0, N) {
+        int32_t sum = shl32((int32_t)x[i], 12), sum1 = 0;
+#pragma unroll
+        for (int j = 0; j < CELT_LPC_ORDER; j += 2) {
+            sum = c_mac16(sum, a[j], x[i - j - 1]);
+            sum1 = c_mac16(sum1, a[j + 1], x[i - j - 2]);
+        }
+        y[i] = c_sround16(wadd(sum, sum1), 12);
     }
+    lsync(L);
 }
 
-// celt/celt_lpc.c celt_iir (the 4-way unrolled form computes the same values)
-DNI void celt_iir(const int32_t *_x, const int16_t *den, int32_t *_y, int N, int ord, int16_t *mem, int16_t *y)
+// celt/celt_lpc.c celt_iir, in place on x (the 4-way unrolled form computes the
+// same values), with the saturation of the extrapolated signal.  Four samples
+// at a time with the filter memory (y, negated and rounded outputs) in
+// registers, as in silk_lpc_synth; every lane runs it and the first one stores.
+DNI void celt_iir(Lanes L, int32_t *x, const int16_t *den, int N, const int16_t *mem)
 {
-    ROLLED for (int i = 0; i < ord; i++) y[i] = (int16_t)-mem[ord - i - 1];
-    ROLLED for (int i = ord; i < N + ord; i++) y[i] = 0;
-    ROLLED for (int i = 0; i < N; i++) {
-        int32_t sum = _x[i];
-        ROLLED for (int j = 0; j < ord; j++) sum = c_mac16(sum, den[ord - j - 1], y[i + j]);
-        y[i + ord] = (int16_t)-c_sround16(sum, 12);
-        _y[i] = sum;
+    int32_t a[CELT_LPC_ORDER], y[CELT_LPC_ORDER];   // y[0] oldest
+#pragma unroll
+    for (int j = 0; j < CELT_LPC_ORDER; j++) {
+        a[j] = den[j];
+        y[j] = (int16_t)-mem[CELT_LPC_ORDER - 1 - j];
     }
-    ROLLED for (int i = 0; i < ord; i++) mem[i] = (int16_t)_y[N - i - 1];
+    int32_t ahead[4];
+#pragma unroll
+    for (int s = 0; s < 4; s++) ahead[s] = x[s];
+    ROLLED for (int i = 0; i < N; i += 4) {
+        int32_t v[4], o[4];
+        const int nx = i + 4 < N ? i + 4 : i;
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+            v[s] = ahead[s];
+            ahead[s] = x[nx + s];
+        }
+        lsync(L);   // every lane has read what the first lane overwrites below
+#pragma unroll
+        for (int j = CELT_LPC_ORDER - 1; j >= 0; j--) {
+#pragma unroll
+            for (int s = 0; s < 4; s++)
+                if (j >= s) v[s] = c_mac16(v[s], a[j], y[CELT_LPC_ORDER - 1 + s - j]);
+        }
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+#pragma unroll
+            for (int t = 0; t < s; t++) v[s] = c_mac16(v[s], a[s - 1 - t], o[t]);
+            o[s] = (int16_t)-c_sround16(v[s], 12);
+        }
+#pragma unroll
+        for (int j = 0; j < CELT_LPC_ORDER - 4; j++) y[j] = y[j + 4];
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+            y[CELT_LPC_ORDER - 4 + s] = o[s];
+            if (L.id == 0) x[i + s] = c_sat(v[s], CELT_SIG_SAT);
+        }
+    }
+    lsync(L);
 }
 
+// Syy: 1 plus the energy of the first len samples of y.
 DNI void find_best_pitch(const int32_t *xcorr, const int16_t *y, int len, int max_pitch, int *best_pitch,
-                         int yshift, int32_t maxcorr)
+                         int yshift, int32_t maxcorr, int32_t Syy)
 {
-    int32_t Syy = 1;
     int16_t best_num[2] = {-1, -1};
     int32_t best_den[2] = {0, 0};
     int xshift = c_ilog2(maxcorr) - 14;
     best_pitch[0] = 0;
     best_pitch[1] = 1;
-    ROLLED for (int j = 0; j < len; j++) Syy = wadd(Syy, c_mul16(y[j], y[j]) >> yshift);
     ROLLED for (int i = 0; i < max_pitch; i++) {
         if (xcorr[i] > 0) {
             int16_t xcorr16 = (int16_t)c_vshr(xcorr[i], xshift);
@@ -2013,30 +2077,35 @@ DNI void find_best_pitch(const int32_t *xcorr, const int16_t *y, int len, int ma
     }
 }
 
-DNI void pitch_downsample(int32_t *x0, int32_t *x1, int16_t *x_lp, int len, int C, int16_t *xx)
+DNI void pitch_downsample(Lanes L, int32_t *x0, int32_t *x1, int16_t *x_lp, int len, int C, int16_t *xx, int32_t *ac)
 {
-    int32_t ac[5];
     int16_t tmp = 32767, lpc[4], lpc2[5];
     const int16_t c1 = 26214;   // QCONST16(.8f, 15)
-    int32_t maxabs = c_maxabs32(x0, len);
-    if (C == 2) maxabs = max32(maxabs, c_maxabs32(x1, len));
+    int32_t maxabs = c_maxabs_lanes(L, x0, len);
+    if (C == 2) maxabs = max32(maxabs, c_maxabs_lanes(L, x1, len));
     if (maxabs < 1) maxabs = 1;
     int shift = c_ilog2(maxabs) - 10;
     if (shift < 0) shift = 0;
     if (C == 2) shift++;
-    ROLLED for (int i = 1; i < len >> 1; i++)
-        x_lp[i] = (int16_t)((x0[2 * i - 1] >> (shift + 2)) + (x0[2 * i + 1] >> (shift + 2)) + (x0[2 * i] >> (shift + 1)));
-    x_lp[0] = (int16_t)((x0[1] >> (shift + 2)) + (x0[0] >> (shift + 1)));
-    if (C == 2) {
-        ROLLED for (int i = 1; i < len >> 1; i++)
-            x_lp[i] = (int16_t)(x_lp[i] + (x1[2 * i - 1] >> (shift + 2)) + (x1[2 * i + 1] >> (shift + 2)) +
-                                (x1[2 * i] >> (shift + 1)));
-        x_lp[0] = (int16_t)(x_lp[0] + (x1[1] >> (shift + 2)) + (x1[0] >> (shift + 1)));
+    LFOR(L, i, 0, len >> 1) {
+        int32_t v = (x0[2 * i + 1] >> (shift + 2)) + (x0[2 * i] >> (shift + 1));
+        if (i) v += x0[2 * i - 1] >> (shift + 2);
+        if (C == 2) {
+            v += (x1[2 * i + 1] >> (shift + 2)) + (x1[2 * i] >> (shift + 1));
+            if (i) v += x1[2 * i - 1] >> (shift + 2);
+        }
+        x_lp[i] = (int16_t)v;
     }
-    celt_autocorr(x_lp, ac, 0, 0, 4, len >> 1, xx);
-    ac[0] = wadd(ac[0], ac[0] >> 13);
-    ROLLED for (int i = 1; i <= 4; i++) ac[i] = wsub(ac[i], c_mul16_32_q15(2 * i * i, ac[i]));
-    celt_lpc(lpc, ac, 4);
+    lsync(L);
+    celt_autocorr(L, x_lp, ac, 0, 0, 4, len >> 1, xx);
+    int32_t acl[5];
+#pragma unroll
+    for (int i = 0; i < 5; i++) acl[i] = ac[i];
+    acl[0] = wadd(acl[0], acl[0] >> 13);
+#pragma unroll
+    for (int i = 1; i <= 4; i++) acl[i] = wsub(acl[i], c_mul16_32_q15(2 * i * i, acl[i]));
+    lpc[0] = lpc[1] = lpc[2] = lpc[3] = 0;
+    celt_lpc(lpc, acl, 4);
     ROLLED for (int i = 0; i < 4; i++) {
         tmp = (int16_t)c_mul16_q15(29491, tmp);   // QCONST16(.9f, 15)
         lpc[i] = (int16_t)c_mul16_q15(lpc[i], tmp);
@@ -2046,87 +2115,109 @@ DNI void pitch_downsample(int32_t *x0, int32_t *x1, int16_t *x_lp, int len, int 
     lpc2[2] = (int16_t)(lpc[2] + c_mul16_q15(c1, lpc[1]));
     lpc2[3] = (int16_t)(lpc[3] + c_mul16_q15(c1, lpc[2]));
     lpc2[4] = (int16_t)c_mul16_q15(c1, lpc[3]);
-    // celt_fir5 in place
-    int32_t m0 = 0, m1 = 0, m2 = 0, m3 = 0, m4 = 0;
-    ROLLED for (int i = 0; i < len >> 1; i++) {
+    // celt_fir5 of the unfiltered samples, through xx
+    lsync(L);
+    LFOR(L, i, 0, len >> 1) {
         int32_t sum = shl32((int32_t)x_lp[i], 12);
-        sum = c_mac16(sum, lpc2[0], m0);
-        sum = c_mac16(sum, lpc2[1], m1);
-        sum = c_mac16(sum, lpc2[2], m2);
-        sum = c_mac16(sum, lpc2[3], m3);
-        sum = c_mac16(sum, lpc2[4], m4);
-        m4 = m3; m3 = m2; m2 = m1; m1 = m0;
-        m0 = x_lp[i];
-        x_lp[i] = (int16_t)c_pshr(sum, 12);
+#pragma unroll
+        for (int j = 0; j < 5; j++)
+            if (i > j) sum = c_mac16(sum, lpc2[j], x_lp[i - 1 - j]);
+        xx[i] = (int16_t)c_pshr(sum, 12);
     }
+    lsync(L);
+    LFOR(L, i, 0, len >> 1) x_lp[i] = xx[i];
+    lsync(L);
 }
 
-DNI void pitch_search(Lanes L, const int16_t *x_lp, int16_t *y, int len, int max_pitch, int *pitch,
-                      CeltScratch *w)
+// Sum of squares of y[0 .. len), each shifted, plus 1 (find_best_pitch's Syy).
+DFN int32_t c_energy_lanes(const Lanes &L, const int16_t *y, int len, int shift)
+{
+    int32_t s = 0;
+    LFOR(L, j, 0, len) s = wadd(s, c_mul16(y[j], y[j]) >> shift);
+    return wadd(1, lsum(L, s));
+}
+
+// The pitch, on every lane.  (len >> 2 and len >> 1 are multiples of 4.)
+DNI int pitch_search(Lanes L, const int16_t *x_lp, int16_t *y, int len, int max_pitch, CeltScratch *w)
 {
     int lag = len + max_pitch;
     int best_pitch[2] = {0, 0};
     int16_t *x_lp4 = w->x_lp4, *y_lp4 = w->y_lp4;
     int32_t *xcorr = w->xcorr;
-    ROLLED for (int j = 0; j < len >> 2; j++) x_lp4[j] = x_lp[2 * j];
-    ROLLED for (int j = 0; j < lag >> 2; j++) y_lp4[j] = y[2 * j];
-    int32_t xmax = c_maxabs16(x_lp4, len >> 2), ymax = c_maxabs16(y_lp4, lag >> 2);
+    LFOR(L, j, 0, len >> 2) x_lp4[j] = x_lp[2 * j];
+    LFOR(L, j, 0, lag >> 2) y_lp4[j] = y[2 * j];
+    lsync(L);
+    int32_t xmax = c_maxabs_lanes(L, x_lp4, len >> 2), ymax = c_maxabs_lanes(L, y_lp4, lag >> 2);
     int shift = c_ilog2(max32(1, max32(xmax, ymax))) - 11;
     if (shift > 0) {
-        ROLLED for (int j = 0; j < len >> 2; j++) x_lp4[j] = (int16_t)(x_lp4[j] >> shift);
-        ROLLED for (int j = 0; j < lag >> 2; j++) y_lp4[j] = (int16_t)(y_lp4[j] >> shift);
+        lsync(L);
+        LFOR(L, j, 0, len >> 2) x_lp4[j] = (int16_t)(x_lp4[j] >> shift);
+        LFOR(L, j, 0, lag >> 2) y_lp4[j] = (int16_t)(y_lp4[j] >> shift);
         shift *= 2;
     } else {
         shift = 0;
     }
     lsync(L);
     // celt_pitch_xcorr: every lag is an independent dot product
-    LFOR(L, i, 0, max_pitch >> 2) {
-        int32_t s = 0;
-        ROLLED for (int j = 0; j < len >> 2; j++) s = c_mac16(s, x_lp4[j], y_lp4[i + j]);
-        xcorr[i] = s;
-    }
-    lsync(L);
     int32_t maxcorr = 1;
-    ROLLED for (int i = 0; i < max_pitch >> 2; i++) maxcorr = max32(maxcorr, xcorr[i]);
-    find_best_pitch(xcorr, y_lp4, len >> 2, max_pitch >> 2, best_pitch, 0, maxcorr);
-    lsync(L);
-    LFOR(L, i, 0, max_pitch >> 1) {
-        xcorr[i] = 0;
-        int d0 = i - 2 * best_pitch[0], d1 = i - 2 * best_pitch[1];
-        if (!((d0 < 0 ? -d0 : d0) > 2 && (d1 < 0 ? -d1 : d1) > 2)) {
-            int32_t s = 0;
-            ROLLED for (int j = 0; j < len >> 1; j++) s = wadd(s, c_mul16(x_lp[j], y[i + j]) >> shift);
-            xcorr[i] = max32(-1, s);
-        }
+    LFOR(L, i, 0, max_pitch >> 2) {
+        xcorr[i] = c_dot4(x_lp4, y_lp4 + i, len >> 2);
+        maxcorr = max32(maxcorr, xcorr[i]);
     }
-    lsync(L);
+    maxcorr = lmax(L, maxcorr);
+    int32_t Syy = c_energy_lanes(L, y_lp4, len >> 2, 0);
+    lead(L, [&]() CUO_INLINE { find_best_pitch(xcorr, y_lp4, len >> 2, max_pitch >> 2, best_pitch, 0, maxcorr, Syy); });
+    best_pitch[0] = lbcast(L, best_pitch[0]);
+    best_pitch[1] = lbcast(L, best_pitch[1]);
     // libopus tracks max(1, raw sums); the -1 floor and the zeroed lags cannot exceed 1
     maxcorr = 1;
-    ROLLED for (int i = 0; i < max_pitch >> 1; i++) maxcorr = max32(maxcorr, xcorr[i]);
-    find_best_pitch(xcorr, y, len >> 1, max_pitch >> 1, best_pitch, shift + 1, maxcorr);
-    int offset;
-    if (best_pitch[0] > 0 && best_pitch[0] < (max_pitch >> 1) - 1) {
-        int32_t a = xcorr[best_pitch[0] - 1], b = xcorr[best_pitch[0]], c = xcorr[best_pitch[0] + 1];
-        if ((c - a) > c_mul16_32_q15(22938, b - a)) offset = 1;          // QCONST16(.7f, 15)
-        else if ((a - c) > c_mul16_32_q15(22938, b - c)) offset = -1;
-        else offset = 0;
-    } else {
-        offset = 0;
+    LFOR(L, i, 0, max_pitch >> 1) {
+        int32_t v = 0;
+        int d0 = i - 2 * best_pitch[0], d1 = i - 2 * best_pitch[1];
+        if (!((d0 < 0 ? -d0 : d0) > 2 && (d1 < 0 ? -d1 : d1) > 2)) {
+            int32_t s0 = 0, s1 = 0;
+            ROLLED for (int j = 0; j < len >> 1; j += 4) {
+                s0 = wadd(s0, c_mul16(x_lp[j], y[i + j]) >> shift);
+                s1 = wadd(s1, c_mul16(x_lp[j + 1], y[i + j + 1]) >> shift);
+                s0 = wadd(s0, c_mul16(x_lp[j + 2], y[i + j + 2]) >> shift);
+                s1 = wadd(s1, c_mul16(x_lp[j + 3], y[i + j + 3]) >> shift);
+            }
+            v = max32(-1, wadd(s0, s1));
+        }
+        xcorr[i] = v;
+        maxcorr = max32(maxcorr, v);
     }
-    *pitch = 2 * best_pitch[0] - offset;
+    maxcorr = lmax(L, maxcorr);
+    Syy = c_energy_lanes(L, y, len >> 1, shift + 1);
+    int pitch = 0;
+    lead(L, [&]() CUO_INLINE {
+        find_best_pitch(xcorr, y, len >> 1, max_pitch >> 1, best_pitch, shift + 1, maxcorr, Syy);
+        int offset;
+        if (best_pitch[0] > 0 && best_pitch[0] < (max_pitch >> 1) - 1) {
+            int32_t a = xcorr[best_pitch[0] - 1], b = xcorr[best_pitch[0]], c = xcorr[best_pitch[0] + 1];
+            if ((c - a) > c_mul16_32_q15(22938, b - a)) offset = 1;          // QCONST16(.7f, 15)
+            else if ((a - c) > c_mul16_32_q15(22938, b - c)) offset = -1;
+            else offset = 0;
+        } else {
+            offset = 0;
+        }
+        pitch = 2 * best_pitch[0] - offset;
+    });
+    return lbcast(L, pitch);
 }
 
-DNI void prefilter_and_fold(CeltDec *st, int N, CeltScratch *w)
+DNI void prefilter_and_fold(Lanes L, CeltDec *st, int N, CeltScratch *w)
 {
     ROLLED for (int c = 0; c < st->channels; c++) {
         int32_t *dm = st->decode_mem[c];
-        comb_filter(w->etmp, dm + CELT_DEC_BUF - N, st->postfilter_period_old, st->postfilter_period, CELT_OVERLAP,
-                    (int16_t)-st->postfilter_gain_old, (int16_t)-st->postfilter_gain, st->postfilter_tapset_old,
-                    st->postfilter_tapset, 0, 0);
-        ROLLED for (int i = 0; i < CELT_OVERLAP / 2; i++)
+        comb_filter_lanes(L, w->etmp, dm + CELT_DEC_BUF - N, st->postfilter_period_old, st->postfilter_period,
+                          CELT_OVERLAP, (int16_t)-st->postfilter_gain_old, (int16_t)-st->postfilter_gain,
+                          st->postfilter_tapset_old, st->postfilter_tapset, 0, 0);
+        lsync(L);
+        LFOR(L, i, 0, CELT_OVERLAP / 2)
             dm[CELT_DEC_BUF - N + i] = wadd(c_mul16_32_q15(T_celt_window[i], w->etmp[CELT_OVERLAP - 1 - i]),
                                             c_mul16_32_q15(T_celt_window[CELT_OVERLAP - i - 1], w->etmp[i]));
+        lsync(L);
     }
 }
 
@@ -2137,18 +2228,18 @@ DNI void celt_decode_lost(Lanes L, CeltDec *st, int N, int LM, CeltScratch *w)
     const int16_t *eB = T_celt_eBands;
     int32_t *out_syn[2];
     ROLLED for (int c = 0; c < C; c++) out_syn[c] = st->decode_mem[c] + CELT_DEC_BUF - N;
-    int loss_duration = st->loss_duration;
-    int start = st->start;
-    int noise_based = loss_duration >= 40 || start != 0 || st->skip_plc;
+    const int loss_duration = st->loss_duration;
+    const int start = st->start;
+    const int noise_based = loss_duration >= 40 || start != 0 || st->skip_plc;
     if (noise_based) {
-        int end = st->end;
-        int effEnd = imax(start, imin(end, T_CELT_EFFEBANDS));
+        const int end = st->end;
+        const int effEnd = imax(start, imin(end, T_CELT_EFFEBANDS));
         int16_t *X = w->X;
         ROLLED for (int c = 0; c < C; c++) lshift_copy(L, st->decode_mem[c], CELT_DEC_BUF - N + CELT_OVERLAP, N);
-        if (st->prefilter_and_fold) prefilter_and_fold(st, N, w);
+        if (st->prefilter_and_fold) prefilter_and_fold(L, st, N, w);
         int16_t decay = loss_duration == 0 ? 1536 : 512;   // QCONST16(1.5f / .5f, DB_SHIFT)
         ROLLED for (int c = 0; c < C; c++)
-            ROLLED for (int i = start; i < end; i++) {
+            LFOR(L, i, start, end) {
                 int32_t a = st->backgroundLogE[c * CELT_NB + i];
                 int32_t b = st->oldBandE[c * CELT_NB + i] - decay;
                 st->oldBandE[c * CELT_NB + i] = (int16_t)(a > b ? a : b);
@@ -2156,121 +2247,125 @@ DNI void celt_decode_lost(Lanes L, CeltDec *st, int N, int LM, CeltScratch *w)
         uint32_t seed = st->rng;
         ROLLED for (int c = 0; c < C; c++) {
             ROLLED for (int i = start; i < effEnd; i++) {
-                int boffs = N * c + (eB[i] << LM);
-                int blen = (eB[i + 1] - eB[i]) << LM;
-                ROLLED for (int j = 0; j < blen; j++) {
-                    seed = c_lcg_rand(seed);
-                    X[boffs + j] = (int16_t)((int32_t)seed >> 20);
-                }
+                const int boffs = N * c + (eB[i] << LM);
+                const int blen = (eB[i + 1] - eB[i]) << LM;
+                LFOR(L, j, 0, blen) X[boffs + j] = (int16_t)((int32_t)(T_lcg.a[j + 1] * seed + T_lcg.c[j + 1]) >> 20);
+                seed = T_lcg.a[blen] * seed + T_lcg.c[blen];
+                lsync(L);
                 renormalise_vector(L, X + boffs, blen, 32767);
             }
         }
-        st->rng = seed;
-        lsync(L);
         celt_synthesis(L, w, X, out_syn, st->oldBandE, start, effEnd, C, C, 0, LM, 0);
-        st->prefilter_and_fold = 0;
-        st->skip_plc = 1;
+        lead(L, [&]() CUO_INLINE {
+            st->rng = seed;
+            st->prefilter_and_fold = 0;
+            st->skip_plc = 1;
+        });
     } else {
         int16_t fade = 32767;
         int pitch_index;
         if (loss_duration == 0) {
-            pitch_downsample(st->decode_mem[0], st->decode_mem[1], w->lp_pitch_buf, CELT_DEC_BUF, C, w->ac_xx);
-            lsync(L);
-            pitch_search(L, w->lp_pitch_buf + (720 >> 1), w->lp_pitch_buf, CELT_DEC_BUF - 720, 720 - 100,
-                         &pitch_index, w);
-            pitch_index = 720 - pitch_index;
-            st->last_pitch_index = pitch_index;
+            pitch_downsample(L, st->decode_mem[0], st->decode_mem[1], w->lp_pitch_buf, CELT_DEC_BUF, C, w->ac_xx, w->etmp);
+            pitch_index = 720 - pitch_search(L, w->lp_pitch_buf + (720 >> 1), w->lp_pitch_buf, CELT_DEC_BUF - 720,
+                                             720 - 100, w);
         } else {
             pitch_index = st->last_pitch_index;
             fade = 26214;   // QCONST16(.8f, 15)
         }
-        int exc_length = imin(2 * pitch_index, CELT_MAX_PERIOD);
+        const int exc_length = imin(2 * pitch_index, CELT_MAX_PERIOD);
         int16_t *exc = w->exc + CELT_LPC_ORDER;
         const int16_t *window = T_celt_window;
         ROLLED for (int c = 0; c < C; c++) {
             int32_t *buf = st->decode_mem[c];
             int16_t *lpc = st->lpc[c];
-            int32_t S1 = 0;
-            ROLLED for (int i = 0; i < CELT_MAX_PERIOD + CELT_LPC_ORDER; i++)
+            lsync(L);
+            LFOR(L, i, 0, CELT_MAX_PERIOD + CELT_LPC_ORDER)
                 exc[i - CELT_LPC_ORDER] = c_sround16(buf[CELT_DEC_BUF - CELT_MAX_PERIOD - CELT_LPC_ORDER + i], 12);
+            lsync(L);
             if (loss_duration == 0) {
-                int32_t ac[CELT_LPC_ORDER + 1];
-                celt_autocorr(exc, ac, window, CELT_OVERLAP, CELT_LPC_ORDER, CELT_MAX_PERIOD, w->ac_xx);
-                ac[0] = wadd(ac[0], ac[0] >> 13);
-                ROLLED for (int i = 1; i <= CELT_LPC_ORDER; i++) ac[i] = wsub(ac[i], c_mul16_32_q15(2 * i * i, ac[i]));
-                celt_lpc(lpc, ac, CELT_LPC_ORDER);
-                ROLLED while (1) {
-                    int16_t tmp = 32767;
-                    int32_t sum = 4096;   // QCONST16(1., SIG_SHIFT)
-                    ROLLED for (int i = 0; i < CELT_LPC_ORDER; i++) sum += lpc[i] < 0 ? -lpc[i] : lpc[i];
-                    if (sum < 65535) break;
-                    ROLLED for (int i = 0; i < CELT_LPC_ORDER; i++) {
-                        tmp = (int16_t)c_mul16_q15(32440, tmp);   // QCONST16(.99f, 15)
-                        lpc[i] = (int16_t)c_mul16_q15(lpc[i], tmp);
+                int32_t *ac = w->etmp;
+                celt_autocorr(L, exc, ac, window, CELT_OVERLAP, CELT_LPC_ORDER, CELT_MAX_PERIOD, w->ac_xx);
+                lead(L, [&]() CUO_INLINE {
+                    ac[0] = wadd(ac[0], ac[0] >> 13);
+                    ROLLED for (int i = 1; i <= CELT_LPC_ORDER; i++) ac[i] = wsub(ac[i], c_mul16_32_q15(2 * i * i, ac[i]));
+                    celt_lpc(lpc, ac, CELT_LPC_ORDER);
+                    ROLLED while (1) {
+                        int16_t tmp = 32767;
+                        int32_t sum = 4096;   // QCONST16(1., SIG_SHIFT)
+                        ROLLED for (int i = 0; i < CELT_LPC_ORDER; i++) sum += lpc[i] < 0 ? -lpc[i] : lpc[i];
+                        if (sum < 65535) break;
+                        ROLLED for (int i = 0; i < CELT_LPC_ORDER; i++) {
+                            tmp = (int16_t)c_mul16_q15(32440, tmp);   // QCONST16(.99f, 15)
+                            lpc[i] = (int16_t)c_mul16_q15(lpc[i], tmp);
+                        }
                     }
-                }
+                });
             }
-            celt_fir(exc + CELT_MAX_PERIOD - exc_length, lpc, w->fir_tmp, exc_length, CELT_LPC_ORDER);
-            ROLLED for (int i = 0; i < exc_length; i++) exc[CELT_MAX_PERIOD - exc_length + i] = w->fir_tmp[i];
+            celt_fir(L, exc + CELT_MAX_PERIOD - exc_length, lpc, w->fir_tmp, exc_length);
+            LFOR(L, i, 0, exc_length) exc[CELT_MAX_PERIOD - exc_length + i] = w->fir_tmp[i];
+            lsync(L);
             int16_t decay;
             {
-                int32_t E1 = 1, E2 = 1;
-                int shift = imax(0, 2 * c_zlog2(c_maxabs16(&exc[CELT_MAX_PERIOD - exc_length], exc_length)) - 20);
-                int decay_length = exc_length >> 1;
-                ROLLED for (int i = 0; i < decay_length; i++) {
+                int shift = imax(0, 2 * c_zlog2(c_maxabs_lanes(L, &exc[CELT_MAX_PERIOD - exc_length], exc_length)) - 20);
+                const int decay_length = exc_length >> 1;
+                int32_t E1 = 0, E2 = 0;
+                LFOR(L, i, 0, decay_length) {
                     int16_t e = exc[CELT_MAX_PERIOD - decay_length + i];
                     E1 = wadd(E1, c_mul16(e, e) >> shift);
                     e = exc[CELT_MAX_PERIOD - 2 * decay_length + i];
                     E2 = wadd(E2, c_mul16(e, e) >> shift);
                 }
+                E1 = wadd(1, lsum(L, E1));
+                E2 = wadd(1, lsum(L, E2));
                 E1 = min32(E1, E2);
                 decay = (int16_t)c_sqrt(c_frac_div32(E1 >> 1, E2));
             }
-            ROLLED for (int i = 0; i < CELT_DEC_BUF - N; i++) buf[i] = buf[i + N];
-            int extrapolation_offset = CELT_MAX_PERIOD - pitch_index;
-            int extrapolation_len = N + CELT_OVERLAP;
+            lshift_copy(L, buf, CELT_DEC_BUF - N, N);
+            const int extrapolation_offset = CELT_MAX_PERIOD - pitch_index;
+            const int extrapolation_len = N + CELT_OVERLAP;
             int16_t attenuation = (int16_t)c_mul16_q15(fade, decay);
-            ROLLED for (int i = 0, j = 0; i < extrapolation_len; i++, j++) {
-                if (j >= pitch_index) {
-                    j -= pitch_index;
-                    attenuation = (int16_t)c_mul16_q15(attenuation, decay);
+            // period after period of the excitation, each weaker than the last
+            int32_t S1 = 0;
+            ROLLED for (int b = 0; b < extrapolation_len; b += pitch_index) {
+                LFOR(L, j, 0, imin(pitch_index, extrapolation_len - b)) {
+                    buf[CELT_DEC_BUF - N + b + j] = shl32((int32_t)(int16_t)c_mul16_q15(attenuation,
+                                                          exc[extrapolation_offset + j]), 12);
+                    int16_t tmp = c_sround16(buf[CELT_DEC_BUF - CELT_MAX_PERIOD - N + extrapolation_offset + j], 12);
+                    S1 = wadd(S1, c_mul16(tmp, tmp) >> 10);
                 }
-                buf[CELT_DEC_BUF - N + i] = shl32((int32_t)(int16_t)c_mul16_q15(attenuation,
-                                                  exc[extrapolation_offset + j]), 12);
-                int16_t tmp = c_sround16(buf[CELT_DEC_BUF - CELT_MAX_PERIOD - N + extrapolation_offset + j], 12);
-                S1 = wadd(S1, c_mul16(tmp, tmp) >> 10);
+                attenuation = (int16_t)c_mul16_q15(attenuation, decay);
             }
-            {
-                int16_t lpc_mem[CELT_LPC_ORDER];
-                ROLLED for (int i = 0; i < CELT_LPC_ORDER; i++) lpc_mem[i] = c_sround16(buf[CELT_DEC_BUF - N - 1 - i], 12);
-                celt_iir(buf + CELT_DEC_BUF - N, lpc, buf + CELT_DEC_BUF - N, extrapolation_len, CELT_LPC_ORDER,
-                         lpc_mem, w->iir_y);
-                ROLLED for (int i = 0; i < extrapolation_len; i++)
-                    buf[CELT_DEC_BUF - N + i] = c_sat(buf[CELT_DEC_BUF - N + i], CELT_SIG_SAT);
+            S1 = lsum(L, S1);
+            lsync(L);
+            int16_t lpc_mem[CELT_LPC_ORDER];
+#pragma unroll
+            for (int i = 0; i < CELT_LPC_ORDER; i++) lpc_mem[i] = c_sround16(buf[CELT_DEC_BUF - N - 1 - i], 12);
+            celt_iir(L, buf + CELT_DEC_BUF - N, lpc, extrapolation_len, lpc_mem);
+            int32_t S2 = 0;
+            LFOR(L, i, 0, extrapolation_len) {
+                int16_t tmp = c_sround16(buf[CELT_DEC_BUF - N + i], 12);
+                S2 = wadd(S2, c_mul16(tmp, tmp) >> 10);
             }
-            {
-                int32_t S2 = 0;
-                ROLLED for (int i = 0; i < extrapolation_len; i++) {
-                    int16_t tmp = c_sround16(buf[CELT_DEC_BUF - N + i], 12);
-                    S2 = wadd(S2, c_mul16(tmp, tmp) >> 10);
-                }
-                if (!(S1 > (S2 >> 2))) {
-                    ROLLED for (int i = 0; i < extrapolation_len; i++) buf[CELT_DEC_BUF - N + i] = 0;
-                } else if (S1 < S2) {
-                    int16_t ratio = (int16_t)c_sqrt(c_frac_div32((S1 >> 1) + 1, S2 + 1));
-                    ROLLED for (int i = 0; i < CELT_OVERLAP; i++) {
-                        int16_t tmp_g = (int16_t)(32767 - c_mul16_q15(window[i], (int16_t)(32767 - ratio)));
-                        buf[CELT_DEC_BUF - N + i] = c_mul16_32_q15(tmp_g, buf[CELT_DEC_BUF - N + i]);
-                    }
-                    ROLLED for (int i = CELT_OVERLAP; i < extrapolation_len; i++)
-                        buf[CELT_DEC_BUF - N + i] = c_mul16_32_q15(ratio, buf[CELT_DEC_BUF - N + i]);
+            S2 = lsum(L, S2);
+            lsync(L);
+            if (!(S1 > (S2 >> 2))) {
+                LFOR(L, i, 0, extrapolation_len) buf[CELT_DEC_BUF - N + i] = 0;
+            } else if (S1 < S2) {
+                const int16_t ratio = (int16_t)c_sqrt(c_frac_div32((S1 >> 1) + 1, S2 + 1));
+                LFOR(L, i, 0, extrapolation_len) {
+                    const int16_t tmp_g = i < CELT_OVERLAP
+                        ? (int16_t)(32767 - c_mul16_q15(window[i], (int16_t)(32767 - ratio))) : ratio;
+                    buf[CELT_DEC_BUF - N + i] = c_mul16_32_q15(tmp_g, buf[CELT_DEC_BUF - N + i]);
                 }
             }
+            lsync(L);
         }
-        st->prefilter_and_fold = 1;
+        lead(L, [&]() CUO_INLINE {
+            st->last_pitch_index = pitch_index;
+            st->prefilter_and_fold = 1;
+        });
     }
-    st->loss_duration = imin(10000, loss_duration + (1 << LM));
-    lsync(L);
+    lead(L, [&]() CUO_INLINE { st->loss_duration = imin(10000, loss_duration + (1 << LM)); });
 }
 
 // ------------------------------------------------------------------ frame decode
@@ -2326,9 +2421,8 @@ DNI int celt_decode(Lanes L, CeltDec *st, const uint8_t *data, int len, int16_t 
     int effEnd = end;
     if (effEnd > T_CELT_EFFEBANDS) effEnd = T_CELT_EFFEBANDS;
     if (data == 0 || len <= 1) {
-        // concealment (mode transitions, lost packets): serial extrapolation
-        // and state updates in place, on the first lane as a group of one
-        lead(L, [&]() CUO_INLINE { celt_decode_lost(lone(L), st, N, LM, w); });
+        // concealment (mode transitions, lost packets)
+        celt_decode_lost(L, st, N, LM, w);
         deemphasis(L, out_syn[0], out_syn[1], pcm, N, CC, st->preemph_memD, accum);
         return frame_size;
     }
@@ -2463,8 +2557,8 @@ DNI int celt_decode(Lanes L, CeltDec *st, const uint8_t *data, int len, int16_t 
                           st->rng);
         if (silence)
             ROLLED for (int i = 0; i < C * CELT_NB; i++) oldBandE[i] = -28672;   // -QCONST16(28.f, DB_SHIFT)
-        if (st->prefilter_and_fold) prefilter_and_fold(st, N, w);
     });
+    if (st->prefilter_and_fold) prefilter_and_fold(L, st, N, w);
     PHASE_BEGIN(t_sy);
     celt_synthesis(L, w, X, out_syn, oldBandE, start, effEnd, C, CC, isTransient, LM, silence);
     PHASE_END(PH_CELT_SYNTH, t_sy, L.id);

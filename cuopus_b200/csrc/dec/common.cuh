@@ -457,20 +457,6 @@ DFN int16_t c_sig2word16(int32_t x)
     return (int16_t)x;
 }
 
-// celt/mathops.h celt_maxabs16 / celt_maxabs32 (scalar)
-DFN int32_t c_maxabs16(const int16_t *x, int len)
-{
-    int16_t mx = 0, mn = 0;
-    ROLLED for (int i = 0; i < len; i++) { mx = x[i] > mx ? x[i] : mx; mn = x[i] < mn ? x[i] : mn; }
-    return max32(mx, -(int32_t)mn);
-}
-DFN int32_t c_maxabs32(const int32_t *x, int len)
-{
-    int32_t mx = 0, mn = 0;
-    ROLLED for (int i = 0; i < len; i++) { mx = max32(mx, x[i]); mn = min32(mn, x[i]); }
-    return max32(mx, -mn);
-}
-
 // celt/mathops.c isqrt32 (bit-by-bit integer square root)
 DFN unsigned c_isqrt32(uint32_t val)
 {

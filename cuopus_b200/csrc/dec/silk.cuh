@@ -563,25 +563,22 @@ DNI void silk_lpc_analysis_filter(Lanes L, int16_t *out, const int16_t *in,
     lsync(L);
 }
 
-// silk/sum_sqr_shift.c
-DNI void silk_sum_sqr_shift(int32_t *energy, int *shift, const int16_t *x, int len)
+// silk/sum_sqr_shift.c, on every lane (the sums wrap, so the lanes' partial
+// sums give the serial values)
+DNI void silk_sum_sqr_shift(Lanes L, int32_t *energy, int *shift, const int16_t *x, int len)
 {
-    int i, shft = 31 - s_clz32(len);
-    int32_t nrg = len;
-    ROLLED for (i = 0; i < len - 1; i += 2) {
-        uint32_t t = (uint32_t)s_smulbb(x[i], x[i]);
-        t = (uint32_t)s_smlabb((int32_t)t, x[i + 1], x[i + 1]);
-        nrg = (int32_t)((uint32_t)nrg + (t >> shft));
+    int shft = 31 - s_clz32(len);
+    int32_t nrg = 0;
+    ROLLED for (int pass = 0; pass < 2; pass++) {
+        uint32_t sum = 0;
+        LFOR(L, q, 0, (len + 1) >> 1) {
+            uint32_t t = (uint32_t)s_smulbb(x[2 * q], x[2 * q]);
+            if (2 * q + 1 < len) t = (uint32_t)s_smlabb((int32_t)t, x[2 * q + 1], x[2 * q + 1]);
+            sum += t >> shft;
+        }
+        nrg = lsum(L, (int32_t)sum);
+        if (pass == 0) shft = imax(0, shft + 3 - s_clz32(wadd(nrg, len)));
     }
-    if (i < len) nrg = (int32_t)((uint32_t)nrg + ((uint32_t)s_smulbb(x[i], x[i]) >> shft));
-    shft = imax(0, shft + 3 - s_clz32(nrg));
-    nrg = 0;
-    ROLLED for (i = 0; i < len - 1; i += 2) {
-        uint32_t t = (uint32_t)s_smulbb(x[i], x[i]);
-        t = (uint32_t)s_smlabb((int32_t)t, x[i + 1], x[i + 1]);
-        nrg = (int32_t)((uint32_t)nrg + (t >> shft));
-    }
-    if (i < len) nrg = (int32_t)((uint32_t)nrg + ((uint32_t)s_smulbb(x[i], x[i]) >> shft));
     *shift = shft;
     *energy = nrg;
 }
@@ -1173,6 +1170,36 @@ DNI void silk_plc_update(SilkChan *c, const SilkCtrl *ctrl)
     p->nb_subfr = c->nb_subfr;
 }
 
+// s_rand k steps on is the affine map seed -> a[k] seed + c[k] mod 2^32.
+struct SilkRandPowers {
+    uint32_t a[SILK_MAX_FRAME + 1], c[SILK_MAX_FRAME + 1];
+    constexpr SilkRandPowers() : a(), c()
+    {
+        a[0] = 1;
+        c[0] = 0;
+        for (int k = 1; k <= SILK_MAX_FRAME; k++) {
+            a[k] = 196314165u * a[k - 1];
+            c[k] = 196314165u * c[k - 1] + 907633515u;
+        }
+    }
+};
+TABG(SilkRandPowers, T_silk_rand) = SilkRandPowers();
+DFN int32_t silk_rand_at(int32_t seed, int k) { return (int32_t)(T_silk_rand.a[k] * (uint32_t)seed + T_silk_rand.c[k]); }
+
+// LPC synthesis of a whole frame (lost frames and comfort noise); v and exc are
+// different arrays.
+DFN void silk_lpc_synth_frame(const Lanes &L, int order, int32_t *hist, const int16_t *A_Q12, const int32_t *exc,
+                              int32_t *v, int n)
+{
+    if (order == 16) silk_lpc_synth<16>(L, hist, A_Q12, exc, v, n);
+    else silk_lpc_synth<10>(L, hist, A_Q12, exc, v, n);
+}
+
+// silk_PLC_conceal.  Every lane works out the gains and the lanes split the
+// sample loops: the LTP excitation in blocks shorter than the lag, its random
+// samples by the generator's powers, the LPC synthesis as in a received frame.
+// (On the first lane alone the LPC synthesis by itself took 360 k cycles per
+// 20 ms.)
 DNI void silk_plc_conceal(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *frame, SilkScratch *w)
 {
     // HARM_ATT_Q15 {32440, 31130}, RAND_ATT_V_Q15 {31130, 26214}, RAND_ATT_UV_Q15
@@ -1180,98 +1207,94 @@ DNI void silk_plc_conceal(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *frame, 
     SilkPLC *p = &c->sPLC;
     int32_t *sLTP_Q14 = w->sLTP_Q15;
     int16_t *sLTP = w->sLTP;
-    // The serial parts (energies, gains, the LPC chirp in place, the LTP
-    // excitation and the LPC synthesis) run on the first lane; the lanes split
-    // the LPC analysis filtering between them.  What the first lane computes
-    // for the second serial part stays in its registers.
-    int32_t prevGain_Q10[2] = {0, 0};
-    const int32_t *rand_ptr = nullptr;
-    int16_t *B_Q14 = p->LTPCoef_Q14;
-    int16_t rand_scale_Q14 = 0;
-    int32_t harm_Gain_Q15 = 0, rand_Gain_Q15 = 0;
+    const int S = c->subfr_length;
+    int32_t prevGain_Q10[2];
+    prevGain_Q10[0] = p->prevGain_Q16[0] >> 6;
+    prevGain_Q10[1] = p->prevGain_Q16[1] >> 6;
+    // silk_PLC_energy
+    int32_t energy1, energy2;
+    int shift1, shift2;
+    int16_t *eb = w->plc_exc;
+    LFOR(L, i, 0, 2 * S)
+        eb[i] = (int16_t)s_sat16(s_smulww(c->exc_Q14[i + (c->nb_subfr - 2) * S], prevGain_Q10[i >= S]) >> 8);
+    lsync(L);
+    silk_sum_sqr_shift(L, &energy1, &shift1, eb, S);
+    silk_sum_sqr_shift(L, &energy2, &shift2, &eb[S], S);
+    const int32_t *rand_ptr;
+    if ((energy1 >> shift2) < (energy2 >> shift1))
+        rand_ptr = &c->exc_Q14[imax(0, (p->nb_subfr - 1) * p->subfr_length - 128)];
+    else
+        rand_ptr = &c->exc_Q14[imax(0, p->nb_subfr * p->subfr_length - 128)];
+    int16_t B_Q14[5];
+#pragma unroll
+    for (int i = 0; i < 5; i++) B_Q14[i] = p->LTPCoef_Q14[i];
+    int16_t rand_scale_Q14 = p->randScale_Q14;
+    const int first_loss = c->lossCnt == 0, voiced = c->prevSignalType == SIG_VOICED;
+    const int32_t harm_Gain_Q15 = first_loss ? 32440 : 31130;
+    int32_t rand_Gain_Q15 = voiced ? (first_loss ? 31130 : 26214) : (first_loss ? 32440 : 29491);
+    int32_t invGain_Q30 = 0;
     lead(L, [&]() CUO_INLINE {
-        prevGain_Q10[0] = p->prevGain_Q16[0] >> 6;
-        prevGain_Q10[1] = p->prevGain_Q16[1] >> 6;
         if (c->first_frame_after_reset) ROLLED for (int i = 0; i < 16; i++) p->prevLPC_Q12[i] = 0;
-
-        // silk_PLC_energy
-        int32_t energy1, energy2;
-        int shift1, shift2;
-        {
-            int16_t *eb = w->plc_exc;
-            ROLLED for (int k = 0; k < 2; k++)
-                ROLLED for (int i = 0; i < c->subfr_length; i++)
-                    eb[k * c->subfr_length + i] = (int16_t)s_sat16(s_smulww(
-                        c->exc_Q14[i + (k + c->nb_subfr - 2) * c->subfr_length], prevGain_Q10[k]) >> 8);
-            silk_sum_sqr_shift(&energy1, &shift1, eb, c->subfr_length);
-            silk_sum_sqr_shift(&energy2, &shift2, &eb[c->subfr_length], c->subfr_length);
-        }
-        if ((energy1 >> shift2) < (energy2 >> shift1))
-            rand_ptr = &c->exc_Q14[imax(0, (p->nb_subfr - 1) * p->subfr_length - 128)];
-        else
-            rand_ptr = &c->exc_Q14[imax(0, p->nb_subfr * p->subfr_length - 128)];
-        rand_scale_Q14 = p->randScale_Q14;
-        const int first_loss = c->lossCnt == 0;
-        harm_Gain_Q15 = first_loss ? 32440 : 31130;
-        rand_Gain_Q15 = c->prevSignalType == SIG_VOICED ? (first_loss ? 31130 : 26214)
-                                                        : (first_loss ? 32440 : 29491);
         silk_bwexpander(p->prevLPC_Q12, c->LPC_order, 64881);   // SILK_FIX_CONST(0.99, 16)
-        if (c->lossCnt == 0) {
-            rand_scale_Q14 = 1 << 14;
-            if (c->prevSignalType == SIG_VOICED) {
-                ROLLED for (int i = 0; i < 5; i++) rand_scale_Q14 = (int16_t)(rand_scale_Q14 - B_Q14[i]);
-                rand_scale_Q14 = rand_scale_Q14 > 3277 ? rand_scale_Q14 : 3277;
-                rand_scale_Q14 = (int16_t)(s_smulbb(rand_scale_Q14, p->prevLTP_scale_Q14) >> 14);
-            } else {
-                int32_t invGain_Q30 = silk_lpc_inv_pred_gain(p->prevLPC_Q12, c->LPC_order, w->sw.A);
-                int32_t down = min32((1 << 30) >> 3, invGain_Q30);
-                down = max32((1 << 30) >> 8, down);
-                down = shl32(down, 3);
-                rand_Gain_Q15 = s_smulwb(down, rand_Gain_Q15) >> 14;
-            }
-        }
+        if (first_loss && !voiced) invGain_Q30 = silk_lpc_inv_pred_gain(p->prevLPC_Q12, c->LPC_order, w->sw.A);
     });
-    int16_t A_Q12[16];
-    ROLLED for (int i = 0; i < c->LPC_order; i++) A_Q12[i] = p->prevLPC_Q12[i];
-    int lag = s_rshift_round(p->pitchL_Q8, 8);
+    if (first_loss) {
+        rand_scale_Q14 = 1 << 14;
+        if (voiced) {
+#pragma unroll
+            for (int i = 0; i < 5; i++) rand_scale_Q14 = (int16_t)(rand_scale_Q14 - B_Q14[i]);
+            rand_scale_Q14 = rand_scale_Q14 > 3277 ? rand_scale_Q14 : 3277;
+            rand_scale_Q14 = (int16_t)(s_smulbb(rand_scale_Q14, p->prevLTP_scale_Q14) >> 14);
+        } else {
+            int32_t down = min32((1 << 30) >> 3, lbcast(L, invGain_Q30));
+            down = max32((1 << 30) >> 8, down);
+            down = shl32(down, 3);
+            rand_Gain_Q15 = s_smulwb(down, rand_Gain_Q15) >> 14;
+        }
+    }
+    const int16_t *A_Q12 = p->prevLPC_Q12;
+    int32_t pitchL_Q8 = p->pitchL_Q8;
+    int lag = s_rshift_round(pitchL_Q8, 8);
     int idx = c->ltp_mem_length - lag - c->LPC_order - 2;
     silk_lpc_analysis_filter(L, &sLTP[idx], &c->outBuf[idx], A_Q12, c->ltp_mem_length - idx, c->LPC_order);
     int32_t inv_gain_Q30 = s_inverse32_varq(p->prevGain_Q16[1], 46);
     inv_gain_Q30 = min32(inv_gain_Q30, 0x7FFFFFFF >> 1);
     LFOR(L, i, idx + c->LPC_order, c->ltp_mem_length) sLTP_Q14[i] = s_smulwb(inv_gain_Q30, sLTP[i]);
-    lead(L, [&]() CUO_INLINE {
-        int32_t rand_seed = p->rand_seed;
-        int sLTP_buf_idx = c->ltp_mem_length;
-        ROLLED for (int k = 0; k < c->nb_subfr; k++) {
-            const int32_t *pl = &sLTP_Q14[sLTP_buf_idx - lag + 2];
-            ROLLED for (int i = 0; i < c->subfr_length; i++) {
+    lsync(L);
+    const int32_t rand_seed = p->rand_seed;
+    ROLLED for (int k = 0; k < c->nb_subfr; k++) {
+        int32_t *out = &sLTP_Q14[c->ltp_mem_length + k * S];
+        const int32_t *pl = out - lag + 2;
+        const int blk = imax(lag - 2, 1);   // as in silk_decode_core
+        ROLLED for (int s0 = 0; s0 < S; s0 += blk) {
+            LFOR(L, i, s0, imin(s0 + blk, S)) {
                 int32_t pr = 2;
                 pr = s_smlawb(pr, pl[i], B_Q14[0]);
                 pr = s_smlawb(pr, pl[i - 1], B_Q14[1]);
                 pr = s_smlawb(pr, pl[i - 2], B_Q14[2]);
                 pr = s_smlawb(pr, pl[i - 3], B_Q14[3]);
                 pr = s_smlawb(pr, pl[i - 4], B_Q14[4]);
-                rand_seed = s_rand(rand_seed);
-                int ri = (rand_seed >> 25) & 127;
-                sLTP_Q14[sLTP_buf_idx] = shl32(s_smlawb(pr, rand_ptr[ri], rand_scale_Q14), 2);
-                sLTP_buf_idx++;
+                const int ri = (silk_rand_at(rand_seed, k * S + i + 1) >> 25) & 127;
+                out[i] = shl32(s_smlawb(pr, rand_ptr[ri], rand_scale_Q14), 2);
             }
-            ROLLED for (int j = 0; j < 5; j++) B_Q14[j] = (int16_t)(s_smulbb(harm_Gain_Q15, B_Q14[j]) >> 15);
-            rand_scale_Q14 = (int16_t)(s_smulbb(rand_scale_Q14, rand_Gain_Q15) >> 15);
-            p->pitchL_Q8 = s_smlawb(p->pitchL_Q8, p->pitchL_Q8, 655);
-            p->pitchL_Q8 = min32(p->pitchL_Q8, shl32(s_smulbb(18, c->fs_kHz), 8));
-            lag = s_rshift_round(p->pitchL_Q8, 8);
+            lsync(L);
         }
-        int32_t *sl = &sLTP_Q14[c->ltp_mem_length - 16];
-        ROLLED for (int i = 0; i < 16; i++) sl[i] = c->sLPC_Q14_buf[i];
-        ROLLED for (int i = 0; i < c->frame_length; i++) {
-            int32_t pr = c->LPC_order >> 1;
-            ROLLED for (int j = 0; j < c->LPC_order; j++) pr = s_smlawb(pr, sl[16 + i - j - 1], A_Q12[j]);
-            sl[16 + i] = s_add_sat32(sl[16 + i], s_lshift_sat32(pr, 4));
-            frame[i] = (int16_t)s_sat16(s_sat16(s_rshift_round(s_smulww(sl[16 + i], prevGain_Q10[1]), 8)));
-        }
-        ROLLED for (int i = 0; i < 16; i++) c->sLPC_Q14_buf[i] = sl[c->frame_length + i];
-        p->rand_seed = rand_seed;
+#pragma unroll
+        for (int j = 0; j < 5; j++) B_Q14[j] = (int16_t)(s_smulbb(harm_Gain_Q15, B_Q14[j]) >> 15);
+        rand_scale_Q14 = (int16_t)(s_smulbb(rand_scale_Q14, rand_Gain_Q15) >> 15);
+        pitchL_Q8 = s_smlawb(pitchL_Q8, pitchL_Q8, 655);
+        pitchL_Q8 = min32(pitchL_Q8, shl32(s_smulbb(18, c->fs_kHz), 8));
+        lag = s_rshift_round(pitchL_Q8, 8);
+    }
+    int32_t *v = w->CNG_sig_Q14;
+    silk_lpc_synth_frame(L, c->LPC_order, c->sLPC_Q14_buf, A_Q12, &sLTP_Q14[c->ltp_mem_length], v, c->frame_length);
+    LFOR(L, i, 0, c->frame_length)
+        frame[i] = (int16_t)s_sat16(s_rshift_round(s_smulww(v[i], prevGain_Q10[1]), 8));
+    lead(L, [&]() CUO_INLINE {
+        p->pitchL_Q8 = pitchL_Q8;
+#pragma unroll
+        for (int i = 0; i < 5; i++) p->LTPCoef_Q14[i] = B_Q14[i];
+        p->rand_seed = silk_rand_at(rand_seed, c->frame_length);
         p->randScale_Q14 = rand_scale_Q14;
         ROLLED for (int i = 0; i < 4; i++) ctrl->pitchL[i] = lag;
     });
@@ -1292,47 +1315,50 @@ DNI void silk_plc(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *frame, int lost
     }
 }
 
-DNI void silk_plc_glue_frames(SilkChan *c, int16_t *frame, int length)
+DNI void silk_plc_glue_frames(Lanes L, SilkChan *c, int16_t *frame, int length)
 {
     SilkPLC *p = &c->sPLC;
-    if (c->lossCnt) {
-        silk_sum_sqr_shift(&p->conc_energy, &p->conc_energy_shift, frame, length);
-        p->last_frame_lost = 1;
-    } else {
-        if (p->last_frame_lost) {
-            int32_t energy;
-            int energy_shift;
-            silk_sum_sqr_shift(&energy, &energy_shift, frame, length);
-            if (energy_shift > p->conc_energy_shift)
-                p->conc_energy = p->conc_energy >> (energy_shift - p->conc_energy_shift);
-            else if (energy_shift < p->conc_energy_shift)
-                energy = energy >> (p->conc_energy_shift - energy_shift);
-            if (energy > p->conc_energy) {
-                int32_t LZ = s_clz32(p->conc_energy) - 1;
-                p->conc_energy = shl32(p->conc_energy, LZ);
-                energy = energy >> imax(24 - LZ, 0);
-                int32_t frac_Q24 = p->conc_energy / imax(energy, 1);
-                int32_t gain_Q16 = shl32(s_sqrt_approx(frac_Q24), 4);
-                int32_t slope_Q16 = ((1 << 16) - gain_Q16) / length;
-                slope_Q16 = shl32(slope_Q16, 2);
-                ROLLED for (int i = 0; i < length; i++) {
-                    frame[i] = (int16_t)s_smulwb(gain_Q16, frame[i]);
-                    gain_Q16 += slope_Q16;
-                    if (gain_Q16 > (1 << 16)) break;
-                }
+    if (!c->lossCnt && !p->last_frame_lost) return;
+    int32_t energy;
+    int energy_shift;
+    silk_sum_sqr_shift(L, &energy, &energy_shift, frame, length);
+    lead(L, [&]() CUO_INLINE {
+        if (c->lossCnt) {
+            p->conc_energy = energy;
+            p->conc_energy_shift = energy_shift;
+            p->last_frame_lost = 1;
+            return;
+        }
+        if (energy_shift > p->conc_energy_shift)
+            p->conc_energy = p->conc_energy >> (energy_shift - p->conc_energy_shift);
+        else if (energy_shift < p->conc_energy_shift)
+            energy = energy >> (p->conc_energy_shift - energy_shift);
+        if (energy > p->conc_energy) {
+            int32_t LZ = s_clz32(p->conc_energy) - 1;
+            p->conc_energy = shl32(p->conc_energy, LZ);
+            energy = energy >> imax(24 - LZ, 0);
+            int32_t frac_Q24 = p->conc_energy / imax(energy, 1);
+            int32_t gain_Q16 = shl32(s_sqrt_approx(frac_Q24), 4);
+            int32_t slope_Q16 = ((1 << 16) - gain_Q16) / length;
+            slope_Q16 = shl32(slope_Q16, 2);
+            ROLLED for (int i = 0; i < length; i++) {
+                frame[i] = (int16_t)s_smulwb(gain_Q16, frame[i]);
+                gain_Q16 += slope_Q16;
+                if (gain_Q16 > (1 << 16)) break;
             }
         }
         p->last_frame_lost = 0;
-    }
+    });
 }
 
 // silk/CNG.c
 // The comfort-noise generation of silk_CNG (only after a lost frame): its own
 // function, so the code of the per-frame update stays small.
-DNI void silk_cng_generate(SilkChan *c, int16_t *frame, int length, SilkScratch *w)
+DNI void silk_cng_generate(Lanes L, SilkChan *c, int16_t *frame, int length, SilkScratch *w)
 {
     SilkCNG *g = &c->sCNG;
-    int32_t *sig = w->CNG_sig_Q14;
+    int32_t *sig = w->CNG_sig_Q14, *v = w->sLTP_Q15;
+    int16_t *A_Q12 = w->sw.res_Q10;
     int32_t gain_Q16 = s_smulww(c->sPLC.randScale_Q14, c->sPLC.prevGain_Q16[1]);
     if (gain_Q16 >= (1 << 21) || g->CNG_smth_Gain_Q16 > (1 << 23)) {
         gain_Q16 = s_smultt(gain_Q16, gain_Q16);
@@ -1347,23 +1373,16 @@ DNI void silk_cng_generate(SilkChan *c, int16_t *frame, int length, SilkScratch 
     // silk_CNG_exc
     int exc_mask = 255;
     ROLLED while (exc_mask > length) exc_mask >>= 1;
-    int32_t seed = g->rand_seed;
-    ROLLED for (int i = 0; i < length; i++) {
-        seed = s_rand(seed);
-        sig[16 + i] = g->CNG_exc_buf_Q14[(seed >> 24) & exc_mask];
-    }
-    g->rand_seed = seed;
-    int16_t A_Q12[16];
-    silk_nlsf2a(A_Q12, g->CNG_smth_NLSF_Q15, c->LPC_order, &w->sw);
-    ROLLED for (int i = 0; i < 16; i++) sig[i] = g->CNG_synth_state[i];
-    ROLLED for (int i = 0; i < length; i++) {
-        int32_t pr = c->LPC_order >> 1;
-        ROLLED for (int j = 0; j < c->LPC_order; j++) pr = s_smlawb(pr, sig[16 + i - j - 1], A_Q12[j]);
-        sig[16 + i] = s_add_sat32(sig[16 + i], s_lshift_sat32(pr, 4));
-        frame[i] = (int16_t)s_sat16((int32_t)frame[i] +
-            s_sat16(s_rshift_round(s_smulww(sig[16 + i], gain_Q10), 8)));
-    }
-    ROLLED for (int i = 0; i < 16; i++) g->CNG_synth_state[i] = sig[length + i];
+    const int32_t seed = g->rand_seed;
+    LFOR(L, i, 0, length) sig[i] = g->CNG_exc_buf_Q14[(silk_rand_at(seed, i + 1) >> 24) & exc_mask];
+    lead(L, [&]() CUO_INLINE {
+        g->rand_seed = silk_rand_at(seed, length);
+        silk_nlsf2a(A_Q12, g->CNG_smth_NLSF_Q15, c->LPC_order, &w->sw);
+    });
+    silk_lpc_synth_frame(L, c->LPC_order, g->CNG_synth_state, A_Q12, sig, v, length);
+    LFOR(L, i, 0, length)
+        frame[i] = (int16_t)s_sat16((int32_t)frame[i] + s_sat16(s_rshift_round(s_smulww(v[i], gain_Q10), 8)));
+    lsync(L);
 }
 
 DNI void silk_cng(Lanes L, SilkChan *c, const SilkCtrl *ctrl, int16_t *frame, int length, SilkScratch *w)
@@ -1403,11 +1422,12 @@ DNI void silk_cng(Lanes L, SilkChan *c, const SilkCtrl *ctrl, int16_t *frame, in
             }
         });
     }
-    lead(L, [&]() CUO_INLINE {
-        if (c->lossCnt) silk_cng_generate(c, frame, length, w);
-        else
-            ROLLED for (int i = 0; i < c->LPC_order; i++) g->CNG_synth_state[i] = 0;
-    });
+    if (c->lossCnt) {
+        silk_cng_generate(L, c, frame, length, w);
+    } else {
+        LFOR(L, i, 0, c->LPC_order) g->CNG_synth_state[i] = 0;
+        lsync(L);
+    }
 }
 
 // ------------------------------------------------------------------ frame
@@ -1461,10 +1481,8 @@ DNI void silk_decode_frame(Lanes L, SilkChan *c, RangeDec *rd, int16_t *pOut, in
     PHASE_BEGIN(t_cn);
     silk_cng(L, c, ctrl, pOut, Lf, w);
     PHASE_END(PH_SILK_CNG, t_cn, L.id);
-    lead(L, [&]() CUO_INLINE {
-        silk_plc_glue_frames(c, pOut, Lf);
-        c->lagPrev = ctrl->pitchL[c->nb_subfr - 1];
-    });
+    silk_plc_glue_frames(L, c, pOut, Lf);
+    lead(L, [&]() CUO_INLINE { c->lagPrev = ctrl->pitchL[c->nb_subfr - 1]; });
     *pN = Lf;
 }
 
