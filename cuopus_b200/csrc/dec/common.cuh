@@ -61,6 +61,7 @@ struct LaneSim;
 void lanesim_sync(LaneSim *s, int id);
 int32_t lanesim_sum(LaneSim *s, int id, int32_t v);
 uint32_t lanesim_or(LaneSim *s, int id, uint32_t v);
+int32_t lanesim_get(LaneSim *s, int id, int32_t v, int src);
 int32_t lanesim_max(LaneSim *s, int id, int32_t v);
 void lanesim_scan_affine(LaneSim *s, int id, uint32_t *a, uint32_t *b);
 void lanesim_bcast(LaneSim *s, int id, void *p, int bytes);
@@ -130,6 +131,20 @@ DFN int32_t lbcast(const Lanes &L, int32_t v)
     if (L.sim) lanesim_bcast(L.sim, L.id, &v, (int)sizeof v);
 #else
     (void)L;
+#endif
+    return v;
+}
+
+// v of lane src of the group (src may differ between the lanes).
+DFN int32_t lget(const Lanes &L, int32_t v, int src)
+{
+#ifdef __CUDA_ARCH__
+    v = __shfl_sync(L.mask, v, (int)(threadIdx.x & 31) - L.id + src);
+#elif defined(CUO_LANE_SIM)
+    if (L.sim) v = lanesim_get(L.sim, L.id, v, src);
+#else
+    (void)L;
+    (void)src;
 #endif
     return v;
 }

@@ -302,16 +302,14 @@ DNI int16_t *silk_iir_fir(Lanes L, SilkResampler *S, int16_t *out, const int16_t
         in += nIn;
         inLen -= nIn;
         if (inLen > 0) {
-            int16_t keep[8];
-            ROLLED for (int i = 0; i < 8; i++) keep[i] = buf[(nIn << 1) + i];
-            lsync(L);
-            LFOR(L, i, 0, 8) buf[i] = keep[i];
+            // nIn is at least 16 here: the eight move down without overlap
+            LFOR(L, i, 0, 8) buf[i] = buf[(nIn << 1) + i];
             lsync(L);
         } else {
             break;
         }
     }
-    ROLLED for (int i = 0; i < 8; i++) S->sFIR[i] = buf[(nIn << 1) + i];
+    LFOR(L, i, 0, 8) S->sFIR[i] = buf[(nIn << 1) + i];
     lsync(L);
     return out;
 }
@@ -351,48 +349,49 @@ DFN void silk_bwexpander_32(int32_t *ar, int d, int32_t chirp_Q16)
     ar[d - 1] = s_smulww(chirp_Q16, ar[d - 1]);
 }
 
-// silk/LPC_inv_pred_gain.c (QA = 24); returns 0 when the filter is unstable
-DNI int32_t silk_lpc_inv_pred_gain(const int16_t *A_Q12, int order, int32_t *A)
+// silk/LPC_inv_pred_gain.c (QA = 24); returns 0 when the filter is unstable.
+// Every lane steps down the order; the lanes split a step's coefficient pairs.
+DNI int32_t silk_lpc_inv_pred_gain(Lanes L, const int16_t *A_Q12, int order, int32_t *A)
 {
     const int32_t A_LIMIT = 16773022;   // SILK_FIX_CONST(0.99975, 24)
     const int32_t MIN_INVG = 107374;    // SILK_FIX_CONST(1 / MAX_PREDICTION_POWER_GAIN, 30)
     int32_t DC = 0;
-    ROLLED for (int k = 0; k < order; k++) {
+    lsync(L);
+    LFOR(L, k, 0, order) {
         DC += A_Q12[k];
         A[k] = shl32((int32_t)A_Q12[k], 12);
     }
+    DC = lsum(L, DC);
+    lsync(L);
     if (DC >= 4096) return 0;
     int32_t invGain_Q30 = 1 << 30;
-    int k;
-    ROLLED for (k = order - 1; k > 0; k--) {
-        if (A[k] > A_LIMIT || A[k] < -A_LIMIT) return 0;
-        int32_t rc_Q31 = -shl32(A[k], 7);
+    ROLLED for (int k = order - 1;; k--) {
+        const int32_t Ak = A[k];
+        if (Ak > A_LIMIT || Ak < -A_LIMIT) return 0;
+        int32_t rc_Q31 = -shl32(Ak, 7);
         int32_t rc_mult1_Q30 = (1 << 30) - s_smmul(rc_Q31, rc_Q31);
         invGain_Q30 = shl32(s_smmul(invGain_Q30, rc_mult1_Q30), 2);
         if (invGain_Q30 < MIN_INVG) return 0;
+        if (k == 0) return invGain_Q30;
         int mult2Q = 32 - s_clz32(s_abs(rc_mult1_Q30));
         int32_t rc_mult2 = s_inverse32_varq(rc_mult1_Q30, mult2Q + 30);
-        ROLLED for (int n = 0; n < (k + 1) >> 1; n++) {
+        uint32_t over = 0;
+        LFOR(L, n, 0, (k + 1) >> 1) {
             int32_t t1 = A[n], t2 = A[k - n - 1];
             int64_t v = s_rshift_round64(s_smull(s_sub_sat32(t1,
                 (int32_t)s_rshift_round64(s_smull(t2, rc_Q31), 31)), rc_mult2), mult2Q);
-            if (v > 2147483647LL || v < -2147483648LL) return 0;
-            A[n] = (int32_t)v;
-            v = s_rshift_round64(s_smull(s_sub_sat32(t2,
+            int64_t u = s_rshift_round64(s_smull(s_sub_sat32(t2,
                 (int32_t)s_rshift_round64(s_smull(t1, rc_Q31), 31)), rc_mult2), mult2Q);
-            if (v > 2147483647LL || v < -2147483648LL) return 0;
-            A[k - n - 1] = (int32_t)v;
+            over |= v != (int32_t)v || u != (int32_t)u;
+            A[n] = (int32_t)v;
+            A[k - n - 1] = (int32_t)u;
         }
+        if (lor(L, over)) return 0;
+        lsync(L);
     }
-    if (A[k] > A_LIMIT || A[k] < -A_LIMIT) return 0;
-    int32_t rc_Q31 = -shl32(A[0], 7);
-    int32_t rc_mult1_Q30 = (1 << 30) - s_smmul(rc_Q31, rc_Q31);
-    invGain_Q30 = shl32(s_smmul(invGain_Q30, rc_mult1_Q30), 2);
-    if (invGain_Q30 < MIN_INVG) return 0;
-    return invGain_Q30;
 }
 
-// silk/LPC_fit.c
+// silk/LPC_fit.c, the first lane alone: coefficients that do not fit in 16 bits
 DNI void silk_lpc_fit(int16_t *a_QOUT, int32_t *a_QIN, int QOUT, int QIN, int d)
 {
     int i, k, idx = 0;
@@ -421,48 +420,76 @@ DNI void silk_lpc_fit(int16_t *a_QOUT, int32_t *a_QIN, int QOUT, int QIN, int d)
     }
 }
 
-// silk/NLSF2A.c (QA = 16): NLSF -> LPC via the P/Q polynomial expansion
-DFN void silk_nlsf2a_poly(int32_t *out, const int32_t *cLSF, int dd)
+// silk/NLSF2A.c (QA = 16): NLSF -> LPC via the P/Q polynomial expansion, in
+// registers: out[0 .. DD] from every second element of cLSF
+template <int DD> DFN void silk_nlsf2a_poly(int32_t *out, const int32_t *cLSF)
 {
-    out[0] = 1 << 16;
-    out[1] = -cLSF[0];
-    ROLLED for (int k = 1; k < dd; k++) {
-        int32_t ftmp = cLSF[2 * k];
-        out[k + 1] = wsub(shl32(out[k - 1], 1), (int32_t)s_rshift_round64(s_smull(ftmp, out[k]), 16));
-        ROLLED for (int n = k; n > 1; n--)
-            out[n] = wadd(out[n], wsub(out[n - 2], (int32_t)s_rshift_round64(s_smull(ftmp, out[n - 1]), 16)));
-        out[1] = wsub(out[1], ftmp);
+    int32_t o[DD + 1], f[DD];
+#pragma unroll
+    for (int k = 0; k < DD; k++) f[k] = cLSF[2 * k];
+    o[0] = 1 << 16;
+    o[1] = -f[0];
+#pragma unroll
+    for (int k = 1; k < DD; k++) {
+        o[k + 1] = wsub(shl32(o[k - 1], 1), (int32_t)s_rshift_round64(s_smull(f[k], o[k]), 16));
+#pragma unroll
+        for (int n = k; n > 1; n--)
+            o[n] = wadd(o[n], wsub(o[n - 2], (int32_t)s_rshift_round64(s_smull(f[k], o[n - 1]), 16)));
+        o[1] = wsub(o[1], f[k]);
     }
+#pragma unroll
+    for (int k = 0; k <= DD; k++) out[k] = o[k];
 }
 
 // ordering16 / ordering10 of silk/NLSF2A.c
 TABC(uint8_t, T_nlsf2a_ord16[16]) = {0, 15, 8, 7, 4, 11, 12, 3, 2, 13, 10, 5, 6, 9, 14, 1};
 TABC(uint8_t, T_nlsf2a_ord10[10]) = {0, 9, 6, 3, 4, 5, 8, 1, 2, 7};
 
-DNI void silk_nlsf2a(int16_t *a_Q12, const int16_t *NLSF, int d, SilkWork *sw)
+// On every lane: the lanes split the tables and the coefficients, one lane per
+// polynomial.  The serial form on one lane took 45 k cycles, NLSF_MEASURED.
+DNI void silk_nlsf2a(Lanes L, int16_t *a_Q12, const int16_t *NLSF, int d, SilkWork *sw)
 {
     const uint8_t *ordering = d == 16 ? T_nlsf2a_ord16 : T_nlsf2a_ord10;
     int32_t *cos_LSF_QA = sw->cos_LSF_QA, *P = sw->P, *Q = sw->Q, *a32_QA1 = sw->a32_QA1;
-    ROLLED for (int k = 0; k < d; k++) {
+    lsync(L);
+    LFOR(L, k, 0, d) {
         int32_t f_int = NLSF[k] >> 8;
         int32_t f_frac = NLSF[k] - shl32(f_int, 8);
         int32_t cos_val = T_silk_LSFCosTab_FIX_Q12[f_int];
         int32_t delta = T_silk_LSFCosTab_FIX_Q12[f_int + 1] - cos_val;
         cos_LSF_QA[ordering[k]] = s_rshift_round(wadd(shl32(cos_val, 8), wmul(delta, f_frac)), 4);
     }
-    int dd = d >> 1;
-    silk_nlsf2a_poly(P, &cos_LSF_QA[0], dd);
-    silk_nlsf2a_poly(Q, &cos_LSF_QA[1], dd);
-    ROLLED for (int k = 0; k < dd; k++) {
+    lsync(L);
+    const int dd = d >> 1;
+    LFOR(L, q, 0, 2) {
+        int32_t *out = q ? Q : P;
+        if (d == 16) silk_nlsf2a_poly<8>(out, cos_LSF_QA + q);
+        else silk_nlsf2a_poly<5>(out, cos_LSF_QA + q);
+    }
+    lsync(L);
+    int32_t top = 0;
+    LFOR(L, k, 0, dd) {
         int32_t Ptmp = wadd(P[k + 1], P[k]);
         int32_t Qtmp = wsub(Q[k + 1], Q[k]);
-        a32_QA1[k] = wsub(-Qtmp, Ptmp);
-        a32_QA1[d - k - 1] = wsub(Qtmp, Ptmp);
+        const int32_t lo = wsub(-Qtmp, Ptmp), hi = wsub(Qtmp, Ptmp);
+        a32_QA1[k] = lo;
+        a32_QA1[d - k - 1] = hi;
+        top = max32(top, max32(s_abs(lo), s_abs(hi)));
     }
-    silk_lpc_fit(a_Q12, a32_QA1, 12, 17, d);
-    ROLLED for (int i = 0; silk_lpc_inv_pred_gain(a_Q12, d, sw->A) == 0 && i < 16; i++) {
-        silk_bwexpander_32(a32_QA1, d, 65536 - shl32(2, i));
-        ROLLED for (int k = 0; k < d; k++) a_Q12[k] = (int16_t)s_rshift_round(a32_QA1[k], 5);
+    top = lmax(L, top);
+    lsync(L);
+    // silk_LPC_fit: usually every coefficient fits and is just rounded
+    if (s_rshift_round(top, 5) > 32767) {
+        lead(L, [&]() CUO_INLINE { silk_lpc_fit(a_Q12, a32_QA1, 12, 17, d); });
+    } else {
+        LFOR(L, k, 0, d) a_Q12[k] = (int16_t)s_rshift_round(a32_QA1[k], 5);
+        lsync(L);
+    }
+    ROLLED for (int i = 0; silk_lpc_inv_pred_gain(L, a_Q12, d, sw->A) == 0 && i < 16; i++) {
+        lead(L, [&]() CUO_INLINE {
+            silk_bwexpander_32(a32_QA1, d, 65536 - shl32(2, i));
+            ROLLED for (int k = 0; k < d; k++) a_Q12[k] = (int16_t)s_rshift_round(a32_QA1[k], 5);
+        });
     }
 }
 
@@ -524,28 +551,37 @@ DFN void silk_nlsf_unpack(int16_t *ec_ix, uint8_t *pred_Q8, const NlsfCB &cb, in
     }
 }
 
-// silk/NLSF_decode.c
-DNI void silk_nlsf_decode(int16_t *pNLSF_Q15, const int8_t *NLSFIndices, const NlsfCB &cb, SilkWork *sw)
+// silk/NLSF_decode.c, on every lane (the residuals' prediction on the first)
+DNI void silk_nlsf_decode(Lanes L, int16_t *pNLSF_Q15, const int8_t *NLSFIndices, const NlsfCB &cb, SilkWork *sw)
 {
     uint8_t *pred_Q8 = sw->pred_Q8;
     int16_t *ec_ix = sw->ec_ix, *res_Q10 = sw->res_Q10;
-    silk_nlsf_unpack(ec_ix, pred_Q8, cb, NLSFIndices[0]);
-    int32_t out_Q10 = 0;
-    ROLLED for (int i = cb.order - 1; i >= 0; i--) {
-        int32_t pred_Q10 = s_smulbb(out_Q10, (int16_t)pred_Q8[i]) >> 8;
-        out_Q10 = shl32(NLSFIndices[i + 1], 10);
-        if (out_Q10 > 0) out_Q10 -= 102;            // SILK_FIX_CONST(NLSF_QUANT_LEVEL_ADJ, 10)
-        else if (out_Q10 < 0) out_Q10 += 102;
-        out_Q10 = s_smlawb(pred_Q10, out_Q10, cb.quantStepSize_Q16);
-        res_Q10[i] = (int16_t)out_Q10;
-    }
+    lead(L, [&]() CUO_INLINE {
+        silk_nlsf_unpack(ec_ix, pred_Q8, cb, NLSFIndices[0]);
+        int32_t out_Q10 = 0;
+        ROLLED for (int i = cb.order - 1; i >= 0; i--) {
+            int32_t pred_Q10 = s_smulbb(out_Q10, (int16_t)pred_Q8[i]) >> 8;
+            out_Q10 = shl32(NLSFIndices[i + 1], 10);
+            if (out_Q10 > 0) out_Q10 -= 102;            // SILK_FIX_CONST(NLSF_QUANT_LEVEL_ADJ, 10)
+            else if (out_Q10 < 0) out_Q10 += 102;
+            out_Q10 = s_smlawb(pred_Q10, out_Q10, cb.quantStepSize_Q16);
+            res_Q10[i] = (int16_t)out_Q10;
+        }
+    });
     const uint8_t *el = &cb.CB1_NLSF_Q8[NLSFIndices[0] * cb.order];
     const int16_t *w = &cb.CB1_Wght_Q9[NLSFIndices[0] * cb.order];
-    ROLLED for (int i = 0; i < cb.order; i++) {
+    LFOR(L, i, 0, cb.order) {
         int32_t t = wadd(shl32((int32_t)res_Q10[i], 14) / w[i], shl32((int16_t)el[i], 7));
         pNLSF_Q15[i] = (int16_t)s_limit(t, 0, 32767);
     }
-    silk_nlsf_stabilize(pNLSF_Q15, cb.deltaMin_Q15, cb.order);
+    lsync(L);
+    // silk_NLSF_stabilize leaves values that keep their distances alone
+    int tight = 0;
+    LFOR(L, i, 0, cb.order + 1) {
+        const int32_t above = i < cb.order ? pNLSF_Q15[i] : 1 << 15, below = i > 0 ? pNLSF_Q15[i - 1] : 0;
+        tight |= above - (below + cb.deltaMin_Q15[i]) < 0;
+    }
+    if (lor(L, (uint32_t)tight)) lead(L, [&]() CUO_INLINE { silk_nlsf_stabilize(pNLSF_Q15, cb.deltaMin_Q15, cb.order); });
 }
 
 // silk/LPC_analysis_filter.c, split over lanes (each output is independent)
@@ -881,44 +917,50 @@ DNI void silk_gains_dequant(int32_t *gain_Q16, const int8_t *ind, int32_t *prev_
     }
 }
 
-DNI void silk_decode_parameters(SilkChan *c, SilkCtrl *ctrl, int condCoding, SilkWork *sw)
+// On every lane; ends with a barrier.
+DNI void silk_decode_parameters(Lanes L, SilkChan *c, SilkCtrl *ctrl, int condCoding, SilkWork *sw)
 {
     int16_t *pNLSF_Q15 = sw->pNLSF_Q15, *pNLSF0_Q15 = sw->pNLSF0_Q15;
     SilkIndices *ix = &c->indices;
-    silk_gains_dequant(ctrl->Gains_Q16, ix->GainsIndices, &c->LastGainIndex, condCoding == CODE_COND,
-                       c->nb_subfr);
-    NlsfCB cb = silk_nlsf_cb(c->LPC_order);
-    silk_nlsf_decode(pNLSF_Q15, ix->NLSFIndices, cb, sw);
-    silk_nlsf2a(ctrl->PredCoef_Q12[1], pNLSF_Q15, c->LPC_order, sw);
-    if (c->first_frame_after_reset == 1) ix->NLSFInterpCoef_Q2 = 4;
+    const int order = c->LPC_order;
+    NlsfCB cb = silk_nlsf_cb(order);
+    silk_nlsf_decode(L, pNLSF_Q15, ix->NLSFIndices, cb, sw);
+    silk_nlsf2a(L, ctrl->PredCoef_Q12[1], pNLSF_Q15, order, sw);
+    lead(L, [&]() CUO_INLINE {
+        silk_gains_dequant(ctrl->Gains_Q16, ix->GainsIndices, &c->LastGainIndex, condCoding == CODE_COND,
+                           c->nb_subfr);
+        if (c->first_frame_after_reset == 1) ix->NLSFInterpCoef_Q2 = 4;
+    });
     if (ix->NLSFInterpCoef_Q2 < 4) {
-        ROLLED for (int i = 0; i < c->LPC_order; i++)
+        LFOR(L, i, 0, order)
             pNLSF0_Q15[i] = (int16_t)(c->prevNLSF_Q15[i] +
                 ((ix->NLSFInterpCoef_Q2 * (pNLSF_Q15[i] - c->prevNLSF_Q15[i])) >> 2));
-        silk_nlsf2a(ctrl->PredCoef_Q12[0], pNLSF0_Q15, c->LPC_order, sw);
+        silk_nlsf2a(L, ctrl->PredCoef_Q12[0], pNLSF0_Q15, order, sw);
     } else {
-        ROLLED for (int i = 0; i < c->LPC_order; i++) ctrl->PredCoef_Q12[0][i] = ctrl->PredCoef_Q12[1][i];
+        LFOR(L, i, 0, order) ctrl->PredCoef_Q12[0][i] = ctrl->PredCoef_Q12[1][i];
     }
-    ROLLED for (int i = 0; i < c->LPC_order; i++) c->prevNLSF_Q15[i] = pNLSF_Q15[i];
-    if (c->lossCnt) {
-        silk_bwexpander(ctrl->PredCoef_Q12[0], c->LPC_order, 63570);
-        silk_bwexpander(ctrl->PredCoef_Q12[1], c->LPC_order, 63570);
-    }
-    if (ix->signalType == SIG_VOICED) {
-        silk_decode_pitch(ix->lagIndex, ix->contourIndex, ctrl->pitchL, c->fs_kHz, c->nb_subfr);
-        const int8_t *cbk = ix->PERIndex == 0 ? T_silk_LTP_gain_vq_0
-                          : (ix->PERIndex == 1 ? T_silk_LTP_gain_vq_1 : T_silk_LTP_gain_vq_2);
-        ROLLED for (int k = 0; k < c->nb_subfr; k++) {
-            int I = ix->LTPIndex[k];
-            ROLLED for (int i = 0; i < 5; i++) ctrl->LTPCoef_Q14[k * 5 + i] = (int16_t)shl32(cbk[I * 5 + i], 7);
+    LFOR(L, i, 0, order) c->prevNLSF_Q15[i] = pNLSF_Q15[i];
+    lead(L, [&]() CUO_INLINE {
+        if (c->lossCnt) {
+            silk_bwexpander(ctrl->PredCoef_Q12[0], order, 63570);
+            silk_bwexpander(ctrl->PredCoef_Q12[1], order, 63570);
         }
-        ctrl->LTP_scale_Q14 = T_silk_LTPScales_table_Q14[ix->LTP_scaleIndex];
-    } else {
-        ROLLED for (int k = 0; k < c->nb_subfr; k++) ctrl->pitchL[k] = 0;
-        ROLLED for (int k = 0; k < 5 * c->nb_subfr; k++) ctrl->LTPCoef_Q14[k] = 0;
-        ix->PERIndex = 0;
-        ctrl->LTP_scale_Q14 = 0;
-    }
+        if (ix->signalType == SIG_VOICED) {
+            silk_decode_pitch(ix->lagIndex, ix->contourIndex, ctrl->pitchL, c->fs_kHz, c->nb_subfr);
+            const int8_t *cbk = ix->PERIndex == 0 ? T_silk_LTP_gain_vq_0
+                              : (ix->PERIndex == 1 ? T_silk_LTP_gain_vq_1 : T_silk_LTP_gain_vq_2);
+            ROLLED for (int k = 0; k < c->nb_subfr; k++) {
+                int I = ix->LTPIndex[k];
+                ROLLED for (int i = 0; i < 5; i++) ctrl->LTPCoef_Q14[k * 5 + i] = (int16_t)shl32(cbk[I * 5 + i], 7);
+            }
+            ctrl->LTP_scale_Q14 = T_silk_LTPScales_table_Q14[ix->LTP_scaleIndex];
+        } else {
+            ROLLED for (int k = 0; k < c->nb_subfr; k++) ctrl->pitchL[k] = 0;
+            ROLLED for (int k = 0; k < 5 * c->nb_subfr; k++) ctrl->LTPCoef_Q14[k] = 0;
+            ix->PERIndex = 0;
+            ctrl->LTP_scale_Q14 = 0;
+        }
+    });
 }
 
 // ------------------------------------------------------------------ synthesis
@@ -999,6 +1041,103 @@ DNI void silk_lpc_synth(Lanes L, int32_t *hist, const int16_t *A_Q12, const int3
 #pragma unroll
     for (int t = 0; t < 16; t++) hist[t] = win[t];
     lsync(L);
+}
+
+// The same recursion with the taps on older outputs split over eight lanes of
+// the group (wider groups repeat them): lane s + 4 h sums the window positions
+// of parity h for sample s of the four, the halves are added and every lane
+// gets the four sums; it carries the in-block part on by itself.  A mad.hi
+// issues once in 6.6 cycles, so the 58 of a block held one lane for 380 cycles;
+// split they take 53 and the exchange 50.  (20 ms at 16 kHz: 52 k cycles with
+// one lane's sums, LPC_MEASURED.)
+template <int ORD>
+DNI void silk_lpc_synth_lanes(Lanes L, int32_t *hist, const int16_t *A_Q12, const int32_t *exc, int32_t *v, int n)
+{
+    constexpr int FIRST = 16 - ORD, T = ORD / 2;   // first window position with a tap; positions of a parity
+    const int s = L.id & 3, half = (L.id >> 2) & 1;
+    int32_t coef[T], win[T], a[3];   // win: this lane's positions FIRST + 2 t + half
+#pragma unroll
+    for (int t = 0; t < T; t++) {
+        const int m = FIRST + 2 * t + half, j = 15 + s - m;
+        coef[t] = j < ORD ? shl32((int32_t)A_Q12[j], 16) : 0;
+        win[t] = hist[m];
+    }
+#pragma unroll
+    for (int j = 0; j < 3; j++) a[j] = shl32((int32_t)A_Q12[j], 16);
+    int32_t ahead[4];   // the next four inputs, loaded while these four are computed
+#pragma unroll
+    for (int k = 0; k < 4; k++) ahead[k] = exc[k];
+    ROLLED for (int i = 0; i < n; i += 4) {
+        int32_t e[4], o[4];
+        const int nx = i + 4 < n ? i + 4 : i;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            e[k] = ahead[k];
+            ahead[k] = exc[nx + k];
+        }
+        int32_t p0 = half ? 0 : ORD >> 1, p1 = 0;
+#pragma unroll
+        for (int t = 0; t < T; t++) {
+            if (t & 1) p1 = s_smlawh(p1, win[t], coef[t]);
+            else p0 = s_smlawh(p0, win[t], coef[t]);
+        }
+        p0 = wadd(p0, p1);
+        p0 = wadd(p0, lget(L, p0, L.id ^ 4));
+        int32_t p[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) p[k] = lget(L, p0, k);
+        const int32_t h1 = p[1], h2 = p[2], h3 = p[3];
+        o[0] = wadd(e[0], shl32(p[0], 4));
+        p[1] = s_smlawh(h1, o[0], a[0]);
+        o[1] = wadd(e[1], shl32(p[1], 4));
+        p[2] = s_smlawh(s_smlawh(h2, o[0], a[1]), o[1], a[0]);
+        o[2] = wadd(e[2], shl32(p[2], 4));
+        p[3] = s_smlawh(s_smlawh(s_smlawh(h3, o[0], a[2]), o[1], a[1]), o[2], a[0]);
+        o[3] = wadd(e[3], shl32(p[3], 4));
+        uint32_t far_p = 0, far_e = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            far_p |= (uint32_t)p[k] + (1u << 26);
+            far_e |= (uint32_t)e[k] + (1u << 30);
+        }
+        if ((far_p >> 27) | (far_e >> 31)) {
+            ROLLED for (int k = 0; k < 4; k++) {   // k is the sample: its sum from the exact ones before it
+                int32_t q = k == 0 ? p[0] : k == 1 ? h1 : k == 2 ? h2 : h3;
+                if (k > 2) q = s_smlawh(q, o[0], a[2]);
+                if (k > 1) q = s_smlawh(q, k == 2 ? o[0] : o[1], a[1]);
+                if (k > 0) q = s_smlawh(q, k == 1 ? o[0] : k == 2 ? o[1] : o[2], a[0]);
+                const int32_t x = s_add_sat32(k == 0 ? e[0] : k == 1 ? e[1] : k == 2 ? e[2] : e[3],
+                                              s_lshift_sat32(q, 4));
+                if (k == 0) o[0] = x;
+                else if (k == 1) o[1] = x;
+                else if (k == 2) o[2] = x;
+                else o[3] = x;
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < T - 2; t++) win[t] = win[t + 2];
+        win[T - 2] = half ? o[1] : o[0];
+        win[T - 1] = half ? o[3] : o[2];
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[i + k] = o[k];
+    }
+    lsync(L);   // every lane has read the window and the lanes have written v
+    LFOR(L, t, 0, 16) hist[t] = v[n - 16 + t];
+    lsync(L);
+}
+
+// LPC synthesis of n samples (a multiple of 4, at least 16); v and exc are
+// different arrays.
+DFN void silk_lpc_synth_any(const Lanes &L, int order, int32_t *hist, const int16_t *A_Q12, const int32_t *exc,
+                            int32_t *v, int n)
+{
+    if (L.n >= 8) {
+        if (order == 16) silk_lpc_synth_lanes<16>(L, hist, A_Q12, exc, v, n);
+        else silk_lpc_synth_lanes<10>(L, hist, A_Q12, exc, v, n);
+    } else {
+        if (order == 16) silk_lpc_synth<16>(L, hist, A_Q12, exc, v, n);
+        else silk_lpc_synth<10>(L, hist, A_Q12, exc, v, n);
+    }
 }
 
 // silk/decode_core.c: excitation, LTP and LPC synthesis for one frame
@@ -1118,8 +1257,7 @@ DNI void silk_decode_core(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *xq, con
         PHASE_END(PH_SILK_LTP, t_ltp, L.id);
         PHASE_BEGIN(t_lpc);
         int32_t *v = w->sLPC_Q14;
-        if (c->LPC_order == 16) silk_lpc_synth<16>(L, c->sLPC_Q14_buf, A_Q12, pres, v, c->subfr_length);
-        else silk_lpc_synth<10>(L, c->sLPC_Q14_buf, A_Q12, pres, v, c->subfr_length);
+        silk_lpc_synth_any(L, c->LPC_order, c->sLPC_Q14_buf, A_Q12, pres, v, c->subfr_length);
         LFOR(L, i, 0, c->subfr_length) pxq[i] = (int16_t)s_sat16(s_rshift_round(s_smulww(v[i], Gain_Q10), 8));
         pexc += c->subfr_length;
         pxq += c->subfr_length;
@@ -1186,15 +1324,6 @@ struct SilkRandPowers {
 TABG(SilkRandPowers, T_silk_rand) = SilkRandPowers();
 DFN int32_t silk_rand_at(int32_t seed, int k) { return (int32_t)(T_silk_rand.a[k] * (uint32_t)seed + T_silk_rand.c[k]); }
 
-// LPC synthesis of a whole frame (lost frames and comfort noise); v and exc are
-// different arrays.
-DFN void silk_lpc_synth_frame(const Lanes &L, int order, int32_t *hist, const int16_t *A_Q12, const int32_t *exc,
-                              int32_t *v, int n)
-{
-    if (order == 16) silk_lpc_synth<16>(L, hist, A_Q12, exc, v, n);
-    else silk_lpc_synth<10>(L, hist, A_Q12, exc, v, n);
-}
-
 // silk_PLC_conceal.  Every lane works out the gains and the lanes split the
 // sample loops: the LTP excitation in blocks shorter than the lag, its random
 // samples by the generator's powers, the LPC synthesis as in a received frame.
@@ -1232,11 +1361,9 @@ DNI void silk_plc_conceal(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *frame, 
     const int first_loss = c->lossCnt == 0, voiced = c->prevSignalType == SIG_VOICED;
     const int32_t harm_Gain_Q15 = first_loss ? 32440 : 31130;
     int32_t rand_Gain_Q15 = voiced ? (first_loss ? 31130 : 26214) : (first_loss ? 32440 : 29491);
-    int32_t invGain_Q30 = 0;
     lead(L, [&]() CUO_INLINE {
         if (c->first_frame_after_reset) ROLLED for (int i = 0; i < 16; i++) p->prevLPC_Q12[i] = 0;
         silk_bwexpander(p->prevLPC_Q12, c->LPC_order, 64881);   // SILK_FIX_CONST(0.99, 16)
-        if (first_loss && !voiced) invGain_Q30 = silk_lpc_inv_pred_gain(p->prevLPC_Q12, c->LPC_order, w->sw.A);
     });
     if (first_loss) {
         rand_scale_Q14 = 1 << 14;
@@ -1246,7 +1373,7 @@ DNI void silk_plc_conceal(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *frame, 
             rand_scale_Q14 = rand_scale_Q14 > 3277 ? rand_scale_Q14 : 3277;
             rand_scale_Q14 = (int16_t)(s_smulbb(rand_scale_Q14, p->prevLTP_scale_Q14) >> 14);
         } else {
-            int32_t down = min32((1 << 30) >> 3, lbcast(L, invGain_Q30));
+            int32_t down = min32((1 << 30) >> 3, silk_lpc_inv_pred_gain(L, p->prevLPC_Q12, c->LPC_order, w->sw.A));
             down = max32((1 << 30) >> 8, down);
             down = shl32(down, 3);
             rand_Gain_Q15 = s_smulwb(down, rand_Gain_Q15) >> 14;
@@ -1287,7 +1414,7 @@ DNI void silk_plc_conceal(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *frame, 
         lag = s_rshift_round(pitchL_Q8, 8);
     }
     int32_t *v = w->CNG_sig_Q14;
-    silk_lpc_synth_frame(L, c->LPC_order, c->sLPC_Q14_buf, A_Q12, &sLTP_Q14[c->ltp_mem_length], v, c->frame_length);
+    silk_lpc_synth_any(L, c->LPC_order, c->sLPC_Q14_buf, A_Q12, &sLTP_Q14[c->ltp_mem_length], v, c->frame_length);
     LFOR(L, i, 0, c->frame_length)
         frame[i] = (int16_t)s_sat16(s_rshift_round(s_smulww(v[i], prevGain_Q10[1]), 8));
     lead(L, [&]() CUO_INLINE {
@@ -1375,11 +1502,9 @@ DNI void silk_cng_generate(Lanes L, SilkChan *c, int16_t *frame, int length, Sil
     ROLLED while (exc_mask > length) exc_mask >>= 1;
     const int32_t seed = g->rand_seed;
     LFOR(L, i, 0, length) sig[i] = g->CNG_exc_buf_Q14[(silk_rand_at(seed, i + 1) >> 24) & exc_mask];
-    lead(L, [&]() CUO_INLINE {
-        g->rand_seed = silk_rand_at(seed, length);
-        silk_nlsf2a(A_Q12, g->CNG_smth_NLSF_Q15, c->LPC_order, &w->sw);
-    });
-    silk_lpc_synth_frame(L, c->LPC_order, g->CNG_synth_state, A_Q12, sig, v, length);
+    lead(L, [&]() CUO_INLINE { g->rand_seed = silk_rand_at(seed, length); });
+    silk_nlsf2a(L, A_Q12, g->CNG_smth_NLSF_Q15, c->LPC_order, &w->sw);
+    silk_lpc_synth_any(L, c->LPC_order, g->CNG_synth_state, A_Q12, sig, v, length);
     LFOR(L, i, 0, length)
         frame[i] = (int16_t)s_sat16((int32_t)frame[i] + s_sat16(s_rshift_round(s_smulww(v[i], gain_Q10), 8)));
     lsync(L);
@@ -1440,8 +1565,8 @@ DNI void silk_decode_frame(Lanes L, SilkChan *c, RangeDec *rd, int16_t *pOut, in
     int Lf = c->frame_length;
     if (lostFlag == LOSS_NONE || (lostFlag == LOSS_LBRR && c->LBRR_flags[c->nFramesDecoded] == 1)) {
         int16_t *pulses = w->pulses;
-        // side information, pulses and parameters: entropy decoding and
-        // state updates in place, on the first lane
+        // side information and pulses: entropy decoding and state updates in
+        // place, on the first lane
         lead_rd(L, rd, [&]() CUO_INLINE {
             ctrl->LTP_scale_Q14 = 0;
             PHASE_BEGIN(t_ix);
@@ -1451,10 +1576,10 @@ DNI void silk_decode_frame(Lanes L, SilkChan *c, RangeDec *rd, int16_t *pOut, in
             silk_decode_pulses(rd, pulses, c->indices.signalType, c->indices.quantOffsetType, c->frame_length,
                                &w->sw);
             PHASE_END(PH_SILK_PULSES, t_pu, L.id);
-            PHASE_BEGIN(t_pa);
-            silk_decode_parameters(c, ctrl, condCoding, &w->sw);
-            PHASE_END(PH_SILK_PARAMS, t_pa, L.id);
         });
+        PHASE_BEGIN(t_pa);
+        silk_decode_parameters(L, c, ctrl, condCoding, &w->sw);
+        PHASE_END(PH_SILK_PARAMS, t_pa, L.id);
         PHASE_BEGIN(t_co);
         silk_decode_core(L, c, ctrl, pOut, pulses, w);
         PHASE_END(PH_SILK_CORE, t_co, L.id);

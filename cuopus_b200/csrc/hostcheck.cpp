@@ -160,7 +160,7 @@ void hc_imdct(const int32_t *in, int32_t *out, int shift, int stride)
 void hc_nlsf2a(int16_t *a_Q12, const int16_t *nlsf, int d)
 {
     cuo::SilkWork sw;
-    cuo::silk_nlsf2a(a_Q12, nlsf, d, &sw);
+    cuo::silk_nlsf2a(cuo::Lanes{0, 1, 1u}, a_Q12, nlsf, d, &sw);
 }
 
 // The decoder's SILK resampler to 48 kHz (all-pass up2 + FIR interpolation),

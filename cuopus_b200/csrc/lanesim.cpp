@@ -223,6 +223,16 @@ int32_t lanesim_max(LaneSim *s, int id, int32_t v)
     return t;
 }
 
+int32_t lanesim_get(LaneSim *s, int id, int32_t v, int src) NOINSTR;
+int32_t lanesim_get(LaneSim *s, int id, int32_t v, int src)
+{
+    s->xv[id] = v;
+    lanesim_sync(s, id);
+    v = s->xv[src];
+    lanesim_sync(s, id);
+    return v;
+}
+
 uint32_t lanesim_or(LaneSim *s, int id, uint32_t v) NOINSTR;
 uint32_t lanesim_or(LaneSim *s, int id, uint32_t v)
 {
