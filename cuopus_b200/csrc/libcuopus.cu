@@ -151,18 +151,11 @@ int default_width()
     return p;
 }
 
-// Decoder warps per SM of the library's own launches (CUOPUS_WARPS_PER_SM).
-// At 32 lanes per chain the default is 5, fewer than the GPU holds (8 at
-// 128-thread blocks): the decoder waits on instruction fetch when more of its
-// warps share an SM, so each chain decodes faster and the longest chains
-// finish sooner (the occupancy autotuner measured 5 per SM best on the mixed
-// batch).  At narrower widths a warp decodes several chains and the default
-// is every resident group (the 2 h file in 1 s chains at 8 lanes per chain
-// decoded in 151 ms with every group, 232 ms at 5 warps per SM).  Returns the
-// cuopus_batch.max_groups value for `width` lanes per chain (0 = all).
+// cuopus_batch.max_groups for `width` lanes per chain at CUOPUS_WARPS_PER_SM
+// decoder warps per SM; 0 (every resident group) when that is not set.
 int default_max_groups(int width)
 {
-    int wps = env_i("CUOPUS_WARPS_PER_SM", width == 32 ? 5 : 0);
+    int wps = env_i("CUOPUS_WARPS_PER_SM", 0);
     if (G.sm_count <= 0 || wps <= 0) return 0;
     return wps * G.sm_count * (32 / width);
 }
@@ -562,30 +555,59 @@ int plan_files(const uint8_t *const *oggs, const size_t *ns, int nfiles, bool re
 // threads against 200 ms at 128; whole streams at 32 lanes: equal).
 const int FILE_BLOCK = 64;
 
-// Lanes per chain of a file batch (CUOPUS_STRIDE, when set, decides).  A
-// batch's decode time is about max(longest chain, total work / decoder
-// groups) / per-group speed.  At 32 lanes a group decodes about 3x faster
-// than at 8 (lane-split loops), but 8 lanes give 6.4x the groups (every
-// resident group at 8 against 5 warps per SM at 32): long or uneven chains
-// (whole streams) decode faster at 32, many short chains (a long file cut in
-// 1 s chains) at 8.  Chain cost: its TOC samples x channels.
-int choose_width(const Plan &P)
+// Launch shape of a file batch: lanes per chain and decoder groups
+// (CUOPUS_STRIDE and CUOPUS_WARPS_PER_SM, when set, decide).  More lanes decode a
+// chain faster, fewer lanes put more chains on the GPU, and more warps on an SM
+// slow each other down, because each of them fetches its own part of a program
+// larger than the SM's instruction caches.  A shape's time is estimated as
+// max(longest chain, total work / groups, what a group with a second chain has
+// to do) / speed; the last term is taken at 0.7, since chains speed up as groups
+// run dry.  Chain cost: its TOC samples x channels.  Speeds are per group,
+// relative to 32 lanes at 4 warps per SM, from files of 300 to 5400 one-second
+// chains (ms at 32 lanes / 16 / 8):
+//   speech, 300 chains 19 / 26 / 42, 1800 58 / 42 / 50, 5400 160 / 113 / 81;
+//   mono and stereo mixed, 1085 chains 92 / 116 / 188 (105 at 5 warps per SM,
+//   138 at 8), 2070 165 / 140 / 230, 3100 248 / 207 / 272;
+//   voice, 600 chains 18 at 4 warps per SM (two rounds), 11.5 at 5;
+//   at 8 lanes, speech of 7200 chains 106 at 8 warps per SM and 112 at 12, voice
+//   of 5400 53 and 36 (two rounds at 8).
+struct LaunchShape {
+    int width, warps_per_sm;   // 0 warps: every resident group
+    double speed;
+};
+const LaunchShape SHAPES[] = {{32, 4, 1.0}, {32, 5, 0.8}, {16, 4, 0.62}, {16, 6, 0.55}, {8, 8, 0.37}, {8, 0, 0.33}};
+
+long long shape_groups(const LaunchShape &s)
 {
-    const char *e = getenv("CUOPUS_STRIDE");
-    if (e && atoi(e) > 0) return default_width();
-    double sum = 0.0, mx = 0.0;
-    for (size_t c = 0; c < P.first.size(); c++) {
-        double w = (double)P.cap[c] * (double)P.chans[c];
-        sum += w;
-        mx = std::max(mx, w);
+    const long long resident = resident_groups(FILE_BLOCK, s.width);
+    const long long asked = (long long)s.warps_per_sm * G.sm_count * (32 / s.width);
+    return s.warps_per_sm > 0 ? std::min(resident, asked) : resident;
+}
+
+// Sets width and max_groups (0: every resident group).
+void choose_launch(const Plan &P, int32_t &width, int32_t &max_groups)
+{
+    const char *e = getenv("CUOPUS_STRIDE"), *ew = getenv("CUOPUS_WARPS_PER_SM");
+    const int want_width = e && atoi(e) > 0 ? default_width() : 0;
+    std::vector<double> cost(P.first.size());
+    double sum = 0.0;
+    for (size_t c = 0; c < cost.size(); c++) sum += cost[c] = (double)P.cap[c] * (double)P.chans[c];
+    std::sort(cost.begin(), cost.end(), std::greater<double>());
+    double best = -1.0;
+    width = want_width > 0 ? want_width : 32;
+    max_groups = default_max_groups(width);
+    for (const LaunchShape &s : SHAPES) {
+        if (want_width && s.width != want_width) continue;
+        const long long g = std::max(shape_groups(s), 1LL);
+        double t = cost.empty() ? 0.0 : std::max(cost[0], sum / (double)g);
+        if ((long long)cost.size() > g) t = std::max(t, 0.7 * (cost[g - 1] + cost[g]));
+        t /= s.speed;
+        if (best >= 0.0 && t >= best) continue;
+        best = t;
+        width = s.width;
+        max_groups = s.warps_per_sm > 0 ? (int32_t)g : 0;
     }
-    long long g32 = default_max_groups(32);
-    if (g32 <= 0) g32 = resident_groups(FILE_BLOCK, 32);
-    long long g8 = resident_groups(FILE_BLOCK, 8);
-    const double speed32 = 3.0;   // per-group speed at 32 lanes relative to 8
-    double t32 = std::max(mx, sum / (double)std::max(g32, 1LL)) / speed32;
-    double t8 = std::max(mx, sum / (double)std::max(g8, 1LL));
-    return t8 < t32 ? 8 : 32;
+    if (ew && atoi(ew) > 0) max_groups = default_max_groups(width);
 }
 
 // fn(begin, end) over [0, n) in up to `threads` contiguous ranges, the first
@@ -667,9 +689,8 @@ int run_plan(const Plan &P, cudaStream_t st, Err &err, int16_t *direct_out = nul
     b.res = (uint32_t *)G.res.p;
     b.nchains = (int32_t)nch;
     if ((rc = ensure_occupancy(err))) return rc;
-    b.width = choose_width(P);
     b.block = FILE_BLOCK;
-    b.max_groups = default_max_groups(b.width);
+    choose_launch(P, b.width, b.max_groups);
     G.last_width = b.width;
     // longest chains first through the device queue, by the fitted additive
     // cost of their packets (CUOPUS_ORDER=samples: by decoded samples x channels)

@@ -65,3 +65,20 @@ def test_predictions_around_a_block(cuda, n):
     y = m.predict_raw(cuda.from_numpy(x).cuda()).cpu().numpy()
     want = mlp_port.forward(m.params.cpu().numpy().astype(np.float64), x.astype(np.float64))
     assert np.allclose(y, want, rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("files", [1, 60, 110, 420])
+def test_launch_shapes_decode_the_same(cuda, files, monkeypatch):
+    """The launch shape follows the number of chains (7 per file: 32, 16 and 8
+    lanes, and fewer warps per SM than fit); the samples do not."""
+    from cuopus_b200 import cuopus_native as cn
+    with open(os.path.join(ROOT, "tests", "golden", "streams", "mixed_stereo_b.opus"), "rb") as f:
+        data = f.read()
+    (want, ch), = cn.decode_ogg_to_int16([data])
+    got = cn.decode_ogg_to_int16([data] * files)
+    assert all(c == ch and cuda.equal(t, want) for t, c in got)
+    for width in ("8", "16", "32"):
+        monkeypatch.setenv("CUOPUS_STRIDE", width)
+        (t, _), = cn.decode_ogg_to_int16([data])
+        assert cn.last_stats()["width"] == int(width) and cuda.equal(t, want)
