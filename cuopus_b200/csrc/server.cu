@@ -161,7 +161,8 @@ struct Wave {
 struct cuopus_server {
     cuopus_server_config cfg{};
     int dev = 0;
-    int width = 32, block = 128, groups = 0;
+    int width = 32, block = 128, groups = 0, sms = 0;
+    bool auto_width = false;                       // lanes per chain chosen wave by wave
     uint8_t *arena = nullptr;
     RangeAlloc ra;
     std::vector<Wave> waves;
@@ -183,6 +184,7 @@ struct cuopus_server {
     bool admit_locked();
     bool worth_launching_locked();
     bool build_wave_locked(Wave &w);
+    int wave_width(size_t nch) const;
     void finish_wave(Wave &w);
 };
 
@@ -380,8 +382,8 @@ void cuopus_server::run()
                 a.res = (cuo::ChainResult *)(d + t.res);
                 a.slots = (cuo::ChainSlot *)w.slots;
                 a.nchains = (int)nch;
-                a.width = width;
-                int gpb = block / width;
+                a.width = wave_width(nch);
+                int gpb = block / a.width;
                 int blocks = (int)((nch + gpb - 1) / gpb);
                 w.d_res = (uint32_t *)(d + t.res);
                 w.t_launch = now_ms();
@@ -438,6 +440,22 @@ void cuopus_server::run()
             }
         cv_done.notify_all();
     }
+}
+
+// Lanes per chain of a wave of nch chains (server thread).  Wide groups decode a
+// chain faster (a second of mixed audio 18 ms at 32 lanes, 33 at 16, 60 at 8),
+// narrow ones keep more chains on the GPU: with the chains of the waves in
+// flight counted in, 32 lanes up to ten chains per SM, 16 up to 24, then 8 (the
+// file entry points' measurements: 1085 chains 92 ms at 32 lanes and 116 at 16,
+// 2070 165 and 140, 5400 160, 113 and 81 at 8).  24 files together, 531 s: 230 ms
+// with 8 lanes throughout, 79 so.
+int cuopus_server::wave_width(size_t nch) const
+{
+    if (!auto_width) return width;
+    size_t load = nch;
+    for (const Wave &w : waves)
+        if (w.busy) load += w.chains.size();
+    return load <= 10 * (size_t)sms ? 32 : load <= 24 * (size_t)sms ? 16 : width;
 }
 
 // Check a finished wave's chains; complete the requests whose chains are all
@@ -506,15 +524,16 @@ extern "C" int cuopus_server_create(const cuopus_server_config *cfg, cuopus_serv
     if (s->cfg.seg_s <= 0) s->cfg.seg_s = 1.0;
     if (s->cfg.preroll_ms < 0) s->cfg.preroll_ms = 250.0;
     if (s->cfg.preroll_ms == 0 && !(cfg && cfg->preroll_ms == 0)) s->cfg.preroll_ms = 250.0;
-    // chains of a few seconds at most: many short chains decode faster at 8
-    // lanes on every resident group than at 32 (the file entry points' rule)
+    // chains of a few seconds at most: the slots are for 8 lanes on every resident
+    // group, and each wave picks its own width (wave_width)
+    s->auto_width = s->cfg.width <= 0 && s->cfg.seg_s <= 4.0;
     s->width = s->cfg.width > 0 ? s->cfg.width : (s->cfg.seg_s <= 4.0 ? 8 : 32);
     s->block = s->cfg.block > 0 ? s->cfg.block : 64;
     if ((s->width & (s->width - 1)) || s->width > 32 || s->block % s->width || s->block > 128 || s->block % 32)
         return fail(errbuf, errcap, 3, "bad width %d / block %d", s->width, s->block);
     cudaError_t e = cudaGetDevice(&s->dev);
     if (e != cudaSuccess) return fail(errbuf, errcap, 2, "cudaGetDevice: %s", cudaGetErrorString(e));
-    int sms = 0, per_sm = 0;
+    int per_sm = 0, &sms = s->sms;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->dev);
     e = cuo::decode_kernel_occupancy(s->block, s->width, &per_sm);
     if (e != cudaSuccess) return fail(errbuf, errcap, 2, "occupancy: %s", cudaGetErrorString(e));
