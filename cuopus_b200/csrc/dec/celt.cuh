@@ -267,8 +267,10 @@ DFN const int16_t *fft_bitrev(int shift)
     return shift == 0 ? T_fft0_bitrev : shift == 1 ? T_fft1_bitrev : shift == 2 ? T_fft2_bitrev : T_fft3_bitrev;
 }
 
-// celt/mdct.c clt_mdct_backward_c
-DNI void mdct_backward(Lanes L, const int32_t *in, int32_t *out, int shift, int stride)
+// celt/mdct.c clt_mdct_backward_c.  With `twin`, a second output buffer gets the
+// same transform (a mono frame in a stereo stream): what precedes the
+// overlap-add is done once and copied.
+DNI void mdct_backward(Lanes L, const int32_t *in, int32_t *out, int shift, int stride, int32_t *twin = nullptr)
 {
     int N = T_CELT_MDCT_N;
     const int16_t *trig = T_celt_mdct_trig;
@@ -304,9 +306,15 @@ DNI void mdct_backward(Lanes L, const int32_t *in, int32_t *out, int shift, int 
         yp0[1] = yi;
     }
     lsync(L);
+    if (twin) {
+        LFOR(L, i, 0, N2) twin[CELT_OVERLAP / 2 + i] = yp[i];
+        lsync(L);
+    }
     const int16_t *w = T_celt_window;
-    LFOR(L, i, 0, CELT_OVERLAP / 2) {
-        int32_t *xp1 = out + CELT_OVERLAP - 1 - i, *yp1 = out + i;
+    LFOR(L, q, 0, twin ? CELT_OVERLAP : CELT_OVERLAP / 2) {
+        const int i = q < CELT_OVERLAP / 2 ? q : q - CELT_OVERLAP / 2;
+        int32_t *o = q < CELT_OVERLAP / 2 ? out : twin;
+        int32_t *xp1 = o + CELT_OVERLAP - 1 - i, *yp1 = o + i;
         int32_t x1 = *xp1, x2 = *yp1;
         int16_t w1 = w[i], w2 = w[CELT_OVERLAP - 1 - i];
         *yp1 = wsub(c_mul16_32_q15(w2, x2), c_mul16_32_q15(w1, x1));
@@ -317,30 +325,59 @@ DNI void mdct_backward(Lanes L, const int32_t *in, int32_t *out, int shift, int 
 
 // ------------------------------------------------------------------ synthesis helpers
 
-// celt/bands.c denormalise_bands (downsample 1)
+// Band of a bin of the shortest frame (eBands inverted).
+struct BandOf {
+    uint8_t b[101];
+    constexpr BandOf() : b()
+    {
+        const int e[22] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16, 20, 24, 28, 34, 40, 48, 60, 78, 100};
+        for (int k = 0; k < 21; k++)
+            for (int u = e[k]; u < e[k + 1]; u++) b[u] = (uint8_t)k;
+        b[100] = 21;
+    }
+};
+TABC(BandOf, T_band_of) = BandOf();
+TABG(BandOf, T_band_of_lanes) = BandOf();   // for lookups that differ between the lanes
+
+// celt/bands.c denormalise_bands (downsample 1).  The lanes work out the bands'
+// gains and shifts first (gain << 8 | shift + 2, in band_gain), then scale the
+// bins, four in flight each.
 DNI void denormalise_bands(Lanes L, const int16_t *X, int32_t *freq, const int16_t *bandLogE, int start,
-                           int end, int M, int silence)
+                           int end, int LM, int silence, int32_t *band_gain)
 {
     const int16_t *eB = T_celt_eBands;
-    int N = M * T_CELT_SHORTMDCT;
-    int bound = M * eB[end];
-    if (silence) { bound = 0; start = end = 0; }
-    LFOR(L, i, 0, M * eB[start]) freq[i] = 0;
-    ROLLED for (int b = start; b < end; b++) {
-        int j0 = M * eB[b], j1 = M * eB[b + 1];
+    const int N = T_CELT_SHORTMDCT << LM;
+    int bound = eB[end] << LM, low = eB[start] << LM;
+    if (silence) bound = low = 0;
+    LFOR(L, b, start, end) {
         int16_t lg = c_sat16(wadd(bandLogE[b], shl32((int32_t)T_celt_eMeans[b], 6)));
         int shift = 16 - (lg >> 10);
         int16_t g;
         if (shift > 31) { shift = 0; g = 0; }
         else g = (int16_t)c_exp2_frac((int16_t)(lg & 1023));
-        if (shift < 0) {
-            if (shift <= -2) { g = 16384; shift = -2; }
-            LFOR(L, j, j0, j1) freq[j] = shl32(c_mul16(X[j], g), -shift);
-        } else {
-            LFOR(L, j, j0, j1) freq[j] = c_mul16(X[j], g) >> shift;
+        if (shift <= -2) { g = 16384; shift = -2; }
+        band_gain[b] = shl32((int32_t)g, 8) | (shift + 2);
+    }
+    lsync(L);
+    ROLLED for (int j0 = L.id; j0 < N; j0 += 4 * L.n) {
+        int32_t x[4], g[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int j = j0 + k * L.n;
+            x[k] = 0;
+            g[k] = 2;
+            if (j >= low && j < bound) {
+                x[k] = X[j];
+                g[k] = band_gain[T_band_of_lanes.b[j >> LM]];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int j = j0 + k * L.n, shift = (g[k] & 0xff) - 2;
+            const int32_t v = c_mul16(x[k], g[k] >> 8);
+            if (j < N) freq[j] = shift < 0 ? shl32(v, -shift) : v >> shift;
         }
     }
-    LFOR(L, i, bound, N) freq[i] = 0;
     lsync(L);
 }
 
@@ -523,22 +560,19 @@ DNI void celt_synthesis(Lanes L, CeltScratch *w, const int16_t *X, int32_t **out
     else { B = 1; NB = T_CELT_SHORTMDCT << LM; shift = T_CELT_MAXLM - LM; }
     int32_t *freq = w->freq;
     if (CC == 2 && C == 1) {
-        denormalise_bands(L, X, freq, oldBandE, start, effEnd, M, silence);
-        int32_t *freq2 = out_syn[1] + CELT_OVERLAP / 2;
-        LFOR(L, i, 0, N) freq2[i] = freq[i];
-        lsync(L);
-        ROLLED for (int b = 0; b < B; b++) mdct_backward(L, &freq2[b], out_syn[0] + NB * b, shift, B);
-        ROLLED for (int b = 0; b < B; b++) mdct_backward(L, &freq[b], out_syn[1] + NB * b, shift, B);
+        denormalise_bands(L, X, freq, oldBandE, start, effEnd, LM, silence, w->bits1);
+        ROLLED for (int b = 0; b < B; b++)
+            mdct_backward(L, &freq[b], out_syn[0] + NB * b, shift, B, out_syn[1] + NB * b);
     } else if (CC == 1 && C == 2) {
         int32_t *freq2 = out_syn[0] + CELT_OVERLAP / 2;
-        denormalise_bands(L, X, freq, oldBandE, start, effEnd, M, silence);
-        denormalise_bands(L, X + N, freq2, oldBandE + CELT_NB, start, effEnd, M, silence);
+        denormalise_bands(L, X, freq, oldBandE, start, effEnd, LM, silence, w->bits1);
+        denormalise_bands(L, X + N, freq2, oldBandE + CELT_NB, start, effEnd, LM, silence, w->bits1);
         LFOR(L, i, 0, N) freq[i] = wadd(freq[i] >> 1, freq2[i] >> 1);
         lsync(L);
         ROLLED for (int b = 0; b < B; b++) mdct_backward(L, &freq[b], out_syn[0] + NB * b, shift, B);
     } else {
         ROLLED for (int c = 0; c < CC; c++) {
-            denormalise_bands(L, X + c * N, freq, oldBandE + c * CELT_NB, start, effEnd, M, silence);
+            denormalise_bands(L, X + c * N, freq, oldBandE + c * CELT_NB, start, effEnd, LM, silence, w->bits1);
             ROLLED for (int b = 0; b < B; b++) mdct_backward(L, &freq[b], out_syn[c] + NB * b, shift, B);
         }
     }
@@ -649,9 +683,9 @@ DFN int pulses2bits(int band, int LM, int pulses)
     return pulses == 0 ? 0 : cache[pulses] + 1;
 }
 
-DFN void init_caps(int32_t *cap, int LM, int C)
+DFN void init_caps(const Lanes &L, int32_t *cap, int LM, int C)
 {
-    ROLLED for (int i = 0; i < CELT_NB; i++) {
+    LFOR(L, i, 0, CELT_NB) {
         int N = (T_celt_eBands[i + 1] - T_celt_eBands[i]) << LM;
         cap[i] = (T_celt_cache_caps[CELT_NB * (2 * LM + C - 1) + i] + 64) * C * N >> 2;
     }
@@ -1555,19 +1589,6 @@ DNI void stereo_merge(Lanes L, int16_t *X, int16_t *Y, int16_t mid, int N)
     lsync(L);
 }
 
-// Band of a bin of the shortest frame (eBands inverted).
-struct BandOf {
-    uint8_t b[101];
-    constexpr BandOf() : b()
-    {
-        const int e[22] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16, 20, 24, 28, 34, 40, 48, 60, 78, 100};
-        for (int k = 0; k < 21; k++)
-            for (int u = e[k]; u < e[k + 1]; u++) b[u] = (uint8_t)k;
-        b[100] = 21;
-    }
-};
-TABC(BandOf, T_band_of) = BandOf();
-
 // celt/bands.c quant_all_bands, decoder path (encode = 0, resynth = 1, no theta
 // RDO), with quant_band_stereo.  A band takes one pass through quant_band or
 // two: mono, stereo of two samples and a band coded mid only: X; dual stereo: X
@@ -1636,7 +1657,8 @@ DNI void quant_all_bands_dec(Lanes L, int start, int end, int16_t *X_, int16_t *
             lowband_scratch = 0;
         }
         if (last) lowband_scratch = 0;
-        if (lowband_offset != 0 && (spread != SPREAD_AGGRESSIVE || B > 1 || tf_change < 0)) {
+        // (a band of one bin takes a sign and neither folds nor looks at the masks)
+        if (N > 1 && lowband_offset != 0 && (spread != SPREAD_AGGRESSIVE || B > 1 || tf_change < 0)) {
             effective_lowband = imax(0, M * eB[lowband_offset] - norm_offset - N);
             // the bands the folding source covers, from the lowest at or below its
             // first bin to the one its last bin is in (of the bands decoded)
@@ -2443,6 +2465,7 @@ DNI int celt_decode(Lanes L, CeltDec *st, const uint8_t *data, int len, int16_t 
     // stay in the scratch).
     enum { H_SILENCE, H_PF_GAIN, H_PF_PITCH, H_PF_TAPSET, H_TRANSIENT, H_SPREAD, H_AC_RSV, H_TRIM, H_BITS, H_N };
     int32_t hv[H_N] = {0};
+    init_caps(L, w->cap, LM, C);
     lead_rd(L, dec, [&]() CUO_INLINE {
         if (st->loss_duration == 0) st->skip_plc = 0;
         int32_t total_bits = len * 8;
@@ -2484,7 +2507,6 @@ DNI int celt_decode(Lanes L, CeltDec *st, const uint8_t *data, int len, int16_t 
         int spread_decision = SPREAD_NORMAL;
         if (tell + 4 <= total_bits) spread_decision = rd_icdf(dec, T_celt_spread_icdf, 5);
         int32_t *cap = w->cap, *offsets = w->offsets;
-        init_caps(cap, LM, C);
         int dynalloc_logp = 6;
         total_bits <<= 3;
         RangeDec d = *dec;   // in registers for the boosts

@@ -213,7 +213,7 @@ int hc_alloc(const uint8_t *buf, uint32_t len, int start, int end, const int32_t
     int32_t cap[21], pulses[21] = {}, ebits[21] = {}, fine_priority[21] = {}, balance = 0;
     int intensity = 0, dual_stereo = 0;
     cuo::RangeDec d;
-    cuo::init_caps(cap, LM, C);
+    cuo::init_caps(cuo::Lanes{0, 1, 1u}, cap, LM, C);
     cuo::rd_init(&d, buf, len);
     int coded = cuo::clt_compute_allocation(cuo::Lanes{0, 1, 1u}, start, end, offsets, cap, alloc_trim, &intensity, &dual_stereo, total,
                                             &balance, pulses, ebits, fine_priority, C, LM, &d, &w);
@@ -244,7 +244,7 @@ int hc_bands(const uint8_t *buf, uint32_t len, int start, int end, const int32_t
     memset(w.X, 0, sizeof w.X);
     memset(w.collapse_masks, 0, sizeof w.collapse_masks);
     cuo::RangeDec d;
-    cuo::init_caps(cap, LM, C);
+    cuo::init_caps(cuo::Lanes{0, 1, 1u}, cap, LM, C);
     cuo::rd_init(&d, buf, len);
     int32_t bits = (int32_t)(len * 8 << 3) - (int32_t)cuo::rd_tell_frac(&d) - 1;
     int coded = cuo::clt_compute_allocation(cuo::Lanes{0, 1, 1u}, start, end, offsets, cap, alloc_trim, &intensity, &dual_stereo, bits,
@@ -272,7 +272,7 @@ int hc_energy(const uint8_t *buf, uint32_t len, int start, int end, int intra, c
     cuo::RangeDec d;
     cuo::rd_init(&d, buf, len);
     cuo::unquant_coarse_energy(start, end, oldE, intra, &d, C, LM);
-    cuo::init_caps(cap, LM, C);
+    cuo::init_caps(cuo::Lanes{0, 1, 1u}, cap, LM, C);
     int32_t bits = (int32_t)(len * 8 << 3) - (int32_t)cuo::rd_tell_frac(&d) - 1;
     cuo::clt_compute_allocation(cuo::Lanes{0, 1, 1u}, start, end, offsets, cap, alloc_trim, &intensity, &dual_stereo, bits, &balance,
                                 pulses, ebits, fine_priority, C, LM, &d, &w);
