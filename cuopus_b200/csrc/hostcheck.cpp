@@ -188,6 +188,33 @@ void hc_silk_lpc_synth(int order, int32_t *hist, const int16_t *A_Q12, const int
     else cuo::silk_lpc_synth<10>(L, hist, A_Q12, exc, v, n);
 }
 
+// The pulse vector of a codeword; returns its sum of squares.
+int32_t hc_cwrsi(int n, int k, uint32_t idx, int32_t *y) { return cuo::cwrsi(n, k, idx, y); }
+
+// One rotation pass over x, its residue classes one after the other.
+void hc_exp_rotation_pass(int16_t *x, int len, int stride, int c, int s)
+{
+    for (int r = 0; r < stride; r++) cuo::exp_rotation_class(x, len, stride, c, s, r);
+}
+
+// 2x up-sampling of len samples, S the six states.
+void hc_silk_up2(int32_t *S, int16_t *out, const int16_t *in, int len)
+{
+    cuo::silk_up2_hq(cuo::Lanes{0, 1, 1u}, S, out, in, len);
+}
+
+// n symbols of buf with the table icdf (up to 20 entries, ending in 0): by
+// entry (rows 0) or from rows of four (rows 1); the final range goes last.
+void hc_icdf(const uint8_t *buf, uint32_t len, const uint8_t *icdf, int entries, int rows, int n, uint32_t *out)
+{
+    cuo::RangeDec d;
+    cuo::rd_init(&d, buf, len);
+    uint32_t row[6];
+    cuo::hot_row(row, 6, icdf, entries);
+    for (int i = 0; i < n; i++) out[i] = (uint32_t)(rows ? cuo::rdi_icdf_row(&d, row) : cuo::rd_icdf(&d, icdf, 8));
+    out[n] = d.rng;
+}
+
 // The decoder's comb (post-)filter in place on buf + off: the serial form
 // (lanes = 0) or the block-parallel form the decoder runs (lanes = 1, here
 // with a single lane walking the same blocks).

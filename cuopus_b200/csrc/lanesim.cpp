@@ -71,6 +71,9 @@ struct LaneSim {
     uint32_t *pkt_nsamp, *pkt_rng;
     ChainResult *res;
     int fec;
+    // or one function of the decoder that every lane runs instead
+    void (*body)(const Lanes &L, void *arg);
+    void *arg;
     // hazard detector (barrier-only schedule): the slot as the barrier released
     // (s0) and as the previous lane arrived (sp)
     int detect;
@@ -278,8 +281,9 @@ NOINSTR static void sim_lane_main(unsigned lo, unsigned hi, int id)
     L.mask = s->n == 32 ? 0xffffffffu : ((1u << s->n) - 1u);
     L.sim = s;
     s->busy = 0;
-    decode_chain(L, s->slot, s->data, s->off, s->len, s->first, s->npkts, s->channels, s->out, s->trim, s->keep,
-                 L.id == 0 ? s->pkt_nsamp : nullptr, L.id == 0 ? s->pkt_rng : nullptr, s->res, nullptr, s->fec);
+    if (s->body) s->body(L, s->arg);
+    else decode_chain(L, s->slot, s->data, s->off, s->len, s->first, s->npkts, s->channels, s->out, s->trim, s->keep,
+                      L.id == 0 ? s->pkt_nsamp : nullptr, L.id == 0 ? s->pkt_rng : nullptr, s->res, nullptr, s->fec);
     s->busy = 1;
     s->state[id] = FINISHED;
     int left = 0;
@@ -446,6 +450,62 @@ NOINSTR long long ls_decode_chains(const uint8_t *data, const uint64_t *off, con
     pthread_mutex_destroy(&j.mu);
     if (hazards) *hazards = j.hazards;
     return (long long)j.switches;
+}
+
+// Run body on `width` fiber lanes, switching as ls_decode_chains does; 0, or
+// -1 on bad arguments or no memory.
+NOINSTR static int ls_run(void (*body)(const cuo::Lanes &, void *), void *arg, int width, int max_run, uint64_t seed)
+{
+    if (width < 1 || width > cuo::SIM_MAX_LANES || (width & (width - 1)) || max_run < 0) return -1;
+    cuo::LaneSim *s = (cuo::LaneSim *)calloc(1, sizeof(cuo::LaneSim));
+    bool ok = s != nullptr;
+    for (int i = 0; ok && i < width; i++) ok = (s->stack[i] = (char *)malloc(cuo::SIM_STACK)) != nullptr;
+    if (ok) {
+        s->n = width;
+        s->max_run = max_run;
+        s->rng = seed | 1;
+        s->body = body;
+        s->arg = arg;
+        cuo::sim_decode(s);
+    }
+    if (s)
+        for (int i = 0; i < width; i++) free(s->stack[i]);
+    free(s);
+    return ok ? 0 : -1;
+}
+
+struct ls_lpc_args {
+    int order, n;
+    int32_t *hist;
+    const int16_t *A_Q12;
+    const int32_t *exc;
+    int32_t *v;
+};
+
+// The LPC synthesis the group's width selects (hostcheck.cpp has the one-lane form).
+int ls_silk_lpc_synth(int order, int32_t *hist, const int16_t *A_Q12, const int32_t *exc, int32_t *v, int n, int width,
+                      int max_run, uint64_t seed)
+{
+    ls_lpc_args a = {order, n, hist, A_Q12, exc, v};
+    return ls_run([](const cuo::Lanes &L, void *p) {
+        const ls_lpc_args *a = (const ls_lpc_args *)p;
+        cuo::silk_lpc_synth_any(L, a->order, a->hist, a->A_Q12, a->exc, a->v, a->n);
+    }, &a, width, max_run, seed);
+}
+
+struct ls_shift_args {
+    int32_t *buf;
+    int n, shift;
+};
+
+// lshift_copy of n + shift elements.
+int ls_lshift_copy(int32_t *buf, int n, int shift, int width, int max_run, uint64_t seed)
+{
+    ls_shift_args a = {buf, n, shift};
+    return ls_run([](const cuo::Lanes &L, void *p) {
+        const ls_shift_args *a = (const ls_shift_args *)p;
+        cuo::lshift_copy(L, a->buf, a->n, a->shift);
+    }, &a, width, max_run, seed);
 }
 
 }
