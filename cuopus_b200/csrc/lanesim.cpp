@@ -508,4 +508,26 @@ int ls_lshift_copy(int32_t *buf, int n, int shift, int width, int max_run, uint6
     }, &a, width, max_run, seed);
 }
 
+struct ls_deemph_args {
+    const int32_t *in;
+    int16_t *pcm;
+    int n, channels;
+    int32_t *mem;
+    int accum;
+};
+
+// Deemphasis of n samples a channel (in: one channel after the other).
+int ls_deemphasis(const int32_t *in, int16_t *pcm, int n, int channels, int32_t *mem, int accum, int width, int max_run,
+                  uint64_t seed)
+{
+    if (n > 960 || n % 8) return -1;
+    static cuo::Quad x[2][240], t[2][240];
+    for (int c = 0; c < channels; c++) memcpy(x[c], in + c * n, sizeof(int32_t) * n);
+    ls_deemph_args a = {in, pcm, n, channels, mem, accum};
+    return ls_run([](const cuo::Lanes &L, void *p) {
+        const ls_deemph_args *a = (const ls_deemph_args *)p;
+        cuo::deemphasis(L, x[0][0].v, x[1][0].v, a->pcm, a->n, a->channels, a->mem, a->accum, t[0][0].v, t[1][0].v);
+    }, &a, width, max_run, seed);
+}
+
 }

@@ -204,3 +204,26 @@ def test_rotation_by_residue_classes(hc, n, stride, top):
         _rotation(want, stride, c, s)
         hc.hc_exp_rotation_pass(_ptr(x), n, stride, c, s)
         assert x.tolist() == want
+
+
+@pytest.mark.parametrize("width,max_run", [(1, 0), (2, 0), (8, 0), (8, 2), (32, 0)])
+@pytest.mark.parametrize("n,channels", [(120, 1), (120, 2), (480, 2), (960, 1), (960, 2)])
+@pytest.mark.parametrize("accum,top", [(0, 1 << 20), (1, 1 << 27), (0, 300000000)])
+def test_deemphasis_by_recursion_and_lanes(ls, width, max_run, n, channels, accum, top):
+    rng = np.random.default_rng(n + channels + top)
+    x = rng.integers(-top, top, (channels, n)).astype(np.int32)
+    pcm = rng.integers(-32768, 32768, n * channels).astype(np.int16)
+    mem = rng.integers(-top, top, 2).astype(np.int32)
+    want, want_mem = pcm.astype(np.int64), [int(v) for v in mem]
+    for c in range(channels):
+        m = want_mem[c]
+        for j in range(n):
+            v = _wrap(int(x[c, j]) + m)
+            m = _wrap(27853 * v >> 15)      # celt/celt_decoder.c, coef0 = .85 in 15 bits
+            s = max(-32768, min(32767, v + 2048 >> 12))
+            q = j * channels + c
+            want[q] = max(-32768, min(32767, s + int(want[q]))) if accum else s
+        want_mem[c] = m
+    assert ls.ls_deemphasis(_ptr(x), _ptr(pcm), n, channels, _ptr(mem), accum, width, max_run, ctypes.c_uint64(n)) == 0
+    assert pcm.tolist() == want.tolist()
+    assert mem.tolist() == want_mem
