@@ -3,10 +3,11 @@
 // FIXED_POINT decoder.
 //
 // Execution model.  One Opus chain is decoded by a group of `width` lanes of a
-// warp (width 1..32).  All lanes of the group execute the scalar decoder code
-// redundantly on identical data (they stay converged, and every store writes
-// the same value), while loops whose iterations are independent are split
-// across the lanes with LFOR and closed with lsync().  Big per-chain arrays
+// warp (width 1..32).  Serial code either runs on every lane, redundantly on
+// identical data and storing only values that no lane reads before the next
+// barrier, or on the group's first lane alone (lead); loops whose iterations
+// are independent are split across the lanes with LFOR and closed with
+// lsync().  Nothing relies on the lanes staying in step.  Big per-chain arrays
 // live in a per-slot work area in global memory that every lane addresses
 // identically; small temporaries stay in registers.  The same source compiles
 // for the host with width 1 (g++), which the host-side parity tests use.
@@ -25,8 +26,9 @@
 // ROLLED before a loop keeps it a loop.  The decoder is one large body of code
 // whose warps each run a different part of it, so its size is paid for in
 // instruction fetch: every loop that does not ask for unrolling by name is
-// kept rolled, and the kernel is then compiled at full optimisation (385 KB of
-// kernel code; 764 KB with the compiler's own unrolling).
+// kept rolled, and the kernel is then compiled at full optimisation (490 KB of
+// code each of its two instances; when the loops were first rolled, 385 KB
+// against 764 KB with the compiler's own unrolling).
 #ifdef __CUDACC__
 #define ROLLED _Pragma("unroll 1")
 #define DFN static __device__ __forceinline__

@@ -3,12 +3,14 @@
 // The kernel is one large body of codec paths (SILK, CELT, hybrid, PLC), each
 // warp at a different place in it, so instruction fetch is paid for by size.
 // It is compiled at full optimisation with its loops rolled (ROLLED in
-// dec/common.cuh): 385 KB of kernel code.  Built at NVVM -O1 and ptxas -O1 to
-// keep it small (342 KB) the arrays that the unrolled loops index stayed in
-// local memory: the LPC recursion took 2,300 cycles a sample (160 now) and
-// 64 one-second voice clips took 29.0 ms (14.8 now); at -O3 with the
-// compiler's own unrolling (764 KB) a loaded GPU was slower than either (30
-// files, 1,085 s: 172 ms against 122 and 117 ms).
+// dec/common.cuh): 490 KB of code each instance.  Built at NVVM -O1 and ptxas
+// -O1 to keep it small (342 KB) the arrays that the unrolled loops index stayed
+// in local memory: the LPC recursion took 2,300 cycles a sample and 64
+// one-second voice clips 29.0 ms; at -O3 with rolled loops (385 KB then) they
+// took 14.8 ms, and at -O3 with the compiler's own unrolling (764 KB) a loaded
+// GPU was slower than either (30 files, 1,085 s: 172 ms against 122 and 117 ms).
+// What was added since (lane-split CELT bands, parameters and concealment) pays
+// for its size: 8.2 ms and 87 ms for the same two.
 #define CUO_DECODE_KERNEL_TU 1
 #include <cuda_runtime.h>
 #include <stdio.h>

@@ -254,7 +254,8 @@ int cuopus_order_weights(int32_t width, double *w);
 typedef struct cuopus_server cuopus_server;
 typedef struct cuopus_server_config {
     int64_t budget_bytes;   /* device arena for admitted requests (0 = 40 GiB) */
-    int32_t width;          /* lanes per chain (0 = 8 for chains of up to 4 s, else 32) */
+    int32_t width;          /* lanes per chain (0 = for chains of up to 4 s (seg_s), 32, 16 or
+                               8 by the chains in flight, wave by wave; else 32) */
     int32_t block;          /* threads per block (0 = 64) */
     int32_t max_inflight;   /* decode waves in flight (0 = 8); with two or more in flight a
                                wave waits until it is half full or its oldest chain has
@@ -329,8 +330,9 @@ int cuopus_last_stats(cuopus_stats *s);
 
 /* Extension: bytes of device state per decoder slot, and the number of lanes
  * per chain cuopus_decode_batch uses when its width is 0 (CUOPUS_STRIDE,
- * default 32).  The file entry points choose 32 or 8 lanes per call from the
- * chains' lengths unless CUOPUS_STRIDE is set (cuopus_stats.width reports it). */
+ * default 32).  The file entry points choose 32, 16 or 8 lanes per call from the
+ * chains' number and lengths unless CUOPUS_STRIDE is set (cuopus_stats.width
+ * reports it). */
 long long cuopus_slot_bytes(void);
 int cuopus_default_width(void);
 
