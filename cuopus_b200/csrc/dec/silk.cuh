@@ -1201,10 +1201,14 @@ DNI void silk_decode_core(Lanes L, SilkChan *c, SilkCtrl *ctrl, int16_t *xq, con
         }
         prev_gain_Q16 = ctrl->Gains_Q16[k];
         if (c->lossCnt && c->prevSignalType == SIG_VOICED && ix->signalType != SIG_VOICED && k < 2) {
-            ROLLED for (int i = 0; i < 5; i++) B_Q14[i] = 0;
-            B_Q14[2] = 4096;   // SILK_FIX_CONST(0.25, 14)
+            // the middle tap passes through zero, and the LTP loop below reads it
+            // with no barrier in between when the gain stays the same
+            lead(L, [&]() CUO_INLINE {
+                ROLLED for (int i = 0; i < 5; i++) B_Q14[i] = 0;
+                B_Q14[2] = 4096;   // SILK_FIX_CONST(0.25, 14)
+                ctrl->pitchL[k] = c->lagPrev;
+            });
             signalType = SIG_VOICED;
-            ctrl->pitchL[k] = c->lagPrev;
         }
         if (signalType == SIG_VOICED) {
             lag = ctrl->pitchL[k];

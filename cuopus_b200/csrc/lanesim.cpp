@@ -37,6 +37,22 @@
 
 #define NOINSTR __attribute__((no_instrument_function))
 
+// Race detector of the test build (tests/lane_race_hooks.cpp): which lane runs,
+// and where every lane has passed a __syncwarp.  The exchanges (lsum, lget,
+// lbcast, ...) hold the lanes together too but order no memory: on the device
+// they are shuffles.
+#ifdef CUO_LANE_RACE
+extern "C" void lanerace_begin(void *base, size_t size);
+extern "C" void lanerace_lane(int id);
+extern "C" void lanerace_barrier();
+extern "C" unsigned long long lanerace_end();
+#else
+static inline void lanerace_begin(void *, size_t) {}
+static inline void lanerace_lane(int) {}
+static inline void lanerace_barrier() {}
+static inline unsigned long long lanerace_end() { return 0; }
+#endif
+
 namespace cuo {
 
 enum { SIM_MAX_LANES = 32, SIM_STACK = 1 << 20 };
@@ -112,6 +128,7 @@ NOINSTR static void sim_switch(LaneSim *s)
     int from = s->cur, to = cand[sim_rand(s) % (uint64_t)k];
     s->cur = to;
     s->switches++;
+    lanerace_lane(to);
     s->busy = 0;
     swapcontext(&s->ctx[from], &s->ctx[to]);
     s->busy = 1;
@@ -175,14 +192,14 @@ NOINSTR static void sim_detect(LaneSim *s, int id, void *where)
     sim_where(s->prev_at[id], sizeof s->prev_at[id]);
 }
 
-void lanesim_sync(LaneSim *s, int id) NOINSTR;
-void lanesim_sync(LaneSim *s, int id)
+NOINSTR static void sim_meet(LaneSim *s, int id, bool memory)
 {
     s->busy = 1;
     uint64_t g = s->gen;
     if (s->detect) sim_detect(s, id, __builtin_return_address(0));
     if (++s->arrived == s->n) {   // the last lane in releases the others
         if (s->detect) memcpy(s->s0, s->slot, sizeof(ChainSlot));
+        if (memory) lanerace_barrier();
         s->arrived = 0;
         s->gen++;
         for (int i = 0; i < s->n; i++)
@@ -204,14 +221,17 @@ void lanesim_sync(LaneSim *s, int id)
     s->busy = 0;
 }
 
+void lanesim_sync(LaneSim *s, int id) NOINSTR;
+void lanesim_sync(LaneSim *s, int id) { sim_meet(s, id, true); }
+
 int32_t lanesim_sum(LaneSim *s, int id, int32_t v) NOINSTR;
 int32_t lanesim_sum(LaneSim *s, int id, int32_t v)
 {
     s->xv[id] = v;
-    lanesim_sync(s, id);
+    sim_meet(s, id, false);
     uint32_t t = 0;
     for (int i = 0; i < s->n; i++) t += (uint32_t)s->xv[i];
-    lanesim_sync(s, id);          // nobody refills xv before every lane has read it
+    sim_meet(s, id, false);          // nobody refills xv before every lane has read it
     return (int32_t)t;
 }
 
@@ -219,10 +239,10 @@ int32_t lanesim_max(LaneSim *s, int id, int32_t v) NOINSTR;
 int32_t lanesim_max(LaneSim *s, int id, int32_t v)
 {
     s->xv[id] = v;
-    lanesim_sync(s, id);
+    sim_meet(s, id, false);
     int32_t t = v;
     for (int i = 0; i < s->n; i++) t = s->xv[i] > t ? s->xv[i] : t;
-    lanesim_sync(s, id);
+    sim_meet(s, id, false);
     return t;
 }
 
@@ -230,9 +250,9 @@ int32_t lanesim_get(LaneSim *s, int id, int32_t v, int src) NOINSTR;
 int32_t lanesim_get(LaneSim *s, int id, int32_t v, int src)
 {
     s->xv[id] = v;
-    lanesim_sync(s, id);
+    sim_meet(s, id, false);
     v = s->xv[src];
-    lanesim_sync(s, id);
+    sim_meet(s, id, false);
     return v;
 }
 
@@ -240,10 +260,10 @@ uint32_t lanesim_or(LaneSim *s, int id, uint32_t v) NOINSTR;
 uint32_t lanesim_or(LaneSim *s, int id, uint32_t v)
 {
     s->xv[id] = (int32_t)v;
-    lanesim_sync(s, id);
+    sim_meet(s, id, false);
     uint32_t t = 0;
     for (int i = 0; i < s->n; i++) t |= (uint32_t)s->xv[i];
-    lanesim_sync(s, id);
+    sim_meet(s, id, false);
     return t;
 }
 
@@ -252,13 +272,13 @@ void lanesim_scan_affine(LaneSim *s, int id, uint32_t *a, uint32_t *b)
 {
     s->xa[id] = *a;
     s->xb[id] = *b;
-    lanesim_sync(s, id);
+    sim_meet(s, id, false);
     uint32_t A = 1, B = 0;        // maps of lanes 0 .. id-1, lane 0's applied first
     for (int i = 0; i < id; i++) {
         B = s->xa[i] * B + s->xb[i];
         A = s->xa[i] * A;
     }
-    lanesim_sync(s, id);
+    sim_meet(s, id, false);
     *a = A;
     *b = B;
 }
@@ -267,9 +287,9 @@ void lanesim_bcast(LaneSim *s, int id, void *p, int bytes) NOINSTR;
 void lanesim_bcast(LaneSim *s, int id, void *p, int bytes)
 {
     if (id == 0) memcpy(s->xbytes, p, (size_t)bytes);
-    lanesim_sync(s, id);
+    sim_meet(s, id, false);
     if (id != 0) memcpy(p, s->xbytes, (size_t)bytes);
-    lanesim_sync(s, id);
+    sim_meet(s, id, false);
 }
 
 NOINSTR static void sim_lane_main(unsigned lo, unsigned hi, int id)
@@ -311,6 +331,7 @@ NOINSTR static void sim_decode(LaneSim *s)
         makecontext(&s->ctx[i], (void (*)())sim_lane_main, 3, (unsigned)(p & 0xffffffffu), (unsigned)(p >> 32), i);
     }
     s->cur = (int)(sim_rand(s) % (uint64_t)s->n);
+    lanerace_lane(s->cur);
     s->budget = sim_run_length(s);
     if (s->detect) {
         memcpy(s->s0, s->slot, sizeof(ChainSlot));
@@ -371,6 +392,7 @@ NOINSTR static void *ls_worker(void *arg)
         s->off = j->off;
         s->len = j->len;
         s->fec = j->fec;
+        lanerace_begin(slot, sizeof(cuo::ChainSlot));
         s->detect = j->max_run == 0 && j->detect;
         if (s->detect) {
             s->s0 = (unsigned char *)malloc(sizeof(cuo::ChainSlot));
@@ -396,8 +418,10 @@ NOINSTR static void *ls_worker(void *arg)
             unsigned long long before = s->hazards;
             s->hazards = 0;
             cuo::sim_decode(s);
+            lanerace_barrier();       // the launch's next chain starts behind one
             s->hazards += before;
         }
+        s->hazards += lanerace_end();
         pthread_mutex_lock(&j->mu);
         j->switches += s->switches;
         j->hazards += s->hazards;
