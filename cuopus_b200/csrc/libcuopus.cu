@@ -754,11 +754,15 @@ int resample(const int16_t *in, int64_t avail, int64_t n_out, float *out, cudaSt
     if (n_out <= 0) return RC_OK;
     int rc = ensure_taps(st, err);
     if (rc) return rc;
-    if ((rc = ensure_occupancy(err))) return rc;
-    const int run = cuo::rs_run(n_out, G.sm_count);
+    // the SM count by itself: this runs on a server's thread too, without the
+    // lock that the file calls' occupancy table is kept under
+    int dev = 0, sms = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int run = cuo::rs_run(n_out, sms);
     long long tiles = (n_out + cuo::rs_tile(run) - 1) / cuo::rs_tile(run);
     if (tiles > 0x7fffffffLL) return err.set(RC_ARG, "resample length too large");
-    const long long blocks = std::min<long long>(tiles, (long long)G.sm_count * cuo::RS_BLOCKS);
+    const long long blocks = std::min<long long>(tiles, (long long)sms * cuo::RS_BLOCKS);
     if (run == 9)
         cuo::k_resample48to16<9><<<(unsigned)blocks, cuo::RS_THREADS, 0, st>>>(in, avail, n_out, out, chans);
     else
@@ -875,6 +879,7 @@ extern "C" void cuopus_release_workspaces(void)
     G.hpin.p = nullptr;
     G.hpin.cap = 0;
     G.dev_bytes = 0;
+    std::lock_guard<std::mutex> taps(g_taps_mu);
     G.taps_dev = -1;
 }
 
