@@ -80,9 +80,9 @@ int main()
     });
     std::thread calls([&] {
         t_dev = 1;
+        cuopus_release_workspaces();
         for (int i = 0; i < 100; i++)
             if (cuopus_warmup(nullptr, 0) || cuopus_resample48to16(&in, 3 * n, n, &out, nullptr, nullptr, 0)) failed++;
-        cuopus_release_workspaces();
     });
     server.join();
     calls.join();
