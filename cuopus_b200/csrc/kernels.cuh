@@ -186,9 +186,12 @@ __global__ void __launch_bounds__(128, MIN_BLOCKS) k_decode_chains(DecodeArgs a)
 //   * RUN outputs of a half per thread: each staged pair is read once (73
 //     8-byte reads for 18 outputs at RUN = 9) and the threads' stride of
 //     3 RUN pairs is odd, so the reads do not conflict in the banks.  RUN = 9
-//     once two blocks per SM have work (rs_run), 3 below: a short input is
-//     over in one block's latency, which the run sets (1,000 to 1,000,000
-//     samples: 14-15 us a call with RUN = 3, 16-17 with 9).
+//     once four of the five blocks that an SM holds have a tile (rs_run), 3
+//     below: a short input is over in one block's latency, which the run sets,
+//     and few blocks of nine leave SMs idle.  Microseconds a call with RUN = 3
+//     and 9: 0.1 to 2 M samples 13.9-15.5 and 15.7-17.4, 2.1 M 15.0 and 16.6,
+//     3 M 15.5 and 15.8, 4 M 16.6 and 17.5, 4.5 M 17.5 and 16.8, 6 M 18.8 and
+//     18.4, 10 M 24.0 and 23.4, 20 M 34.7 and 32.1.
 //   * Interior tiles read the input as aligned words, neighbouring lanes
 //     neighbouring words, whose pairs go to shared memory without conflicts (a
 //     16-byte vector per lane stored them 16 to a bank), and a block loads the
@@ -200,7 +203,7 @@ __global__ void __launch_bounds__(128, MIN_BLOCKS) k_decode_chains(DecodeArgs a)
 // stores free of conflicts, 158 us with the next tile's loads in flight.
 enum { RS_TAPS = 49, RS_PAD = 24, RS_THREADS = 128, RS_BLOCKS = 5 };
 constexpr int rs_tile(int run) { return 2 * RS_THREADS * run; }   // outputs per block
-inline int rs_run(long long n_out, int sms) { return n_out >= 2ll * sms * rs_tile(9) ? 9 : 3; }
+inline int rs_run(long long n_out, int sms) { return n_out >= 4ll * sms * rs_tile(9) ? 9 : 3; }
 
 __constant__ uint64_t c_rs_taps[RS_TAPS];   // each tap twice, a pair of floats
 

@@ -1,7 +1,7 @@
 // The library's host code (libcuopus.cu) on a CUDA runtime made here, with two
 // devices and no GPU: threads that reach it without a common lock, under
 // ThreadSanitizer (tests/test_host_threads.py).  Exit status 0 when the launches
-// are the ones each device asks for; a data race makes it 66.
+// are the ones that each device and size ask for; a data race makes it 66.
 #include <atomic>
 #include <stdint.h>
 #include <stdio.h>
@@ -92,5 +92,13 @@ int main()
     }
     // one set of occupancies: the decoder ran on device 1 only
     if (g_occupancy_calls != 24) printf("%d occupancy queries, not 24\n", g_occupancy_calls.load()), failed++;
+    // the form of the resampler: tiles of 768 outputs until four blocks an SM have one of 2304
+    t_dev = 0;
+    for (const long long tiles : {3ll * 148, 4ll * 148 - 1, 4ll * 148}) {
+        const long long outs = 2304 * tiles;
+        if (cuopus_resample48to16(&in, 3 * outs, outs, &out, nullptr, nullptr, 0)) failed++;
+        const unsigned want = tiles < 4 * 148 ? 5 * 148 : (unsigned)tiles;
+        if (g_grid[0] != want) printf("%lld outputs: grid %u, not %u\n", outs, g_grid[0].load(), want), failed++;
+    }
     return failed ? 1 : 0;
 }
