@@ -61,7 +61,7 @@ def _run(cmd):
 
 def build_libcuopus(force=False):
     deps = _sources("libcuopus.cu", "decode_kernel.cu", "costmodel.cu", "server.cu", "kernels.cuh", "ogg_demux.cpp",
-                    "ogg_demux.h", "ordercost.cpp", "ordercost.h", "ordercost_coef.inc", "dec") + \
+                    "ogg_demux.h", "ordercost.cpp", "ordercost.h", "ordercost_coef.inc", "launch_shape.h", "dec") + \
         [os.path.join(ROOT, "include", "cuopus.h")]
     if not force and not _stale(LIBCUOPUS, deps):
         return LIBCUOPUS
@@ -92,7 +92,7 @@ def build_libcuopus(force=False):
 def build_hostcheck(force=False):
     """The host build, and a second one whose lane-split loops run backwards
     (a test that their iterations are independent)."""
-    deps = _sources("hostcheck.cpp", "dec")
+    deps = _sources("hostcheck.cpp", "launch_shape.h", "dec")
     for target, extra in ((HOSTCHECK, []), (HOSTCHECK_REV, ["-DCUO_LFOR_REVERSE"])):
         if not force and not _stale(target, deps):
             continue

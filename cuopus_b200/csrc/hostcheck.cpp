@@ -10,6 +10,7 @@
 
 #define CUO_FRAME_EVENTS 1
 #include "dec/chain.cuh"
+#include "launch_shape.h"
 
 // Frame events of the host build (CUO_FRAME_EVENTS): counters the tests read
 // with hc_frame_events to show which branches of the frame decode their
@@ -118,6 +119,9 @@ int hc_decode_chains(const uint8_t *data, const uint64_t *off, const uint32_t *l
     return hc_decode_chains_fec(data, off, len, first, npkts, channels, nchains, pcm, pcm_off, trim, keep, rec_off,
                                 pkt_nsamp, pkt_rng, res, nthreads, 0);
 }
+
+// Lanes per chain of a server wave (launch_shape.h).
+int hc_server_wave_width(size_t load, int sms, int narrow) { return cuo_host::server_wave_width(load, sms, narrow); }
 
 unsigned long hc_slot_bytes(void) { return sizeof(cuo::ChainSlot); }
 

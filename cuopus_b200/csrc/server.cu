@@ -42,6 +42,7 @@
 #include "../../include/cuopus.h"
 #define CUO_NO_RESAMPLE_KERNEL 1
 #include "kernels.cuh"
+#include "launch_shape.h"
 #include "ogg_demux.h"
 
 namespace {
@@ -442,20 +443,14 @@ void cuopus_server::run()
     }
 }
 
-// Lanes per chain of a wave of nch chains (server thread).  Wide groups decode a
-// chain faster (a second of mixed audio 18 ms at 32 lanes, 33 at 16, 60 at 8),
-// narrow ones keep more chains on the GPU: with the chains of the waves in
-// flight counted in, 32 lanes up to ten chains per SM, 16 up to 24, then 8 (the
-// file entry points' measurements: 1085 chains 92 ms at 32 lanes and 116 at 16,
-// 2070 165 and 140, 5400 160, 113 and 81 at 8).  24 files together, 531 s: 230 ms
-// with 8 lanes throughout, 79 so.
+// Lanes per chain of a wave of nch chains (server thread).
 int cuopus_server::wave_width(size_t nch) const
 {
     if (!auto_width) return width;
     size_t load = nch;
     for (const Wave &w : waves)
         if (w.busy) load += w.chains.size();
-    return load <= 10 * (size_t)sms ? 32 : load <= 24 * (size_t)sms ? 16 : width;
+    return cuo_host::server_wave_width(load, sms, width);
 }
 
 // Check a finished wave's chains; complete the requests whose chains are all
