@@ -120,6 +120,21 @@ int hc_decode_chains(const uint8_t *data, const uint64_t *off, const uint32_t *l
                                 pkt_nsamp, pkt_rng, res, nthreads, 0);
 }
 
+// The launch shape (launch_shape.h) for n chains of the given costs, the longest
+// first: 100 * lanes + warps per SM, 0 when no shape has want_width lanes.  The
+// groups are those of `sms` SMs with `resident` warps each at 32 and 16 lanes
+// and `resident8` at 8.
+int hc_choose_shape(const double *cost, int n, int want_width, int sms, int resident, int resident8)
+{
+    const auto groups = [&](const cuo_host::LaunchShape &s) {
+        const int most = s.width == 8 ? resident8 : resident;
+        const int warps = s.warps_per_sm > 0 && s.warps_per_sm < most ? s.warps_per_sm : most;
+        return (long long)warps * sms * (32 / s.width);
+    };
+    const cuo_host::LaunchShape *s = cuo_host::choose_shape(std::vector<double>(cost, cost + n), want_width, groups);
+    return s ? 100 * s->width + s->warps_per_sm : 0;
+}
+
 // Lanes per chain of a server wave (launch_shape.h).
 int hc_server_wave_width(size_t load, int sms, int narrow) { return cuo_host::server_wave_width(load, sms, narrow); }
 

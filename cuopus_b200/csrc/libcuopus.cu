@@ -33,6 +33,7 @@
 
 #include "../../include/cuopus.h"
 #include "kernels.cuh"
+#include "launch_shape.h"
 #include "ogg_demux.h"
 #include "ordercost.h"
 
@@ -555,57 +556,29 @@ int plan_files(const uint8_t *const *oggs, const size_t *ns, int nfiles, bool re
 // threads against 200 ms at 128; whole streams at 32 lanes: equal).
 const int FILE_BLOCK = 64;
 
-// Launch shape of a file batch: lanes per chain and decoder groups
-// (CUOPUS_STRIDE and CUOPUS_WARPS_PER_SM, when set, decide).  More lanes decode a
-// chain faster, fewer lanes put more chains on the GPU, and more warps on an SM
-// slow each other down, because each of them fetches its own part of a program
-// larger than the SM's instruction caches.  A shape's time is estimated as
-// max(longest chain, total work / groups, what a group with a second chain has
-// to do) / speed; the last term is taken at 0.7, since chains speed up as groups
-// run dry.  Chain cost: its TOC samples x channels.  Speeds are per group,
-// relative to 32 lanes at 4 warps per SM, from files of 300 to 5400 one-second
-// chains (ms at 32 lanes / 16 / 8):
-//   speech, 300 chains 19 / 26 / 42, 1800 58 / 42 / 50, 5400 160 / 113 / 81;
-//   mono and stereo mixed, 1085 chains 92 / 116 / 188 (105 at 5 warps per SM,
-//   138 at 8), 2070 165 / 140 / 230, 3100 248 / 207 / 272;
-//   voice, 600 chains 18 at 4 warps per SM (two rounds), 11.5 at 5;
-//   at 8 lanes, speech of 7200 chains 106 at 8 warps per SM and 112 at 12, voice
-//   of 5400 53 and 36 (two rounds at 8).
-struct LaunchShape {
-    int width, warps_per_sm;   // 0 warps: every resident group
-    double speed;
-};
-const LaunchShape SHAPES[] = {{32, 4, 1.0}, {32, 5, 0.8}, {16, 4, 0.62}, {16, 6, 0.55}, {8, 8, 0.37}, {8, 0, 0.33}};
-
-long long shape_groups(const LaunchShape &s)
+// Decoder groups of a launch shape (launch_shape.h) on this GPU.
+long long shape_groups(const cuo_host::LaunchShape &s)
 {
     const long long resident = resident_groups(FILE_BLOCK, s.width);
     const long long asked = (long long)s.warps_per_sm * G.sm_count * (32 / s.width);
-    return s.warps_per_sm > 0 ? std::min(resident, asked) : resident;
+    return std::max(s.warps_per_sm > 0 ? std::min(resident, asked) : resident, 1LL);
 }
 
-// Sets width and max_groups (0: every resident group).
+// Launch shape of a file batch: sets width and max_groups (0: every resident
+// group).  CUOPUS_STRIDE and CUOPUS_WARPS_PER_SM, when set, decide.  Chain cost:
+// its TOC samples x channels.
 void choose_launch(const Plan &P, int32_t &width, int32_t &max_groups)
 {
     const char *e = getenv("CUOPUS_STRIDE"), *ew = getenv("CUOPUS_WARPS_PER_SM");
     const int want_width = e && atoi(e) > 0 ? default_width() : 0;
     std::vector<double> cost(P.first.size());
-    double sum = 0.0;
-    for (size_t c = 0; c < cost.size(); c++) sum += cost[c] = (double)P.cap[c] * (double)P.chans[c];
+    for (size_t c = 0; c < cost.size(); c++) cost[c] = (double)P.cap[c] * (double)P.chans[c];
     std::sort(cost.begin(), cost.end(), std::greater<double>());
-    double best = -1.0;
     width = want_width > 0 ? want_width : 32;
     max_groups = default_max_groups(width);
-    for (const LaunchShape &s : SHAPES) {
-        if (want_width && s.width != want_width) continue;
-        const long long g = std::max(shape_groups(s), 1LL);
-        double t = cost.empty() ? 0.0 : std::max(cost[0], sum / (double)g);
-        if ((long long)cost.size() > g) t = std::max(t, 0.7 * (cost[g - 1] + cost[g]));
-        t /= s.speed;
-        if (best >= 0.0 && t >= best) continue;
-        best = t;
-        width = s.width;
-        max_groups = s.warps_per_sm > 0 ? (int32_t)g : 0;
+    if (const cuo_host::LaunchShape *s = cuo_host::choose_shape(cost, want_width, shape_groups)) {
+        width = s->width;
+        max_groups = s->warps_per_sm > 0 ? (int32_t)shape_groups(*s) : 0;
     }
     if (ew && atoi(ew) > 0) max_groups = default_max_groups(width);
 }
