@@ -386,61 +386,10 @@ DNI void denormalise_bands(Lanes L, const int16_t *X, int32_t *freq, const int16
     lsync(L);
 }
 
-// celt/celt.c comb_filter (in place when y == x): the IIR recursion over lag T
-// is kept serial.
 // gains[3][3] of celt/celt.c (comb filter taps per tapset)
 TABC(int16_t, T_comb_gains[3][3]) = {{10048, 7112, 4248}, {15200, 8784, 0}, {26208, 3280, 0}};
 
-DNI void comb_filter(int32_t *y, int32_t *x, int T0, int T1, int N, int16_t g0, int16_t g1, int tapset0,
-                     int tapset1, const int16_t *window, int overlap)
-{
-    const int16_t (*gains)[3] = T_comb_gains;
-    if (g0 == 0 && g1 == 0) {
-        if (x != y) ROLLED for (int i = 0; i < N; i++) y[i] = x[i];
-        return;
-    }
-    T0 = imax(T0, 15);
-    T1 = imax(T1, 15);
-    int16_t g00 = (int16_t)c_mul16_p15(g0, gains[tapset0][0]);
-    int16_t g01 = (int16_t)c_mul16_p15(g0, gains[tapset0][1]);
-    int16_t g02 = (int16_t)c_mul16_p15(g0, gains[tapset0][2]);
-    int16_t g10 = (int16_t)c_mul16_p15(g1, gains[tapset1][0]);
-    int16_t g11 = (int16_t)c_mul16_p15(g1, gains[tapset1][1]);
-    int16_t g12 = (int16_t)c_mul16_p15(g1, gains[tapset1][2]);
-    int32_t x0, x1 = x[-T1 + 1], x2 = x[-T1], x3 = x[-T1 - 1], x4 = x[-T1 - 2];
-    if (g0 == g1 && T0 == T1 && tapset0 == tapset1) overlap = 0;
-    int i;
-    ROLLED for (i = 0; i < overlap; i++) {
-        x0 = x[i - T1 + 2];
-        int16_t f = (int16_t)c_mul16_q15(window[i], window[i]);
-        int32_t v = x[i];
-        v = wadd(v, c_mul16_32_q15((int16_t)c_mul16_q15(32767 - f, g00), x[i - T0]));
-        v = wadd(v, c_mul16_32_q15((int16_t)c_mul16_q15(32767 - f, g01), wadd(x[i - T0 + 1], x[i - T0 - 1])));
-        v = wadd(v, c_mul16_32_q15((int16_t)c_mul16_q15(32767 - f, g02), wadd(x[i - T0 + 2], x[i - T0 - 2])));
-        v = wadd(v, c_mul16_32_q15((int16_t)c_mul16_q15(f, g10), x2));
-        v = wadd(v, c_mul16_32_q15((int16_t)c_mul16_q15(f, g11), wadd(x1, x3)));
-        v = wadd(v, c_mul16_32_q15((int16_t)c_mul16_q15(f, g12), wadd(x0, x4)));
-        y[i] = c_sat(v, CELT_SIG_SAT);
-        x4 = x3; x3 = x2; x2 = x1; x1 = x0;
-    }
-    if (g1 == 0) {
-        if (x != y) ROLLED for (int k = overlap; k < N; k++) y[k] = x[k];
-        return;
-    }
-    // comb_filter_const_c
-    int32_t *yy = y + i, *xx = x + i;
-    int Nc = N - i;
-    x4 = xx[-T1 - 2]; x3 = xx[-T1 - 1]; x2 = xx[-T1]; x1 = xx[-T1 + 1];
-    ROLLED for (int k = 0; k < Nc; k++) {
-        x0 = xx[k - T1 + 2];
-        int32_t v = wadd(wadd(wadd(xx[k], c_mul16_32_q15(g10, x2)), c_mul16_32_q15(g11, wadd(x1, x3))),
-                         c_mul16_32_q15(g12, wadd(x0, x4)));
-        yy[k] = c_sat(v, CELT_SIG_SAT);
-        x4 = x3; x3 = x2; x2 = x1; x1 = x0;
-    }
-}
-
-// comb_filter split across the lanes.  In place (y == x) output i reads the
+// celt/celt.c comb_filter split across the lanes.  In place (y == x) output i reads the
 // input at i and outputs at i - T - 2 .. i - T + 2 (T >= 15), so a block of
 // min(T0, T1) - 2 consecutive outputs depends only on earlier blocks: the
 // blocks run in order with a barrier between them and the outputs of a block
