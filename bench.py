@@ -764,6 +764,11 @@ def main():
     if args.impl == "reference":
         if rank != 0:
             return 0
+        from oracle.corpus import REF_LIB
+        if not os.path.exists(REF_LIB):
+            print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/libopus_ref.so is not built: no reference "
+                              "tree to compile libopus from (make -C oracle REF=<reference tree>)"}), flush=True)
+            return 0
         files, seg = load_inputs(args.workload, args.count)
         rates, els = [], []
         for i in range(args.warmup + args.steps):
