@@ -11,6 +11,12 @@
 // GPU was slower than either (30 files, 1,085 s: 172 ms against 122 and 117 ms).
 // What was added since (lane-split CELT bands, parameters and concealment) pays
 // for its size: 8.2 ms and 87 ms for the same two.
+//
+// An early build decoded wrong stereo samples at ptxas -O2 and -O3: serial code
+// that every lane ran updated group memory in place, which is in order only while
+// the lanes of a group stay in step.  Such code now runs on the first lane (lead,
+// dec/common.cuh); tests/test_lanes.py and tests/test_lane_races.py check it on
+// the host, tests/test_against_golden_gpu.py the samples of this build.
 #define CUO_DECODE_KERNEL_TU 1
 #include <cuda_runtime.h>
 #include <stdio.h>
@@ -34,7 +40,9 @@ namespace cuo {
 // long chains that set an uneven batch's step, with few warps per SM: they
 // run the instance with the full register budget (255), which decodes each
 // chain faster (the mixed batch at 5 warps per SM: 2,401-2,496 ms against
-// 2,798-2,803 with the register cap).
+// 2,798-2,803 with the register cap).  Those figures are from the build of -O1;
+// on this one the 2 h file's chains take 90.3 ms at 8 warps per SM, and 88.0 when
+// 8-lane groups run the full-register instance, which does not pay for a rule.
 static bool dense_instance(int width) { return width <= 8; }
 
 cudaError_t decode_kernel_occupancy(int block, int width, int *blocks_per_sm)

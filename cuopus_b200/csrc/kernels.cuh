@@ -200,7 +200,8 @@ __global__ void __launch_bounds__(128, MIN_BLOCKS) k_decode_chains(DecodeArgs a)
 //     shared memory.
 // 172,800,001 samples: 395 us as four outputs per thread with scalar FMAs on
 // shared reads that conflicted 4 ways; 266 us packed, 200 us with the staging
-// stores free of conflicts, 158 us with the next tile's loads in flight.
+// stores free of conflicts, 158 us with the next tile's loads in flight (158-169
+// a call, by box).
 enum { RS_TAPS = 49, RS_PAD = 24, RS_THREADS = 128, RS_BLOCKS = 5 };
 constexpr int rs_tile(int run) { return 2 * RS_THREADS * run; }   // outputs per block
 inline int rs_run(long long n_out, int sms) { return n_out >= 4ll * sms * rs_tile(9) ? 9 : 3; }

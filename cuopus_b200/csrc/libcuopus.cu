@@ -566,7 +566,8 @@ long long shape_groups(const cuo_host::LaunchShape &s)
 
 // Launch shape of a file batch: sets width and max_groups (0: every resident
 // group).  CUOPUS_STRIDE and CUOPUS_WARPS_PER_SM, when set, decide.  Chain cost:
-// its TOC samples x channels.
+// its TOC samples x channels, which takes a stereo CELT second for two SILK ones
+// (it takes as long as five).
 void choose_launch(const Plan &P, int32_t &width, int32_t &max_groups)
 {
     const char *e = getenv("CUOPUS_STRIDE"), *ew = getenv("CUOPUS_WARPS_PER_SM");

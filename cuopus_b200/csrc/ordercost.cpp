@@ -3,13 +3,13 @@
 // The file entry points pull chains from a device queue in a host-given
 // order, longest first (list scheduling).  When the chains of a call are few
 // per decoder group (the 2 h file in 1 s chains: 7,200 chains on 4,736 groups
-// of 8 lanes), the makespan depends on which chains go first, and a chain's
+// of 8 lanes when this was fitted), the makespan depends on which chains go first, and a chain's
 // sample count does not tell them apart: a second of hybrid costs more than a
 // second of SILK.  The cost of a chain is modelled as the sum of its packets'
 // costs (plus a constant), each packet a non-negative combination of the
 // features below, so chain costs are prefix-sum differences.  The weights are
 // fitted by non-negative least squares to per-chain device times measured on
-// a training corpus (cuopus_b200/fit_order_cost.py writes ordercost_coef.inc);
+// a training corpus (cuopus_b200/ordercost.py writes ordercost_coef.inc);
 // they change no decoded sample, only the order in which chains start.
 //
 // Features of one packet (TOC of RFC 6716 section 3.1):

@@ -22,7 +22,9 @@ struct OrderCost {
         return packet + per_byte * len + nf * frame[toc >> 3][(toc >> 2) & 1][out_channels == 2];
     }
 };
-// Weights for chains decoded by groups of `width` lanes (8 and below, or 32).
+// Weights for chains decoded by groups of `width` lanes: one set for 32 lanes, one
+// for fewer (fitted at 8).  Both were fitted when a stereo CELT second took twice
+// as long as a SILK second; it takes more than five times as long now.
 const double *order_coefficients(int width);
 // False while the weights are the unfitted default (cost = decoded duration).
 bool order_model_fitted();

@@ -223,7 +223,7 @@ int cuopus_mlp_train(float *params_dev, const float *x_dev, const float *t_dev, 
  * sum over a chain's packets of non-negative weights times the packet's
  * features, plus a constant per chain.  The weights are fitted by
  * non-negative least squares to per-chain device times of a training corpus,
- * one set for 8 lanes per chain and one for 32.  Host pointers; the tables are
+ * one set for up to 16 lanes per chain and one for 32.  Host pointers; the tables are
  * those of cuopus_batch.  feat receives nchains x CUOPUS_ORDER_FEATURES values:
  * 1 (chain constant), packets, bytes / 100, frames per (mode, duration) class
  * and TOC stereo bit (SILK 10/20/40/60 ms, hybrid 10/20, CELT 2.5/5/10/20;
