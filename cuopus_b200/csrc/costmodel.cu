@@ -53,75 +53,93 @@ __device__ __forceinline__ int toc_bw(int config)   // 0 NB, 1 MB, 2 WB, 3 SWB, 
     return b == 0 ? 0 : b + 1;
 }
 
-__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v)
+// Features of 32 chains a block, G lanes for each; feat[c * 16 + k].  A packet
+// costs two dependent loads (offset and length, then its TOC bytes), so a chain's
+// packets go to its lanes, 2 G in flight; one thread per chain walked them one
+// after the other (4096 chains of 0.5-2 s, features and predictions: 617 us, 66
+// now).  The sums are whole numbers, so their order does not matter.  Then each
+// warp works out one feature of all 32 chains at a time: with a chain's sixteen
+// in a warp of its own, five lanes of which took logarithms, 40,000 chains of one
+// packet took 64 us a call, one thread per chain 28, this 28.
+template <int G>
+__global__ void __launch_bounds__(32 * G)
+k_chain_features(const uint8_t *__restrict__ data, const uint64_t *__restrict__ off, const uint32_t *__restrict__ len,
+                 const uint32_t *__restrict__ first, const uint32_t *__restrict__ npkts,
+                 const uint8_t *__restrict__ channels, int nchains, float *__restrict__ feat)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// One warp per chain; feat[c * 16 + k].  A packet costs three dependent loads
-// (offset and length, then its TOC bytes), so the chain's packets go to the
-// lanes, 32 in flight; one thread per chain walked them one after the other
-// (4096 chains of 0.5-2 s, features and predictions: 617 us, 73 now).  The
-// sums are whole numbers, so their order does not matter.
-__global__ void k_chain_features(const uint8_t *__restrict__ data, const uint64_t *__restrict__ off,
-                                 const uint32_t *__restrict__ len, const uint32_t *__restrict__ first,
-                                 const uint32_t *__restrict__ npkts, const uint8_t *__restrict__ channels,
-                                 int nchains, float *__restrict__ feat)
-{
-    const int lane = threadIdx.x & 31;
-    const int c = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (c >= nchains) return;
     enum { BYTES, FRAMES, Q, SILK, HYBRID, CELT, F25, F5, F10, F20, F40, BW, STEREO, SUMS };
+    __shared__ unsigned long long sums[SUMS][32];
+    const int lane = threadIdx.x % G, own = threadIdx.x / G;
+    const long long c0 = (long long)blockIdx.x * 32, c = c0 + own;
     unsigned long long sum[SUMS] = {};
-    const uint32_t n = npkts[c];
-    for (uint64_t k = lane; k < n; k += 32) {
-        const uint64_t p = (uint64_t)first[c] + k;
-        const uint32_t L = len[p];
-        sum[BYTES] += L;
-        if (!L) continue;
-        const uint8_t *b = data + off[p];
-        const int toc = b[0], cfg = toc >> 3, code = toc & 3;
-        const int nf = code == 0 ? 1 : code < 3 ? 2 : (L > 1 ? (b[1] & 63) : 0);
-        const int qms = toc_qms(cfg), mode = toc_mode(cfg);
-        sum[FRAMES] += nf;
-        sum[Q] += (unsigned)(nf * qms);
-        sum[SILK] += mode == 0 ? nf : 0;
-        sum[HYBRID] += mode == 1 ? nf : 0;
-        sum[CELT] += mode == 2 ? nf : 0;
-        sum[F25] += qms == 10 ? nf : 0;
-        sum[F5] += qms == 20 ? nf : 0;
-        sum[F10] += qms == 40 ? nf : 0;
-        sum[F20] += qms == 80 ? nf : 0;
-        sum[F40] += qms > 80 ? nf : 0;
-        sum[BW] += (unsigned)(nf * toc_bw(cfg));
-        sum[STEREO] += (toc >> 2) & 1;
-    }
+    const uint32_t n = c < nchains ? npkts[c] : 0;
+    const uint64_t p0 = n ? first[c] : 0;
+    // two packets a step, their loads side by side
+    for (uint64_t k = lane; k < n; k += 2 * G) {
+        uint32_t L[2], toc[2], count[2];
+        uint64_t at[2];
 #pragma unroll
-    for (int i = 0; i < SUMS; i++) sum[i] = warp_sum(sum[i]);
-    // feature `lane` on its lane: a logarithm, the channels, or a fraction
-    const double frames = (double)sum[FRAMES], bytes = (double)sum[BYTES], secs = (double)sum[Q] / 4000.0;
-    const double fr = frames > 0 ? 1.0 / frames : 0.0;
-    if (lane >= F) return;
-    float v;
-    if (lane < 4 || lane == 15) {
-        const double x = lane == 0 ? (double)n : lane == 1 ? bytes : lane == 2 ? frames : lane == 3 ? secs
-                       : secs > 0 ? bytes / secs : 0.0;
-        v = (float)log1p(x);
-    } else if (lane == 4) {
-        v = (float)(channels[c] - 1);
-    } else if (lane < 13) {
-        unsigned long long k = 0;
+        for (int u = 0; u < 2; u++) {
+            const bool in = k + u * G < n;
+            L[u] = in ? len[p0 + k + u * G] : 0;
+            at[u] = in ? off[p0 + k + u * G] : 0;
+        }
 #pragma unroll
-        for (int i = SILK; i <= F40; i++) k = lane - 5 == i - SILK ? sum[i] : k;
-        v = (float)((double)k * fr);
-    } else if (lane == 13) {
-        v = (float)((double)sum[BW] * fr * 0.25);
-    } else {
-        v = (float)(n ? (double)sum[STEREO] / n : 0.0);
+        for (int u = 0; u < 2; u++) {
+            toc[u] = L[u] > 0 ? data[at[u]] : 0;
+            count[u] = L[u] > 1 ? data[at[u] + 1] & 63 : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            if (!L[u]) continue;
+            const int cfg = toc[u] >> 3, code = toc[u] & 3;
+            const int nf = code == 0 ? 1 : code < 3 ? 2 : count[u];
+            const int qms = toc_qms(cfg), mode = toc_mode(cfg);
+            sum[BYTES] += L[u];
+            sum[FRAMES] += nf;
+            sum[Q] += (unsigned)(nf * qms);
+            sum[SILK] += mode == 0 ? nf : 0;
+            sum[HYBRID] += mode == 1 ? nf : 0;
+            sum[CELT] += mode == 2 ? nf : 0;
+            sum[F25] += qms == 10 ? nf : 0;
+            sum[F5] += qms == 20 ? nf : 0;
+            sum[F10] += qms == 40 ? nf : 0;
+            sum[F20] += qms == 80 ? nf : 0;
+            sum[F40] += qms > 80 ? nf : 0;
+            sum[BW] += (unsigned)(nf * toc_bw(cfg));
+            sum[STEREO] += (toc[u] >> 2) & 1;
+        }
     }
-    feat[(size_t)c * F + lane] = v;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < SUMS; i++) {
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], o);
+        if (lane == 0) sums[i][own] = sum[i];
+    }
+    __syncthreads();
+    // feature k (the same on all lanes of the warp) of chain c0 + j: a logarithm, the
+    // channels, or a fraction
+    for (int i = threadIdx.x; i < 32 * F; i += 32 * G) {
+        const int k = i >> 5, j = i & 31;
+        if (c0 + j >= nchains) continue;
+        float v;
+        if (k < 4 || k == 15) {
+            const double bytes = (double)sums[BYTES][j], secs = (double)sums[Q][j] / 4000.0;
+            const double x = k == 0 ? (double)npkts[c0 + j] : k == 1 ? bytes : k == 2 ? (double)sums[FRAMES][j]
+                           : k == 3 ? secs : secs > 0 ? bytes / secs : 0.0;
+            v = (float)log1p(x);
+        } else if (k == 4) {
+            v = (float)(channels[c0 + j] - 1);
+        } else if (k < 14) {
+            const double frames = (double)sums[FRAMES][j], fr = frames > 0 ? 1.0 / frames : 0.0;
+            v = k < 13 ? (float)((double)sums[SILK + k - 5][j] * fr) : (float)((double)sums[BW][j] * fr * 0.25);
+        } else {
+            const uint32_t pk = npkts[c0 + j];
+            v = (float)(pk ? (double)sums[STEREO][j] / pk : 0.0);
+        }
+        feat[(size_t)(c0 + j) * F + k] = v;
+    }
 }
 
 // ------------------------------------------------------------------ network
@@ -341,9 +359,26 @@ extern "C" int cuopus_chain_features(const cuopus_batch *b, float *feat_dev, voi
         return set_err(errbuf, errcap, 3, "chain_features: NULL argument", cudaSuccess);
     if (b->nchains <= 0) return 0;
     cudaStream_t st = (cudaStream_t)cuda_stream;
-    const long long blocks = ((long long)b->nchains * 32 + THREADS - 1) / THREADS;
-    k_chain_features<<<(unsigned)blocks, THREADS, 0, st>>>(b->data, b->off, b->len, b->first, b->npkts, b->channels,
-                                                           b->nchains, feat_dev);
+    int dev = 0, sms = 0;
+    CKM(cudaGetDevice(&dev), "cudaGetDevice");
+    CKM(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
+    const unsigned blocks = (unsigned)(((long long)b->nchains + 31) / 32);
+    // Lanes per chain: as many as keep all chains on the GPU at once.  Microseconds
+    // a call at 32 / 16 / 8 / 4 / 2 lanes:
+    //    4,096 chains of 60 packets 32 / 32 / 34 / 38 / 47, of 400 60 / 74 / 110 / 149 / 268;
+    //    9,472 of 1                 37 / 31 / 29 / 30 / 31, of 60 38 / 34 / 35 / 38 / 47;
+    //   16,384 of 1                 42 / 31 / 27 / 26 / 27, of 60 51 / 42 / 38 / 45 / 61;
+    //   40,000 of 1                 67 / 41 / 32 / 29 / 29, of 60 91 / 80 / 72 / 69 / 78;
+    //  200,000 of 1                240 / 109 / 59 / 47 / 44, of 16 278 / 138 / 94 / 89 / 95.
+    const auto launch = [&](auto kernel, int lanes) {
+        kernel<<<blocks, 32 * lanes, 0, st>>>(b->data, b->off, b->len, b->first, b->npkts, b->channels, b->nchains,
+                                              feat_dev);
+    };
+    if (b->nchains <= 32ll * sms) launch(k_chain_features<32>, 32);
+    else if (b->nchains <= 64ll * sms) launch(k_chain_features<16>, 16);
+    else if (b->nchains <= 128ll * sms) launch(k_chain_features<8>, 8);
+    else if (b->nchains <= 512ll * sms) launch(k_chain_features<4>, 4);
+    else launch(k_chain_features<2>, 2);
     CKM(cudaGetLastError(), "chain_features launch");
     CKM(cudaStreamSynchronize(st), "chain_features");
     return 0;
