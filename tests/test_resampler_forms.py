@@ -19,3 +19,21 @@ def test_resampler_where_its_forms_meet(cuda, n_out):
     assert cn.lib().cuopus_resample48to16(ctypes.c_void_p(d.data_ptr() + 2), len(x), n_out, ctypes.c_void_p(y.data_ptr()),
                                           ctypes.c_void_p(cuda.cuda.current_stream().cuda_stream), None, 0) == 0
     assert np.array_equal(y.cpu().numpy(), pipeline.resample(x, n_out))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("seconds", [7.0, 100.0])
+def test_interleaved_channels_in_both_forms(cuda, seconds):
+    """A stereo file to 16 kHz, below and above that line: each channel is the
+    restatement's resampling of the int16 decode's channel."""
+    from cuopus_b200 import cuopus_native as cn
+    from oracle import pipeline
+    from perf import cases
+    f = cases._files(dict(files=1, min_s=seconds, max_s=seconds, content="stereo"), 3)
+    (pcm, ch), = cn.decode_ogg_to_int16(f)
+    (got, ch16), = cn.decode_ogg_to_f16k_channels(f)
+    assert ch == ch16 == 2
+    pcm, got = pcm.cpu().numpy().reshape(-1, 2), got.cpu().numpy().reshape(-1, 2)
+    assert len(got) == (len(pcm) - 48) // 3
+    for c in range(2):
+        assert np.array_equal(got[:, c], pipeline.resample(np.ascontiguousarray(pcm[:, c]), len(got)))
